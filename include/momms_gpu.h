@@ -119,8 +119,9 @@ int momms_sgemm(int64_t m, int64_t n, int64_t k, const float* alpha, const float
  * unit stride along one index with the other stride a multiple of 2 elements
  * and a 16-byte aligned base (other layouts would need a repack copy). The
  * split-k scratch is one device-global array of MOMMS_NOALLOC_SCRATCH_BYTES
- * (160 partial tiles of 128 x 128 doubles plus 1024 tile counters) that every
- * GPU loading this library holds until the process exits; a problem whose
+ * (160 partial tiles of 128 x 128 doubles plus 1024 tile counters) and 1 KB of
+ * further counters that every GPU loading this library holds until the process
+ * exits; a problem whose
  * split-k plan needs more than that is rejected with MOMMS_ERR_INVALID_ARG.
  * All calls on a device share that array and it keeps the last call's
  * contents, so calls that overlap on the GPU (other streams, or other host

@@ -24,17 +24,7 @@
 namespace momms {
 namespace grouped {
 
-struct DProblem {
-  int64_t m, n, k;
-  double alpha, beta;
-  double* c;
-  int64_t rsc, csc;
-  int tiles_m, tiles_n, splits, flags;  // flags: bit 0 A x-contiguous, bit 1 B x-contiguous
-  int64_t kb_split;
-  int64_t unit_begin;
-  int64_t part_offset;     // elements into the partials buffer
-  int64_t counter_offset;  // entries into the counters buffer
-};
+using dmma::DProblem;
 
 struct SProblem {
   ffma::Operands o;
@@ -57,112 +47,35 @@ __device__ __forceinline__ int find_problem(const P* probs, int nprobs, int64_t 
   return lo;
 }
 
-// Decodes unit u of the f64 group: its problem, output tile and k-blocks.
-struct DUnit {
-  int pi, tm, tn, sp;
-  int64_t tile, kb0, kb1;
+// A table of problems, ordered by their first unit, as a source of units.
+struct Many {
+  const CUtensorMap* maps;
+  const DProblem* probs;
+  int nprobs;
+  long long units;
+  __device__ __forceinline__ long long total() const { return units; }
+  template <typename F>
+  __device__ __forceinline__ void unit(long long u, F&& fn) const {
+    const int pi = find_problem(probs, nprobs, u);
+    const DProblem& P = probs[pi];
+    const int64_t local = u - P.unit_begin;
+    dmma::Unit w;
+    w.sp = (int)(local % P.splits);
+    w.tile = local / P.splits;
+    w.tm = (int)(w.tile % P.tiles_m);
+    w.tn = (int)(w.tile / P.tiles_m);
+    w.kb0 = w.sp * P.kb_split;
+    w.kb1 = min(ceil_div_dev(P.k, dmma::BK), w.kb0 + P.kb_split);
+    fn(P, &maps[2 * pi], &maps[2 * pi + 1], w);
+  }
 };
-__device__ __forceinline__ DUnit decode_dunit(const DProblem* probs, int nprobs, int64_t u) {
-  using namespace dmma;
-  DUnit d;
-  d.pi = find_problem(probs, nprobs, u);
-  const DProblem& P = probs[d.pi];
-  const int64_t local = u - P.unit_begin;
-  d.sp = (int)(local % P.splits);
-  d.tile = local / P.splits;
-  d.tm = (int)(d.tile % P.tiles_m);
-  d.tn = (int)(d.tile / P.tiles_m);
-  const int64_t kblocks = ceil_div_dev(P.k, BK);
-  d.kb0 = d.sp * P.kb_split;
-  d.kb1 = min(kblocks, d.kb0 + P.kb_split);
-  return d;
-}
 
-// Units are handed out dynamically: the producer lane takes the next unit
-// from a global counter (units are numbered largest problem first, so this
-// is longest-processing-time-first list scheduling, balanced by the actual
-// unit durations rather than a cost model) and tags the first pipeline stage
-// it fills for that unit with the unit's index; the DMMA warps read the tag
-// when they reach that stage. An index of -1 ends the kernel. The last CTA
-// to finish resets the counter, so a captured plan relaunches as is.
-__global__ void __launch_bounds__(dmma::THREADS, 1)
+// Every plain f64 problem's units, dealt dynamically (dgemm_body); the last
+// CTA resets the unit counter, so a captured plan relaunches as is.
+__global__ void __launch_bounds__(dmma::THREADS, dmma::CTAS_PER_SM)
     dgemm_grouped_kernel(const CUtensorMap* __restrict__ maps, const DProblem* __restrict__ probs, int nprobs,
-                         int64_t total_units, double* partials, unsigned* counters, unsigned long long* next_unit,
-                         unsigned* status) {
-  using namespace dmma;
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ long long s_stage_unit[STAGES];  // unit starting at each stage, -1: end
-  const Smem sm = setup_smem(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int stage = 0;
-  uint32_t phase = 0;
-  if (warp == CONSUMER_WARPS) {
-    if (lane == 0) {
-      bool ok = true;
-      for (;;) {
-        const long long u = (long long)atomicAdd(next_unit, 1ull);
-        if (u >= total_units) break;
-        const DUnit d = decode_dunit(probs, nprobs, u);
-        const DProblem& P = probs[d.pi];
-        // the tag is written while the stage is free (every DMMA warp read
-        // the previous tag before releasing it) and published by the
-        // stage's arrive (release) to the warps' wait (acquire)
-        if (!mbar_wait_bounded(&sm.empty[stage], phase ^ 1)) {
-          report_status(status, DEV_TIMEOUT_EMPTY);
-          ok = false;
-          break;
-        }
-        s_stage_unit[stage] = u;
-        if (!produce_unit(&maps[2 * d.pi], &maps[2 * d.pi + 1], P.flags & 1, (P.flags >> 1) & 1, d.tm, d.tn, d.kb0,
-                          d.kb1, sm.sA, sm.sB, sm.full, sm.empty, stage, phase, status)) {
-          ok = false;
-          break;
-        }
-      }
-      if (ok) {
-        if (mbar_wait_bounded(&sm.empty[stage], phase ^ 1)) {
-          s_stage_unit[stage] = -1;
-          mbar_arrive(&sm.full[stage]);
-        } else {
-          report_status(status, DEV_TIMEOUT_EMPTY);
-        }
-      }
-      // the last CTA out resets the unit counter for the next launch
-      __threadfence();
-      const unsigned long long done = atomicAdd(next_unit + 1, 1ull);
-      if (done == (unsigned long long)gridDim.x - 1) {
-        next_unit[0] = 0ull;
-        next_unit[1] = 0ull;
-        __threadfence();
-      }
-    }
-    return;
-  }
-  const int wm = warp >> 2, wn = warp & 3;
-  for (;;) {
-    if (!mbar_wait_bounded(&sm.full[stage], phase)) {
-      report_status(status, DEV_TIMEOUT_FULL);
-      return;
-    }
-    const long long u = s_stage_unit[stage];
-    if (u < 0) break;
-    const DUnit d = decode_dunit(probs, nprobs, u);
-    const DProblem& P = probs[d.pi];
-    const int64_t row_base = (int64_t)d.tm * BM + wm * 64, col_base = (int64_t)d.tn * BN + wn * 32;
-    const uint32_t live = live_mask(row_base, col_base, P.m, P.n);
-    double acc[8][4][2];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    if (!consume_unit(P.flags & 1, (P.flags >> 1) & 1, d.kb0, d.kb1, live, sm.sA, sm.sB, sm.full, sm.empty, stage,
-                      phase, wm, wn, lane, acc, status))
-      return;
-    const Epi e{P.m, P.n, P.alpha, P.beta, P.c, P.rsc, P.csc};
-    finish_unit(e, acc, row_base + (lane >> 2), col_base + 2 * (lane & 3), P.splits, d.sp,
-                P.splits > 1 ? partials + P.part_offset + (size_t)d.tile * P.splits * BM * BN : nullptr,
-                P.splits > 1 ? counters + P.counter_offset + d.tile : nullptr, threadIdx.x, sm.s_last);
-  }
+                         int64_t total_units, unsigned long long* next_unit, unsigned* status) {
+  dmma::dgemm_body(Many{maps, probs, nprobs, total_units}, next_unit, status);
 }
 
 template <int TM, typename Off>
@@ -252,15 +165,6 @@ struct Plan {
   std::vector<PlanProblem> other;
   // two or more emulated problems with fixed slice counts: one slice launch
   OzakiBatch* ozb = nullptr;
-  // operands copied to column-major scratch before each launch (f64
-  // operands whose strides do not suit TMA)
-  struct Repack {
-    DevMat src;
-    int64_t rows, cols;
-    void* dst;
-    int64_t ld;
-  };
-  std::vector<Repack> repacks;
   // captured graph
   cudaGraphExec_t graph = nullptr;
   std::vector<void*> allocs;
@@ -362,107 +266,35 @@ int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_
   // ---- f64 group ----
   if (!dlist.empty()) {
     using namespace dmma;
-    struct Cost {
-      int idx;
-      double tile_cost;
-      int tiles;
-      int64_t kblocks;
-    };
-    std::vector<Cost> cs;
-    for (int i : dlist) {
-      const momms_gemm_desc& d = descs[i];
-      const int tiles = (int)(ceil_div(d.m, BM) * ceil_div(d.n, BN));
-      // live 8x8 blocks of an average tile, times k-blocks
-      const double live = (double)std::min<int64_t>(d.m, BM) * std::min<int64_t>(d.n, BN) / 64.0;
-      const int64_t kb = ceil_div(d.k, BK);
-      cs.push_back(Cost{i, live * (double)kb, tiles, kb});
-    }
     std::vector<grouped::DProblem> probs;
     std::vector<CUtensorMap> maps;
-    std::vector<std::pair<double, int>> order;  // (unit cost, index into cs)
-    std::vector<int> splits(cs.size());
-    for (size_t j = 0; j < cs.size(); ++j) {
-      const momms_gemm_desc& d = descs[cs[j].idx];
-      // the same split count as a single launch of this shape: a problem's
-      // result does not depend on the batch it is in
-      splits[j] = splits_f64(d.m, d.n, d.k, ds->sm_count);
-      order.push_back({cs[j].tile_cost / splits[j], (int)j});
-    }
-    std::sort(order.begin(), order.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+    // the same plan as a single launch of this shape: a problem's result does
+    // not depend on the batch it is in; costliest units first
+    std::vector<std::pair<F64Plan, int>> order;
+    for (int i : dlist) order.push_back({f64_plan(descs[i].m, descs[i].n, descs[i].k, ds->sm_count), i});
+    std::sort(order.begin(), order.end(),
+              [](const auto& a, const auto& b) { return a.first.unit_cost > b.first.unit_cost; });
     int64_t units = 0, parts = 0, ctrs = 0;
     for (auto& oc : order) {
-      const Cost& c = cs[oc.second];
-      const momms_gemm_desc& d = descs[c.idx];
-      grouped::DProblem P;
-      memset(&P, 0, sizeof(P));
-      P.m = d.m; P.n = d.n; P.k = d.k;
-      P.alpha = d.alpha; P.beta = d.beta;
-      P.c = static_cast<double*>(d.c.ptr);
-      P.rsc = d.c.rs; P.csc = d.c.cs;
-      P.tiles_m = (int)ceil_div(d.m, BM);
-      P.tiles_n = (int)ceil_div(d.n, BN);
-      int s = splits[oc.second];
-      P.kb_split = ceil_div(c.kblocks, s);
-      s = (int)ceil_div(c.kblocks, P.kb_split);
-      P.splits = s;
-      P.unit_begin = units;
-      units += (int64_t)c.tiles * s;
-      if (s > 1) {
-        P.part_offset = parts;
-        P.counter_offset = ctrs;
-        parts += (int64_t)c.tiles * s * BM * BN;
-        ctrs += c.tiles;
-      }
-      // tensor maps in each operand's own orientation (repacked copies for
-      // strides TMA cannot take, exactly as a single launch does)
-      CUtensorMap ma, mb;
+      const F64Plan& fp = oc.first;
+      const momms_gemm_desc& d = descs[oc.second];
       const DevGemm gv = devgemm_of(d);  // packed operands: their column-major copies
-      DevMat a = gv.a, b = gv.b;
-      int oa = dmma_orient(a, d.m, d.k, true), ob = dmma_orient(b, d.k, d.n, false);
-      if (oa == 2) {
-        const int64_t ld = round_up(d.m, 2);
-        void* dst = nullptr;
-        int rc = plan_alloc(p, &dst, (size_t)ld * d.k * 8);
-        if (rc) { plan_free(p); return rc; }
-        p->repacks.push_back(Plan::Repack{a, d.m, d.k, dst, ld});
-        a = DevMat{dst, 1, ld};
-        oa = 0;
-      }
-      if (ob == 2) {
-        const int64_t ld = round_up(d.k, 2);
-        void* dst = nullptr;
-        int rc = plan_alloc(p, &dst, (size_t)ld * d.n * 8);
-        if (rc) { plan_free(p); return rc; }
-        p->repacks.push_back(Plan::Repack{b, d.k, d.n, dst, ld});
-        b = DevMat{dst, 1, ld};
-        ob = 1;
-      }
-      const bool a_xc = (oa == 0), b_xc = (ob == 0);
-      uint64_t dims[2], strides[1];
-      uint32_t box[2];
-      if (a_xc) {
-        dims[0] = d.m; dims[1] = d.k; strides[0] = (uint64_t)(d.k == 1 ? round_up(d.m * 8, 16) : a.cs * 8);
-        box[0] = 16; box[1] = BK;
-      } else {
-        dims[0] = d.k; dims[1] = d.m; strides[0] = (uint64_t)(d.m == 1 ? round_up(d.k * 8, 16) : a.rs * 8);
-        box[0] = BK; box[1] = BM;
-      }
-      int rc = encode_tiled(&ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, a.ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-      if (!rc) {
-        if (b_xc) {
-          dims[0] = d.n; dims[1] = d.k; strides[0] = (uint64_t)(d.k == 1 ? round_up(d.n * 8, 16) : b.rs * 8);
-          box[0] = 16; box[1] = BK;
-        } else {
-          dims[0] = d.k; dims[1] = d.n; strides[0] = (uint64_t)(d.n == 1 ? round_up(d.k * 8, 16) : b.cs * 8);
-          box[0] = BK; box[1] = BN;
-        }
-        rc = encode_tiled(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, b.ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-      }
+      grouped::DProblem P;
+      CUtensorMap ma, mb;
+      const int rc = dmma_problem(gv, fp, &P, &ma, &mb);
       if (rc) {
         plan_free(p);
         return rc;
       }
-      P.flags = (a_xc ? 1 : 0) | (b_xc ? 2 : 0);
+      P.unit_begin = units;
+      units += fp.units();
+      if (P.splits > 1) {
+        // offsets until the buffers exist
+        P.partials = reinterpret_cast<double*>(parts * sizeof(double));
+        P.counters = reinterpret_cast<unsigned*>(ctrs * sizeof(unsigned));
+        parts += fp.units() * TILE_ELEMS;
+        ctrs += fp.tiles();
+      }
       probs.push_back(P);
       maps.push_back(ma);
       maps.push_back(mb);
@@ -477,6 +309,11 @@ int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_
     if (!rc) { p->d_counters = static_cast<unsigned*>(buf); rc = plan_alloc(p, &buf, 2 * sizeof(unsigned long long)); }
     if (!rc) p->d_next = static_cast<unsigned long long*>(buf);
     if (rc) { plan_free(p); return rc; }
+    for (grouped::DProblem& P : probs)
+      if (P.splits > 1) {
+        P.partials = p->d_partials + reinterpret_cast<size_t>(P.partials) / sizeof(double);
+        P.counters = p->d_counters + reinterpret_cast<size_t>(P.counters) / sizeof(unsigned);
+      }
     size_t off = p->host_tables.size();
     rc = plan_upload(p, p->d_probs, probs.data(), probs.size() * sizeof(grouped::DProblem));
     if (!rc && async) pending.push_back({p->d_probs, {off, probs.size() * sizeof(grouped::DProblem)}});
@@ -614,16 +451,12 @@ int plan_launch(Plan* p, cudaStream_t s, int max_sms) {
   if (!ds) return MOMMS_ERR_NO_DEVICE;
   if (ds->device != p->device) return fail(MOMMS_ERR_INVALID_ARG, "plan belongs to device %d", p->device);
   cudaError_t e;
-  for (const Plan::Repack& r : p->repacks) {
-    int rc = repack_colmajor(r.src, r.rows, r.cols, 8, r.dst, r.ld, s);
-    if (rc) return rc;
-  }
   if (p->nd) {
     const int sms = (max_sms > 0 && max_sms < ds->sm_count) ? max_sms : ds->sm_count;
-    const int grid = (int)std::min<int64_t>(p->d_units, sms);
+    const int grid = (int)std::min<int64_t>(p->d_units, (int64_t)dmma::CTAS_PER_SM * sms);
     KernelTimer kt(MOMMS_KERNEL_DGEMM_DMMA, s);
     grouped::dgemm_grouped_kernel<<<grid, dmma::THREADS, dmma::SMEM_BYTES, s>>>(
-        p->d_maps, p->d_probs, p->nd, p->d_units, p->d_partials, p->d_counters, p->d_next, ds->status);
+        p->d_maps, p->d_probs, p->nd, p->d_units, p->d_next, ds->status);
     note_launch();
     if ((e = launch_status()) != cudaSuccess) return cuda_fail(e, "grouped f64 launch");
   }

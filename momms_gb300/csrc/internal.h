@@ -242,20 +242,50 @@ void tf32_operand_planes(const float* x, int64_t sr, int64_t sp, int64_t R, int6
 int repack_colmajor(const DevMat& src, int64_t rows, int64_t cols, size_t elem, void* dst, int64_t ld,
                     cudaStream_t s);
 
-// How the f64 kernels stage an operand: 0 = TMA with the non-k index
-// contiguous, 1 = TMA with k contiguous, 2 = needs a column-major repack.
-int dmma_orient(const DevMat& v, int64_t rows, int64_t cols, bool x_is_rows);
+// How the f64 kernels stage an operand: strides along x (the non-k index) and
+// k, the staged layout (xc: x contiguous), and whether TMA can address it
+// (16-byte aligned base, one unit stride, the other a multiple of 16 bytes);
+// others are staged by 8-byte cp.async.
+struct DmmaOrient {
+  int64_t sx, sk;
+  bool xc, tma;
+};
+DmmaOrient dmma_orient(const DevMat& v, int64_t rows, int64_t cols, bool x_is_rows);
 
-// Launch configuration of a plain f64 / f32 problem: the output tile
-// (0 = the kernel's 128 x 128 tile, 1 = its small tile: FFMA 64 x 64) and the
-// k-split count, from the tuning table (momms_autotune, keyed by shape
-// bucket) or the model. Depends only on the shape and the SM count.
+// Launch configuration of a plain problem: the output tile (f32: 0 = 128 x
+// 128, 1 = 64 x 64; f64: 0) and the k-split count, from the tuning table
+// (momms_autotune, keyed by shape bucket) or the model. Depends only on the
+// shape and the SM count.
 struct PlainCfg {
   int tile;
   int splits;
 };
 PlainCfg plain_cfg(int dtype, int64_t m, int64_t n, int64_t k, int sm_count);
-int splits_f64(int64_t m, int64_t n, int64_t k, int sm_count);
+
+// How a plain f64 problem is cut: square output tiles of ts = 32, 16 or 8, k
+// in `splits` ranges of kb_split k-blocks of 16. Depends only on the shape, the tuning table and
+// the SM count.
+struct F64Plan {
+  int ts, tiles_m, tiles_n, splits;
+  int64_t kb_split;
+  int64_t tiles() const { return (int64_t)tiles_m * tiles_n; }
+  int64_t units() const { return tiles() * splits; }
+  double unit_cost;  // FP64-pipe clocks of one SM per unit
+};
+F64Plan f64_plan(int64_t m, int64_t n, int64_t k, int sm_count);
+namespace dmma {
+struct DProblem;
+}
+// The kernels' description of a problem under a plan (partials and counters
+// are the caller's), with the tensor maps of the operands TMA stages.
+int dmma_problem(const DevGemm& g, const F64Plan& plan, dmma::DProblem* P, CUtensorMap* tmA, CUtensorMap* tmB);
+// What a split plan of the model may use, the same for every caller: partial
+// tiles within 160 of 128 x 128 doubles (counted on the 128 grid), and the
+// 1280 counters that two splits of so many 32 x 32 tiles take.
+constexpr int64_t kSplitTileCap = 160, kSplitCounterCap = 1280;
+inline bool f64_split_fits(int64_t m, int64_t n, int splits) {
+  return ((m + 127) / 128) * ((n + 127) / 128) * splits <= kSplitTileCap;
+}
 
 // Emulated problems of a plan run together: each problem's preparation and
 // recombination, and ONE persistent slice-kernel launch (CTA pairs) over all
