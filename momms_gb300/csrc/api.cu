@@ -327,11 +327,14 @@ int gemm_impl(const momms_gemm_desc* d, cudaStream_t s) {
     host[i] = ops[i]->mem == MOMMS_MEM_HOST || (ops[i]->mem == MOMMS_MEM_AUTO && !is_device_ptr(ops[i]->ptr));
   const bool any_packed = packed_of(d->a) || packed_of(d->b);
   const bool any_host0 = host[0] || host[1] || host[2];
+  bool tight = false;
   if (any_host0) {
     // Larger than the staging budget: stream the operands through in blocks
     // (the reference's out-of-core PartM / PartN, src/exper/out_of_core.rs:77-87).
     const uint64_t budget = staging_budget();
-    if (incore_bytes(*d, host) > budget) {
+    const size_t incore = incore_bytes(*d, host);
+    tight = incore + kFreeScratch > budget;
+    if (incore > budget) {
       if (any_packed) return fail(MOMMS_ERR_UNSUPPORTED, "streamed (out-of-core) calls take no packed operands");
       BlockPlan plan;
       rc = plan_blocks(*d, host, budget, &plan);
@@ -347,6 +350,7 @@ int gemm_impl(const momms_gemm_desc* d, cudaStream_t s) {
   g.k = d->k;
   g.alpha = d->alpha;
   g.beta = d->beta;
+  g.tight = tight;
   Staged st[3];
   DevMat* dm[3] = {&g.a, &g.b, &g.c};
   const bool any_host = host[0] || host[1] || host[2];

@@ -4,12 +4,16 @@
 // this header with the host compiler and compare every result with exact
 // rational rounding.
 #pragma once
+#include <stdint.h>
 #include <string.h>
 
 #ifndef __CUDACC__
 #define __host__
 #define __device__
 #define __forceinline__ inline
+#define MOMMS_UNROLL
+#else
+#define MOMMS_UNROLL _Pragma("unroll")
 #endif
 
 namespace momms {
@@ -105,6 +109,68 @@ __host__ __device__ __forceinline__ double wide_to_double(long long P0, long lon
   unsigned __int128 u = (uh << (64 - s)) | (unsigned __int128)(ul >> s);
   if (ul & ((1ull << s) - 1)) u |= 1u;  // sticky
   return i128_to_double(neg ? -(__int128)u : (__int128)u, scale + s);
+}
+
+__host__ __device__ __forceinline__ uint32_t funnel_left(uint32_t hi, uint32_t lo, int n) {  // 0 <= n < 32
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, (uint32_t)n);
+#else
+  return n ? (hi << n) | (lo >> (32 - n)) : hi;
+#endif
+}
+
+// Nearest double to R * 2^scale, R an NW-word two's complement integer (least
+// word first, NW >= 4) other than the most negative one. The magnitude's
+// leading word and the two below it are normalised to 64 bits with everything
+// below as a sticky bit; about 30 instructions. Magnitudes below 2^64 and
+// results outside the normal range take i128_to_double, on the same words and
+// a sticky bit (at least 65 bits where anything lies below them, more than the
+// 53 + 2 the rounding looks at).
+template <int NW>
+__host__ __device__ __forceinline__ double words_to_double(const uint32_t (&w)[NW], int scale) {
+  static_assert(NW >= 4, "at least 128 bits");
+  const uint32_t neg = (uint32_t)((int32_t)w[NW - 1] >> 31);  // all ones when negative
+  uint32_t u[NW];
+  unsigned long long c = neg & 1u;
+  MOMMS_UNROLL
+  for (int i = 0; i < NW; ++i) {
+    c += w[i] ^ neg;
+    u[i] = (uint32_t)c;
+    c >>= 32;
+  }
+  // the leading words at h, h - 1, h - 2 (h >= 2)
+  uint32_t t2 = u[2], t1 = u[1], t0 = u[0], below = 0, sticky = 0;
+  int h = 2;
+  MOMMS_UNROLL
+  for (int i = 3; i < NW; ++i) {
+    below |= u[i - 3];
+    if (u[i] != 0) {
+      t2 = u[i];
+      t1 = u[i - 1];
+      t0 = u[i - 2];
+      sticky = below;
+      h = i;
+    }
+  }
+  const int lz = t2 ? clz64(t2) - 32 : 0;
+  const uint32_t nh = funnel_left(t2, t1, lz);
+  const uint32_t nl = funnel_left(t1, t0, lz) | (((t0 << lz) | sticky) != 0 ? 1u : 0u);
+  const int E = 32 * h + 31 - lz + scale;  // the leading bit weighs 2^E
+  if (t2 != 0 && E >= -1022 && E < 1023) {
+    unsigned long long m = (((unsigned long long)nh << 32) | nl) >> 11;  // 53 bits
+    if ((nl & 0x7ffu) + ((uint32_t)m & 1u) > 0x400u) ++m;
+    // the leading bit adds one to the exponent field, and so does a carry
+    unsigned long long b = m + ((unsigned long long)(uint32_t)(E + 1022) << 52);
+    b |= (unsigned long long)(neg & 0x80000000u) << 32;
+    double r;
+    memcpy(&r, &b, sizeof(r));
+    return r;
+  }
+  const unsigned long long top = ((unsigned long long)t2 << 32) | t1;
+  const unsigned long long lo = (top << 33) | ((unsigned long long)t0 << 1) | (sticky ? 1u : 0u);
+  // 97 bits at most: the negated value is formed in integers
+  const __int128 mag = (__int128)(((unsigned __int128)(top >> 31) << 64) | lo);
+  return i128_to_double(neg ? -mag : mag, scale + 32 * (h - 2) - 1);
 }
 
 }  // namespace momms

@@ -128,6 +128,8 @@ struct DevGemm {
   DevMat a, b, c;
   Staging* staging = nullptr;
   const PackedOperand* pk[2] = {nullptr, nullptr};  // packed A, B (their DevMat is the plain copy, if any)
+  bool tight = false;  // emulated: scratch within work_bytes (ozaki_scratch)
+  int64_t whole_m = 0, whole_n = 0;  // a block of a streamed product: that product's sizes
 };
 
 // DevGemm of a descriptor whose operands are device views or packs.
@@ -188,8 +190,9 @@ int stage_out(const momms_operand& op, size_t es, const Staged& st, cudaStream_t
 int run_device_gemm(const DevGemm& g, const momms_gemm_desc& d, cudaStream_t s);
 
 // Device bytes a mode needs beyond the operands for an m x n x k problem
-// (slice planes, group sums, split-k partials); an upper bound.
-size_t work_bytes(int dtype, int precision, int slices, int64_t m, int64_t n, int64_t k);
+// (slice planes, group sums, split-k partials); an upper bound. `tight`: for
+// a call that runs with DevGemm::tight.
+size_t work_bytes(int dtype, int precision, int slices, int64_t m, int64_t n, int64_t k, bool tight);
 
 // ---- Out-of-core blocking (outofcore.cu) ----
 // Block sizes of a streamed call: C in mb x nb blocks, k in slabs of kb,
@@ -223,8 +226,10 @@ constexpr int kOzakiMaxSlices = 15;
 // Ozaki FP64 emulation: target relative error (0 = FP64 level) and slice count
 // (0 = chosen from the target). *slices_used receives the count actually used.
 int launch_dgemm_ozaki(const DevGemm& g, double target_rel_err, int slices, int* slices_used, cudaStream_t s);
-// Accumulation groups (int32 sum planes) of an ns-slice product with this k.
-int ozaki_group_count(int ns, int64_t k);
+// Bytes of operand and group planes a call holds: `tight`, never above the
+// digit form's; otherwise the residue form may take kFreeScratch instead.
+constexpr size_t kFreeScratch = 512u << 20;
+double ozaki_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight);
 // Exponents of the R rows of a view x (element (r, p) at x[r*sr + p*sp],
 // p < K) into exps[R], using maxbits[R] as scratch; and the ns digit planes
 // [ns][R][kp] of the view under those exponents.

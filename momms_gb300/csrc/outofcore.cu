@@ -44,7 +44,7 @@ size_t slot_bytes(int64_t rows, int64_t cols, size_t es) {
 
 size_t block_footprint(const momms_gemm_desc& d, const bool host[3], int64_t mb, int64_t nb, int64_t kb) {
   const size_t es = esize(d.dtype);
-  size_t bytes = work_bytes(d.dtype, d.precision, d.slices, mb, nb, kb) + kSlack;
+  size_t bytes = work_bytes(d.dtype, d.precision, d.slices, mb, nb, kb, true) + kSlack;
   if (host[0]) bytes += 2 * slot_bytes(mb, kb, es);
   if (host[1]) bytes += 2 * slot_bytes(kb, nb, es);
   if (host[2]) bytes += 2 * slot_bytes(mb, nb, es);
@@ -73,30 +73,26 @@ double block_traffic(const momms_gemm_desc& d, const bool host[3], int64_t bm, i
 
 }  // namespace
 
-size_t work_bytes(int dtype, int precision, int slices, int64_t m, int64_t n, int64_t k) {
+size_t work_bytes(int dtype, int precision, int slices, int64_t m, int64_t n, int64_t k, bool tight) {
   const double M = (double)m, N = (double)n, K = (double)k;
   double bytes;
   if (precision == MOMMS_PREC_OZAKI) {
     const int s = slices > 0 ? slices : 8;  // FP64-level targets take up to 8 slices
-    // digit planes of A and B, one int32 sum plane per accumulation group
-    // (tile-blocked: m and n padded to whole 128 x 256 tiles)
-    const double groups = (double)ozaki_group_count(s, k);
-    const double Mp = (double)round_up(m, 128), Np = (double)round_up(n, 256);
-    bytes = 2.0 * s * (M + N) * (double)round_up(std::min<int64_t>(k, kOzakiMaxK), 8) + 4.0 * groups * Mp * Np +
-            12.0 * (M + N);
+    // operand planes of A and B and the products' group planes
+    bytes = ozaki_scratch(s, m, n, k, tight) + 12.0 * (M + N);
   } else if (precision == MOMMS_PREC_SPLIT_TF32) {
     bytes = 8.0 * (M + N) * (double)round_up(k, 4);
   } else {
     (void)dtype;
     (void)K;
-    bytes = 21.0 * 1024 * 1024;  // split-k partials: at most one 128 x 128 tile per SM
+    bytes = 21.0 * 1024 * 1024;  // split-k partials (kSplitTileCap)
   }
   return (size_t)bytes;
 }
 
 size_t incore_bytes(const momms_gemm_desc& d, const bool host[3]) {
   const size_t es = esize(d.dtype);
-  size_t bytes = work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k) + kSlack;
+  size_t bytes = work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k, true) + kSlack;
   if (host[0]) bytes += slot_bytes(d.m, d.k, es);
   if (host[1]) bytes += slot_bytes(d.k, d.n, es);
   if (host[2]) bytes += slot_bytes(d.m, d.n, es);
@@ -341,6 +337,9 @@ int gemm_streamed(const momms_gemm_desc& d, const bool host[3], const BlockPlan&
     block_of(0, tk, &r0, &c0, &rows, &cols);
     g.k = cols;
     g.alpha = d.alpha;
+    g.tight = true;  // the blocks were sized for it
+    g.whole_m = d.m;
+    g.whole_n = d.n;
     g.beta = (tk.pb == 0) ? d.beta : 1.0;  // later k slabs accumulate (src/composables/part.rs:96-110)
     DevMat* dm[3] = {&g.a, &g.b, &g.c};
     int q_used[3] = {-1, -1, -1};

@@ -36,6 +36,7 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "crt_kernels.cuh"
 #include "exact_round.cuh"
 #include "ozaki_elem.cuh"
 #include "planes.cuh"
@@ -57,6 +58,8 @@ static_assert((kMaxK / 64) * 64 * (1ll << (2 * kDigitBits)) < (1ll << 31), "int3
 constexpr double kGroupLimit = 2147483647.0;
 // one TMEM chunk's bound: integers up to 2^24 are exact in FP32
 constexpr double kChunkBound = 16777216.0;
+// the residue form runs from this k (crt_applies)
+constexpr int64_t kCrtMinK = 128;
 
 // Everything in the pre-pass runs on integer bit patterns: GB300's FP64 pipe
 // is about 1 TFLOP/s, so FP64 arithmetic per element would dominate.
@@ -718,9 +721,174 @@ int launch_combine(CombineParams cp, int64_t j0, int64_t j1, int sm_count, cudaS
 }
 }  // namespace
 
-int ozaki_group_count(int ns, int64_t k) {
+namespace {
+// ---- The residue form (crt_elem.cuh) ---------------------------------------
+#define MOMMS_CRT_NS(X) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15)
+
+// Moduli that hold an ns-slice product over k: P > 2 |R|, |R| <= k 2^(16 ns),
+// with 2 % to spare for the quotient's rounding (crt::kFracBits).
+int crt_moduli(int ns, int64_t k) {
+  const double need = 16.0 * ns + log2((double)k) + 1.0 + 0.03;
+  double have = 0.0;
+  int n = 0;
+  while (n < crt::kMaxModuli && have < need) have += log2((double)crt::kModuli[n++]);
+  return n;
+}
+// Whether an ns-slice product runs by residues: where the model below says it
+// is the faster form. From the sizes alone (those of the whole product, where
+// it is streamed in blocks), so that a product gives the same bits alone, in a
+// batch, streamed and from packed operands. The rates are measured ones (n^2 =
+// entries of C; ps per entry or per operand element):
+//  * slice products 1.8 PFLOP/s, and per group and entry what of the epilogue
+//    they do not hide: 0.53 ps (digits: 4 bytes of plane), 0.2 ps (residues);
+//  * recombination 7.4 ps (7 digit groups), 10.4 ps (16 moduli);
+//  * operand planes 2 bytes per slice or modulus, 8 read, at 6 TB/s;
+//  * 20 us that the residue planes take longer where they do not fill the GPU.
+// Both forms at 8192 x 8192, 7 slices, ms per call: k = 128 1.33 (digits) and
+// 1.40, 256 1.61 and 1.56, 1024 3.17 and 2.48, 8192 20.9 and 13.1; at 65536 x
+// 256 x 256 0.64 and 0.75.
+bool crt_applies(int ns, int64_t m, int64_t n, int64_t k) {
+  if (ns < 5 || k < kCrtMinK) return false;
+  const int N = crt_moduli(ns, k);
   Schedule sc;
-  return ozaki_schedule(ns, k, &sc) ? sc.ng : sp::MAX_GROUPS;
+  if (!ozaki_schedule(ns, k, &sc)) return true;
+  const double mn = (double)m * n, ops = (double)(m + n) * k, mma = 2.0 * mn * k / 1.8e3;  // ps per product
+  const double digits = sc.np * mma + 0.53 * sc.ng * mn + mn * (2.7 + 0.67 * sc.ng) + ops * (8 + 2 * ns) / 6.0;
+  const double residues = N * mma + 0.2 * N * mn + mn * 0.65 * N + ops * (8 + 2 * N) / 6.0 + 20e6;
+  return residues < digits;
+}
+
+// Scratch of an emulated product, operand planes and group planes: the digit
+// form's, or the residue form's with `per` moduli per pass.
+double plane_bytes(int64_t m, int64_t n) { return (double)round_up(m, sp::BM) * (double)round_up(n, sp::BN); }
+double digit_scratch(int ns, int64_t m, int64_t n, int64_t k) {
+  Schedule sc;
+  const double ng = ozaki_schedule(ns, k, &sc) ? sc.ng : sp::MAX_GROUPS;
+  return 2.0 * ns * (double)(m + n) * (double)round_up(std::min(k, kMaxK), 8) + 4.0 * ng * plane_bytes(m, n);
+}
+double crt_scratch(int per, int moduli, int64_t m, int64_t n, int64_t k) {
+  return 2.0 * per * (double)(m + n) * (double)round_up(std::min(k, kMaxK), 8) + moduli * plane_bytes(m, n);
+}
+// The residue form keeps to the digit form's scratch (or kFreeScratch bytes, unless
+// `tight`) by walking the moduli in several passes, each with its own operand
+// planes: at 8192^3 two passes of 9 and 8 moduli instead of 4.6 GB of planes,
+// for one more read of the operands (0.2 of 13 ms).
+int crt_per_pass(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
+  const int N = crt_moduli(ns, k);
+  const double limit = std::max(digit_scratch(ns, m, n, k), tight ? 0.0 : (double)kFreeScratch);
+  int per = N;
+  while (per > 1 && crt_scratch(per, N, m, n, k) > limit) --per;
+  const int passes = (int)ceil_div(N, per);
+  return (int)ceil_div(N, passes);
+}
+
+// Residue planes l0..l1-1 of an operand view, or of a packed operand's digits.
+void crt_planes(int ns, const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K, __half* out, int64_t ldp,
+                int64_t plane_elems, const int* exps, int l0, int l1, cudaStream_t s) {
+  KernelTimer kt(MOMMS_KERNEL_PREP, s);
+  switch (ns) {
+#define X(NS) \
+  case NS: crt::launch_residues<NS>(x, sr, sp, R, K, out, ldp, plane_elems, exps, l0, l1, s); break;
+    MOMMS_CRT_NS(X)
+#undef X
+    default: refuse_launch(cudaErrorInvalidValue);
+  }
+  note_launch();
+}
+void crt_planes_of_pack(const PackedOperand& P, int64_t R, __half* out, int l0, int l1, int sm_count, cudaStream_t s) {
+  KernelTimer kt(MOMMS_KERNEL_PREP, s);
+  const __half* d = static_cast<const __half*>(P.planes);
+  switch (P.np) {
+#define X(NS) \
+  case NS: crt::launch_residues_of_digits<NS>(d, R * P.kp, out, l0, l1, sm_count, s); break;
+    MOMMS_CRT_NS(X)
+#undef X
+    default: refuse_launch(cudaErrorInvalidValue);
+  }
+  note_launch();
+}
+
+// The slice kernel's parameters for moduli l0..l1-1: one group of one pair
+// each. A k-block of a pair is at most 64 * 2^7 * 2^7, so a chunk holds 16.
+void crt_slice_params(int64_t m, int64_t k, int l0, int l1, sp::Params* p) {
+  memset(p, 0, sizeof(*p));
+  p->m = m;
+  p->kelems = 64;
+  p->kblocks = (int)ceil_div(k, 64);
+  p->tiles_m = (int)ceil_div(m, sp::BM);
+  p->ngroups = l1 - l0;
+  p->chunk_cap = kChunkCap;
+  p->residue = 1;
+  for (int g = 0; g < l1 - l0; ++g) {
+    p->group_begin[g] = g;
+    p->pair_a[g] = p->pair_b[g] = (uint8_t)g;
+    p->pair_w[g] = (64 << 14) >> (kChunkUnitLog2 + 6);
+    p->mod[g].p = (float)crt::kModuli[l0 + g];
+    p->mod[g].inv = (float)(1.0 / crt::kModuli[l0 + g]);
+  }
+  p->group_begin[l1 - l0] = l1 - l0;
+}
+
+void crt_combine_params(const DevGemm& g, int ns, int moduli, const void* res, int64_t plane, int64_t mpad,
+                        const int* rexp, const int* cexp, crt::CombineParams* cp) {
+  memset(cp, 0, sizeof(*cp));
+  cp->res = static_cast<const uint8_t*>(res);
+  cp->plane = plane;
+  cp->mpad = mpad;
+  cp->moduli = moduli;
+  cp->scale_off = -16 * ns;
+  cp->alpha_sign = g.alpha == 1.0 ? 1 : (g.alpha == -1.0 ? -1 : 0);
+  cp->beta_zero = (g.beta == 0.0);
+  cp->m = g.m;
+  cp->row_exp = rexp;
+  cp->col_exp = cexp;
+  cp->alpha = g.alpha;
+  cp->beta = g.beta;
+  cp->c = static_cast<double*>(g.c.ptr);
+  cp->rsc = g.c.rs;
+  cp->csc = g.c.cs;
+  crt::make_weights(moduli, &cp->wt);
+}
+
+// One recombination launch over columns [j0, j1) of C (j0 a multiple of 4) on stream Y.
+int launch_crt_combine(crt::CombineParams& cp, int ns, int64_t j0, int64_t j1, int sm_count, cudaStream_t Y) {
+  cp.j0 = j0;
+  cp.j1 = j1;
+  const int64_t bx = ceil_div(cp.m, 256), quads = ceil_div(j1 - j0, 4);
+  const int64_t by = std::min<int64_t>({quads, 65535, std::max<int64_t>(1, (int64_t)sm_count * 16 / bx)});
+  {
+    KernelTimer kt(MOMMS_KERNEL_COMBINE, Y);
+    const dim3 grid((unsigned)bx, (unsigned)by);
+    // the moduli that ns slices take for k from kCrtMinK to kMaxK
+    switch (ns * 100 + cp.moduli) {
+#define X(NS, N) case NS * 100 + N: crt::combine_kernel<crt::words_of(NS), N><<<grid, 256, 0, Y>>>(cp); break;
+      X(5, 12) X(5, 13) X(6, 14) X(6, 15) X(7, 16) X(7, 17) X(8, 18) X(8, 19) X(9, 20) X(9, 21) X(10, 22) X(10, 23)
+      X(11, 24) X(11, 25) X(11, 26) X(12, 27) X(12, 28) X(13, 29) X(13, 30) X(14, 31) X(14, 32) X(14, 33) X(15, 34)
+      X(15, 35)
+#undef X
+      default: refuse_launch(cudaErrorInvalidValue);
+    }
+  }
+  note_launch();
+  const cudaError_t e = launch_status();
+  return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "Ozaki launch");
+}
+
+// Tensor maps of K-major operand planes [planes][rows][kp] (`box_rows` rows per box).
+int plane_map(CUtensorMap* map, const void* base, int64_t k, int64_t rows, int planes, int64_t kp, size_t plane_elems,
+              int box_rows) {
+  uint64_t dims[3] = {(uint64_t)k, (uint64_t)rows, (uint64_t)planes};
+  uint64_t strides[2] = {(uint64_t)kp * 2, (uint64_t)plane_elems * 2};
+  uint32_t box[3] = {64, (uint32_t)box_rows, 1};  // 128-byte k-blocks
+  return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+}  // namespace
+
+double ozaki_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
+  const double d = digit_scratch(ns, m, n, k);
+  const int64_t kk = std::min(k, kMaxK);
+  if (!crt_applies(ns, m, n, kk)) return d;
+  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, m, n, kk, tight), crt_moduli(ns, kk), m, n, kk));
 }
 
 namespace {
@@ -1200,60 +1368,43 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
 
   const int64_t kp = round_up(k, 8);  // 16-byte rows of fp16
   const size_t a_plane = (size_t)m * kp, b_plane = (size_t)n * kp;
+  // The form: digit planes (one pass; packed operands bring theirs), or
+  // residue planes in passes of `per` moduli.
+  const bool crt = crt_applies(ns, g.whole_m ? g.whole_m : m, g.whole_n ? g.whole_n : n, k);
+  const int N = crt ? crt_moduli(ns, k) : ns;
+  const int per = crt ? crt_per_pass(ns, m, n, k, g.tight) : ns;
+  const int passes = (int)ceil_div(N, per);
+  const bool own_a = crt || !PA, own_b = crt || !PB;
   __half* planes_buf = nullptr;
-  const size_t own = (PA ? 0 : (size_t)ns * a_plane) + (PB ? 0 : (size_t)ns * b_plane);
+  const size_t own = (own_a ? (size_t)per * a_plane : 0) + (own_b ? (size_t)per * b_plane : 0);
   if (own && (ce = scratch_alloc(&planes_buf, own * sizeof(__half), s)) != cudaSuccess)
     return cuda_fail(ce, "Ozaki slice planes");
   ScratchGuard free_planes(planes_buf, s);
-  const __half* pa = PA ? static_cast<const __half*>(PA->planes) : planes_buf;
-  const __half* pb = PB ? static_cast<const __half*>(PB->planes) : planes_buf + (PA ? 0 : (size_t)ns * a_plane);
-  if (!PA) ozaki_operand_planes(ns, A, g.a.rs, g.a.cs, m, k, const_cast<__half*>(pa), kp, rexp, s);
+  const __half* pa = own_a ? planes_buf : static_cast<const __half*>(PA->planes);
+  const __half* pb = own_b ? planes_buf + (own_a ? (size_t)per * a_plane : 0) : static_cast<const __half*>(PB->planes);
 
   if (k > kMaxK) return fail(MOMMS_ERR_UNSUPPORTED, "Ozaki emulation supports k <= %lld per launch", (long long)kMaxK);
-  CUtensorMap tmA;
-  {
-    uint64_t dims[3] = {(uint64_t)k, (uint64_t)m, (uint64_t)ns};
-    uint64_t strides[2] = {(uint64_t)kp * 2, (uint64_t)a_plane * 2};
-    uint32_t box[3] = {64, (uint32_t)sp::BM, 1};  // 128-byte k-blocks
-    rc = encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, pa, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-  }
-
   sp::Params p;
   Schedule sch;
-  if (!slice_params(ns, m, k, &p, &sch)) return fail(MOMMS_ERR_UNSUPPORTED, "Ozaki schedule needs too many groups");
-  const int np = sch.np, ng = sch.ng;
+  if (!crt && !slice_params(ns, m, k, &p, &sch))
+    return fail(MOMMS_ERR_UNSUPPORTED, "Ozaki schedule needs too many groups");
+  const int np = crt ? N : sch.np, ng = crt ? N : sch.ng;
   call_info().slices = ns;
   call_info().pairs = np;
   call_info().groups = ng;
 
-  int* sbuf = nullptr;
+  char* sbuf = nullptr;
   // group planes tile-blocked (sp::Params::sbuf): m and n padded to whole
-  // 128 x 256 tiles, each tile one contiguous block
+  // 128 x 256 tiles, each tile one contiguous block of int32 or residue bytes
   const int64_t mpad = round_up(m, (int64_t)sp::BM);
-  const size_t plane = (size_t)mpad * (size_t)round_up(n, (int64_t)sp::BN);
-  if ((ce = scratch_alloc(&sbuf, (size_t)ng * plane * sizeof(int), s)) != cudaSuccess)
-    return cuda_fail(ce, "Ozaki group sums");
+  const size_t plane = (size_t)mpad * (size_t)round_up(n, (int64_t)sp::BN), word = crt ? 1 : sizeof(int);
+  if ((ce = scratch_alloc(&sbuf, (size_t)ng * plane * word, s)) != cudaSuccess) return cuda_fail(ce, "Ozaki group sums");
   ScratchGuard free_sbuf(sbuf, s);
-  p.plane = (int64_t)plane;
-  p.status = ds->status;
   CombineParams cp;
-  combine_params(g, ns, sch, sbuf, (int64_t)plane, mpad, rexp, cexp, &cp);
+  crt::CombineParams ccp;
+  if (crt) crt_combine_params(g, ns, N, sbuf, (int64_t)plane, mpad, rexp, cexp, &ccp);
+  else combine_params(g, ns, sch, reinterpret_cast<const int*>(sbuf), (int64_t)plane, mpad, rexp, cexp, &cp);
 
-  // The second stream starts after everything above (scratch, A, the
-  // choice), and so does the verify stream V, which runs the bound kernel
-  // and, under verification, the recombinations.
-  cudaStream_t V = verify ? ds->aux2 : nullptr;
-  Events ev;
-  if (nch > 1 || verify) {
-    rc = ev.create(nch);
-    if (!rc) {
-      ce = cudaEventRecord(ev.fork, s);
-      if (ce == cudaSuccess && nch > 1) ce = cudaStreamWaitEvent(ds->aux, ev.fork, 0);
-      if (ce == cudaSuccess && verify) ce = cudaStreamWaitEvent(V, ev.fork, 0);
-      if (ce != cudaSuccess) rc = cuda_fail(ce, "Ozaki chunk streams");
-    }
-  }
   // Recombination of chunk c (columns j0..j1 of C) on stream Y: with C staged
   // from host memory and one chunk, in column ranges each copied back while
   // the next is computed.
@@ -1261,77 +1412,114 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     const int64_t j0 = cut[c], j1 = cut[c + 1], w = j1 - j0;
     cudaError_t e = defer_c ? cudaStreamWaitEvent(Y, ev_c[c], 0) : wait_operand(g, 2, Y);
     if (e != cudaSuccess) return cuda_fail(e, "operand staging");
-    const int64_t nsub = (nch == 1 && stg && stg->writeback) ? std::min<int64_t>(4, w) : 1;
+    const int64_t nsub = (nch == 1 && stg && stg->writeback && w >= 16) ? 4 : 1;
     for (int64_t q = 0; q < nsub; ++q) {
-      const int64_t c0 = j0 + w * q / nsub, c1 = j0 + w * (q + 1) / nsub;
-      int r2 = launch_combine(cp, c0, c1, ds->sm_count, Y);
+      const int64_t c0 = j0 + w * q / nsub / 4 * 4, c1 = q + 1 < nsub ? j0 + w * (q + 1) / nsub / 4 * 4 : j1;
+      int r2 = crt ? launch_crt_combine(ccp, ns, c0, c1, ds->sm_count, Y) : launch_combine(cp, c0, c1, ds->sm_count, Y);
       if (!r2) r2 = columns_done(g, c0, c1, Y);
       if (r2) return r2;
     }
     return MOMMS_OK;
   };
-  for (int c = 0; c < nch && !rc; ++c) {
-    const int64_t j0 = cut[c], j1 = cut[c + 1], w = j1 - j0;
-    if (w <= 0) continue;
-    cudaStream_t X = (c & 1) ? ds->aux : s;
-    // B's columns j0..j1: exponents and digit planes
-    ce = defer_b ? cudaStreamWaitEvent(X, ev_b[c], 0) : wait_operand(g, 1, X);
-    if (ce != cudaSuccess) {
-      rc = cuda_fail(ce, "operand staging");
-      break;
+
+  cudaStream_t V = verify ? ds->aux2 : nullptr;
+  Events ev;
+  if (nch > 1 || verify) rc = ev.create(nch);
+  for (int pass = 0; pass < passes && !rc; ++pass) {
+    const int l0 = pass * per, l1 = std::min(N, l0 + per);
+    const bool last = pass + 1 == passes;
+    // A's planes of this pass (on s, after every slice launch of the pass
+    // before), and a packed B's
+    if (crt) {
+      if (PA) crt_planes_of_pack(*PA, m, const_cast<__half*>(pa), l0, l1, ds->sm_count, s);
+      else crt_planes(ns, A, g.a.rs, g.a.cs, m, k, const_cast<__half*>(pa), kp, (int64_t)a_plane, rexp, l0, l1, s);
+      if (PB) crt_planes_of_pack(*PB, n, const_cast<__half*>(pb), l0, l1, ds->sm_count, s);
+      crt_slice_params(m, k, l0, l1, &p);
+    } else if (!PA) {
+      ozaki_operand_planes(ns, A, g.a.rs, g.a.cs, m, k, const_cast<__half*>(pa), kp, rexp, s);
     }
-    const double* Bc = B + j0 * g.b.cs;
-    if (!PB) {
-      if (!b_exps_ready) rc = ozaki_operand_exponents(Bc, g.b.cs, g.b.rs, w, k, maxbits + m + j0, cexp_w + j0, X);
+    p.plane = (int64_t)plane;
+    p.status = ds->status;
+    CUtensorMap tmA;
+    rc = plane_map(&tmA, pa, k, m, l1 - l0, kp, a_plane, sp::BM);
+    if (rc) break;
+    // The second stream starts after everything above (scratch, A, the
+    // choice), and so does the verify stream V, which runs the bound kernel
+    // and, under verification, the recombinations.
+    if (nch > 1 || (verify && pass == 0)) {
+      ce = cudaEventRecord(ev.fork, s);
+      if (ce == cudaSuccess && nch > 1) ce = cudaStreamWaitEvent(ds->aux, ev.fork, 0);
+      if (ce == cudaSuccess && verify && pass == 0) ce = cudaStreamWaitEvent(V, ev.fork, 0);
+      if (ce != cudaSuccess) rc = cuda_fail(ce, "Ozaki chunk streams");
+    }
+    for (int c = 0; c < nch && !rc; ++c) {
+      const int64_t j0 = cut[c], j1 = cut[c + 1], w = j1 - j0;
+      if (w <= 0) continue;
+      cudaStream_t X = (c & 1) ? ds->aux : s;
+      // B's columns j0..j1: exponents and planes
+      const double* Bc = B + j0 * g.b.cs;
+      if (pass == 0) {
+        ce = defer_b ? cudaStreamWaitEvent(X, ev_b[c], 0) : wait_operand(g, 1, X);
+        if (ce != cudaSuccess) {
+          rc = cuda_fail(ce, "operand staging");
+          break;
+        }
+        if (!PB && !b_exps_ready)
+          rc = ozaki_operand_exponents(Bc, g.b.cs, g.b.rs, w, k, maxbits + m + j0, cexp_w + j0, X);
+        if (rc) break;
+      }
+      if (!PB && crt) {
+        crt_planes(ns, Bc, g.b.cs, g.b.rs, w, k, const_cast<__half*>(pb) + j0 * kp, kp, (int64_t)b_plane, cexp_w + j0,
+                   l0, l1, X);
+      } else if (!PB) {
+        KernelTimer kt(MOMMS_KERNEL_PREP, X);
+        ozaki_planes(ns, Bc, g.b.cs, g.b.rs, w, k, const_cast<__half*>(pb) + j0 * kp, kp, (int64_t)b_plane,
+                     cexp_w + j0, X);
+        note_launch();
+      }
+      if (verify && pass == 0) {
+        // B's magnitudes for the bound (verify implies B is not packed)
+        rc = enqueue_magnitudes(Bc, g.b.cs, g.b.rs, w, k, cexp_w + j0, bw.mag_b + j0 * bw.kp, bw.kp, bw.sum_b + j0, X);
+        if (rc) break;
+        if ((ce = cudaEventRecord(ev.mag[c], X)) != cudaSuccess ||
+            (ce = cudaStreamWaitEvent(V, ev.mag[c], 0)) != cudaSuccess) {
+          rc = cuda_fail(ce, "Ozaki bound events");
+          break;
+        }
+      }
+      CUtensorMap tmB, tmB_half;  // half: one CTA's share of the B tile for the pair kernel
+      rc = plane_map(&tmB, pb + j0 * kp, k, w, l1 - l0, kp, b_plane, sp::BN);
+      if (!rc) rc = plane_map(&tmB_half, pb + j0 * kp, k, w, l1 - l0, kp, b_plane, sp::BN / 2);
       if (rc) break;
-      KernelTimer kt(MOMMS_KERNEL_PREP, X);
-      ozaki_planes(ns, Bc, g.b.cs, g.b.rs, w, k, const_cast<__half*>(pb) + j0 * kp, kp, (int64_t)b_plane,
-                   cexp_w + j0, X);
+      p.n = w;
+      p.tiles_n = (int)ceil_div(w, sp::BN);
+      // j0 is a multiple of the tile width: the chunk's tile blocks start here
+      p.sbuf = reinterpret_cast<int*>(sbuf + (crt ? (size_t)l0 * plane : 0) + (size_t)(j0 * mpad) * word);
+      {
+        KernelTimer kt(MOMMS_KERNEL_SLICE_OZAKI, X);
+        int variant = 0;
+        ce = sp::launch_slice<0, sp::EPI_OZAKI>(tmA, tmB, tmB_half, p, ds->sm_count, X, &variant);
+        if (ce == cudaSuccess) ce = launch_status();
+        if (ce != cudaSuccess) {
+          rc = cuda_fail(ce, "Ozaki slice launch");
+          break;
+        }
+        call_info().slice_variant = variant;
+      }
       note_launch();
-    }
-    if (verify) {
-      // B's magnitudes for the bound (verify implies B is not packed)
-      rc = enqueue_magnitudes(Bc, g.b.cs, g.b.rs, w, k, cexp_w + j0, bw.mag_b + j0 * bw.kp, bw.kp, bw.sum_b + j0, X);
-      if (rc) break;
-      if ((ce = cudaEventRecord(ev.mag[c], X)) != cudaSuccess || (ce = cudaStreamWaitEvent(V, ev.mag[c], 0)) != cudaSuccess) {
-        rc = cuda_fail(ce, "Ozaki bound events");
-        break;
+      if (!last) continue;
+      if (verify) {
+        // the recombination waits for the bound's verdict (below)
+        if ((ce = cudaEventRecord(ev.prod[c], X)) != cudaSuccess) rc = cuda_fail(ce, "Ozaki chunk streams");
+      } else {
+        rc = combine_chunk(c, X);
       }
     }
-    CUtensorMap tmB, tmB_half;
-    {
-      const __half* pbc = pb + j0 * kp;
-      uint64_t dimsb[3] = {(uint64_t)k, (uint64_t)w, (uint64_t)ns};
-      uint64_t stridesb[2] = {(uint64_t)kp * 2, (uint64_t)b_plane * 2};
-      uint32_t boxb[3] = {64, (uint32_t)sp::BN, 1};
-      rc = encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, pbc, dimsb, stridesb, boxb,
-                        CU_TENSOR_MAP_SWIZZLE_128B);
-      if (rc) break;
-      uint32_t boxh[3] = {64, (uint32_t)(sp::BN / 2), 1};  // one CTA's half of the B tile for the pair kernel
-      rc = encode_tiled(&tmB_half, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, pbc, dimsb, stridesb, boxh,
-                        CU_TENSOR_MAP_SWIZZLE_128B);
-      if (rc) break;
-    }
-    p.n = w;
-    p.tiles_n = (int)ceil_div(w, sp::BN);
-    p.sbuf = sbuf + j0 * mpad;  // j0 is a multiple of the tile width: the chunk's tile blocks start here
-    {
-      KernelTimer kt(MOMMS_KERNEL_SLICE_OZAKI, X);
-      int variant = 0;
-      ce = sp::launch_slice<0, sp::EPI_OZAKI>(tmA, tmB, tmB_half, p, ds->sm_count, X, &variant);
-      if (ce == cudaSuccess) ce = launch_status();
-      if (ce != cudaSuccess) {
-        rc = cuda_fail(ce, "Ozaki slice launch");
-        break;
-      }
-      call_info().slice_variant = variant;
-    }
-    note_launch();
-    if (verify) {
-      // the recombination waits for the bound's verdict (below)
-      if ((ce = cudaEventRecord(ev.prod[c], X)) != cudaSuccess) rc = cuda_fail(ce, "Ozaki chunk streams");
-    } else {
-      rc = combine_chunk(c, X);
+    if (!last && nch > 1 && !rc) {
+      // the next pass reuses A's planes: s waits for the second stream's products
+      ce = cudaEventRecord(ev.join, ds->aux);
+      if (ce == cudaSuccess) ce = cudaStreamWaitEvent(s, ev.join, 0);
+      if (ce != cudaSuccess) rc = cuda_fail(ce, "Ozaki chunk streams");
     }
   }
 
@@ -1487,10 +1675,13 @@ struct OzakiBatch {
     unsigned long long* maxbits = nullptr;
     int* exps = nullptr;
     __half* planes = nullptr;
-    int* sbuf = nullptr;
+    char* sbuf = nullptr;
     int64_t kp = 0;
     size_t a_plane = 0, b_plane = 0;
+    int planes_each = 0;  // digit or residue planes per operand
+    bool crt = false;
     CombineParams cp;
+    crt::CombineParams ccp;
   };
   std::vector<Prob> probs;
   sp::Params* d_params = nullptr;  // device problem table
@@ -1505,8 +1696,11 @@ bool sp_pairs_available(int* clusters) {
 }
 
 bool ozaki_batchable(const DevGemm& g, int slices) {
-  return slices > 0 && slices <= kOzakiMaxSlices && !g.pk[0] && !g.pk[1] && g.k <= kMaxK && g.m > 0 && g.n > 0 &&
-         g.k > 0;
+  if (!(slices > 0 && slices <= kOzakiMaxSlices && !g.pk[0] && !g.pk[1] && g.k <= kMaxK && g.m > 0 && g.n > 0 &&
+        g.k > 0))
+    return false;
+  // residues only where one pass holds them all
+  return !crt_applies(slices, g.m, g.n, g.k) || crt_per_pass(slices, g.m, g.n, g.k, false) == crt_moduli(slices, g.k);
 }
 
 void ozaki_batch_destroy(OzakiBatch* b) {
@@ -1542,8 +1736,8 @@ int ozaki_batch_create(const DevGemm* gs, const int* slices, int count, cudaStre
   for (int i = 0; i < count; ++i) {
     order[(size_t)i] = i;
     const DevGemm& g = gs[i];
-    cost[(size_t)i] = (double)ceil_div(g.m, 2 * sp::BM) * ceil_div(g.n, sp::BN) * ceil_div(g.k, 64) * slices[i] *
-                      (slices[i] + 1);
+    cost[(size_t)i] = (double)ceil_div(g.m, 2 * sp::BM) * ceil_div(g.n, sp::BN) * ceil_div(g.k, 64) *
+                      (crt_applies(slices[i], g.m, g.n, g.k) ? 2 * crt_moduli(slices[i], g.k) : slices[i] * (slices[i] + 1));
   }
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[(size_t)x] > cost[(size_t)y]; });
   int rc = MOMMS_OK;
@@ -1556,27 +1750,32 @@ int ozaki_batch_create(const DevGemm* gs, const int* slices, int count, cudaStre
     const int64_t m = P.g.m, n = P.g.n, k = P.g.k;
     sp::Params& prm = params[(size_t)oi];
     Schedule sch;
-    if (!slice_params(P.ns, m, k, &prm, &sch)) {
+    P.crt = crt_applies(P.ns, m, n, k);
+    P.planes_each = P.crt ? crt_moduli(P.ns, k) : P.ns;
+    if (P.crt) {
+      crt_slice_params(m, k, 0, P.planes_each, &prm);
+    } else if (!slice_params(P.ns, m, k, &prm, &sch)) {
       rc = fail(MOMMS_ERR_UNSUPPORTED, "Ozaki schedule needs too many groups");
       break;
     }
+    const int ng = P.crt ? P.planes_each : sch.ng;
     P.kp = round_up(k, 8);
     P.a_plane = (size_t)m * P.kp;
     P.b_plane = (size_t)n * P.kp;
     const int64_t mpad = round_up(m, (int64_t)sp::BM);
     const size_t plane = (size_t)mpad * (size_t)round_up(n, (int64_t)sp::BN);
     const size_t eb = (size_t)round_up((m + n) * 12, 256);
-    const size_t pb = (size_t)round_up((int64_t)(P.ns * (P.a_plane + P.b_plane) * 2), 256);
-    rc = alloc(&P.mem, eb + pb + (size_t)sch.ng * plane * 4);
+    const size_t pb = (size_t)round_up((int64_t)(P.planes_each * (P.a_plane + P.b_plane) * 2), 256);
+    rc = alloc(&P.mem, eb + pb + (size_t)ng * plane * (P.crt ? 1 : 4));
     if (rc) break;
     char* base = static_cast<char*>(P.mem);
     P.maxbits = reinterpret_cast<unsigned long long*>(base);
     P.exps = reinterpret_cast<int*>(P.maxbits + (m + n));
     P.planes = reinterpret_cast<__half*>(base + eb);
-    P.sbuf = reinterpret_cast<int*>(base + eb + pb);
+    P.sbuf = base + eb + pb;
     prm.n = n;
     prm.tiles_n = (int)ceil_div(n, sp::BN);
-    prm.sbuf = P.sbuf;
+    prm.sbuf = reinterpret_cast<int*>(P.sbuf);
     prm.plane = (int64_t)plane;
     prm.gchunk = prm.ngroups;  // a batch fills the GPU without splitting a tile's groups
     prm.status = ds->status;
@@ -1586,20 +1785,14 @@ int ozaki_batch_create(const DevGemm* gs, const int* slices, int count, cudaStre
     }
     prm.unit_begin = b->units;
     b->units += (int64_t)((prm.tiles_m + 1) / 2) * prm.tiles_n;
-    combine_params(P.g, P.ns, sch, P.sbuf, (int64_t)plane, mpad, P.exps, P.exps + m, &P.cp);
-    // A [ns][m][kp] and B [ns][n][kp], 128-byte k-blocks, each CTA of a pair
-    // staging half of the 256-row B tile
-    uint64_t dims[3] = {(uint64_t)k, (uint64_t)m, (uint64_t)P.ns};
-    uint64_t strides[2] = {(uint64_t)P.kp * 2, (uint64_t)P.a_plane * 2};
-    uint32_t box[3] = {64, (uint32_t)sp::BM, 1};
-    rc = encode_tiled(&maps[2 * (size_t)oi], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, P.planes, dims, strides, box,
-                      CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) break;
-    uint64_t dimsb[3] = {(uint64_t)k, (uint64_t)n, (uint64_t)P.ns};
-    uint64_t stridesb[2] = {(uint64_t)P.kp * 2, (uint64_t)P.b_plane * 2};
-    uint32_t boxh[3] = {64, (uint32_t)(sp::BN / 2), 1};
-    rc = encode_tiled(&maps[2 * (size_t)oi + 1], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, P.planes + P.ns * P.a_plane,
-                      dimsb, stridesb, boxh, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (P.crt) crt_combine_params(P.g, P.ns, P.planes_each, P.sbuf, (int64_t)plane, mpad, P.exps, P.exps + m, &P.ccp);
+    else combine_params(P.g, P.ns, sch, reinterpret_cast<const int*>(P.sbuf), (int64_t)plane, mpad, P.exps, P.exps + m, &P.cp);
+    // A [planes][m][kp] and B [planes][n][kp], each CTA of a pair staging half
+    // of the 256-row B tile
+    rc = plane_map(&maps[2 * (size_t)oi], P.planes, k, m, P.planes_each, P.kp, P.a_plane, sp::BM);
+    if (!rc)
+      rc = plane_map(&maps[2 * (size_t)oi + 1], P.planes + P.planes_each * P.a_plane, k, n, P.planes_each, P.kp,
+                     P.b_plane, sp::BN / 2);
   }
   if (!rc) rc = alloc(reinterpret_cast<void**>(&b->d_params), params.size() * sizeof(sp::Params));
   if (!rc) rc = alloc(reinterpret_cast<void**>(&b->d_maps), maps.size() * sizeof(CUtensorMap));
@@ -1632,8 +1825,14 @@ int ozaki_batch_launch(OzakiBatch* b, cudaStream_t s, int max_sms) {
     int rc = ozaki_operand_exponents(A, g.a.rs, g.a.cs, g.m, g.k, P.maxbits, P.exps, s);
     if (!rc) rc = ozaki_operand_exponents(B, g.b.cs, g.b.rs, g.n, g.k, P.maxbits + g.m, P.exps + g.m, s);
     if (rc) return rc;
-    ozaki_operand_planes(P.ns, A, g.a.rs, g.a.cs, g.m, g.k, P.planes, P.kp, P.exps, s);
-    ozaki_operand_planes(P.ns, B, g.b.cs, g.b.rs, g.n, g.k, P.planes + P.ns * P.a_plane, P.kp, P.exps + g.m, s);
+    __half* pb = P.planes + P.planes_each * P.a_plane;
+    if (P.crt) {
+      crt_planes(P.ns, A, g.a.rs, g.a.cs, g.m, g.k, P.planes, P.kp, (int64_t)P.a_plane, P.exps, 0, P.planes_each, s);
+      crt_planes(P.ns, B, g.b.cs, g.b.rs, g.n, g.k, pb, P.kp, (int64_t)P.b_plane, P.exps + g.m, 0, P.planes_each, s);
+    } else {
+      ozaki_operand_planes(P.ns, A, g.a.rs, g.a.cs, g.m, g.k, P.planes, P.kp, P.exps, s);
+      ozaki_operand_planes(P.ns, B, g.b.cs, g.b.rs, g.n, g.k, pb, P.kp, P.exps + g.m, s);
+    }
   }
   // one persistent slice launch over every problem's tiles
   int clusters = 0;
@@ -1656,7 +1855,8 @@ int ozaki_batch_launch(OzakiBatch* b, cudaStream_t s, int max_sms) {
   note_launch();
   if (e != cudaSuccess) return cuda_fail(e, "grouped Ozaki slice launch");
   for (auto& P : b->probs) {
-    const int rc = launch_combine(P.cp, 0, P.g.n, ds->sm_count, s);
+    const int rc = P.crt ? launch_crt_combine(P.ccp, P.ns, 0, P.g.n, ds->sm_count, s)
+                         : launch_combine(P.cp, 0, P.g.n, ds->sm_count, s);
     if (rc) return rc;
   }
   return MOMMS_OK;

@@ -12,6 +12,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "exact_round.cuh"
 
 namespace momms {
@@ -42,6 +44,37 @@ __host__ __device__ __forceinline__ int exponent_of_max(unsigned long long b) {
   return (63 - clz64(b)) - 1073;                      // subnormal
 }
 
+template <int NS>
+struct Word {  // an integer type for kDigitBits * NS bits and the rounding carry
+  using type = typename std::conditional<(kDigitBits * NS <= 62), unsigned long long, unsigned __int128>::type;
+};
+
+__host__ __device__ __forceinline__ bool is_negative(double v) {
+#ifdef __CUDA_ARCH__
+  return __double_as_longlong(v) < 0;
+#else
+  unsigned long long b;
+  memcpy(&b, &v, sizeof b);
+  return (b >> 63) != 0;
+#endif
+}
+
+// X = round(|v| * 2^(bits*NS - e)) as an integer, halves up; 0 for every
+// element of a row holding a NaN or an infinity (e == INT32_MAX).
+template <int NS, typename U>
+__host__ __device__ __forceinline__ U scaled_integer(double v, int e) {
+  const unsigned long long ab = abs_bits(v);
+  const unsigned long long frac = ab & ((1ull << 52) - 1);
+  const int be = (int)(ab >> 52);
+  const unsigned long long M = be ? (frac | (1ull << 52)) : frac;
+  const int E = be ? be - 1075 : -1074;  // |v| = M * 2^E
+  const int sh = E - e + kDigitBits * NS;
+  if (e == INT32_MAX) return 0;
+  if (sh >= 0) return (U)M << sh;
+  if (sh > -64) return (U)((M >> (-sh)) + ((M >> (-sh - 1)) & 1ull));
+  return 0;
+}
+
 // Signed digits of v * 2^-e at kDigitBits bits each, nearest rounding at the
 // last digit: X = round(|v| * 2^(bits*NS - e)) as an integer, written as
 //   X = sum_{pos < NS-1} d_pos 2^(bits*pos) + top 2^(bits*(NS-1))
@@ -58,18 +91,7 @@ __host__ __device__ __forceinline__ U offset_digits(double v, int e) {
   U H = 0;
 #pragma unroll
   for (int pos = 0; pos < NS - 1; ++pos) H |= (U)half << (bits * pos);
-  const unsigned long long ab = abs_bits(v);
-  const unsigned long long frac = ab & ((1ull << 52) - 1);
-  const int be = (int)(ab >> 52);
-  const unsigned long long M = be ? (frac | (1ull << 52)) : frac;
-  const int E = be ? be - 1075 : -1074;  // |v| = M * 2^E
-  const int sh = E - e + bits * NS;
-  U X;
-  if (e == INT32_MAX) X = 0;
-  else if (sh >= 0) X = (U)M << sh;
-  else if (sh > -64) X = (U)((M >> (-sh)) + ((M >> (-sh - 1)) & 1ull));
-  else X = 0;
-  return X + H;
+  return scaled_integer<NS, U>(v, e) + H;
 }
 
 // |v| 2^-e for the bound: as bf16 rounded toward zero (0 below bf16's normal

@@ -72,10 +72,15 @@ double estimate_s(const momms_gemm_desc& d) {
   return flops / rate;
 }
 
-size_t footprint_of(const momms_gemm_desc& d) {
+// Operands and work space. A request whose work space would pass the budget
+// only in the larger form it may take (work_bytes) is charged the whole budget.
+size_t footprint_of(const momms_gemm_desc& d, uint64_t budget) {
   const size_t es = d.dtype == MOMMS_DTYPE_F64 ? 8 : 4;
   const double m = (double)d.m, n = (double)d.n, k = (double)d.k;
-  return (size_t)(es * (m * k + k * n + m * n)) + work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k);
+  const size_t ops = (size_t)(es * (m * k + k * n + m * n));
+  const size_t most = ops + work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k, false);
+  if (most <= budget) return most;
+  return std::max<size_t>(ops + work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k, true), budget);
 }
 
 }  // namespace
@@ -341,7 +346,7 @@ int momms_server_submit(momms_server server, const momms_gemm_desc* desc, uint64
         return fail(MOMMS_ERR_INVALID_ARG, "served requests keep their operands resident in device memory");
       }
     }
-  const size_t fp = footprint_of(*desc);
+  const size_t fp = footprint_of(*desc, sv->cfg.hbm_budget_bytes);
   std::lock_guard<std::mutex> lk(sv->mu);
   if (sv->stop) return fail(MOMMS_ERR_SHUTDOWN, "server is stopping");
   if (fp > sv->cfg.hbm_budget_bytes) {

@@ -65,7 +65,7 @@ constexpr int EPI_COLS = BN / (EPI_WARPS / 4);   // columns drained per thread
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
 constexpr int TMEM_COLS = 512;  // two 128 x 256 f32 accumulators
 constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 256;
-constexpr int MAX_GROUPS = 160, MAX_PAIRS = 160;
+constexpr int MAX_GROUPS = 160, MAX_PAIRS = 160, MAX_MODULI = 36;
 
 enum { EPI_F32 = 0, EPI_OZAKI = 1, EPI_BOUND = 2 };
 
@@ -94,9 +94,17 @@ struct Params {
   // element (row, col) at (col / BN) * (tiles_m * BM * BN) + (row / BM) * BM * BN
   // + (col % BN) * BM + row % BM, so that each CTA tile is written as one
   // contiguous block
+  // Residue form (residue != 0): group g is one modulus, its sum is reduced
+  // to a symmetric residue r and its plane holds bytes (r + 128) mod 256: four
+  // columns of a row per 32-bit word, word (col / 4, row) of a tile at
+  // (col % BN / 4) * BM + row % BM (the tile's 32 KB block in the same place)
   int* sbuf;
-  int64_t plane;
+  int64_t plane;  // bytes between group planes in the residue form, else ints
   int64_t rsc, csc;
+  int residue;
+  struct Modulus {
+    float p, inv;
+  } mod[MAX_MODULI];
   // EPI_BOUND: row sums of the scaled magnitudes of A (m) and B's columns
   // (n) in units of 2^-40, each term rounded up; the lower-bound factor for
   // the accumulation; k; the two maxima (bit patterns of non-negative floats)
@@ -247,6 +255,193 @@ __device__ __forceinline__ void prefetch_c_rows(const Params& p, int64_t row_of_
     const int64_t col = col0 + j;
     if (col < p.n) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + col * p.csc));
   }
+}
+
+// Symmetric residues of exact integers |v| <= 2^24: at most p/2 and a
+// rounding of the quotient beyond (|r| <= 128). Two at a time: the FP32
+// operations are packed pairs. nq: the nearest integers to -v/p.
+struct ResidueOf {
+  float2 ninv, p;
+  __device__ __forceinline__ explicit ResidueOf(const Params::Modulus& m)
+      : ninv(make_float2(-m.inv, -m.inv)), p(make_float2(m.p, m.p)) {}
+  __device__ __forceinline__ float2 operator()(float2 v) const {
+    const float2 big = make_float2(12582912.0f, 12582912.0f), nbig = make_float2(-12582912.0f, -12582912.0f);
+    const float2 nq = add2(fma2(v, ninv, big), nbig);
+    return fma2(nq, p, v);
+  }
+};
+
+// Walks one TMEM chunk (this thread's row, NC columns from taddr) 16 columns
+// at a time, the next batch's load in flight: fn(first column, 16 values).
+template <int NC, typename F>
+__device__ __forceinline__ void for_batches(uint32_t taddr, F&& fn) {
+  uint32_t ra[16], rb[16];
+  tc::ld16(taddr, ra);
+#pragma unroll
+  for (int pc = 0; pc < NC / 16; ++pc) {
+    uint32_t(&cur)[16] = (pc & 1) ? rb : ra;
+    uint32_t(&nxt)[16] = (pc & 1) ? ra : rb;
+    tc::ld_wait(cur);
+    if (pc + 1 < NC / 16) tc::ld16(taddr + (pc + 1) * 16, nxt);
+    fn(pc * 16, cur);
+  }
+}
+
+// The bytes of four symmetric residues, one word. Under the exponent of 2^23
+// a float's low byte is (r + 128) mod 256; modulo 255 a residue of 128 would
+// not survive that (modulo 256 it does), so it becomes -127 first.
+template <bool P255>
+__device__ __forceinline__ uint32_t residue_bytes(float2 a, float2 b) {
+  if (P255) {
+    a.x = a.x > 127.0f ? -127.0f : a.x;
+    a.y = a.y > 127.0f ? -127.0f : a.y;
+    b.x = b.x > 127.0f ? -127.0f : b.x;
+    b.y = b.y > 127.0f ? -127.0f : b.y;
+  }
+  const float2 k = make_float2(8388736.0f, 8388736.0f);
+  a = add2(a, k);
+  b = add2(b, k);
+  return __byte_perm(__byte_perm(__float_as_uint(a.x), __float_as_uint(a.y), 0x0040),
+                     __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x0040), 0x5410);
+}
+
+// One residue group of one tile: its chunks' residues to the plane's words
+// `out` of this thread's row (see Params::sbuf), `live` columns of it. Each
+// chunk's values are reduced in FP32 (three packed operations of the wide FMA
+// pipe per pair; the conversion to int32 of the digit form runs at an eighth
+// of that pipe's rate).
+template <int NC, bool P255, typename Wait, typename Release>
+__device__ __forceinline__ bool residue_group(const Params::Modulus& m, int chunks, uint32_t* out, int live, Wait&& wait,
+                                              Release&& release) {
+  const ResidueOf res(m);
+  auto pair = [](const uint32_t(&v)[16], int j) { return make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])); };
+  if (chunks == 1) {
+    // straight from TMEM to bytes
+    const uint32_t taddr = wait();
+    if (taddr == ~0u) return false;
+    for_batches<NC>(taddr, [&](int j0, const uint32_t(&v)[16]) {
+#pragma unroll
+      for (int j = 0; j < 16; j += 4) {
+        const uint32_t w = residue_bytes<P255>(res(pair(v, j)), res(pair(v, j + 2)));
+        if (j0 + j < live) out[((j0 + j) / 4) * BM] = w;
+      }
+    });
+    release();
+    return true;
+  }
+  // several chunks: the residues, plus 128, are summed as pairs of 16-bit
+  // fields (at most 32 chunks of at most 256), half the registers of FP32 sums
+  uint32_t S[NC / 2];
+#pragma unroll
+  for (int j = 0; j < NC / 2; ++j) S[j] = 0;
+  for (int c = 0; c < chunks; ++c) {
+    const uint32_t taddr = wait();
+    if (taddr == ~0u) return false;
+    for_batches<NC>(taddr, [&](int j0, const uint32_t(&v)[16]) {
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        const float2 r = add2(res(pair(v, j)), make_float2(8388736.0f, 8388736.0f));
+        S[(j0 + j) / 2] += __byte_perm(__float_as_uint(r.x), __float_as_uint(r.y), 0x5410);
+      }
+    });
+    release();
+  }
+  const float nbias = -(8388608.0f + 128.0f * (float)chunks);
+  auto sum = [&](int i) {
+    return add2(make_float2(__uint_as_float(0x4B000000u | (S[i] & 0xffffu)), __uint_as_float(0x4B000000u | (S[i] >> 16))),
+                make_float2(nbias, nbias));
+  };
+#pragma unroll
+  for (int j = 0; j < NC; j += 4) {
+    const uint32_t w = residue_bytes<P255>(res(sum(j / 2)), res(sum(j / 2 + 1)));
+    if (j < live) out[(j / 4) * BM] = w;
+  }
+  return true;
+}
+
+// EPI_OZAKI: publishes a group's exact int32 sums of this thread's row.
+template <int NC>
+__device__ __forceinline__ void publish_sums(int* out, int live, const int (&S)[NC]) {
+#pragma unroll
+  for (int j = 0; j < NC; ++j)
+    if (j < live) out[j * BM] = S[j];
+}
+
+// The epilogue of EPI_OZAKI's groups [g0, g1) of one tile: wait() returns
+// the TMEM address of the next finished chunk or ~0 on a timeout, release()
+// hands its buffer back. Returns false on a timeout.
+template <int NC, typename Wait, typename Release>
+__device__ __forceinline__ bool ozaki_groups(const Params& p, int g0, int g1, int64_t row, int64_t col0, int tm, int tn,
+                                             int col_in_tile, int r_local, Wait&& wait, Release&& release) {
+  const int live = row < p.m ? (int)max((int64_t)0, min((int64_t)NC, p.n - col0)) : 0;
+  const size_t tile = (size_t)tn * ((size_t)p.tiles_m * BM * BN) + (size_t)tm * (BM * BN);
+  for (int g = g0; g < g1; ++g) {
+    const int chunks = p.group_chunks[g];
+    if (p.residue) {
+      uint32_t* out = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(p.sbuf) + (size_t)g * p.plane + tile) +
+                      (size_t)(col_in_tile / 4) * BM + r_local;
+      const bool ok = p.mod[g].p == 255.0f ? residue_group<NC, true>(p.mod[g], chunks, out, live, wait, release)
+                                           : residue_group<NC, false>(p.mod[g], chunks, out, live, wait, release);
+      if (!ok) return false;
+    } else {
+      int S[NC];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) S[j] = 0;
+      for (int c = 0; c < chunks; ++c) {
+        const uint32_t taddr = wait();
+        if (taddr == ~0u) return false;
+        drain_chunk<EPI_OZAKI, NC>(taddr, S);
+        release();
+      }
+      // tile-blocked plane: this CTA's 128 x 256 tile is one contiguous block,
+      // column after column of 128 rows (see the host's plane layout)
+      publish_sums<NC>(p.sbuf + (size_t)g * p.plane + tile + (size_t)col_in_tile * BM + r_local, live, S);
+    }
+  }
+  return true;
+}
+
+// The epilogue of EPI_F32 and EPI_BOUND for one tile (groups [g0, g1)), as ozaki_groups.
+template <int EPI, int NC, typename Wait, typename Release>
+__device__ __forceinline__ bool float_groups(const Params& p, int g0, int g1, int64_t row, int64_t col0, Wait&& wait,
+                                             Release&& release) {
+  // per-thread FP32 sums of finished chunks, rounded to nearest, which keeps
+  // the tensor core's internal accumulation to one chunk at a time
+  float S[NC];
+#pragma unroll
+  for (int j = 0; j < NC; ++j) S[j] = 0.0f;
+  for (int g = g0; g < g1; ++g) {
+    for (int c = 0; c < p.group_chunks[g]; ++c) {
+      const uint32_t taddr = wait();
+      if (taddr == ~0u) return false;
+      drain_chunk<EPI_F32, NC>(taddr, S);
+      release();
+    }
+  }
+  if constexpr (EPI == EPI_BOUND) bound_tile<NC>(p, row, col0, S);
+  if (EPI == EPI_F32 && row < p.m) {
+    // C is read 8 columns at a time, every load of a group issued before
+    // the first use (one memory round trip per group, not per element)
+    float* crow = p.c32 + row * p.rsc;
+#pragma unroll
+    for (int j0 = 0; j0 < NC; j0 += 8) {
+      float c0[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int64_t col = col0 + j0 + j;
+        c0[j] = (p.beta_f != 0.0f && col < p.n) ? crow[col * p.csc] : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int64_t col = col0 + j0 + j;
+        if (col < p.n) {
+          const float v = (float)S[j0 + j] * p.alpha_f;
+          crow[col * p.csc] = (p.beta_f == 0.0f) ? v : fmaf(p.beta_f, c0[j], v);
+        }
+      }
+    }
+  }
+  return true;
 }
 
 template <int KIND, int EPI>
@@ -442,67 +637,28 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int64_t row = (int64_t)tm * BM + r_local;
       const int64_t col0 = (int64_t)tn * BN + h * EPI_COLS;
       if (EPI == EPI_F32) prefetch_c_rows<EPI_COLS>(p, (int64_t)tm * BM + q * 32, col0, lane);
-      // per-thread accumulators of finished chunks: exact int32 digit sums
-      // (Ozaki) or FP32 sums rounded to nearest (split-TF32), which keeps the
-      // tensor core's internal accumulation to one chunk at a time
-      EpiAcc<EPI> S[EPI_COLS];
-#pragma unroll
-      for (int j = 0; j < EPI_COLS; ++j) S[j] = EpiAcc<EPI>(0);
-      for (int g = g_begin(t); g < g_end(t); ++g) {
-        for (int c = 0; c < p.group_chunks[g]; ++c) {
-          if (!mbar_wait_bounded(&tfull[buf], acc_ph[buf])) {
-            report_status(p.status, DEV_TIMEOUT_MMA);
-            *abort_flag = 1;
-            goto epi_done;
-          }
-          tc::fence_after();
-          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + h * EPI_COLS);
-          drain_chunk<EPI, EPI_COLS>(taddr, S);
-          tc::fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[buf]);
-          acc_ph[buf] ^= 1;
-          buf ^= 1;
+      // the next finished chunk's TMEM address (~0: timed out), and its release
+      auto wait = [&]() -> uint32_t {
+        if (!mbar_wait_bounded(&tfull[buf], acc_ph[buf])) {
+          report_status(p.status, DEV_TIMEOUT_MMA);
+          *abort_flag = 1;
+          return ~0u;
         }
-        if (EPI == EPI_OZAKI) {
-          // end of group g: publish the exact int32 sums (column-major plane g)
-          if (row < p.m) {
-            // tile-blocked plane: this CTA's 128 x 256 tile is one contiguous
-            // block, column after column of 128 rows (see the host's plane layout)
-            int* srow = p.sbuf + (size_t)g * p.plane + (size_t)tn * ((size_t)p.tiles_m * BM * BN) +
-                        (size_t)tm * (BM * BN) + (size_t)(h * EPI_COLS) * BM + r_local;
-#pragma unroll
-            for (int j = 0; j < EPI_COLS; ++j) {
-              const int64_t col = col0 + j;
-              if (col < p.n) srow[j * BM] = S[j];
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < EPI_COLS; ++j) S[j] = EpiAcc<EPI>(0);
-        }
-      }
-      if constexpr (EPI == EPI_BOUND) bound_tile<EPI_COLS>(p, row, col0, S);
-      if (EPI == EPI_F32 && row < p.m) {
-        // C is read 8 columns at a time, every load of a group issued before
-        // the first use (one memory round trip per group, not per element)
-        float* crow = p.c32 + row * p.rsc;
-#pragma unroll
-        for (int j0 = 0; j0 < EPI_COLS; j0 += 8) {
-          float c0[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int64_t col = col0 + j0 + j;
-            c0[j] = (p.beta_f != 0.0f && col < p.n) ? crow[col * p.csc] : 0.0f;
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int64_t col = col0 + j0 + j;
-            if (col < p.n) {
-              const float v = (float)S[j0 + j] * p.alpha_f;
-              crow[col * p.csc] = (p.beta_f == 0.0f) ? v : fmaf(p.beta_f, c0[j], v);
-            }
-          }
-        }
+        tc::fence_after();
+        return tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + h * EPI_COLS);
+      };
+      auto release = [&]() {
+        tc::fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[buf]);
+        acc_ph[buf] ^= 1;
+        buf ^= 1;
+      };
+      if constexpr (EPI == EPI_OZAKI) {
+        if (!ozaki_groups<EPI_COLS>(p, g_begin(t), g_end(t), row, col0, tm, tn, h * EPI_COLS, r_local, wait, release))
+          goto epi_done;
+      } else {
+        if (!float_groups<EPI, EPI_COLS>(p, g_begin(t), g_end(t), row, col0, wait, release)) goto epi_done;
       }
     }
   epi_done:;
@@ -773,65 +929,26 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int64_t row = (int64_t)tm * BM + r_local;
       const int64_t col0 = (int64_t)tn * BN + h * EPI_COLS;
       if (EPI == EPI_F32) prefetch_c_rows<EPI_COLS>(P, (int64_t)tm * BM + q * 32, col0, lane);
-      EpiAcc<EPI> S[EPI_COLS];
-#pragma unroll
-      for (int j = 0; j < EPI_COLS; ++j) S[j] = EpiAcc<EPI>(0);
-      for (int g = g0; g < g1; ++g) {
-        for (int c = 0; c < P.group_chunks[g]; ++c) {
-          if (!mbar_wait_bounded(&tfull[buf], acc_ph[buf])) {
-            report_status(status, DEV_TIMEOUT_MMA);
-            *abort_flag = 1;
-            return false;
-          }
-          tc::fence_after();
-          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + h * EPI_COLS);
-          drain_chunk<EPI, EPI_COLS>(taddr, S);
-          tc::fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster_relaxed(tempty_leader[buf]);
-          acc_ph[buf] ^= 1;
-          buf ^= 1;
+      auto wait = [&]() -> uint32_t {
+        if (!mbar_wait_bounded(&tfull[buf], acc_ph[buf])) {
+          report_status(status, DEV_TIMEOUT_MMA);
+          *abort_flag = 1;
+          return ~0u;
         }
-        if (EPI == EPI_OZAKI) {
-          if (row < P.m) {
-            // tile-blocked plane: this CTA's 128 x 256 tile is one contiguous
-            // block, column after column of 128 rows (see the host's plane layout)
-            int* srow = P.sbuf + (size_t)g * P.plane + (size_t)tn * ((size_t)P.tiles_m * BM * BN) +
-                        (size_t)tm * (BM * BN) + (size_t)(h * EPI_COLS) * BM + r_local;
-#pragma unroll
-            for (int j = 0; j < EPI_COLS; ++j) {
-              const int64_t col = col0 + j;
-              if (col < P.n) srow[j * BM] = S[j];
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < EPI_COLS; ++j) S[j] = EpiAcc<EPI>(0);
-        }
-      }
-      if constexpr (EPI == EPI_BOUND) bound_tile<EPI_COLS>(P, row, col0, S);
-      if (EPI == EPI_F32 && row < P.m) {
-        // C is read 8 columns at a time, every load of a group issued before
-        // the first use (one memory round trip per group, not per element)
-        float* crow = P.c32 + row * P.rsc;
-#pragma unroll
-        for (int j0 = 0; j0 < EPI_COLS; j0 += 8) {
-          float c0[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int64_t col = col0 + j0 + j;
-            c0[j] = (P.beta_f != 0.0f && col < P.n) ? crow[col * P.csc] : 0.0f;
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int64_t col = col0 + j0 + j;
-            if (col < P.n) {
-              const float v = (float)S[j0 + j] * P.alpha_f;
-              crow[col * P.csc] = (P.beta_f == 0.0f) ? v : fmaf(P.beta_f, c0[j], v);
-            }
-          }
-        }
-      }
-      return true;
+        tc::fence_after();
+        return tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + h * EPI_COLS);
+      };
+      auto release = [&]() {
+        tc::fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster_relaxed(tempty_leader[buf]);
+        acc_ph[buf] ^= 1;
+        buf ^= 1;
+      };
+      if constexpr (EPI == EPI_OZAKI)
+        return ozaki_groups<EPI_COLS>(P, g0, g1, row, col0, tm, tn, h * EPI_COLS, r_local, wait, release);
+      else
+        return float_groups<EPI, EPI_COLS>(P, g0, g1, row, col0, wait, release);
     };
     bool ok = true;
     for (int64_t r = 0; r * unit_step < units && ok && !aborted(abort_flag); ++r) {

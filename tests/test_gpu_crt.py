@@ -1,0 +1,74 @@
+"""The residue form of the emulated product on the GPU: the result is the exact integer product
+rounded once, so it is within half an ulp (and alpha, beta) of the double-double oracle, over tile
+and chunk edges, layouts, slice counts, passes under a scratch limit, and packed operands."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import momms_gb300 as mg
+from tests import gpu_util as gu
+from tests import oracle_util as ou
+
+pytestmark = pytest.mark.gpu
+
+
+def _call(gpu, A, B, C0, s, alpha=1.0, beta=0.0):
+    C = gu.gemm_device(gpu, A, B, C0, alpha, beta, precision=mg.PREC_OZAKI, slices=s)
+    info = mg.CallInfo()
+    gpu.momms_last_info(ctypes.byref(info))
+    return C, info
+
+
+# one and several TMEM chunks (16 k-blocks of 64), tile remainders in m and n, row and column quads
+@pytest.mark.parametrize("shape", [(2049, 2050, 1024), (1300, 1027, 1025), (1153, 1281, 4001), (2049, 770, 1700)])
+@pytest.mark.parametrize("s", [10, 12, 15])
+def test_within_an_ulp_of_the_exact_product(gpu, shape, s):
+    m, n, k = shape
+    rng = np.random.default_rng(m + n + k + s)
+    A = np.asfortranarray(rng.uniform(-1, 1, (m, k)))
+    B = rng.uniform(-1, 1, (k, n))
+    C, info = _call(gpu, A, B, np.zeros((m, n), order="F"), s)
+    assert info.pairs < s * (s + 1) // 2  # the residue form ran
+    rows = rng.choice(m, 24, replace=False)
+    ref, mag = ou.dd_gemm(np.asfortranarray(A[rows]), np.asfortranarray(B), np.zeros((24, n), order="F"), 1.0, 0.0)
+    # operands rounded at 2^-(8s+1) of their row or column maximum, one rounding of the product
+    tol = 2.0**-53 * np.abs(ref) * 1.01 + k * 2.0 ** (-8 * s) * 1.01 + 2.0**-100 * mag
+    assert np.all(np.abs(C[rows] - ref) <= tol)
+
+
+def test_passes_and_packs_give_the_same_bits(gpu):
+    """Streamed blocks (which hold their scratch to the digit form's by passes over the moduli)
+    and packed operands (residues taken from their digits) against the plain call."""
+    m, n, k, s = 2100, 1900, 2300, 8
+    rng = np.random.default_rng(11)
+    A = np.asfortranarray(rng.uniform(-1, 1, (m, k)))
+    B = np.asfortranarray(rng.uniform(-1, 1, (k, n)))
+    C0 = np.asfortranarray(rng.uniform(-1, 1, (m, n)))
+    want, info = _call(gpu, A, B, C0, s, -1.0, 1.0)
+    assert info.pairs < 36
+    gpu.momms_set_staging_budget(300 << 20)  # 1280 x 1024 blocks of the whole k
+    try:
+        got = gu.gemm_host(gpu, A, B, C0.copy(order="F"), -1.0, 1.0, precision=mg.PREC_OZAKI, slices=s)
+    finally:
+        gpu.momms_set_staging_budget(0)
+    assert np.array_equal(got, want)
+    packs = []
+    for role, x in ((mg.ROLE_A, A), (mg.ROLE_B, B)):
+        t, rs, cs = gu.to_device(x)
+        h = ctypes.c_void_p()
+        src = mg.Operand(t.data_ptr(), rs, cs, mg.MEM_DEVICE, 0)
+        mg.check(gpu.momms_pack(mg.DTYPE_F64, mg.PREC_OZAKI, role, *x.shape, ctypes.byref(src), s, None, ctypes.byref(h)), gpu)
+        packs.append(h)
+    tc, rs, cs = gu.to_device(C0)
+    d = gu.make_desc(mg.DTYPE_F64, m, n, k, -1.0, 1.0, (0, 0, 0), (0, 0, 0), (tc.data_ptr(), rs, cs),
+                     precision=mg.PREC_OZAKI, mem=mg.MEM_DEVICE, slices=s)
+    d.a, d.b = (mg.Operand(h.value, 0, 0, mg.MEM_PACKED, 0) for h in packs)
+    mg.check(gpu.momms_gemm(ctypes.byref(d), None), gpu)
+    import torch
+    torch.cuda.synchronize()
+    assert np.array_equal(tc.cpu().numpy(), want)
+    for h in packs:
+        mg.check(gpu.momms_packed_destroy(h), gpu)
+    bits = ctypes.c_uint32(0)
+    assert gpu.momms_device_status(ctypes.byref(bits)) == mg.OK and bits.value == 0
