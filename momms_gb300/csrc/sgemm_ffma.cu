@@ -11,6 +11,7 @@
 // microkernel's order, d6x8.c:725-885), then acc*alpha, then
 // fma(beta, c, acc).
 #include "ffma_core.cuh"
+#include "ffma_small.cuh"
 #include "internal.h"
 
 namespace momms {
@@ -55,6 +56,27 @@ __global__ void __launch_bounds__(Tile<TM>::THREADS, Tile<TM>::CTAS_PER_SM)
     } else {
       ffma_finish<TM>(p.e, acc, tm, tn, 1, 0, nullptr, nullptr, &s_last);
     }
+  }
+}
+
+template <bool A_XC, bool B_XC>
+__global__ void __launch_bounds__(Small::THREADS, Small::CTAS_PER_SM)
+    sgemm_small_kernel(const __grid_constant__ Params p) {
+  extern __shared__ float4 ffma_smem[];
+  __shared__ int s_last;
+  const int64_t units = p.sched.units();
+  for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
+    int tm, tn, sp;
+    p.sched.decode(u, tm, tn, sp);
+    const int64_t k0 = sp * p.sched.k_per_split, k1 = min(p.o.k, k0 + p.sched.k_per_split);
+    const int64_t m0 = (int64_t)tm * Small::TILE, n0 = (int64_t)tn * Small::TILE;
+    float acc[2][4] = {};
+    small_unit<A_XC, B_XC>(p.o, m0, n0, k0, k1, acc, reinterpret_cast<float*>(ffma_smem));
+    const int64_t tile = u / p.sched.splits;
+    const bool split = p.sched.splits > 1;
+    small_finish(p.e, acc, m0, n0, p.sched.splits, sp,
+                 split ? p.partials + (size_t)tile * p.sched.splits * Small::TILE * Small::TILE : nullptr,
+                 split ? p.counters + tile : nullptr, &s_last);
   }
 }
 
@@ -118,14 +140,20 @@ int sgemm_ffma_impl(const DevGemm& g0, cudaStream_t s, void* (&scratch)[3]) {
   p.e = Epi{g.m, g.n, (float)g.alpha, (float)g.beta, static_cast<float*>(g.c.ptr), g.c.rs, g.c.cs};
   // the tile and split count of this shape (tuning table or model)
   const PlainCfg cfg = plain_cfg(MOMMS_DTYPE_F32, g.m, g.n, g.k, ds->sm_count);
-  const int TMv = cfg.tile == 1 ? 64 : 128;
+  const int64_t kblocks = ceil_div(g.k, BK), kb_split = ceil_div(kblocks, cfg.splits);
+  const int splits = (int)ceil_div(kblocks, kb_split);
+  // Fewer units of 128 x 128 than SMs (few tiles and a short k): 32 x 32 tiles
+  // of the same splits, with the same results. 256 x 300 x 200 28.7 -> 8.2 us,
+  // 512^3 33 -> 22.3 us; with more units (1024^3: 256) the large tile is faster,
+  // 72 against 84 us. (Fewer splits would be faster still, 16.5 us at 512^3, but
+  // round more: longer chains.)
+  const bool small = cfg.tile == 0 && ceil_div(g.m, 128) * ceil_div(g.n, 128) * splits < ds->sm_count;
+  const int TMv = small ? Small::TILE : cfg.tile == 1 ? 64 : 128;
   const int tiles_m = (int)ceil_div(g.m, TMv), tiles_n = (int)ceil_div(g.n, TMv);
   const int64_t tiles = (int64_t)tiles_m * tiles_n;
-  const int64_t kblocks = ceil_div(g.k, BK);
-  const int slots = ds->sm_count * (cfg.tile == 1 ? Tile<64>::CTAS_PER_SM : Tile<128>::CTAS_PER_SM);
-  int splits = cfg.splits;
-  int64_t kb_split = ceil_div(kblocks, splits);
-  splits = (int)ceil_div(kblocks, kb_split);
+  const int slots = ds->sm_count * (small           ? Small::CTAS_PER_SM
+                                    : cfg.tile == 1 ? Tile<64>::CTAS_PER_SM
+                                                    : Tile<128>::CTAS_PER_SM);
   p.sched = TileSched{tiles_m, tiles_n, splits, 8, kb_split * BK};
   call_info().splits = splits;
   p.partials = nullptr;
@@ -144,7 +172,11 @@ int sgemm_ffma_impl(const DevGemm& g0, cudaStream_t s, void* (&scratch)[3]) {
     KernelTimer kt(MOMMS_KERNEL_SGEMM_FFMA, s);
     // one instantiation per (tile, A layout, B layout, offset width, split)
     const int li = offsets_fit_32(p.o) ? 0 : 1, si = splits > 1 ? 1 : 0;
-    if (cfg.tile == 1)
+    if (small) {
+      static const Kern kSmall[2][2] = {{sgemm_small_kernel<false, false>, sgemm_small_kernel<false, true>},
+                                        {sgemm_small_kernel<true, false>, sgemm_small_kernel<true, true>}};
+      kSmall[a_xc][b_xc]<<<grid, Small::THREADS, Small::SMEM_BYTES, s>>>(p);
+    } else if (cfg.tile == 1)
       kernel_table<64>()[a_xc][b_xc][li][si]<<<grid, Tile<64>::THREADS, Tile<64>::SMEM_BYTES, s>>>(p);
     else
       kernel_table<128>()[a_xc][b_xc][li][si]<<<grid, Tile<128>::THREADS, Tile<128>::SMEM_BYTES, s>>>(p);
