@@ -237,9 +237,14 @@ int ozaki_operand_exponents(const double* x, int64_t sr, int64_t sp, int64_t R, 
                             unsigned long long* maxbits, int* exps, cudaStream_t s);
 void ozaki_operand_planes(int ns, const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K, void* planes,
                           int64_t kp, const int* exps, cudaStream_t s);
-// The two TF32 planes [2][R][kp] of an f32 view.
-void tf32_operand_planes(const float* x, int64_t sr, int64_t sp, int64_t R, int64_t K, float* planes, int64_t kp,
-                         cudaStream_t s);
+// The two TF32 planes [2][R][kp] of one or two f32 views (element (r, p) at
+// x[r*sr + p*sp], p < K), in one launch.
+struct F32View {
+  const float* x;
+  int64_t sr, sp, R;
+  float* planes;
+};
+void tf32_operand_planes(const F32View* v, int count, int64_t K, int64_t kp, cudaStream_t s);
 
 // Copy an operand into a column-major device scratch matrix with an even
 // leading dimension (used when its strides or alignment do not suit TMA or

@@ -64,66 +64,133 @@ constexpr int64_t kCrtMinK = 128;
 // Everything in the pre-pass runs on integer bit patterns: GB300's FP64 pipe
 // is about 1 TFLOP/s, so FP64 arithmetic per element would dominate.
 
-// Row maxima of |x(r, p)| as bit patterns, rows contiguous (sr == 1, a
-// column-major A). A block covers 32 rows x 256 of p: lanes along r, the 8
-// warps striding over p, each thread's 32 loads issued before the first
-// maximum; the warps' maxima meet in shared memory and one atomicMax per row
-// posts them (maxbits must start at zero). At 8192^2 this reads at 5.0 TB/s
-// (104-108 us), against 4.0 for the run layout of the other prep kernels
-// (133 us); with p contiguous the run layout is the faster one (132 us,
-// against 230 for a warp per row with lanes along p in this block shape).
-__global__ void __launch_bounds__(256) row_absmax_kernel(const double* __restrict__ x, int64_t sp, int64_t R,
-                                                         int64_t K, unsigned long long* __restrict__ maxbits) {
-  __shared__ unsigned long long red[8][33];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int64_t r = (int64_t)blockIdx.y * 32 + tx, p0 = (int64_t)blockIdx.x * 256;
-  unsigned long long mx = 0;
-  if (r < R) {
-    double v[32];
+// Row maxima of |x(r, p)| as bit patterns (maxbits must start at zero).
+//  * Rows contiguous (sr == 1, a column-major A): a block covers 32 rows x 64
+//    of p per iteration: lanes along r, the 8 warps striding over p, each
+//    thread's 8 (four iterations: 32) loads issued before the first maximum;
+//    the warps' maxima meet in shared memory and one atomicMax per row posts
+//    them. At 8192^2 this reads at 5.0 TB/s (104-108 us), against 4.0 for the
+//    run layout of the other prep passes (133 us).
+//  * p contiguous (or general strides): the run layout of planes.cuh, the
+//    lanes of one row reducing by shuffles, one atomicMax each (132 us, against
+//    230 for a warp per row with lanes along p in the other block shape).
+struct AbsmaxBody {
+  using Tin = double;
+  static constexpr int RUN = 8, kContigLg = planes::kRowsContigLg;
+  template <bool R_CONTIG>
+  static int rows(int lg) { return R_CONTIG ? 32 : planes::run_rows(lg); }
+  template <bool R_CONTIG>
+  static int64_t cols(int lg, int iters) { return (R_CONTIG ? 64 : (int64_t)RUN << lg) * iters; }
+  unsigned long long* maxbits[2];
+
+  template <int LOADS>
+  __device__ __forceinline__ void column_block(const planes::View<double>& v, unsigned long long* out) const {
+    __shared__ unsigned long long red[8][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t p0 = (int64_t)blockIdx.x * (8 * LOADS);
+    for (int64_t rb = (int64_t)blockIdx.y * 32; rb < v.R; rb += (int64_t)gridDim.y * 32) {
+      const int64_t r = rb + tx;
+      unsigned long long mx = 0;
+      if (r < v.R) {
+        double x[LOADS];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int64_t pp = p0 + ty + 8 * j;
-      v[j] = pp < K ? x[r + pp * sp] : 0.0;
+        for (int j = 0; j < LOADS; ++j) {
+          const int64_t pp = p0 + ty + 8 * j;
+          x[j] = pp < v.K ? v.x[r + pp * v.sp] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j) mx = max(mx, abs_bits(x[j]));
+      }
+      red[ty][tx] = mx;
+      __syncthreads();
+      if (ty == 0 && r < v.R) {
+        for (int i = 1; i < 8; ++i) mx = max(mx, red[i][tx]);
+        if (mx) atomicMax(&out[r], mx);
+      }
+      __syncthreads();
     }
+  }
+
+  template <bool R_CONTIG>
+  __device__ __forceinline__ void run(const planes::View<double>& v, int z) const {
+    unsigned long long* out = maxbits[z];
+    if (R_CONTIG) {
+      if (v.iters == planes::PITER) column_block<8 * planes::PITER>(v, out);
+      else column_block<8>(v, out);
+      return;
+    }
+    const planes::Chunk<false> c(v.lg);
+    // the row loop's trip count is the same for every thread of the block, so
+    // every lane reaches the shuffles
+    for (int64_t rb = (int64_t)blockIdx.y * c.rows; rb < v.R; rb += (int64_t)gridDim.y * c.rows) {
+      const int64_t r = rb + c.rl;
+      unsigned long long mx = 0;
+      if (r < v.R) {
+        const double* xr = v.x + r * v.sr;
+#pragma unroll 1
+        for (int it = 0; it < v.iters; ++it) {
+          const int64_t p = planes::run_col(blockIdx.x, c, it, RUN, v.iters);
+          if (p >= v.K) break;
+          double x[RUN];
+          planes::load_run<false, RUN>(xr, v.sp, p, v.K, v.vec, x);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) mx = max(mx, abs_bits(v[j]));
+          for (int i = 0; i < RUN; ++i) mx = max(mx, abs_bits(x[i]));
+        }
+      }
+      for (int o = c.runs >> 1; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (c.ru == 0 && r < v.R && mx) atomicMax(&out[r], mx);
+    }
   }
-  red[ty][tx] = mx;
-  __syncthreads();
-  if (ty == 0 && r < R) {
-    for (int i = 1; i < 8; ++i) mx = max(mx, red[i][tx]);
-    if (mx) atomicMax(&maxbits[r], mx);
-  }
+};
+
+// One operand of a product in the passes below: the R x K view (element (r, p)
+// at x[r*sr + p*sp]; A, or B transposed) and its rows' exponents, either given
+// or as the row maxima they follow from.
+struct Side {
+  const double* x;
+  int64_t sr, sp, R;
+  unsigned long long* maxbits;
+  int* exps;
+};
+Side side_a(const DevGemm& g, unsigned long long* maxbits, int* exps) {
+  return Side{static_cast<const double*>(g.a.ptr), g.a.rs, g.a.cs, g.m, maxbits, exps};
+}
+Side side_b(const DevGemm& g, unsigned long long* maxbits, int* exps) {
+  return Side{static_cast<const double*>(g.b.ptr), g.b.cs, g.b.rs, g.n, maxbits, exps};
+}
+planes::Views<double> views_of(const Side* sides, int count, int64_t K) {
+  planes::Views<double> vs{};
+  for (int i = 0; i < count; ++i) vs.v[i] = planes::make_view(sides[i].x, sides[i].sr, sides[i].sp, sides[i].R, K);
+  return vs;
 }
 
-// Row maxima with p contiguous (or general strides), in the run layout of
-// planes.cuh: the lanes of one row reduce by shuffles and one posts an
-// atomicMax (maxbits must start at zero).
-__global__ void __launch_bounds__(planes::THREADS)
-    row_absmax_runs_kernel(const double* __restrict__ x, int64_t sr, int64_t sp, int64_t R, int64_t K, bool vec,
-                           int lg, unsigned long long* __restrict__ maxbits) {
-  constexpr int RUN = 8;
-  const planes::Chunk<false> c(lg);
-  // the row loop's trip count is the same for every thread of the block, so
-  // every lane reaches the shuffles
-  for (int64_t rb = (int64_t)blockIdx.y * c.rows; rb < R; rb += (int64_t)gridDim.y * c.rows) {
-    const int64_t r = rb + c.rl;
-    unsigned long long mx = 0;
-    if (r < R) {
-      const double* xr = x + r * sr;
-#pragma unroll 1
-      for (int it = 0; it < planes::PITER; ++it) {
-        const int64_t p = planes::run_col(blockIdx.x, c, it, RUN);
-        if (p >= K) break;
-        double v[RUN];
-        planes::load_run<false, RUN>(xr, sp, p, K, vec, v);
-#pragma unroll
-        for (int i = 0; i < RUN; ++i) mx = max(mx, abs_bits(v[i]));
-      }
-    }
-    for (int o = c.runs >> 1; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (c.ru == 0 && r < R && mx) atomicMax(&maxbits[r], mx);
+// A row's exponent: from its maximum, and written out for the passes that
+// follow (`out`, may be null), or as given.
+struct RowExp {
+  const unsigned long long* maxbits;  // null: given
+  const int* exps;
+  int* out;
+  __device__ __forceinline__ int row(int64_t r) const { return maxbits ? exponent_of_max(maxbits[r]) : exps[r]; }
+  __device__ __forceinline__ void first(int64_t r, int e) const {
+    if (out) out[r] = e;
   }
+};
+// from_max: the exponents are not written yet
+RowExp row_exp(const Side& s, bool from_max) {
+  return RowExp{from_max ? s.maxbits : nullptr, s.exps, from_max ? s.exps : nullptr};
+}
+
+// Row maxima of the sides (maxbits zeroed by the caller).
+int enqueue_absmax(const Side* sides, int count, int64_t K, cudaStream_t s) {
+  AbsmaxBody body{};
+  for (int i = 0; i < count; ++i) body.maxbits[i] = sides[i].maxbits;
+  {
+    KernelTimer kt(MOMMS_KERNEL_PREP, s);
+    planes::launch_views(views_of(sides, count, K), count, body, s);
+  }
+  note_launch();
+  const cudaError_t e = launch_status();
+  return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "Ozaki exponents");
 }
 
 __global__ void exps_kernel(const unsigned long long* __restrict__ maxbits, int64_t count, int* __restrict__ exps) {
@@ -145,8 +212,9 @@ struct OzakiSliceOp {
   using Tout = __half;
   using Word = uint32_t;  // one pair's __half2 bits
   using U = typename std::conditional<(kDigitBits * NS <= 62), unsigned long long, unsigned __int128>::type;
-  const int* exps;
-  __device__ __forceinline__ int row(int64_t r) const { return exps[r]; }
+  RowExp re;
+  __device__ __forceinline__ int row(int64_t r) const { return re.row(r); }
+  __device__ __forceinline__ void first(int64_t r, int e) const { re.first(r, e); }
   // 32-bit word w of Y
   __device__ __forceinline__ static uint32_t word(U y, int w) { return (uint32_t)(y >> (32 * w)); }
   __device__ __forceinline__ static uint32_t bits_of(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
@@ -181,23 +249,34 @@ struct OzakiSliceOp {
 };
 
 template <int NS>
-void launch_ozaki_planes(const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K, __half* planes, int64_t ldp,
-                         int64_t plane_elems, const int* exps, cudaStream_t s) {
-  planes::launch_to_planes(x, sr, sp, R, K, planes, ldp, plane_elems, OzakiSliceOp<NS>{exps}, s);
+void launch_ozaki_planes(const Side* sides, int count, int64_t K, __half* const* out, int64_t ldp,
+                         const int64_t* plane_elems, bool from_max, cudaStream_t s) {
+  planes::PlanesBody<double, OzakiSliceOp<NS>> body{};
+  body.ldp = ldp;
+  for (int i = 0; i < count; ++i) {
+    body.planes[i] = out[i];
+    body.plane_elems[i] = plane_elems[i];
+    body.op[i] = OzakiSliceOp<NS>{row_exp(sides[i], from_max)};
+  }
+  planes::launch_to_planes(views_of(sides, count, K), count, body, s);
 }
 
-// Runtime slice count -> the unrolled kernel for it (1..kOzakiMaxSlices).
-void ozaki_planes(int ns, const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K, __half* planes, int64_t ldp,
-                  int64_t plane_elems, const int* exps, cudaStream_t s) {
+// The ns digit planes of the sides (runtime slice count -> the unrolled kernel
+// for it, 1..kOzakiMaxSlices). from_max: the exponents come from the row
+// maxima and are written here.
+void ozaki_planes(int ns, const Side* sides, int count, int64_t K, __half* const* out, int64_t ldp,
+                  const int64_t* plane_elems, bool from_max, cudaStream_t s) {
+  KernelTimer kt(MOMMS_KERNEL_PREP, s);
   switch (ns) {
 #define MOMMS_OZAKI_NS(N) \
-  case N: launch_ozaki_planes<N>(x, sr, sp, R, K, planes, ldp, plane_elems, exps, s); break;
+  case N: launch_ozaki_planes<N>(sides, count, K, out, ldp, plane_elems, from_max, s); break;
     MOMMS_OZAKI_NS(1) MOMMS_OZAKI_NS(2) MOMMS_OZAKI_NS(3) MOMMS_OZAKI_NS(4) MOMMS_OZAKI_NS(5) MOMMS_OZAKI_NS(6)
     MOMMS_OZAKI_NS(7) MOMMS_OZAKI_NS(8) MOMMS_OZAKI_NS(9) MOMMS_OZAKI_NS(10) MOMMS_OZAKI_NS(11) MOMMS_OZAKI_NS(12)
     MOMMS_OZAKI_NS(13) MOMMS_OZAKI_NS(14) MOMMS_OZAKI_NS(15)
 #undef MOMMS_OZAKI_NS
     default: break;
   }
+  note_launch();
 }
 
 // Sampled quantities for the slice-count bound: for sampled (i, j),
@@ -484,16 +563,6 @@ double ozaki_bound(int s, int bits, double q1, double q2) {
   return ldexp(1.0, -bits * s - 1) * (q1 + 0.5 * (s - 1) * q2);
 }
 
-// Row exponents of A (first m) and column exponents of B (next n).
-int compute_exponents(const DevGemm& g, unsigned long long* maxbits, int* exps, cudaStream_t s) {
-  // A viewed as m x k; B viewed transposed, n x k
-  int rc = ozaki_operand_exponents(static_cast<const double*>(g.a.ptr), g.a.rs, g.a.cs, g.m, g.k, maxbits, exps, s);
-  if (!rc)
-    rc = ozaki_operand_exponents(static_cast<const double*>(g.b.ptr), g.b.cs, g.b.rs, g.n, g.k, maxbits + g.m,
-                                 exps + g.m, s);
-  return rc;
-}
-
 // Smallest slice count whose sampled worst-case bound meets the target
 // (0 = FP64 level, 2^-52). Synchronises the stream once to read the sample.
 int choose_slices(const DevGemm& g, const int* rexp, const int* cexp, double target, int bits, cudaStream_t s,
@@ -535,35 +604,26 @@ int choose_slices(const DevGemm& g, const int* rexp, const int* cexp, double tar
 int ozaki_operand_exponents(const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K,
                             unsigned long long* maxbits, int* exps, cudaStream_t s) {
   if (R == 0) return MOMMS_OK;
-  const bool r_contig = (sr == 1 && sp != 1);
-  KernelTimer kt(MOMMS_KERNEL_PREP, s);
   cudaError_t ce = cudaMemsetAsync(maxbits, 0, (size_t)R * sizeof(unsigned long long), s);
   if (ce != cudaSuccess) return cuda_fail(ce, "Ozaki exponents");
-  int launches = 1;
-  if (r_contig) {
-    // rows in launches of at most 65535 row tiles (the grid's y limit)
-    for (int64_t rb = 0; rb < R; rb += (int64_t)65535 * 32, ++launches) {
-      const int64_t rn = std::min<int64_t>(R - rb, (int64_t)65535 * 32);
-      row_absmax_kernel<<<dim3((unsigned)ceil_div(K, 256), (unsigned)ceil_div(rn, 32)), dim3(32, 8), 0, s>>>(
-          x + rb, sp, rn, K, maxbits + rb);
-    }
-  } else {
-    const int lg = planes::run_lanes_log2(K, 8, false, planes::kRowsContigLg);
-    row_absmax_runs_kernel<<<planes::run_grid<false, 8>(R, K, lg), planes::THREADS, 0, s>>>(
-        x, sr, sp, R, K, planes::rows_vector_aligned(x, sr, sp), lg, maxbits);
-    ++launches;
+  const Side side{x, sr, sp, R, maxbits, exps};
+  const int rc = enqueue_absmax(&side, 1, K, s);
+  if (rc) return rc;
+  {
+    KernelTimer kt(MOMMS_KERNEL_PREP, s);
+    exps_kernel<<<(unsigned)ceil_div(R, 256), 256, 0, s>>>(maxbits, R, exps);
   }
-  exps_kernel<<<(unsigned)ceil_div(R, 256), 256, 0, s>>>(maxbits, R, exps);
-  note_launch(launches);
+  note_launch();
   ce = launch_status();
   return ce == cudaSuccess ? MOMMS_OK : cuda_fail(ce, "Ozaki exponents");
 }
 
 void ozaki_operand_planes(int ns, const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K, void* planes,
                           int64_t kp, const int* exps, cudaStream_t s) {
-  KernelTimer kt(MOMMS_KERNEL_PREP, s);
-  ozaki_planes(ns, x, sr, sp, R, K, static_cast<__half*>(planes), kp, R * kp, exps, s);
-  note_launch();
+  const Side side{x, sr, sp, R, nullptr, const_cast<int*>(exps)};
+  __half* out[1] = {static_cast<__half*>(planes)};
+  const int64_t pe[1] = {R * kp};
+  ozaki_planes(ns, &side, 1, K, out, kp, pe, false, s);
 }
 
 int set_attrs_ozaki() {
@@ -782,13 +842,23 @@ int crt_per_pass(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
   return (int)ceil_div(N, passes);
 }
 
-// Residue planes l0..l1-1 of an operand view, or of a packed operand's digits.
-void crt_planes(int ns, const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K, __half* out, int64_t ldp,
-                int64_t plane_elems, const int* exps, int l0, int l1, cudaStream_t s) {
+// Residue planes l0..l1-1 of the sides, or of a packed operand's digits.
+void crt_planes(int ns, const Side* sides, int count, int64_t K, __half* const* out, int64_t ldp,
+                const int64_t* plane_elems, bool from_max, int l0, int l1, cudaStream_t s) {
   KernelTimer kt(MOMMS_KERNEL_PREP, s);
+  const planes::Views<double> vs = views_of(sides, count, K);
+  auto launch = [&](auto body) {
+    body.ldp = ldp;
+    body.l0 = l0, body.l1 = l1;
+    for (int i = 0; i < count; ++i) {
+      body.out[i] = out[i];
+      body.plane_elems[i] = plane_elems[i];
+      body.re[i] = row_exp(sides[i], from_max);
+    }
+    planes::launch_views(vs, count, body, s);
+  };
   switch (ns) {
-#define X(NS) \
-  case NS: crt::launch_residues<NS>(x, sr, sp, R, K, out, ldp, plane_elems, exps, l0, l1, s); break;
+#define X(NS) case NS: launch(crt::ResidueBody<NS, RowExp>{}); break;
     MOMMS_CRT_NS(X)
 #undef X
     default: refuse_launch(cudaErrorInvalidValue);
@@ -957,9 +1027,8 @@ int guaranteed_slices(double target, double q1, double q2, bool uncovered, bool*
 
 // Scratch of the bound: bf16 magnitude planes of A (m rows) and of B
 // transposed (n rows), K-major with row stride kp; the rows' sums of scaled
-// magnitudes (units of 2^-40, m then n, contiguous) and the result words
-// right after them: out[0], out[1] the maxima (float bits), out[2..3] a
-// 64-bit count of covered entries.
+// magnitudes (units of 2^-40, m then n) and the result words: out[0], out[1]
+// the maxima (float bits), out[2..3] a 64-bit count of covered entries.
 struct BoundWork {
   uint16_t* mag_a;
   uint16_t* mag_b;
@@ -970,90 +1039,119 @@ struct BoundWork {
 };
 size_t bound_work_bytes(int64_t m, int64_t n, int64_t k) {
   const int64_t kp = round_up(k, 8);
-  return (size_t)round_up(m * kp * 2, 256) + (size_t)round_up(n * kp * 2, 256) + (size_t)(m + n) * 8 + 16;
+  return (size_t)round_up(m * kp * 2, 256) + (size_t)round_up(n * kp * 2, 256);
 }
-void bound_work_carve(void* base, int64_t m, int64_t n, int64_t k, BoundWork* w) {
+
+// The per-row words of a call's passes, zeroed by one memset where they must
+// start at zero: row maxima (m + n), the bound's sums (m + n) and result words;
+// then the exponents (m + n).
+struct RowWork {
+  unsigned long long* maxbits;
+  unsigned long long* sums;
+  unsigned* out;
+  int* exps;
+};
+constexpr size_t kBoundWords = 4;
+size_t row_work_zero_bytes(int64_t m, int64_t n) { return (size_t)(m + n) * 16 + kBoundWords * 4; }
+size_t row_work_bytes(int64_t m, int64_t n) { return row_work_zero_bytes(m, n) + (size_t)(m + n) * 4; }
+RowWork row_work_carve(void* base, int64_t m, int64_t n) {
+  RowWork w;
+  w.maxbits = static_cast<unsigned long long*>(base);
+  w.sums = w.maxbits + (m + n);
+  w.out = reinterpret_cast<unsigned*>(w.sums + (m + n));
+  w.exps = reinterpret_cast<int*>(w.out + kBoundWords);
+  return w;
+}
+void bound_work_carve(void* base, const RowWork& rw, int64_t m, int64_t n, int64_t k, BoundWork* w) {
   char* p = static_cast<char*>(base);
   w->kp = round_up(k, 8);
   w->mag_a = reinterpret_cast<uint16_t*>(p);
   p += round_up(m * w->kp * 2, 256);
   w->mag_b = reinterpret_cast<uint16_t*>(p);
-  p += round_up(n * w->kp * 2, 256);
-  w->sum_a = reinterpret_cast<unsigned long long*>(p);
-  w->sum_b = w->sum_a + m;
-  w->out = reinterpret_cast<unsigned*>(w->sum_b + n);
+  w->sum_a = rw.sums;
+  w->sum_b = rw.sums + m;
+  w->out = rw.out;
 }
 
-// Magnitude plane and row sums of an R x K view (element (r, p) at
-// x[r*sr + p*sp]) under the row exponents, in the run layout of planes.cuh:
-// a thread converts runs of 8 elements of one row (one 16-byte store of bf16
-// each) and adds their fixed-point terms in a register; the lanes of one
-// row (4, or 2^lg) add their terms by shuffles and one of them posts a 64-bit
-// atomicAdd. The sums are exact integers, so they do not depend on the order
-// of the atomics. With `indicator` the kernel writes the 0/1 plane of nonzero
-// elements and no sums.
-template <bool R_CONTIG>
-__global__ void __launch_bounds__(planes::THREADS)
-    magnitude_kernel(const double* __restrict__ x, int64_t sr, int64_t sp, int64_t R, int64_t K, bool vec, int lg,
-                     const int* __restrict__ exps, uint16_t* __restrict__ plane, int64_t ldp,
-                     unsigned long long* __restrict__ sums, bool indicator) {
-  constexpr int RUN = 8;
-  const planes::Chunk<R_CONTIG> c(lg);
-  // the row loop's trip count is the same for every thread of the block
-  // (rows past R only skip their work), so every lane reaches the shuffles
-  for (int64_t rb = (int64_t)blockIdx.y * c.rows; rb < R; rb += (int64_t)gridDim.y * c.rows) {
-    const int64_t r = rb + c.rl;
-    unsigned long long t = 0;
-    if (r < R) {
-      const int e = exps[r];
-      const double* xr = x + r * sr;
-      uint16_t* outr = plane + r * ldp;
+// Magnitude planes and row sums of the sides under their row exponents, in the
+// run layout of planes.cuh: a thread converts runs of 8 elements of one row
+// (one 16-byte store of bf16 each) and adds their fixed-point terms in a
+// register; the lanes of one row (4, or 2^lg) add their terms by shuffles and
+// one of them posts a 64-bit atomicAdd. The sums are exact integers, so they
+// do not depend on the order of the atomics. With `indicator` the pass writes
+// the 0/1 planes of nonzero elements and no sums.
+struct MagnitudeBody {
+  using Tin = double;
+  static constexpr int RUN = 8, kContigLg = planes::kRowsContigLg;
+  template <bool R_CONTIG>
+  static int rows(int lg) { return planes::run_rows(lg); }
+  template <bool R_CONTIG>
+  static int64_t cols(int lg, int iters) { return ((int64_t)RUN << lg) * iters; }
+  RowExp re[2];
+  uint16_t* plane[2];
+  unsigned long long* sums[2];
+  int64_t ldp;
+  int indicator;
+
+  template <bool R_CONTIG>
+  __device__ __forceinline__ void run(const planes::View<double>& v, int z) const {
+    const planes::Chunk<R_CONTIG> c(v.lg);
+    // the row loop's trip count is the same for every thread of the block
+    // (rows past R only skip their work), so every lane reaches the shuffles
+    for (int64_t rb = (int64_t)blockIdx.y * c.rows; rb < v.R; rb += (int64_t)gridDim.y * c.rows) {
+      const int64_t r = rb + c.rl;
+      unsigned long long t = 0;
+      if (r < v.R) {
+        const int e = re[z].row(r);
+        if (blockIdx.x == 0 && c.ru == 0) re[z].first(r, e);
+        const double* xr = v.x + r * v.sr;
+        uint16_t* outr = plane[z] + r * ldp;
 #pragma unroll 1
-      for (int it = 0; it < planes::PITER; ++it) {
-        const int64_t p = planes::run_col(blockIdx.x, c, it, RUN);
-        if (p >= K) break;
-        double v[RUN];
-        planes::load_run<R_CONTIG, RUN>(xr, sp, p, K, vec, v);
-        uint32_t w[RUN / 2];
+        for (int it = 0; it < v.iters; ++it) {
+          const int64_t p = planes::run_col(blockIdx.x, c, it, RUN, v.iters);
+          if (p >= v.K) break;
+          double x[RUN];
+          planes::load_run<R_CONTIG, RUN>(xr, v.sp, p, v.K, v.vec, x);
+          uint32_t w[RUN / 2];
 #pragma unroll
-        for (int q = 0; q < RUN / 2; ++q) {
-          uint16_t b0, b1;
-          unsigned long long f0, f1;
-          magnitude(v[2 * q], e, indicator, &b0, &f0);
-          magnitude(v[2 * q + 1], e, indicator, &b1, &f1);
-          w[q] = (uint32_t)b0 | ((uint32_t)b1 << 16);
-          t += f0 + f1;
+          for (int q = 0; q < RUN / 2; ++q) {
+            uint16_t b0, b1;
+            unsigned long long f0, f1;
+            magnitude(x[2 * q], e, indicator != 0, &b0, &f0);
+            magnitude(x[2 * q + 1], e, indicator != 0, &b1, &f1);
+            w[q] = (uint32_t)b0 | ((uint32_t)b1 << 16);
+            t += f0 + f1;
+          }
+          *reinterpret_cast<uint4*>(outr + p) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        *reinterpret_cast<uint4*>(outr + p) = make_uint4(w[0], w[1], w[2], w[3]);
       }
+      if (indicator) continue;
+      // a row's lanes differ in the top lg lane bits (rows contiguous) or in the low lg bits
+      if (R_CONTIG) {
+        for (int o = 16; o >= (32 >> v.lg); o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      } else {
+        for (int o = c.runs >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      }
+      if (c.ru == 0 && r < v.R && t) atomicAdd(&sums[z][r], t);
     }
-    if (indicator) continue;
-    // a row's lanes differ in the top lg lane bits (rows contiguous) or in the low lg bits
-    if (R_CONTIG) {
-      for (int o = 16; o >= (32 >> lg); o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    } else {
-      for (int o = c.runs >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    if (c.ru == 0 && r < R && t) atomicAdd(&sums[r], t);
   }
-}
+};
 
-int enqueue_magnitudes(const double* x, int64_t sr, int64_t sp, int64_t R, int64_t K, const int* exps,
-                       uint16_t* plane, int64_t kp, unsigned long long* sums, cudaStream_t s, bool indicator = false) {
-  if (R == 0) return MOMMS_OK;
-  const bool r_contig = (sr == 1 && sp != 1);
-  const bool vec = planes::rows_vector_aligned(x, sr, sp);
-  if (kp % 8 || (reinterpret_cast<uintptr_t>(plane) & 15))
-    return fail(MOMMS_ERR_INVALID_ARG, "Ozaki bound magnitudes: plane rows not 16-byte aligned");
-  const int lg = planes::run_lanes_log2(K, 8, r_contig, planes::kRowsContigLg);
+int enqueue_magnitudes(const Side* sides, int count, int64_t K, uint16_t* const* plane, int64_t kp,
+                       unsigned long long* const* sums, bool from_max, cudaStream_t s, bool indicator = false) {
+  MagnitudeBody body{};
+  body.ldp = kp;
+  body.indicator = indicator ? 1 : 0;
+  for (int i = 0; i < count; ++i) {
+    if (kp % 8 || (reinterpret_cast<uintptr_t>(plane[i]) & 15))
+      return fail(MOMMS_ERR_INVALID_ARG, "Ozaki bound magnitudes: plane rows not 16-byte aligned");
+    body.re[i] = row_exp(sides[i], from_max);
+    body.plane[i] = plane[i];
+    body.sums[i] = sums ? sums[i] : nullptr;
+  }
   {
     KernelTimer kt(MOMMS_KERNEL_PREP, s);
-    if (r_contig)
-      magnitude_kernel<true><<<planes::run_grid<true, 8>(R, K, lg), planes::THREADS, 0, s>>>(
-          x, sr, sp, R, K, vec, lg, exps, plane, kp, sums, indicator);
-    else
-      magnitude_kernel<false><<<planes::run_grid<false, 8>(R, K, lg), planes::THREADS, 0, s>>>(
-          x, sr, sp, R, K, vec, lg, exps, plane, kp, sums, indicator);
+    planes::launch_views(views_of(sides, count, K), count, body, s);
   }
   note_launch();
   const cudaError_t e = launch_status();
@@ -1129,15 +1227,7 @@ int enqueue_bound_kernel(const BoundWork& w, int64_t m, int64_t n, int64_t k, bo
 // term below FP32's range (relative to 2^(e_i+f_j)): no slice count can vouch
 // for it. Entries with no nonzero term are exact (their digits are all zero).
 // Synchronises `s`.
-struct OperandViews {
-  const double* a;
-  int64_t a_rs, a_cs;
-  const double* b;
-  int64_t b_rs, b_cs;
-  const int* rexp;
-  const int* cexp;
-};
-int bound_result(const BoundWork& w, const OperandViews& v, int64_t m, int64_t n, int64_t k, DeviceState* ds,
+int bound_result(const BoundWork& w, const Side (&sides)[2], int64_t m, int64_t n, int64_t k, DeviceState* ds,
                  cudaStream_t s, float* q1, float* q2, bool* uncovered) {
   unsigned words[4] = {0, 0, 0, 0};
   cudaError_t ce = cudaMemcpyAsync(words, w.out, sizeof(words), cudaMemcpyDeviceToHost, s);
@@ -1153,8 +1243,8 @@ int bound_result(const BoundWork& w, const OperandViews& v, int64_t m, int64_t n
   // indicator pass (sparse operands, or terms beyond FP32's range)
   ce = cudaMemsetAsync(w.out + 2, 0, 8, s);
   if (ce != cudaSuccess) return cuda_fail(ce, "Ozaki bound");
-  int rc = enqueue_magnitudes(v.a, v.a_rs, v.a_cs, m, k, v.rexp, w.mag_a, w.kp, nullptr, s, true);
-  if (!rc) rc = enqueue_magnitudes(v.b, v.b_cs, v.b_rs, n, k, v.cexp, w.mag_b, w.kp, nullptr, s, true);
+  uint16_t* const mag[2] = {w.mag_a, w.mag_b};
+  int rc = enqueue_magnitudes(sides, 2, k, mag, w.kp, nullptr, false, s, true);
   if (!rc) rc = enqueue_bound_kernel(w, m, n, k, true, ds->status, ds->sm_count, s);
   if (rc) return rc;
   unsigned long long nonzero = 0;
@@ -1289,21 +1379,33 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   if (!rc && defer_c) rc = copy_columns(g, 2, cut[nch - 1], cut[nch], &ev_c[nch - 1]);
   if (rc) return rc;
 
-  // exponents of the unpacked operands: [m + n] u64 maxima, [m + n] int exponents
+  // row maxima, bound sums and exponents of the unpacked operands
   void* ebuf = nullptr;
-  if ((ce = scratch_alloc(&ebuf, (size_t)(m + n) * (sizeof(unsigned long long) + sizeof(int)), s)) != cudaSuccess)
-    return cuda_fail(ce, "Ozaki exponents");
+  if ((ce = scratch_alloc(&ebuf, row_work_bytes(m, n), s)) != cudaSuccess) return cuda_fail(ce, "Ozaki exponents");
   ScratchGuard free_ebuf(ebuf, s);
-  unsigned long long* maxbits = static_cast<unsigned long long*>(ebuf);
-  int* exps = reinterpret_cast<int*>(maxbits + (m + n));
+  const RowWork rw = row_work_carve(ebuf, m, n);
+  if ((ce = cudaMemsetAsync(ebuf, 0, row_work_zero_bytes(m, n), s)) != cudaSuccess) return cuda_fail(ce, "Ozaki exponents");
   const double* A = static_cast<const double*>(g.a.ptr);
   const double* B = static_cast<const double*>(g.b.ptr);
+  const Side sides[2] = {side_a(g, rw.maxbits, rw.exps), side_b(g, rw.maxbits + m, rw.exps + m)};
   if ((ce = wait_operand(g, 0, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
-  if (!PA) rc = ozaki_operand_exponents(A, g.a.rs, g.a.cs, m, k, maxbits, exps, s);
-  if (rc) return rc;
-  const int* rexp = PA ? PA->exps : exps;
-  int* cexp_w = exps + m;  // B's column exponents, written per chunk
+  int* cexp_w = rw.exps + m;  // B's column exponents
+  const int* rexp = PA ? PA->exps : rw.exps;
   const int* cexp = PB ? PB->exps : cexp_w;
+  // B's maxima with A's where B is on the device (or will be once its copy,
+  // waited for here, is in); a deferred B's per column chunk. A deferred call's
+  // exponents of A are written now: the sample reads them.
+  const bool whole_b = !PB && !defer_b;
+  if (defer_b) {
+    if (!PA) rc = ozaki_operand_exponents(A, g.a.rs, g.a.cs, m, k, rw.maxbits, rw.exps, s);
+  } else {
+    if (whole_b && (ce = wait_operand(g, 1, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
+    const int first = PA ? 1 : 0, count = (PA ? 0 : 1) + (whole_b ? 1 : 0);
+    if (count) rc = enqueue_absmax(sides + first, count, k, s);
+  }
+  if (rc) return rc;
+  // whether a side's exponents are still to be derived from its maxima
+  bool from_max = !defer_b;
 
   int ns = ns_fixed ? ns_fixed : slices;
   // Automatic count, guaranteed for every entry by the bound kernel (the
@@ -1317,44 +1419,35 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   //    bound's count while C still holds its input.
   const bool automatic = ns <= 0;
   const bool verify = automatic && defer_b;
-  bool b_exps_ready = false;
   int verdict = MOMMS_OK;
   BoundWork bw{};
   void* bw_mem = nullptr;
   if (automatic) {
     if ((ce = scratch_alloc(&bw_mem, bound_work_bytes(m, n, k), s)) != cudaSuccess)
       return cuda_fail(ce, "Ozaki bound scratch");
-    bound_work_carve(bw_mem, m, n, k, &bw);
-    // sums and result words start at zero (they are contiguous); A's
-    // magnitudes on s after A's exponents
-    ce = cudaMemsetAsync(bw.sum_a, 0, (size_t)(m + n) * sizeof(unsigned long long) + 4 * sizeof(unsigned), s);
-    rc = ce == cudaSuccess ? enqueue_magnitudes(A, g.a.rs, g.a.cs, m, k, rexp, bw.mag_a, bw.kp, bw.sum_a, s)
-                           : cuda_fail(ce, "Ozaki bound scratch");
-    if (rc) {
-      cudaFreeAsync(bw_mem, s);
-      return rc;
-    }
+    bound_work_carve(bw_mem, rw, m, n, k, &bw);
   }
+  uint16_t* const mags[2] = {bw.mag_a, bw.mag_b};
+  unsigned long long* const sums[2] = {bw.sum_a, bw.sum_b};
   ScratchGuard free_bw(bw_mem, s);
   if (automatic && !verify) {
-    // all of B's exponents and magnitudes, the bound, the count
-    if ((ce = wait_operand(g, 1, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
-    rc = ozaki_operand_exponents(B, g.b.cs, g.b.rs, n, k, maxbits + m, cexp_w, s);
-    if (!rc) rc = enqueue_magnitudes(B, g.b.cs, g.b.rs, n, k, cexp_w, bw.mag_b, bw.kp, bw.sum_b, s);
+    // the magnitudes (writing the exponents), the bound, the count
+    rc = enqueue_magnitudes(sides, 2, k, mags, bw.kp, sums, from_max, s);
+    from_max = false;
     if (!rc) rc = enqueue_bound_kernel(bw, m, n, k, false, ds->status, ds->sm_count, s);
     float q1f = 0.0f, q2f = 0.0f;
     bool uncovered = false;
     if (!rc)
-      rc = bound_result(bw, OperandViews{A, g.a.rs, g.a.cs, B, g.b.rs, g.b.cs, rexp, cexp_w}, m, n, k, ds, s, &q1f,
-                        &q2f, &uncovered);
+      rc = bound_result(bw, sides, m, n, k, ds, s, &q1f, &q2f, &uncovered);
     if (rc) return rc;
     bool reachable = false;
     ns = guaranteed_slices(target, q1f, q2f, uncovered, &reachable);
     call_info().bound_rel_err = uncovered ? HUGE_VAL : guaranteed_bound(ns, q1f, q2f);
     if (!reachable) verdict = MOMMS_ERR_TARGET_UNREACHABLE;
-    b_exps_ready = true;
   } else if (automatic) {
-    // B at the sampled columns, and their exponents
+    // A's magnitudes; B at the sampled columns, and their exponents
+    rc = enqueue_magnitudes(sides, 1, k, mags, bw.kp, sums, false, s);
+    if (rc) return rc;
     if ((ce = cudaStreamWaitEvent(s, ev_sample, 0)) != cudaSuccess) return cuda_fail(ce, "operand staging");
     {
       KernelTimer kt(MOMMS_KERNEL_PREP, s);
@@ -1429,14 +1522,19 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     const int l0 = pass * per, l1 = std::min(N, l0 + per);
     const bool last = pass + 1 == passes;
     // A's planes of this pass (on s, after every slice launch of the pass
-    // before), and a packed B's
+    // before), with B's where it is one chunk and on the device, and a packed
+    // operand's residues
+    const bool together = whole_b && nch == 1;
+    __half* const outs[2] = {const_cast<__half*>(pa), const_cast<__half*>(pb)};
+    const int64_t pes[2] = {(int64_t)a_plane, (int64_t)b_plane};
+    const int first = PA ? 1 : 0, count = (PA ? 0 : 1) + (together ? 1 : 0);
     if (crt) {
-      if (PA) crt_planes_of_pack(*PA, m, const_cast<__half*>(pa), l0, l1, ds->sm_count, s);
-      else crt_planes(ns, A, g.a.rs, g.a.cs, m, k, const_cast<__half*>(pa), kp, (int64_t)a_plane, rexp, l0, l1, s);
-      if (PB) crt_planes_of_pack(*PB, n, const_cast<__half*>(pb), l0, l1, ds->sm_count, s);
+      if (PA) crt_planes_of_pack(*PA, m, outs[0], l0, l1, ds->sm_count, s);
+      if (PB) crt_planes_of_pack(*PB, n, outs[1], l0, l1, ds->sm_count, s);
+      if (count) crt_planes(ns, sides + first, count, k, outs + first, kp, pes + first, from_max, l0, l1, s);
       crt_slice_params(m, k, l0, l1, &p);
-    } else if (!PA) {
-      ozaki_operand_planes(ns, A, g.a.rs, g.a.cs, m, k, const_cast<__half*>(pa), kp, rexp, s);
+    } else if (count) {
+      ozaki_planes(ns, sides + first, count, k, outs + first, kp, pes + first, from_max, s);
     }
     p.plane = (int64_t)plane;
     p.status = ds->status;
@@ -1456,35 +1554,30 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
       const int64_t j0 = cut[c], j1 = cut[c + 1], w = j1 - j0;
       if (w <= 0) continue;
       cudaStream_t X = (c & 1) ? ds->aux : s;
-      // B's columns j0..j1: exponents and planes
-      const double* Bc = B + j0 * g.b.cs;
-      if (pass == 0) {
-        ce = defer_b ? cudaStreamWaitEvent(X, ev_b[c], 0) : wait_operand(g, 1, X);
-        if (ce != cudaSuccess) {
-          rc = cuda_fail(ce, "operand staging");
-          break;
-        }
-        if (!PB && !b_exps_ready)
-          rc = ozaki_operand_exponents(Bc, g.b.cs, g.b.rs, w, k, maxbits + m + j0, cexp_w + j0, X);
-        if (rc) break;
+      // B's columns j0..j1, where they were not prepared with A: exponents
+      // (a deferred B's) and planes
+      if (pass == 0 && defer_b && (ce = cudaStreamWaitEvent(X, ev_b[c], 0)) != cudaSuccess) {
+        rc = cuda_fail(ce, "operand staging");
+        break;
       }
-      if (!PB && crt) {
-        crt_planes(ns, Bc, g.b.cs, g.b.rs, w, k, const_cast<__half*>(pb) + j0 * kp, kp, (int64_t)b_plane, cexp_w + j0,
-                   l0, l1, X);
-      } else if (!PB) {
-        KernelTimer kt(MOMMS_KERNEL_PREP, X);
-        ozaki_planes(ns, Bc, g.b.cs, g.b.rs, w, k, const_cast<__half*>(pb) + j0 * kp, kp, (int64_t)b_plane,
-                     cexp_w + j0, X);
-        note_launch();
-      }
-      if (verify && pass == 0) {
-        // B's magnitudes for the bound (verify implies B is not packed)
-        rc = enqueue_magnitudes(Bc, g.b.cs, g.b.rs, w, k, cexp_w + j0, bw.mag_b + j0 * bw.kp, bw.kp, bw.sum_b + j0, X);
+      if (!PB && !together) {
+        const Side bs{B + j0 * g.b.cs, g.b.cs, g.b.rs, w, rw.maxbits + m + j0, cexp_w + j0};
+        if (pass == 0 && defer_b) rc = ozaki_operand_exponents(bs.x, bs.sr, bs.sp, w, k, bs.maxbits, bs.exps, X);
         if (rc) break;
-        if ((ce = cudaEventRecord(ev.mag[c], X)) != cudaSuccess ||
-            (ce = cudaStreamWaitEvent(V, ev.mag[c], 0)) != cudaSuccess) {
-          rc = cuda_fail(ce, "Ozaki bound events");
-          break;
+        __half* const out = const_cast<__half*>(pb) + j0 * kp;
+        if (crt) crt_planes(ns, &bs, 1, k, &out, kp, &pes[1], from_max, l0, l1, X);
+        else ozaki_planes(ns, &bs, 1, k, &out, kp, &pes[1], from_max, X);
+        if (verify && pass == 0) {
+          // B's magnitudes for the bound (verify implies B is not packed)
+          uint16_t* const mag = bw.mag_b + j0 * bw.kp;
+          unsigned long long* const sum = bw.sum_b + j0;
+          rc = enqueue_magnitudes(&bs, 1, k, &mag, bw.kp, &sum, false, X);
+          if (rc) break;
+          if ((ce = cudaEventRecord(ev.mag[c], X)) != cudaSuccess ||
+              (ce = cudaStreamWaitEvent(V, ev.mag[c], 0)) != cudaSuccess) {
+            rc = cuda_fail(ce, "Ozaki bound events");
+            break;
+          }
         }
       }
       CUtensorMap tmB, tmB_half;  // half: one CTA's share of the B tile for the pair kernel
@@ -1515,6 +1608,7 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
         rc = combine_chunk(c, X);
       }
     }
+    from_max = false;
     if (!last && nch > 1 && !rc) {
       // the next pass reuses A's planes: s waits for the second stream's products
       ce = cudaEventRecord(ev.join, ds->aux);
@@ -1532,8 +1626,7 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   if (verify && !rc) {
     rc = enqueue_bound_kernel(bw, m, n, k, false, ds->status, ds->sm_count, V);
     if (!rc)
-      rc = bound_result(bw, OperandViews{A, g.a.rs, g.a.cs, B, g.b.rs, g.b.cs, rexp, cexp_w}, m, n, k, ds, V, &q1f,
-                        &q2f, &uncovered);
+      rc = bound_result(bw, sides, m, n, k, ds, V, &q1f, &q2f, &uncovered);
     if (!rc) {
       bool reachable = false;
       const int need = guaranteed_slices(target, q1f, q2f, uncovered, &reachable);
@@ -1609,7 +1702,7 @@ int ozaki_choose_slices(const momms_gemm_desc& d, int* slices, cudaStream_t s) {
   const int64_t nslab = ceil_div(d.k, kMaxK), kb = round_up(ceil_div(d.k, nslab), 64);
   const int64_t kmax = std::min(d.k, kb);
   void* ebuf = nullptr;
-  cudaError_t ce = scratch_alloc(&ebuf, (size_t)(m + n) * (sizeof(unsigned long long) + sizeof(int)), s);
+  cudaError_t ce = scratch_alloc(&ebuf, row_work_bytes(m, n), s);
   if (ce != cudaSuccess) return cuda_fail(ce, "Ozaki exponents");
   ScratchGuard free_ebuf(ebuf, s);
   void* bw_mem = nullptr;
@@ -1617,8 +1710,7 @@ int ozaki_choose_slices(const momms_gemm_desc& d, int* slices, cudaStream_t s) {
     return cuda_fail(ce, "Ozaki bound scratch");
   ScratchGuard free_bw(bw_mem, s);
   BoundWork bw{};
-  unsigned long long* maxbits = static_cast<unsigned long long*>(ebuf);
-  int* exps = reinterpret_cast<int*>(maxbits + (m + n));
+  const RowWork rw = row_work_carve(ebuf, m, n);
   int need = 1, rc = MOMMS_OK;
   bool reachable_all = true;
   for (int64_t p0 = 0; p0 < d.k && !rc; p0 += kb) {
@@ -1628,22 +1720,18 @@ int ozaki_choose_slices(const momms_gemm_desc& d, int* slices, cudaStream_t s) {
     g.k = std::min(kb, d.k - p0);
     g.a = DevMat{static_cast<double*>(d.a.ptr) + p0 * d.a.cs, d.a.rs, d.a.cs};
     g.b = DevMat{static_cast<double*>(d.b.ptr) + p0 * d.b.rs, d.b.rs, d.b.cs};
-    bound_work_carve(bw_mem, m, n, g.k, &bw);
-    rc = compute_exponents(g, maxbits, exps, s);
-    if (!rc) {
-      ce = cudaMemsetAsync(bw.sum_a, 0, (size_t)(m + n) * sizeof(unsigned long long) + 4 * sizeof(unsigned), s);
-      if (ce != cudaSuccess) rc = cuda_fail(ce, "Ozaki bound scratch");
-    }
-    const double* Ap = static_cast<const double*>(g.a.ptr);
-    const double* Bp = static_cast<const double*>(g.b.ptr);
-    if (!rc) rc = enqueue_magnitudes(Ap, g.a.rs, g.a.cs, m, g.k, exps, bw.mag_a, bw.kp, bw.sum_a, s);
-    if (!rc) rc = enqueue_magnitudes(Bp, g.b.cs, g.b.rs, n, g.k, exps + m, bw.mag_b, bw.kp, bw.sum_b, s);
+    bound_work_carve(bw_mem, rw, m, n, g.k, &bw);
+    const Side sides[2] = {side_a(g, rw.maxbits, rw.exps), side_b(g, rw.maxbits + m, rw.exps + m)};
+    uint16_t* const mags[2] = {bw.mag_a, bw.mag_b};
+    unsigned long long* const sums[2] = {bw.sum_a, bw.sum_b};
+    ce = cudaMemsetAsync(ebuf, 0, row_work_zero_bytes(m, n), s);
+    if (ce != cudaSuccess) rc = cuda_fail(ce, "Ozaki bound scratch");
+    if (!rc) rc = enqueue_absmax(sides, 2, g.k, s);
+    if (!rc) rc = enqueue_magnitudes(sides, 2, g.k, mags, bw.kp, sums, true, s);
     if (!rc) rc = enqueue_bound_kernel(bw, m, n, g.k, false, ds->status, ds->sm_count, s);
     float q1 = 0.0f, q2 = 0.0f;
     bool uncovered = false;
-    if (!rc)
-      rc = bound_result(bw, OperandViews{Ap, g.a.rs, g.a.cs, Bp, g.b.rs, g.b.cs, exps, exps + m}, m, n, g.k, ds, s,
-                        &q1, &q2, &uncovered);
+    if (!rc) rc = bound_result(bw, sides, m, n, g.k, ds, s, &q1, &q2, &uncovered);
     if (!rc) {
       bool reachable = false;
       need = std::max(need, guaranteed_slices(d.target_rel_err, q1, q2, uncovered, &reachable));
@@ -1820,19 +1908,14 @@ int ozaki_batch_launch(OzakiBatch* b, cudaStream_t s, int max_sms) {
   // each problem's exponents and digit planes
   for (auto& P : b->probs) {
     const DevGemm& g = P.g;
-    const double* A = static_cast<const double*>(g.a.ptr);
-    const double* B = static_cast<const double*>(g.b.ptr);
-    int rc = ozaki_operand_exponents(A, g.a.rs, g.a.cs, g.m, g.k, P.maxbits, P.exps, s);
-    if (!rc) rc = ozaki_operand_exponents(B, g.b.cs, g.b.rs, g.n, g.k, P.maxbits + g.m, P.exps + g.m, s);
+    const Side sides[2] = {side_a(g, P.maxbits, P.exps), side_b(g, P.maxbits + g.m, P.exps + g.m)};
+    const cudaError_t ce = cudaMemsetAsync(P.maxbits, 0, (size_t)(g.m + g.n) * sizeof(unsigned long long), s);
+    int rc = ce == cudaSuccess ? enqueue_absmax(sides, 2, g.k, s) : cuda_fail(ce, "Ozaki exponents");
     if (rc) return rc;
-    __half* pb = P.planes + P.planes_each * P.a_plane;
-    if (P.crt) {
-      crt_planes(P.ns, A, g.a.rs, g.a.cs, g.m, g.k, P.planes, P.kp, (int64_t)P.a_plane, P.exps, 0, P.planes_each, s);
-      crt_planes(P.ns, B, g.b.cs, g.b.rs, g.n, g.k, pb, P.kp, (int64_t)P.b_plane, P.exps + g.m, 0, P.planes_each, s);
-    } else {
-      ozaki_operand_planes(P.ns, A, g.a.rs, g.a.cs, g.m, g.k, P.planes, P.kp, P.exps, s);
-      ozaki_operand_planes(P.ns, B, g.b.cs, g.b.rs, g.n, g.k, pb, P.kp, P.exps + g.m, s);
-    }
+    __half* const outs[2] = {P.planes, P.planes + P.planes_each * P.a_plane};
+    const int64_t pes[2] = {(int64_t)P.a_plane, (int64_t)P.b_plane};
+    if (P.crt) crt_planes(P.ns, sides, 2, g.k, outs, P.kp, pes, true, 0, P.planes_each, s);
+    else ozaki_planes(P.ns, sides, 2, g.k, outs, P.kp, pes, true, s);
   }
   // one persistent slice launch over every problem's tiles
   int clusters = 0;

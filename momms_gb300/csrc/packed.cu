@@ -158,7 +158,8 @@ int momms_pack(int dtype, int precision, int role, int64_t rows, int64_t cols, c
     if (ce == cudaSuccess) {
       p->planes = p->mem;
       const int64_t sr = role == MOMMS_ROLE_A ? v.rs : v.cs, sp = role == MOMMS_ROLE_A ? v.cs : v.rs;
-      tf32_operand_planes(static_cast<const float*>(v.ptr), sr, sp, R, K, static_cast<float*>(p->planes), p->kp, s);
+      const F32View fv{static_cast<const float*>(v.ptr), sr, sp, R, static_cast<float*>(p->planes)};
+      tf32_operand_planes(&fv, 1, K, p->kp, s);
     }
   }
   if (ce == cudaSuccess) ce = launch_status();

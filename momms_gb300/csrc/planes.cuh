@@ -37,7 +37,7 @@ namespace momms {
 void refuse_launch(cudaError_t e);
 namespace planes {
 
-constexpr int THREADS = 256, PITER = 4;
+constexpr int THREADS = 256, PITER = 4;  // PITER: runs per thread, at most (launch_views)
 
 // A thread's place in a block's chunk of the view: row rl of the chunk's
 // rows, run ru of the runs taken across the chunk per iteration. A warp
@@ -62,9 +62,10 @@ __host__ __device__ __forceinline__ RunPlace run_place(int tid, int lg) {
   return c;
 }
 // First column of the thread's run `it` in block column bx (runs of `run`
-// elements; a block covers runs * run * PITER columns).
-__host__ __device__ __forceinline__ int64_t run_col(int64_t bx, const RunPlace& c, int it, int run) {
-  return (bx * c.runs * PITER + c.ru + (int64_t)c.runs * it) * run;
+// elements; a block covers runs * run * iters columns).
+__host__ __device__ __forceinline__ int64_t run_col(int64_t bx, const RunPlace& c, int it, int run,
+                                                    int iters = PITER) {
+  return (bx * c.runs * iters + c.ru + (int64_t)c.runs * it) * run;
 }
 template <bool R_CONTIG>
 struct Chunk : RunPlace {
@@ -112,45 +113,85 @@ __device__ __forceinline__ void load_run(const Tin* __restrict__ xr, int64_t sp,
   }
 }
 
+// One or two operands of a product in one launch (blockIdx.z): the passes over
+// A and B are independent, and at 512^2 a launch of its own costs each as much
+// as its work.
+template <typename Tin>
+struct View {
+  const Tin* x;
+  int64_t sr, sp, R, K;
+  int r_contig, vec, lg, iters;
+  unsigned bx;  // blocks in x
+};
+template <typename Tin>
+struct Views {
+  View<Tin> v[2];
+};
+// Body: Tin, RUN, kContigLg, rows<R_CONTIG>(lg) and cols<R_CONTIG>(lg, iters)
+// of a block, and run<R_CONTIG>(view, index of the view).
+template <typename Body>
+__global__ void __launch_bounds__(THREADS) views_kernel(const __grid_constant__ Views<typename Body::Tin> vs,
+                                                        const __grid_constant__ Body body) {
+  const View<typename Body::Tin>& v = vs.v[blockIdx.z];
+  if (blockIdx.x >= v.bx) return;
+  if (v.r_contig) body.template run<true>(v, blockIdx.z);
+  else body.template run<false>(v, blockIdx.z);
+}
+__host__ __device__ constexpr int run_rows(int lg) { return (THREADS / 32) << (5 - lg); }
+
 // Op: PLANES, Tout, Word (one pair's value in one plane: two Tout), Ctx
-// row(r) (per-row state) and pack(v0, v1, ctx, Word (&w)[PLANES]).
-template <bool R_CONTIG, typename Tin, typename Op>
-__global__ void __launch_bounds__(THREADS)
-    to_planes_kernel(const Tin* __restrict__ x, int64_t sr, int64_t sp, int64_t R, int64_t K, bool vec, int lg,
-                     typename Op::Tout* __restrict__ planes, int64_t ldp, int64_t plane_elems, Op op) {
+// row(r) (per-row state), first(r, ctx) (called by one thread per row) and
+// pack(v0, v1, ctx, Word (&w)[PLANES]).
+template <typename In, typename Op>
+struct PlanesBody {
+  using Tin = In;
   using Tout = typename Op::Tout;
-  using Word = typename Op::Word;
-  constexpr int RUN = 16 / sizeof(Tout), NP = Op::PLANES;
-  static_assert(sizeof(Word) == 2 * sizeof(Tout), "a word is one pair's value");
-  const Chunk<R_CONTIG> c(lg);
-  // row chunks beyond the grid's y limit are taken in further passes
-  for (int64_t r = (int64_t)blockIdx.y * c.rows + c.rl; r < R; r += (int64_t)gridDim.y * c.rows) {
-    const auto ctx = op.row(r);
-    const Tin* xr = x + r * sr;
-    Tout* outr = planes + r * ldp;
+  static constexpr int RUN = 16 / sizeof(Tout), kContigLg = kRowsContigLgPlanes;
+  template <bool R_CONTIG>
+  static int rows(int lg) { return run_rows(lg); }
+  template <bool R_CONTIG>
+  static int64_t cols(int lg, int iters) { return ((int64_t)RUN << lg) * iters; }
+  Tout* planes[2];
+  int64_t ldp, plane_elems[2];
+  Op op[2];
+
+  template <bool R_CONTIG>
+  __device__ __forceinline__ void run(const View<Tin>& v, int z) const {
+    using Word = typename Op::Word;
+    constexpr int NP = Op::PLANES;
+    static_assert(sizeof(Word) == 2 * sizeof(Tout), "a word is one pair's value");
+    const Chunk<R_CONTIG> c(v.lg);
+    const int64_t pe = plane_elems[z];
+    // row chunks beyond the grid's y limit are taken in further passes
+    for (int64_t r = (int64_t)blockIdx.y * c.rows + c.rl; r < v.R; r += (int64_t)gridDim.y * c.rows) {
+      const auto ctx = op[z].row(r);
+      if (blockIdx.x == 0 && c.ru == 0) op[z].first(r, ctx);
+      const Tin* xr = v.x + r * v.sr;
+      Tout* outr = planes[z] + r * ldp;
 #pragma unroll 1
-    for (int it = 0; it < PITER; ++it) {
-      const int64_t p = run_col(blockIdx.x, c, it, RUN);
-      if (p >= K) break;
-      Tin v[RUN];
-      load_run<R_CONTIG, RUN>(xr, sp, p, K, vec, v);
-      Word w[NP][RUN / 2];
+      for (int it = 0; it < v.iters; ++it) {
+        const int64_t p = run_col(blockIdx.x, c, it, RUN, v.iters);
+        if (p >= v.K) break;
+        Tin x[RUN];
+        load_run<R_CONTIG, RUN>(xr, v.sp, p, v.K, v.vec, x);
+        Word w[NP][RUN / 2];
 #pragma unroll
-      for (int q = 0; q < RUN / 2; ++q) {
-        Word wq[NP];
-        op.pack(v[2 * q], v[2 * q + 1], ctx, wq);
+        for (int q = 0; q < RUN / 2; ++q) {
+          Word wq[NP];
+          op[z].pack(x[2 * q], x[2 * q + 1], ctx, wq);
 #pragma unroll
-        for (int t = 0; t < NP; ++t) w[t][q] = wq[t];
-      }
+          for (int t = 0; t < NP; ++t) w[t][q] = wq[t];
+        }
 #pragma unroll
-      for (int t = 0; t < NP; ++t) {
-        uint4 u;
-        memcpy(&u, w[t], sizeof(u));
-        *reinterpret_cast<uint4*>(outr + t * plane_elems + p) = u;
+        for (int t = 0; t < NP; ++t) {
+          uint4 u;
+          memcpy(&u, w[t], sizeof(u));
+          *reinterpret_cast<uint4*>(outr + t * pe + p) = u;
+        }
       }
     }
   }
-}
+};
 
 // Grid of a run kernel over an R x K view, lg from run_lanes_log2: a block
 // holds 256 >> lg rows of 2^lg runs in either layout (the layouts differ in
@@ -158,9 +199,9 @@ __global__ void __launch_bounds__(THREADS)
 // by the kernels' row loops.
 template <bool R_CONTIG, int RUN>
 inline dim3 run_grid(int64_t R, int64_t K, int lg) {
-  const int64_t rows = (int64_t)(THREADS / 32) << (5 - lg);
   const int64_t runs = (int64_t)1 << lg;
-  return dim3((unsigned)ceil_div_dev(K, runs * RUN * PITER), (unsigned)std::min<int64_t>(ceil_div_dev(R, rows), 65535));
+  return dim3((unsigned)ceil_div_dev(K, runs * RUN * PITER),
+              (unsigned)std::min<int64_t>(ceil_div_dev(R, run_rows(lg)), 65535));
 }
 
 // True when row r of the view starts 16-byte aligned for every r and p is
@@ -170,23 +211,50 @@ inline bool rows_vector_aligned(const Tin* x, int64_t sr, int64_t sp) {
   return sp == 1 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ((sr * (int64_t)sizeof(Tin)) & 15) == 0;
 }
 
-template <typename Tin, typename Op>
-void launch_to_planes(const Tin* x, int64_t sr, int64_t sp, int64_t R, int64_t K, typename Op::Tout* planes,
-                      int64_t ldp, int64_t plane_elems, Op op, cudaStream_t s) {
-  constexpr int RUN = 16 / sizeof(typename Op::Tout);
-  if (ldp % RUN || plane_elems % RUN || (reinterpret_cast<uintptr_t>(planes) & 15)) {
-    refuse_launch(cudaErrorMisalignedAddress);  // the vector stores need 16-byte aligned runs
-    return;
+template <typename Tin>
+inline View<Tin> make_view(const Tin* x, int64_t sr, int64_t sp, int64_t R, int64_t K) {
+  View<Tin> v{};
+  v.x = x, v.sr = sr, v.sp = sp, v.R = R, v.K = K;
+  v.r_contig = (sr == 1 && sp != 1) ? 1 : 0;
+  v.vec = rows_vector_aligned(x, sr, sp) ? 1 : 0;
+  return v;
+}
+
+// Launches a body over `count` views. A thread takes PITER runs, or one where
+// that leaves fewer than four blocks per SM.
+template <typename Body>
+void launch_views(Views<typename Body::Tin> vs, int count, const Body& body, cudaStream_t s) {
+  constexpr int64_t kFewBlocks = 4 * 152;
+  auto rows = [](bool rc, int lg) { return rc ? Body::template rows<true>(lg) : Body::template rows<false>(lg); };
+  auto cols = [](bool rc, int lg, int it) {
+    return rc ? Body::template cols<true>(lg, it) : Body::template cols<false>(lg, it);
+  };
+  int64_t blocks = 0;
+  for (int i = 0; i < count; ++i) {
+    View<typename Body::Tin>& v = vs.v[i];
+    v.lg = run_lanes_log2(v.K, Body::RUN, v.r_contig != 0, Body::kContigLg);
+    blocks += ceil_div_dev(v.K, cols(v.r_contig != 0, v.lg, PITER)) * ceil_div_dev(v.R, rows(v.r_contig != 0, v.lg));
   }
-  const bool r_contig = (sr == 1 && sp != 1);
-  const bool vec = rows_vector_aligned(x, sr, sp);
-  const int lg = run_lanes_log2(K, RUN, r_contig, kRowsContigLgPlanes);
-  if (r_contig)
-    to_planes_kernel<true, Tin, Op>
-        <<<run_grid<true, RUN>(R, K, lg), THREADS, 0, s>>>(x, sr, sp, R, K, vec, lg, planes, ldp, plane_elems, op);
-  else
-    to_planes_kernel<false, Tin, Op>
-        <<<run_grid<false, RUN>(R, K, lg), THREADS, 0, s>>>(x, sr, sp, R, K, vec, lg, planes, ldp, plane_elems, op);
+  dim3 grid(1, 1, (unsigned)count);
+  for (int i = 0; i < count; ++i) {
+    View<typename Body::Tin>& v = vs.v[i];
+    v.iters = blocks < kFewBlocks ? 1 : PITER;
+    v.bx = (unsigned)ceil_div_dev(v.K, cols(v.r_contig != 0, v.lg, v.iters));
+    grid.x = std::max(grid.x, v.bx);
+    grid.y = std::max(grid.y, (unsigned)std::min<int64_t>(ceil_div_dev(v.R, rows(v.r_contig != 0, v.lg)), 65535));
+  }
+  views_kernel<Body><<<grid, THREADS, 0, s>>>(vs, body);
+}
+
+// Both operands' planes (count 2), or one's.
+template <typename Tin, typename Op>
+void launch_to_planes(const Views<Tin>& vs, int count, const PlanesBody<Tin, Op>& body, cudaStream_t s) {
+  for (int i = 0; i < count; ++i)
+    if (body.ldp % body.RUN || body.plane_elems[i] % body.RUN || (reinterpret_cast<uintptr_t>(body.planes[i]) & 15)) {
+      refuse_launch(cudaErrorMisalignedAddress);  // the vector stores need 16-byte aligned runs
+      return;
+    }
+  launch_views(vs, count, body, s);
 }
 
 }  // namespace planes

@@ -19,6 +19,7 @@ struct Tf32SplitOp {
   using Tout = float;
   using Word = uint2;  // one pair's float2 bits
   __device__ __forceinline__ int row(int64_t) const { return 0; }
+  __device__ __forceinline__ void first(int64_t, int) const {}
   __device__ __forceinline__ static void split(float v, float* hi_out, float* lo_out) {
     uint32_t hi, lo;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(v));
@@ -43,10 +44,17 @@ int set_attrs_tf32() {
   return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "cudaFuncSetAttribute(split-TF32)");
 }
 
-void tf32_operand_planes(const float* x, int64_t sr, int64_t sp, int64_t R, int64_t K, float* planes, int64_t kp,
-                         cudaStream_t s) {
+void tf32_operand_planes(const F32View* v, int count, int64_t K, int64_t kp, cudaStream_t s) {
+  planes::Views<float> vs{};
+  planes::PlanesBody<float, Tf32SplitOp> body{};
+  body.ldp = kp;
+  for (int i = 0; i < count; ++i) {
+    vs.v[i] = planes::make_view(v[i].x, v[i].sr, v[i].sp, v[i].R, K);
+    body.planes[i] = v[i].planes;
+    body.plane_elems[i] = v[i].R * kp;
+  }
   KernelTimer kt(MOMMS_KERNEL_PREP, s);
-  planes::launch_to_planes(x, sr, sp, R, K, planes, kp, R * kp, Tf32SplitOp{}, s);
+  planes::launch_to_planes(vs, count, body, s);
   note_launch();
 }
 
@@ -66,14 +74,21 @@ int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   ScratchGuard free_buf(buf, s);
   float* pa = PA ? static_cast<float*>(PA->planes) : static_cast<float*>(buf);
   float* pb = PB ? static_cast<float*>(PB->planes) : static_cast<float*>(buf) + (PA ? 0 : 2 * a_plane);
-  // each operand's split waits only for that operand
-  if (!PA) {
-    if ((ce = wait_operand(g, 0, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
-    tf32_operand_planes(static_cast<const float*>(g.a.ptr), g.a.rs, g.a.cs, g.m, g.k, pa, kp, s);
-  }
-  if (!PB) {
-    if ((ce = wait_operand(g, 1, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
-    tf32_operand_planes(static_cast<const float*>(g.b.ptr), g.b.cs, g.b.rs, g.n, g.k, pb, kp, s);
+  const F32View va{static_cast<const float*>(g.a.ptr), g.a.rs, g.a.cs, g.m, pa};
+  const F32View vb{static_cast<const float*>(g.b.ptr), g.b.cs, g.b.rs, g.n, pb};
+  if (!PA && !PB && !g.staging) {
+    const F32View both[2] = {va, vb};
+    tf32_operand_planes(both, 2, g.k, kp, s);
+  } else {
+    // each operand's split waits only for that operand
+    if (!PA) {
+      if ((ce = wait_operand(g, 0, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
+      tf32_operand_planes(&va, 1, g.k, kp, s);
+    }
+    if (!PB) {
+      if ((ce = wait_operand(g, 1, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
+      tf32_operand_planes(&vb, 1, g.k, kp, s);
+    }
   }
 
   CUtensorMap tmA, tmB, tmB_half;
