@@ -36,17 +36,17 @@ struct ResidueBody {
   int l0, l1;
 
   template <bool R_CONTIG>
-  __device__ __forceinline__ void run(const planes::View<double>& v, int z) const {
+  __device__ __forceinline__ void run(const planes::View<double>& v, int z, const planes::BlockPlace& at) const {
     const planes::Chunk<R_CONTIG> c(v.lg);
     const int64_t pe = plane_elems[z];
-    for (int64_t r = (int64_t)blockIdx.y * c.rows + c.rl; r < v.R; r += (int64_t)gridDim.y * c.rows) {
+    for (int64_t r = (int64_t)at.y * c.rows + c.rl; r < v.R; r += (int64_t)at.ny * c.rows) {
       const int e = re[z].row(r);
-      if (blockIdx.x == 0 && c.ru == 0) re[z].first(r, e);
+      if (at.x == 0 && c.ru == 0) re[z].first(r, e);
       const double* xr = v.x + r * v.sr;
       __half* outr = out[z] + r * ldp;
 #pragma unroll 1
       for (int it = 0; it < v.iters; ++it) {
-        const int64_t p = planes::run_col(blockIdx.x, c, it, RUN, v.iters);
+        const int64_t p = planes::run_col(at.x, c, it, RUN, v.iters);
         if (p >= v.K) break;
         float f[RUN][L];
         {

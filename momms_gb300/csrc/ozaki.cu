@@ -33,6 +33,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "internal.h"
@@ -84,19 +85,24 @@ struct AbsmaxBody {
   unsigned long long* maxbits[2];
 
   template <int LOADS>
-  __device__ __forceinline__ void column_block(const planes::View<double>& v, unsigned long long* out) const {
+  __device__ __forceinline__ void column_block(const planes::View<double>& v, unsigned long long* out, const planes::BlockPlace& at) const {
     __shared__ unsigned long long red[8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t p0 = (int64_t)blockIdx.x * (8 * LOADS);
-    for (int64_t rb = (int64_t)blockIdx.y * 32; rb < v.R; rb += (int64_t)gridDim.y * 32) {
+    const int64_t p0 = (int64_t)at.x * (8 * LOADS);
+    for (int64_t rb = (int64_t)at.y * 32; rb < v.R; rb += (int64_t)at.ny * 32) {
       const int64_t r = rb + tx;
       unsigned long long mx = 0;
       if (r < v.R) {
         double x[LOADS];
+        const double* q = v.x + r + (p0 + ty) * v.sp;
+        const int64_t step = 8 * v.sp;
+        const int left = (int)min((int64_t)(8 * LOADS), v.K - p0) - ty;  // columns from this warp's first
+        if (left > 8 * (LOADS - 1)) {
 #pragma unroll
-        for (int j = 0; j < LOADS; ++j) {
-          const int64_t pp = p0 + ty + 8 * j;
-          x[j] = pp < v.K ? v.x[r + pp * v.sp] : 0.0;
+          for (int j = 0; j < LOADS; ++j) x[j] = __ldg(q + j * step);
+        } else {
+#pragma unroll
+          for (int j = 0; j < LOADS; ++j) x[j] = 8 * j < left ? __ldg(q + j * step) : 0.0;
         }
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) mx = max(mx, abs_bits(x[j]));
@@ -112,24 +118,24 @@ struct AbsmaxBody {
   }
 
   template <bool R_CONTIG>
-  __device__ __forceinline__ void run(const planes::View<double>& v, int z) const {
+  __device__ __forceinline__ void run(const planes::View<double>& v, int z, const planes::BlockPlace& at) const {
     unsigned long long* out = maxbits[z];
     if (R_CONTIG) {
-      if (v.iters == planes::PITER) column_block<8 * planes::PITER>(v, out);
-      else column_block<8>(v, out);
+      if (v.iters == planes::PITER) column_block<8 * planes::PITER>(v, out, at);
+      else column_block<8>(v, out, at);
       return;
     }
     const planes::Chunk<false> c(v.lg);
     // the row loop's trip count is the same for every thread of the block, so
     // every lane reaches the shuffles
-    for (int64_t rb = (int64_t)blockIdx.y * c.rows; rb < v.R; rb += (int64_t)gridDim.y * c.rows) {
+    for (int64_t rb = (int64_t)at.y * c.rows; rb < v.R; rb += (int64_t)at.ny * c.rows) {
       const int64_t r = rb + c.rl;
       unsigned long long mx = 0;
       if (r < v.R) {
         const double* xr = v.x + r * v.sr;
 #pragma unroll 1
         for (int it = 0; it < v.iters; ++it) {
-          const int64_t p = planes::run_col(blockIdx.x, c, it, RUN, v.iters);
+          const int64_t p = planes::run_col(at.x, c, it, RUN, v.iters);
           if (p >= v.K) break;
           double x[RUN];
           planes::load_run<false, RUN>(xr, v.sp, p, v.K, v.vec, x);
@@ -186,9 +192,8 @@ int enqueue_absmax(const Side* sides, int count, int64_t K, cudaStream_t s) {
   for (int i = 0; i < count; ++i) body.maxbits[i] = sides[i].maxbits;
   {
     KernelTimer kt(MOMMS_KERNEL_PREP, s);
-    planes::launch_views(views_of(sides, count, K), count, body, s);
+    note_launch(planes::launch_views(views_of(sides, count, K), count, body, s));
   }
-  note_launch();
   const cudaError_t e = launch_status();
   return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "Ozaki exponents");
 }
@@ -249,8 +254,8 @@ struct OzakiSliceOp {
 };
 
 template <int NS>
-void launch_ozaki_planes(const Side* sides, int count, int64_t K, __half* const* out, int64_t ldp,
-                         const int64_t* plane_elems, bool from_max, cudaStream_t s) {
+int launch_ozaki_planes(const Side* sides, int count, int64_t K, __half* const* out, int64_t ldp,
+                        const int64_t* plane_elems, bool from_max, cudaStream_t s) {
   planes::PlanesBody<double, OzakiSliceOp<NS>> body{};
   body.ldp = ldp;
   for (int i = 0; i < count; ++i) {
@@ -258,7 +263,7 @@ void launch_ozaki_planes(const Side* sides, int count, int64_t K, __half* const*
     body.plane_elems[i] = plane_elems[i];
     body.op[i] = OzakiSliceOp<NS>{row_exp(sides[i], from_max)};
   }
-  planes::launch_to_planes(views_of(sides, count, K), count, body, s);
+  return planes::launch_to_planes(views_of(sides, count, K), count, body, s);
 }
 
 // The ns digit planes of the sides (runtime slice count -> the unrolled kernel
@@ -269,14 +274,13 @@ void ozaki_planes(int ns, const Side* sides, int count, int64_t K, __half* const
   KernelTimer kt(MOMMS_KERNEL_PREP, s);
   switch (ns) {
 #define MOMMS_OZAKI_NS(N) \
-  case N: launch_ozaki_planes<N>(sides, count, K, out, ldp, plane_elems, from_max, s); break;
+  case N: note_launch(launch_ozaki_planes<N>(sides, count, K, out, ldp, plane_elems, from_max, s)); break;
     MOMMS_OZAKI_NS(1) MOMMS_OZAKI_NS(2) MOMMS_OZAKI_NS(3) MOMMS_OZAKI_NS(4) MOMMS_OZAKI_NS(5) MOMMS_OZAKI_NS(6)
     MOMMS_OZAKI_NS(7) MOMMS_OZAKI_NS(8) MOMMS_OZAKI_NS(9) MOMMS_OZAKI_NS(10) MOMMS_OZAKI_NS(11) MOMMS_OZAKI_NS(12)
     MOMMS_OZAKI_NS(13) MOMMS_OZAKI_NS(14) MOMMS_OZAKI_NS(15)
 #undef MOMMS_OZAKI_NS
     default: break;
   }
-  note_launch();
 }
 
 // Sampled quantities for the slice-count bound: for sampled (i, j),
@@ -785,10 +789,12 @@ namespace {
 // ---- The residue form (crt_elem.cuh) ---------------------------------------
 #define MOMMS_CRT_NS(X) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15)
 
-// Moduli that hold an ns-slice product over k: P > 2 |R|, |R| <= k 2^(16 ns),
-// with 2 % to spare for the quotient's rounding (crt::kFracBits).
-int crt_moduli(int ns, int64_t k) {
-  const double need = 16.0 * ns + log2((double)k) + 1.0 + 0.03;
+// Moduli that hold an ns-slice product whose sums of scaled magnitudes
+// (sum_p |a_ip b_pj| 2^-e_i 2^-f_j, at most k) stay within `sum`: P > 2 |R|,
+// |R| <= sum 2^(16 ns), with 2 % to spare for the quotient's rounding
+// (crt::kFracBits). More moduli than R needs do not change the result.
+int crt_moduli(int ns, double sum) {
+  const double need = 16.0 * ns + log2(std::max(sum, (double)kCrtMinK)) + 1.0 + 0.03;
   double have = 0.0;
   int n = 0;
   while (n < crt::kMaxModuli && have < need) have += log2((double)crt::kModuli[n++]);
@@ -797,24 +803,27 @@ int crt_moduli(int ns, int64_t k) {
 // Whether an ns-slice product runs by residues: where the model below says it
 // is the faster form. From the sizes alone (those of the whole product, where
 // it is streamed in blocks), so that a product gives the same bits alone, in a
-// batch, streamed and from packed operands. The rates are measured ones (n^2 =
-// entries of C; ps per entry or per operand element):
-//  * slice products 1.8 PFLOP/s, and per group and entry what of the epilogue
-//    they do not hide: 0.53 ps (digits: 4 bytes of plane), 0.2 ps (residues);
-//  * recombination 7.4 ps (7 digit groups), 10.4 ps (16 moduli);
-//  * operand planes 2 bytes per slice or modulus, 8 read, at 6 TB/s;
-//  * 20 us that the residue planes take longer where they do not fill the GPU.
-// Both forms at 8192 x 8192, 7 slices, ms per call: k = 128 1.33 (digits) and
-// 1.40, 256 1.61 and 1.56, 1024 3.17 and 2.48, 8192 20.9 and 13.1; at 65536 x
-// 256 x 256 0.64 and 0.75.
+// batch, streamed and from packed operands. The rates are measured ones:
+//  * slice products: 0.26 us per 256 x 256 x 64 step of a CTA pair, 76 pairs,
+//    a group's steps in series (7 pairs of digits, or one modulus, each over
+//    all of k: what decides for few tiles), and per group and entry what of
+//    the epilogue they do not hide: 0.53 ps (digits: 4 bytes of plane), 0.2 ps;
+//  * recombination 7.4 ps per entry (7 digit groups), 10.4 ps (16 moduli);
+//  * operand planes 2 bytes per slice or modulus, 8 read, at 6 TB/s.
+// Both forms, 7 slices, ms per call: 8192 x 8192 x 128 1.33 (digits) and 1.40,
+// x 256 1.61 and 1.56, x 1024 3.17 and 2.48, x 8192 20.9 and 13.1; 65536 x 256 x
+// 256 0.64 and 0.75; the slice kernel alone at 512^3 0.030 and 0.014.
 bool crt_applies(int ns, int64_t m, int64_t n, int64_t k) {
   if (ns < 5 || k < kCrtMinK) return false;
   const int N = crt_moduli(ns, k);
   Schedule sc;
   if (!ozaki_schedule(ns, k, &sc)) return true;
-  const double mn = (double)m * n, ops = (double)(m + n) * k, mma = 2.0 * mn * k / 1.8e3;  // ps per product
-  const double digits = sc.np * mma + 0.53 * sc.ng * mn + mn * (2.7 + 0.67 * sc.ng) + ops * (8 + 2 * ns) / 6.0;
-  const double residues = N * mma + 0.2 * N * mn + mn * 0.65 * N + ops * (8 + 2 * N) / 6.0 + 20e6;
+  constexpr double kPairs = 76.0, kStep = 0.26e6;  // ps
+  const double mn = (double)m * n, ops = (double)(m + n) * k;
+  const double tiles = (double)(ceil_div(m, 256) * ceil_div(n, 256)), steps = (double)ceil_div(k, 64) * kStep;
+  auto products = [&](double pairs, double longest) { return steps * std::max(pairs * tiles / kPairs, longest); };
+  const double digits = products(sc.np, ns) + mn * (0.53 * sc.ng + 2.7 + 0.67 * sc.ng) + ops * (8 + 2 * ns) / 6.0;
+  const double residues = products(N, 1.0) + mn * (0.2 * N + 0.65 * N) + ops * (8 + 2 * N) / 6.0;
   return residues < digits;
 }
 
@@ -833,8 +842,7 @@ double crt_scratch(int per, int moduli, int64_t m, int64_t n, int64_t k) {
 // `tight`) by walking the moduli in several passes, each with its own operand
 // planes: at 8192^3 two passes of 9 and 8 moduli instead of 4.6 GB of planes,
 // for one more read of the operands (0.2 of 13 ms).
-int crt_per_pass(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
-  const int N = crt_moduli(ns, k);
+int crt_per_pass(int ns, int N, int64_t m, int64_t n, int64_t k, bool tight) {
   const double limit = std::max(digit_scratch(ns, m, n, k), tight ? 0.0 : (double)kFreeScratch);
   int per = N;
   while (per > 1 && crt_scratch(per, N, m, n, k) > limit) --per;
@@ -855,7 +863,7 @@ void crt_planes(int ns, const Side* sides, int count, int64_t K, __half* const* 
       body.plane_elems[i] = plane_elems[i];
       body.re[i] = row_exp(sides[i], from_max);
     }
-    planes::launch_views(vs, count, body, s);
+    note_launch(planes::launch_views(vs, count, body, s));
   };
   switch (ns) {
 #define X(NS) case NS: launch(crt::ResidueBody<NS, RowExp>{}); break;
@@ -863,7 +871,6 @@ void crt_planes(int ns, const Side* sides, int count, int64_t K, __half* const* 
 #undef X
     default: refuse_launch(cudaErrorInvalidValue);
   }
-  note_launch();
 }
 void crt_planes_of_pack(const PackedOperand& P, int64_t R, __half* out, int l0, int l1, int sm_count, cudaStream_t s) {
   KernelTimer kt(MOMMS_KERNEL_PREP, s);
@@ -899,6 +906,14 @@ void crt_slice_params(int64_t m, int64_t k, int l0, int l1, sp::Params* p) {
   p->group_begin[l1 - l0] = l1 - l0;
 }
 
+// The reconstruction constants of the first n moduli, computed once each.
+const crt::Weights& crt_weights(int n) {
+  static crt::Weights table[crt::kMaxModuli + 1];
+  static std::once_flag once[crt::kMaxModuli + 1];
+  std::call_once(once[n], [n] { crt::make_weights(n, &table[n]); });
+  return table[n];
+}
+
 void crt_combine_params(const DevGemm& g, int ns, int moduli, const void* res, int64_t plane, int64_t mpad,
                         const int* rexp, const int* cexp, crt::CombineParams* cp) {
   memset(cp, 0, sizeof(*cp));
@@ -917,7 +932,7 @@ void crt_combine_params(const DevGemm& g, int ns, int moduli, const void* res, i
   cp->c = static_cast<double*>(g.c.ptr);
   cp->rsc = g.c.rs;
   cp->csc = g.c.cs;
-  crt::make_weights(moduli, &cp->wt);
+  cp->wt = crt_weights(moduli);
 }
 
 // One recombination launch over columns [j0, j1) of C (j0 a multiple of 4) on stream Y.
@@ -958,7 +973,7 @@ double ozaki_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
   const double d = digit_scratch(ns, m, n, k);
   const int64_t kk = std::min(k, kMaxK);
   if (!crt_applies(ns, m, n, kk)) return d;
-  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, m, n, kk, tight), crt_moduli(ns, kk), m, n, kk));
+  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, crt_moduli(ns, kk), m, n, kk, tight), crt_moduli(ns, kk), m, n, kk));
 }
 
 namespace {
@@ -1028,7 +1043,8 @@ int guaranteed_slices(double target, double q1, double q2, bool uncovered, bool*
 // Scratch of the bound: bf16 magnitude planes of A (m rows) and of B
 // transposed (n rows), K-major with row stride kp; the rows' sums of scaled
 // magnitudes (units of 2^-40, m then n) and the result words: out[0], out[1]
-// the maxima (float bits), out[2..3] a 64-bit count of covered entries.
+// the maxima (float bits), out[2..3] a 64-bit count of covered entries, out[4],
+// out[5] the largest row sums (float bits).
 struct BoundWork {
   uint16_t* mag_a;
   uint16_t* mag_b;
@@ -1051,7 +1067,7 @@ struct RowWork {
   unsigned* out;
   int* exps;
 };
-constexpr size_t kBoundWords = 4;
+constexpr size_t kBoundWords = 6;
 size_t row_work_zero_bytes(int64_t m, int64_t n) { return (size_t)(m + n) * 16 + kBoundWords * 4; }
 size_t row_work_bytes(int64_t m, int64_t n) { return row_work_zero_bytes(m, n) + (size_t)(m + n) * 4; }
 RowWork row_work_carve(void* base, int64_t m, int64_t n) {
@@ -1094,21 +1110,21 @@ struct MagnitudeBody {
   int indicator;
 
   template <bool R_CONTIG>
-  __device__ __forceinline__ void run(const planes::View<double>& v, int z) const {
+  __device__ __forceinline__ void run(const planes::View<double>& v, int z, const planes::BlockPlace& at) const {
     const planes::Chunk<R_CONTIG> c(v.lg);
     // the row loop's trip count is the same for every thread of the block
     // (rows past R only skip their work), so every lane reaches the shuffles
-    for (int64_t rb = (int64_t)blockIdx.y * c.rows; rb < v.R; rb += (int64_t)gridDim.y * c.rows) {
+    for (int64_t rb = (int64_t)at.y * c.rows; rb < v.R; rb += (int64_t)at.ny * c.rows) {
       const int64_t r = rb + c.rl;
       unsigned long long t = 0;
       if (r < v.R) {
         const int e = re[z].row(r);
-        if (blockIdx.x == 0 && c.ru == 0) re[z].first(r, e);
+        if (at.x == 0 && c.ru == 0) re[z].first(r, e);
         const double* xr = v.x + r * v.sr;
         uint16_t* outr = plane[z] + r * ldp;
 #pragma unroll 1
         for (int it = 0; it < v.iters; ++it) {
-          const int64_t p = planes::run_col(blockIdx.x, c, it, RUN, v.iters);
+          const int64_t p = planes::run_col(at.x, c, it, RUN, v.iters);
           if (p >= v.K) break;
           double x[RUN];
           planes::load_run<R_CONTIG, RUN>(xr, v.sp, p, v.K, v.vec, x);
@@ -1151,9 +1167,8 @@ int enqueue_magnitudes(const Side* sides, int count, int64_t K, uint16_t* const*
   }
   {
     KernelTimer kt(MOMMS_KERNEL_PREP, s);
-    planes::launch_views(views_of(sides, count, K), count, body, s);
+    note_launch(planes::launch_views(views_of(sides, count, K), count, body, s));
   }
-  note_launch();
   const cudaError_t e = launch_status();
   return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "Ozaki bound magnitudes");
 }
@@ -1227,14 +1242,39 @@ int enqueue_bound_kernel(const BoundWork& w, int64_t m, int64_t n, int64_t k, bo
 // term below FP32's range (relative to 2^(e_i+f_j)): no slice count can vouch
 // for it. Entries with no nonzero term are exact (their digits are all zero).
 // Synchronises `s`.
+// Pinned words the calling thread reads results into: a copy to pageable
+// memory is staged by the driver.
+struct PinnedWords {
+  unsigned* p = nullptr;
+  PinnedWords() {
+    if (cudaMallocHost(&p, 64) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~PinnedWords() {
+    if (p) cudaFreeHost(p);
+  }
+};
 int bound_result(const BoundWork& w, const Side (&sides)[2], int64_t m, int64_t n, int64_t k, DeviceState* ds,
-                 cudaStream_t s, float* q1, float* q2, bool* uncovered) {
-  unsigned words[4] = {0, 0, 0, 0};
-  cudaError_t ce = cudaMemcpyAsync(words, w.out, sizeof(words), cudaMemcpyDeviceToHost, s);
+                 cudaStream_t s, float* q1, float* q2, bool* uncovered, double* sum_most = nullptr) {
+  static thread_local PinnedWords pinned;
+  unsigned local[kBoundWords] = {0, 0, 0, 0};
+  unsigned* words = pinned.p ? pinned.p : local;
+  cudaError_t ce = cudaMemcpyAsync(words, w.out, kBoundWords * sizeof(unsigned), cudaMemcpyDeviceToHost, s);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
   if (ce != cudaSuccess) return cuda_fail(ce, "Ozaki bound");
   memcpy(q1, &words[0], 4);
   memcpy(q2, &words[1], 4);
+  if (sum_most) {
+    // |a'_ip|, |b'_pj| <= 1, so an entry's sum is at most its row's and its
+    // column's; a scaled integer may exceed the element by half a unit (2^-41 at
+    // five slices, the fewest that ask)
+    float rows, cols;
+    memcpy(&rows, &words[4], 4);
+    memcpy(&cols, &words[5], 4);
+    *sum_most = std::min((double)k, 1.0001 * (double)std::min(rows, cols) + 1.0);
+  }
   unsigned long long zeros;
   memcpy(&zeros, &words[2], 8);
   *uncovered = false;
@@ -1419,6 +1459,7 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   //    bound's count while C still holds its input.
   const bool automatic = ns <= 0;
   const bool verify = automatic && defer_b;
+  double sum_most = (double)k;  // bounds every entry's sum of scaled magnitudes (crt_moduli)
   int verdict = MOMMS_OK;
   BoundWork bw{};
   void* bw_mem = nullptr;
@@ -1438,7 +1479,7 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     float q1f = 0.0f, q2f = 0.0f;
     bool uncovered = false;
     if (!rc)
-      rc = bound_result(bw, sides, m, n, k, ds, s, &q1f, &q2f, &uncovered);
+      rc = bound_result(bw, sides, m, n, k, ds, s, &q1f, &q2f, &uncovered, &sum_most);
     if (rc) return rc;
     bool reachable = false;
     ns = guaranteed_slices(target, q1f, q2f, uncovered, &reachable);
@@ -1464,8 +1505,8 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   // The form: digit planes (one pass; packed operands bring theirs), or
   // residue planes in passes of `per` moduli.
   const bool crt = crt_applies(ns, g.whole_m ? g.whole_m : m, g.whole_n ? g.whole_n : n, k);
-  const int N = crt ? crt_moduli(ns, k) : ns;
-  const int per = crt ? crt_per_pass(ns, m, n, k, g.tight) : ns;
+  const int N = crt ? crt_moduli(ns, sum_most) : ns;
+  const int per = crt ? crt_per_pass(ns, N, m, n, k, g.tight) : ns;
   const int passes = (int)ceil_div(N, per);
   const bool own_a = crt || !PA, own_b = crt || !PB;
   __half* planes_buf = nullptr;
@@ -1788,7 +1829,7 @@ bool ozaki_batchable(const DevGemm& g, int slices) {
         g.k > 0))
     return false;
   // residues only where one pass holds them all
-  return !crt_applies(slices, g.m, g.n, g.k) || crt_per_pass(slices, g.m, g.n, g.k, false) == crt_moduli(slices, g.k);
+  return !crt_applies(slices, g.m, g.n, g.k) || crt_per_pass(slices, crt_moduli(slices, g.k), g.m, g.n, g.k, false) == crt_moduli(slices, g.k);
 }
 
 void ozaki_batch_destroy(OzakiBatch* b) {
@@ -1924,7 +1965,7 @@ int ozaki_batch_launch(OzakiBatch* b, cudaStream_t s, int max_sms) {
   if (max_sms > 0) clusters = std::max(1, std::min(clusters, max_sms / 2));
   sp::GroupTable gt{b->d_params, b->d_maps, (int)b->probs.size(), b->units};
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = sp::cluster2_config(sp::P_SMEM_BYTES, attr);
+  cudaLaunchConfig_t cfg = sp::cluster2_config(sp::pair_smem<sp::EPI_OZAKI>(), attr);
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(b->units, clusters)));
   cfg.stream = s;
   cudaError_t e;

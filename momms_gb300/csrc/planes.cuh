@@ -113,29 +113,45 @@ __device__ __forceinline__ void load_run(const Tin* __restrict__ xr, int64_t sp,
   }
 }
 
-// One or two operands of a product in one launch (blockIdx.z): the passes over
+// One or two operands of a product: the passes over
 // A and B are independent, and at 512^2 a launch of its own costs each as much
-// as its work.
+// as its work (launch_views).
 template <typename Tin>
 struct View {
   const Tin* x;
   int64_t sr, sp, R, K;
   int r_contig, vec, lg, iters;
-  unsigned bx;  // blocks in x
+  unsigned nx, ny;  // blocks along the columns and the rows
+};
+// A block's place in its view.
+struct BlockPlace {
+  unsigned x, y, ny;
 };
 template <typename Tin>
 struct Views {
   View<Tin> v[2];
 };
 // Body: Tin, RUN, kContigLg, rows<R_CONTIG>(lg) and cols<R_CONTIG>(lg, iters)
-// of a block, and run<R_CONTIG>(view, index of the view).
+// of a block, and run<R_CONTIG>(view, index of the view, block). The blocks of
+// both views make one row of the grid: none is idle, whatever the two shapes.
 template <typename Body>
 __global__ void __launch_bounds__(THREADS) views_kernel(const __grid_constant__ Views<typename Body::Tin> vs,
                                                         const __grid_constant__ Body body) {
-  const View<typename Body::Tin>& v = vs.v[blockIdx.z];
-  if (blockIdx.x >= v.bx) return;
-  if (v.r_contig) body.template run<true>(v, blockIdx.z);
-  else body.template run<false>(v, blockIdx.z);
+  const unsigned first = vs.v[0].nx * vs.v[0].ny;
+  const int z = blockIdx.x >= first ? 1 : 0;
+  const View<typename Body::Tin>& v = vs.v[z];
+  const unsigned b = blockIdx.x - (z ? first : 0);
+  const BlockPlace at{b % v.nx, b / v.nx, v.ny};
+  if (v.r_contig) body.template run<true>(v, z, at);
+  else body.template run<false>(v, z, at);
+}
+// One view in a launch of its own, compiled for its orientation alone: large
+// operands, whose passes need every register and warp they can get (row maxima
+// of both operands of 8192^3: 240 us in two launches, 340-500 in one).
+template <typename Body, bool R_CONTIG>
+__global__ void __launch_bounds__(THREADS) view_kernel(const __grid_constant__ View<typename Body::Tin> v, int z,
+                                                       const __grid_constant__ Body body) {
+  body.template run<R_CONTIG>(v, z, BlockPlace{blockIdx.x % v.nx, blockIdx.x / v.nx, v.ny});
 }
 __host__ __device__ constexpr int run_rows(int lg) { return (THREADS / 32) << (5 - lg); }
 
@@ -156,21 +172,21 @@ struct PlanesBody {
   Op op[2];
 
   template <bool R_CONTIG>
-  __device__ __forceinline__ void run(const View<Tin>& v, int z) const {
+  __device__ __forceinline__ void run(const View<Tin>& v, int z, const BlockPlace& at) const {
     using Word = typename Op::Word;
     constexpr int NP = Op::PLANES;
     static_assert(sizeof(Word) == 2 * sizeof(Tout), "a word is one pair's value");
     const Chunk<R_CONTIG> c(v.lg);
     const int64_t pe = plane_elems[z];
     // row chunks beyond the grid's y limit are taken in further passes
-    for (int64_t r = (int64_t)blockIdx.y * c.rows + c.rl; r < v.R; r += (int64_t)gridDim.y * c.rows) {
+    for (int64_t r = (int64_t)at.y * c.rows + c.rl; r < v.R; r += (int64_t)at.ny * c.rows) {
       const auto ctx = op[z].row(r);
-      if (blockIdx.x == 0 && c.ru == 0) op[z].first(r, ctx);
+      if (at.x == 0 && c.ru == 0) op[z].first(r, ctx);
       const Tin* xr = v.x + r * v.sr;
       Tout* outr = planes[z] + r * ldp;
 #pragma unroll 1
       for (int it = 0; it < v.iters; ++it) {
-        const int64_t p = run_col(blockIdx.x, c, it, RUN, v.iters);
+        const int64_t p = run_col(at.x, c, it, RUN, v.iters);
         if (p >= v.K) break;
         Tin x[RUN];
         load_run<R_CONTIG, RUN>(xr, v.sp, p, v.K, v.vec, x);
@@ -220,10 +236,11 @@ inline View<Tin> make_view(const Tin* x, int64_t sr, int64_t sp, int64_t R, int6
   return v;
 }
 
-// Launches a body over `count` views. A thread takes PITER runs, or one where
-// that leaves fewer than four blocks per SM.
+// Launches a body over `count` views: one launch for both, each thread taking
+// one run, where PITER runs a thread leave fewer than four blocks per SM, else
+// one launch each. Returns the launches made.
 template <typename Body>
-void launch_views(Views<typename Body::Tin> vs, int count, const Body& body, cudaStream_t s) {
+int launch_views(Views<typename Body::Tin> vs, int count, const Body& body, cudaStream_t s) {
   constexpr int64_t kFewBlocks = 4 * 152;
   auto rows = [](bool rc, int lg) { return rc ? Body::template rows<true>(lg) : Body::template rows<false>(lg); };
   auto cols = [](bool rc, int lg, int it) {
@@ -235,26 +252,36 @@ void launch_views(Views<typename Body::Tin> vs, int count, const Body& body, cud
     v.lg = run_lanes_log2(v.K, Body::RUN, v.r_contig != 0, Body::kContigLg);
     blocks += ceil_div_dev(v.K, cols(v.r_contig != 0, v.lg, PITER)) * ceil_div_dev(v.R, rows(v.r_contig != 0, v.lg));
   }
-  dim3 grid(1, 1, (unsigned)count);
+  unsigned grid = 0;
   for (int i = 0; i < count; ++i) {
     View<typename Body::Tin>& v = vs.v[i];
     v.iters = blocks < kFewBlocks ? 1 : PITER;
-    v.bx = (unsigned)ceil_div_dev(v.K, cols(v.r_contig != 0, v.lg, v.iters));
-    grid.x = std::max(grid.x, v.bx);
-    grid.y = std::max(grid.y, (unsigned)std::min<int64_t>(ceil_div_dev(v.R, rows(v.r_contig != 0, v.lg)), 65535));
+    v.nx = (unsigned)ceil_div_dev(v.K, cols(v.r_contig != 0, v.lg, v.iters));
+    // at most 2^30 blocks a view: the bodies' row loops take the rest
+    v.ny = (unsigned)std::min<int64_t>(ceil_div_dev(v.R, rows(v.r_contig != 0, v.lg)), ((int64_t)1 << 30) / v.nx);
+    grid += v.nx * v.ny;
   }
-  views_kernel<Body><<<grid, THREADS, 0, s>>>(vs, body);
+  if (blocks < kFewBlocks && count > 1) {
+    views_kernel<Body><<<grid, THREADS, 0, s>>>(vs, body);
+    return 1;
+  }
+  for (int i = 0; i < count; ++i) {
+    const View<typename Body::Tin>& v = vs.v[i];
+    if (v.r_contig) view_kernel<Body, true><<<v.nx * v.ny, THREADS, 0, s>>>(v, i, body);
+    else view_kernel<Body, false><<<v.nx * v.ny, THREADS, 0, s>>>(v, i, body);
+  }
+  return count;
 }
 
 // Both operands' planes (count 2), or one's.
 template <typename Tin, typename Op>
-void launch_to_planes(const Views<Tin>& vs, int count, const PlanesBody<Tin, Op>& body, cudaStream_t s) {
+int launch_to_planes(const Views<Tin>& vs, int count, const PlanesBody<Tin, Op>& body, cudaStream_t s) {
   for (int i = 0; i < count; ++i)
     if (body.ldp % body.RUN || body.plane_elems[i] % body.RUN || (reinterpret_cast<uintptr_t>(body.planes[i]) & 15)) {
       refuse_launch(cudaErrorMisalignedAddress);  // the vector stores need 16-byte aligned runs
-      return;
+      return 0;
     }
-  launch_views(vs, count, body, s);
+  return launch_views(vs, count, body, s);
 }
 
 }  // namespace planes

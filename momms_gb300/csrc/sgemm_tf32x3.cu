@@ -54,8 +54,7 @@ void tf32_operand_planes(const F32View* v, int count, int64_t K, int64_t kp, cud
     body.plane_elems[i] = v[i].R * kp;
   }
   KernelTimer kt(MOMMS_KERNEL_PREP, s);
-  planes::launch_to_planes(vs, count, body, s);
-  note_launch();
+  note_launch(planes::launch_to_planes(vs, count, body, s));
 }
 
 int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {

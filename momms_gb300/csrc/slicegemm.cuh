@@ -111,7 +111,7 @@ struct Params {
   const unsigned long long* msum_a;
   const unsigned long long* msum_b;
   float lb_scale, kf;
-  unsigned* bound_out;                // [0], [1]: the maxima
+  unsigned* bound_out;                // [0], [1]: the maxima; [4], [5]: the largest row sum of A's and B's magnitudes
   unsigned long long* bound_count;  // entries counted
   int count_only;
   int64_t unit_begin;  // grouped launches: this problem's first work unit
@@ -172,61 +172,90 @@ __device__ __forceinline__ void drain_chunk(uint32_t taddr, EpiAcc<EPI> (&S)[NC]
 }
 
 // EPI_BOUND: this thread's row against its NC columns, reduced over the warp
-// and posted to the two maxima. Every lane calls it (rows past m contribute 0).
+// and posted to the maxima. Every lane calls it (rows past m contribute 0).
+// `sb`: shared memory for this warp's NC column sums.
+//
+// The maxima need only be upper bounds, so a quotient is a product with the
+// hardware's approximate reciprocal (at most one unit of 2^-23 off), and each
+// maximum is raised by 2^-18 at the end, which covers that and the roundings:
+// six instructions per entry. (With upward-rounded quotients formed where they
+// could raise the maximum, and column sums by shuffle, the epilogue took 25 of
+// the 30 us of a 512 x 512 x 512 bound, 0.23 ms at 8192 x 8192 x 64.)
 template <int NC>
-__device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t col0, const float (&S)[NC]) {
-  static_assert(NC % 32 == 0, "columns are shared out 32 per lane round");
-  float m1 = 0.0f, m2 = 0.0f;
+__device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t col0, const float (&S)[NC], float* sb) {
+  const int lane = threadIdx.x & 31;
+  float m1 = 0.0f, m2 = 0.0f, ma = 0.0f, mb = 0.0f;
   unsigned cnt = 0;
   // columns of this tile inside C (the same for the whole warp)
   const int nvalid = (int)min((int64_t)NC, max((int64_t)0, p.n - col0));
+  const bool rv = row < p.m;
   if (p.count_only) {
-    if (row < p.m) {
+    if (rv) {
 #pragma unroll
       for (int j = 0; j < NC; ++j) cnt += (j < nvalid && S[j] > 0.0f) ? 1u : 0u;
     }
   } else {
-    // The warp's 32 rows share their NC columns: each lane converts the
-    // column sums of every 32nd column once (upward, units of 2^-40) and the
-    // entries take them by shuffle.
-    const int lane = threadIdx.x & 31;
-    float sbl[NC / 32];
 #pragma unroll
-    for (int q = 0; q < NC / 32; ++q)
-      sbl[q] = 32 * q + lane < nvalid ? __fmul_ru(__ull2float_ru(p.msum_b[col0 + 32 * q + lane]), 0x1p-40f) : 0.0f;
-    const bool rv = row < p.m;
-    const float sa = rv ? __fmul_ru(__ull2float_ru(p.msum_a[row]), 0x1p-40f) : 0.0f;
-    // q2 = k / L needs only the row's smallest L: one reciprocal per row.
-    // q1 = (sa + sb) / L: an entry whose (sa + sb), rounded up, is at most
-    // m1 * L rounded down cannot raise m1 (its quotient is at most m1), so
-    // the upward quotient is formed only for the others.
-    float lmin = INFINITY;
+    for (int q = 0; q < NC / 32; ++q) {
+      const float v = 32 * q + lane < nvalid ? __fmul_ru(__ull2float_ru(p.msum_b[col0 + 32 * q + lane]), 0x1p-40f) : 0.0f;
+      sb[32 * q + lane] = v;
+      mb = fmaxf(mb, v);
+    }
+    __syncwarp();
+    if (rv) {
+      const float sa = ma = __fmul_ru(__ull2float_ru(p.msum_a[row]), 0x1p-40f);
+      float smin = INFINITY;
 #pragma unroll
-    for (int j = 0; j < NC; ++j) {
-      const float sb = __shfl_sync(0xffffffffu, sbl[j >> 5], j & 31);
-      const float lb = __fmul_rd(S[j], p.lb_scale);
-      // L = 0: no p with both a_ip and b_pj nonzero (the entry has no
-      // error), or every term below FP32's range: counted, the host tells
-      // the two apart
-      if (rv && j < nvalid) {
-        if (lb > 0.0f) {
-          const float x = __fadd_ru(sa, sb);
-          if (x > __fmul_rd(m1, lb)) m1 = fmaxf(m1, __fmul_ru(x, __frcp_ru(lb)));
-          lmin = fminf(lmin, lb);
-        } else {
-          ++cnt;
+      for (int j = 0; j < NC; j += 4) {
+        const float4 b4 = *reinterpret_cast<const float4*>(sb + j);
+        const float b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          // columns past n count as covered
+          const float s = j + q < nvalid ? S[j + q] : INFINITY;
+          float r;
+          asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(s));
+          m1 = fmaxf(m1, (sa + b[q]) * r);
+          smin = fminf(smin, s);
         }
       }
+      // S = 0: no p with both a_ip and b_pj nonzero (the entry has no error), or
+      // every term below FP32's range: counted, the host tells the two apart.
+      // Such rows (and any whose smallest sum an approximate reciprocal would
+      // take past FP32's range) go through their entries again.
+      if (smin < 0x1p-100f) {
+        m1 = 0.0f;
+        smin = INFINITY;
+#pragma unroll 1
+        for (int j = 0; j < nvalid; ++j) {
+          float s = 0.0f;
+#pragma unroll
+          for (int q = 0; q < NC; ++q) s = q == j ? S[q] : s;
+          if (s > 0.0f) {
+            m1 = fmaxf(m1, __fdiv_ru(sa + sb[j], s));
+            smin = fminf(smin, s);
+          } else {
+            ++cnt;
+          }
+        }
+      }
+      if (smin < INFINITY) m2 = __fdiv_ru(p.kf, smin);
+      // the lower bound is S times lb_scale
+      const float up = __fdiv_ru(1.0f + 0x1p-18f, p.lb_scale);
+      m1 = __fmul_ru(m1, up);
+      m2 = __fmul_ru(m2, up);
     }
-    if (lmin < INFINITY) m2 = __fmul_ru(p.kf, __frcp_ru(lmin));  // >= k / L for every entry of the row
+    __syncwarp();  // before the next tile's column sums
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
     m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    ma = fmaxf(ma, __shfl_xor_sync(0xffffffffu, ma, o));
+    mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, o));
     cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   }
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     // Non-negative floats order like their bit patterns. Every warp of every
     // tile reports here: the maxima only grow, so a warp below the value
     // already posted skips its atomic (same-address atomics serialise in L2;
@@ -235,6 +264,8 @@ __device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t
       const volatile unsigned* cur = p.bound_out;
       if (__float_as_uint(m1) > cur[0]) atomicMax(&p.bound_out[0], __float_as_uint(m1));
       if (__float_as_uint(m2) > cur[1]) atomicMax(&p.bound_out[1], __float_as_uint(m2));
+      if (__float_as_uint(ma) > cur[4]) atomicMax(&p.bound_out[4], __float_as_uint(ma));
+      if (__float_as_uint(mb) > cur[5]) atomicMax(&p.bound_out[5], __float_as_uint(mb));
     }
     if (cnt) atomicAdd(p.bound_count, (unsigned long long)cnt);
   }
@@ -404,7 +435,7 @@ __device__ __forceinline__ bool ozaki_groups(const Params& p, int g0, int g1, in
 // The epilogue of EPI_F32 and EPI_BOUND for one tile (groups [g0, g1)), as ozaki_groups.
 template <int EPI, int NC, typename Wait, typename Release>
 __device__ __forceinline__ bool float_groups(const Params& p, int g0, int g1, int64_t row, int64_t col0, Wait&& wait,
-                                             Release&& release) {
+                                             Release&& release, float* sb) {
   // per-thread FP32 sums of finished chunks, rounded to nearest, which keeps
   // the tensor core's internal accumulation to one chunk at a time
   float S[NC];
@@ -418,7 +449,7 @@ __device__ __forceinline__ bool float_groups(const Params& p, int g0, int g1, in
       release();
     }
   }
-  if constexpr (EPI == EPI_BOUND) bound_tile<NC>(p, row, col0, S);
+  if constexpr (EPI == EPI_BOUND) bound_tile<NC>(p, row, col0, S, sb);
   if (EPI == EPI_F32 && row < p.m) {
     // C is read 8 columns at a time, every load of a group issued before
     // the first use (one memory round trip per group, not per element)
@@ -626,6 +657,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     // ------------------------------ epilogue ------------------------------
     const int q = warp & 3;              // TMEM lane quarter this warp may access
     const int h = (warp - 2) >> 2;       // column group: cols h*EPI_COLS .. +EPI_COLS-1
+    __shared__ float4 s_sums[EPI == EPI_BOUND ? EPI_WARPS * EPI_COLS / 4 : 1];
+    float* sb = reinterpret_cast<float*>(s_sums) + (EPI == EPI_BOUND ? (warp - 2) * EPI_COLS : 0);
     const int r_local = q * 32 + lane;
     int buf = 0;
     uint32_t acc_ph[2] = {0, 0};
@@ -658,7 +691,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!ozaki_groups<EPI_COLS>(p, g_begin(t), g_end(t), row, col0, tm, tn, h * EPI_COLS, r_local, wait, release))
           goto epi_done;
       } else {
-        if (!float_groups<EPI, EPI_COLS>(p, g_begin(t), g_end(t), row, col0, wait, release)) goto epi_done;
+        if (!float_groups<EPI, EPI_COLS>(p, g_begin(t), g_end(t), row, col0, wait, release, sb)) goto epi_done;
       }
     }
   epi_done:;
@@ -688,14 +721,19 @@ __global__ void __launch_bounds__(THREADS, 1)
 //   tfull[b]  (each CTA)  the even CTA's commit, multicast: accumulator b done
 //   tempty[b] (even CTA)  all 16 epilogue warps of the pair: b drained
 // ---------------------------------------------------------------------------
-constexpr int PSTAGES = 7;
 constexpr int P_STAGE_BYTES = A_TILE + B_TILE / 2;  // 32 KB
-constexpr int P_SMEM_BYTES = 1024 + PSTAGES * P_STAGE_BYTES + 256;
+// Stages: seven, or six where the epilogue needs shared memory of its own (the
+// bound's column sums).
+template <int EPI>
+constexpr int pair_stages() { return EPI == EPI_BOUND ? 6 : 7; }
+template <int EPI>
+constexpr int pair_smem() { return 1024 + pair_stages<EPI>() * P_STAGE_BYTES + 256; }
 
 template <int KIND, int EPI, bool GROUPED = false>
 __global__ void __launch_bounds__(THREADS, 1)
     slice_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
                            const __grid_constant__ Params p, const __grid_constant__ GroupTable gt) {
+  constexpr int PSTAGES = pair_stages<EPI>();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + PSTAGES * P_STAGE_BYTES);
@@ -918,6 +956,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     // ------------------------------ epilogue (both CTAs) ------------------------------
     const int q = warp & 3;
     const int h = (warp - 2) >> 2;
+    __shared__ float4 s_sums[EPI == EPI_BOUND ? EPI_WARPS * EPI_COLS / 4 : 1];
+    float* sb = reinterpret_cast<float*>(s_sums) + (EPI == EPI_BOUND ? (warp - 2) * EPI_COLS : 0);
     const int r_local = q * 32 + lane;
     const uint32_t tempty_leader[2] = {mapa_shared(&tempty[0], 0), mapa_shared(&tempty[1], 0)};
     int buf = 0;
@@ -948,7 +988,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       if constexpr (EPI == EPI_OZAKI)
         return ozaki_groups<EPI_COLS>(P, g0, g1, row, col0, tm, tn, h * EPI_COLS, r_local, wait, release);
       else
-        return float_groups<EPI, EPI_COLS>(P, g0, g1, row, col0, wait, release);
+        return float_groups<EPI, EPI_COLS>(P, g0, g1, row, col0, wait, release, sb);
     };
     bool ok = true;
     for (int64_t r = 0; r * unit_step < units && ok && !aborted(abort_flag); ++r) {
@@ -1011,10 +1051,10 @@ inline cudaError_t set_slice_attrs() {
                                        SMEM_BYTES);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(slice_gemm_pair_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             P_SMEM_BYTES);
+                             pair_smem<EPI>());
   if (e == cudaSuccess && EPI == EPI_OZAKI)
     e = cudaFuncSetAttribute(slice_gemm_pair_kernel<KIND, EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             P_SMEM_BYTES);
+                             pair_smem<EPI>());
   return e;
 }
 
@@ -1053,7 +1093,7 @@ inline int slice_variant(int* clusters) {
     int v = SLICE_SINGLE, n = 0;
     if (want_pair) {
       cudaLaunchAttribute attr[1];
-      cudaLaunchConfig_t cfg = cluster2_config(P_SMEM_BYTES, attr);
+      cudaLaunchConfig_t cfg = cluster2_config(pair_smem<EPI>(), attr);
       int c = 0;
       if (cudaOccupancyMaxActiveClusters(&c, (const void*)slice_gemm_pair_kernel<KIND, EPI>, &cfg) != cudaSuccess) {
         cudaGetLastError();
@@ -1092,7 +1132,18 @@ inline cudaError_t launch_slice(const CUtensorMap& tmA, const CUtensorMap& tmB_f
   // can run as separate work units. Pick the split whose schedule of units
   // (group-major, handed out in the kernel's snake order; cost = k-blocks of
   // the unit's pairs plus 8 for its pipeline fill) finishes first.
-  if (EPI == EPI_OZAKI && tile_units < 4 * slots && p.ngroups > 1) {
+  if (EPI == EPI_OZAKI && p.residue && tile_units < 4 * slots) {
+    // groups of equal cost: the makespan is rounds times a unit's
+    double best = -1.0;
+    for (int gc = p.ngroups; gc >= 1; gc = gc == 1 ? 0 : (gc + 1) / 2) {
+      const int64_t units = tile_units * ((p.ngroups + gc - 1) / gc);
+      const double makespan = (double)((units + slots - 1) / slots) * (8.0 + (double)gc * (double)p.kblocks);
+      if (best < 0.0 || makespan < best * 0.97) {
+        best = makespan;
+        q.gchunk = gc;
+      }
+    }
+  } else if (EPI == EPI_OZAKI && tile_units < 4 * slots && p.ngroups > 1) {
     double best = -1.0;
     std::vector<double> load((size_t)slots);
     for (int gc = p.ngroups; gc >= 1; gc = gc == 1 ? 0 : (gc + 1) / 2) {
@@ -1117,7 +1168,7 @@ inline cudaError_t launch_slice(const CUtensorMap& tmA, const CUtensorMap& tmB_f
   const int64_t units = tile_units * ((p.ngroups + q.gchunk - 1) / q.gchunk);
   if (v == SLICE_PAIR) {
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = cluster2_config(P_SMEM_BYTES, attr);
+    cudaLaunchConfig_t cfg = cluster2_config(pair_smem<EPI>(), attr);
     cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(units, clusters)));
     cfg.stream = s;
     return cudaLaunchKernelEx(&cfg, slice_gemm_pair_kernel<KIND, EPI>, tmA, tmB_half, q, GroupTable{});
