@@ -128,7 +128,7 @@ struct DevGemm {
   DevMat a, b, c;
   Staging* staging = nullptr;
   const PackedOperand* pk[2] = {nullptr, nullptr};  // packed A, B (their DevMat is the plain copy, if any)
-  bool tight = false;  // emulated: scratch within work_bytes (ozaki_scratch)
+  bool tight = false;  // scratch within work_bytes (ozaki_scratch, plane_row)
   int64_t whole_m = 0, whole_n = 0;  // a block of a streamed product: that product's sizes
 };
 
@@ -355,5 +355,13 @@ class KernelTimer {
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
+// Row stride of an operand plane of k elements, `unit` of which are 16 bytes:
+// whole 32-byte sectors. TMA takes any multiple of 16 bytes, but a 128-byte
+// row of a tile that starts in the middle of a sector reads five sectors for
+// four: split-TF32 6000 x 3001 x 4099 761 -> 627 us, 16 residue products at
+// 4096 x 4096 x 4097 2188 -> 1761 us (strides of whole 128-byte lines measured
+// the same as whole sectors). A call that must stay within its scratch
+// (DevGemm::tight) keeps to 16 bytes.
+inline int64_t plane_row(int64_t k, int64_t unit, bool tight) { return round_up(k, tight ? unit : 2 * unit); }
 
 }  // namespace momms

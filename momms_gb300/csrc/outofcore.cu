@@ -81,7 +81,7 @@ size_t work_bytes(int dtype, int precision, int slices, int64_t m, int64_t n, in
     // operand planes of A and B and the products' group planes
     bytes = ozaki_scratch(s, m, n, k, tight) + 12.0 * (M + N);
   } else if (precision == MOMMS_PREC_SPLIT_TF32) {
-    bytes = 8.0 * (M + N) * (double)round_up(k, 4);
+    bytes = 8.0 * (M + N) * (double)plane_row(k, 4, tight);
   } else {
     (void)dtype;
     (void)K;

@@ -830,22 +830,22 @@ bool crt_applies(int ns, int64_t m, int64_t n, int64_t k) {
 // Scratch of an emulated product, operand planes and group planes: the digit
 // form's, or the residue form's with `per` moduli per pass.
 double plane_bytes(int64_t m, int64_t n) { return (double)round_up(m, sp::BM) * (double)round_up(n, sp::BN); }
-double digit_scratch(int ns, int64_t m, int64_t n, int64_t k) {
+double digit_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
   Schedule sc;
   const double ng = ozaki_schedule(ns, k, &sc) ? sc.ng : sp::MAX_GROUPS;
-  return 2.0 * ns * (double)(m + n) * (double)round_up(std::min(k, kMaxK), 8) + 4.0 * ng * plane_bytes(m, n);
+  return 2.0 * ns * (double)(m + n) * (double)plane_row(std::min(k, kMaxK), 8, tight) + 4.0 * ng * plane_bytes(m, n);
 }
-double crt_scratch(int per, int moduli, int64_t m, int64_t n, int64_t k) {
-  return 2.0 * per * (double)(m + n) * (double)round_up(std::min(k, kMaxK), 8) + moduli * plane_bytes(m, n);
+double crt_scratch(int per, int moduli, int64_t m, int64_t n, int64_t k, bool tight) {
+  return 2.0 * per * (double)(m + n) * (double)plane_row(std::min(k, kMaxK), 8, tight) + moduli * plane_bytes(m, n);
 }
 // The residue form keeps to the digit form's scratch (or kFreeScratch bytes, unless
 // `tight`) by walking the moduli in several passes, each with its own operand
 // planes: at 8192^3 two passes of 9 and 8 moduli instead of 4.6 GB of planes,
 // for one more read of the operands (0.2 of 13 ms).
 int crt_per_pass(int ns, int N, int64_t m, int64_t n, int64_t k, bool tight) {
-  const double limit = std::max(digit_scratch(ns, m, n, k), tight ? 0.0 : (double)kFreeScratch);
+  const double limit = std::max(digit_scratch(ns, m, n, k, tight), tight ? 0.0 : (double)kFreeScratch);
   int per = N;
-  while (per > 1 && crt_scratch(per, N, m, n, k) > limit) --per;
+  while (per > 1 && crt_scratch(per, N, m, n, k, tight) > limit) --per;
   const int passes = (int)ceil_div(N, per);
   return (int)ceil_div(N, passes);
 }
@@ -970,10 +970,10 @@ int plane_map(CUtensorMap* map, const void* base, int64_t k, int64_t rows, int p
 }  // namespace
 
 double ozaki_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
-  const double d = digit_scratch(ns, m, n, k);
+  const double d = digit_scratch(ns, m, n, k, tight);
   const int64_t kk = std::min(k, kMaxK);
   if (!crt_applies(ns, m, n, kk)) return d;
-  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, crt_moduli(ns, kk), m, n, kk, tight), crt_moduli(ns, kk), m, n, kk));
+  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, crt_moduli(ns, kk), m, n, kk, tight), crt_moduli(ns, kk), m, n, kk, tight));
 }
 
 namespace {
@@ -1054,7 +1054,7 @@ struct BoundWork {
   int64_t kp;
 };
 size_t bound_work_bytes(int64_t m, int64_t n, int64_t k) {
-  const int64_t kp = round_up(k, 8);
+  const int64_t kp = plane_row(k, 8, false);
   return (size_t)round_up(m * kp * 2, 256) + (size_t)round_up(n * kp * 2, 256);
 }
 
@@ -1080,7 +1080,7 @@ RowWork row_work_carve(void* base, int64_t m, int64_t n) {
 }
 void bound_work_carve(void* base, const RowWork& rw, int64_t m, int64_t n, int64_t k, BoundWork* w) {
   char* p = static_cast<char*>(base);
-  w->kp = round_up(k, 8);
+  w->kp = plane_row(k, 8, false);
   w->mag_a = reinterpret_cast<uint16_t*>(p);
   p += round_up(m * w->kp * 2, 256);
   w->mag_b = reinterpret_cast<uint16_t*>(p);
@@ -1500,8 +1500,9 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   }
   if (slices_used) *slices_used = ns;
 
-  const int64_t kp = round_up(k, 8);  // 16-byte rows of fp16
-  const size_t a_plane = (size_t)m * kp, b_plane = (size_t)n * kp;
+  // row strides of the planes: a packed operand's are the pack's
+  const int64_t kp = plane_row(k, 8, g.tight), kpa = PA ? PA->kp : kp, kpb = PB ? PB->kp : kp;
+  const size_t a_plane = (size_t)m * kpa, b_plane = (size_t)n * kpb;
   // The form: digit planes (one pass; packed operands bring theirs), or
   // residue planes in passes of `per` moduli.
   const bool crt = crt_applies(ns, g.whole_m ? g.whole_m : m, g.whole_n ? g.whole_n : n, k);
@@ -1580,7 +1581,7 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     p.plane = (int64_t)plane;
     p.status = ds->status;
     CUtensorMap tmA;
-    rc = plane_map(&tmA, pa, k, m, l1 - l0, kp, a_plane, sp::BM);
+    rc = plane_map(&tmA, pa, k, m, l1 - l0, kpa, a_plane, sp::BM);
     if (rc) break;
     // The second stream starts after everything above (scratch, A, the
     // choice), and so does the verify stream V, which runs the bound kernel
@@ -1622,8 +1623,8 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
         }
       }
       CUtensorMap tmB, tmB_half;  // half: one CTA's share of the B tile for the pair kernel
-      rc = plane_map(&tmB, pb + j0 * kp, k, w, l1 - l0, kp, b_plane, sp::BN);
-      if (!rc) rc = plane_map(&tmB_half, pb + j0 * kp, k, w, l1 - l0, kp, b_plane, sp::BN / 2);
+      rc = plane_map(&tmB, pb + j0 * kpb, k, w, l1 - l0, kpb, b_plane, sp::BN);
+      if (!rc) rc = plane_map(&tmB_half, pb + j0 * kpb, k, w, l1 - l0, kpb, b_plane, sp::BN / 2);
       if (rc) break;
       p.n = w;
       p.tiles_n = (int)ceil_div(w, sp::BN);
@@ -1888,7 +1889,7 @@ int ozaki_batch_create(const DevGemm* gs, const int* slices, int count, cudaStre
       break;
     }
     const int ng = P.crt ? P.planes_each : sch.ng;
-    P.kp = round_up(k, 8);
+    P.kp = plane_row(k, 8, false);
     P.a_plane = (size_t)m * P.kp;
     P.b_plane = (size_t)n * P.kp;
     const int64_t mpad = round_up(m, (int64_t)sp::BM);

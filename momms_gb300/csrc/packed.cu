@@ -135,7 +135,7 @@ int momms_pack(int dtype, int precision, int role, int64_t rows, int64_t cols, c
     }
   } else if (precision == MOMMS_PREC_OZAKI) {
     p->np = slices > 0 ? slices : 7;  // 56 bits: FP64 level for most data
-    p->kp = round_up(K, 8);
+    p->kp = plane_row(K, 8, false);
     const size_t plane_bytes = (size_t)p->np * (size_t)R * (size_t)p->kp * 2;
     const size_t exps_off = round_up((int64_t)plane_bytes, 256);
     p->bytes = exps_off + (size_t)round_up((int64_t)((size_t)R * sizeof(int)), 8) + (size_t)R * sizeof(unsigned long long);
@@ -152,7 +152,7 @@ int momms_pack(int dtype, int precision, int role, int64_t rows, int64_t cols, c
     }
   } else {  // split-TF32
     p->np = 2;
-    p->kp = round_up(K, 4);
+    p->kp = plane_row(K, 4, false);
     p->bytes = 2 * (size_t)R * (size_t)p->kp * 4;
     ce = device_malloc((void**)&p->mem, p->bytes);
     if (ce == cudaSuccess) {

@@ -60,11 +60,11 @@ void tf32_operand_planes(const F32View* v, int count, int64_t K, int64_t kp, cud
 int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   DeviceState* ds = device_state();
   if (!ds) return MOMMS_ERR_NO_DEVICE;
-  const int64_t kp = round_up(g.k, 4);  // 16-byte rows for TMA
-  const size_t a_plane = (size_t)g.m * kp, b_plane = (size_t)g.n * kp;
   // packed operands (momms_pack) bring their planes
   const PackedOperand* PA = g.pk[0];
   const PackedOperand* PB = g.pk[1];
+  const int64_t kp = plane_row(g.k, 4, g.tight), kpa = PA ? PA->kp : kp, kpb = PB ? PB->kp : kp;
+  const size_t a_plane = (size_t)g.m * kpa, b_plane = (size_t)g.n * kpb;
   void* buf = nullptr;
   cudaError_t ce = cudaSuccess;
   const size_t own = (PA ? 0 : 2 * a_plane) + (PB ? 0 : 2 * b_plane);
@@ -93,12 +93,12 @@ int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   CUtensorMap tmA, tmB, tmB_half;
   {
     uint64_t dims[3] = {(uint64_t)g.k, (uint64_t)g.m, 2};
-    uint64_t strides[2] = {(uint64_t)kp * 4, (uint64_t)a_plane * 4};
+    uint64_t strides[2] = {(uint64_t)kpa * 4, (uint64_t)a_plane * 4};
     uint32_t box[3] = {32, (uint32_t)sp::BM, 1};  // 128-byte k-blocks
     int rc = encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, pa, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     uint64_t dimsb[3] = {(uint64_t)g.k, (uint64_t)g.n, 2};
-    uint64_t stridesb[2] = {(uint64_t)kp * 4, (uint64_t)b_plane * 4};
+    uint64_t stridesb[2] = {(uint64_t)kpb * 4, (uint64_t)b_plane * 4};
     uint32_t boxb[3] = {32, (uint32_t)sp::BN, 1};
     rc = encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, pb, dimsb, stridesb, boxb, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
