@@ -7,6 +7,8 @@
 // Markidis et al. 2018, Ootomo & Yokota 2022). The small cross terms are
 // accumulated first. The result stays inside the f32 componentwise bound
 // |dC| <= 2k u_32 (|A||B|) that the plain FFMA path meets.
+#include <cstdlib>
+
 #include "internal.h"
 #include "planes.cuh"
 #include "slicegemm.cuh"
@@ -60,68 +62,70 @@ void tf32_operand_planes(const F32View* v, int count, int64_t K, int64_t kp, cud
 int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   DeviceState* ds = device_state();
   if (!ds) return MOMMS_ERR_NO_DEVICE;
+  // The epilogue's lanes hold consecutive rows of the tile, so C is taken
+  // transposed (C^T = B^T A^T) where its columns are the closer ones: 32-lane
+  // stores of one line instead of 32 (6000 x 3001 x 4099, C by rows: 627 ->
+  // 543 us). Every product and the order of the sums stay the same.
+  const bool flip = std::llabs(g.c.cs) < std::llabs(g.c.rs);
+  const int ia = flip ? 1 : 0, ib = 1 - ia;  // the operand (0 = A, 1 = B) that gives the tile's rows, columns
+  const int64_t rows = flip ? g.n : g.m, cols = flip ? g.m : g.n;
   // packed operands (momms_pack) bring their planes
-  const PackedOperand* PA = g.pk[0];
-  const PackedOperand* PB = g.pk[1];
-  const int64_t kp = plane_row(g.k, 4, g.tight), kpa = PA ? PA->kp : kp, kpb = PB ? PB->kp : kp;
-  const size_t a_plane = (size_t)g.m * kpa, b_plane = (size_t)g.n * kpb;
+  int64_t kp[2];
+  size_t plane[2], own = 0;
+  for (int i = 0; i < 2; ++i) {
+    kp[i] = g.pk[i] ? g.pk[i]->kp : plane_row(g.k, 4, g.tight);
+    plane[i] = (size_t)((i ? g.n : g.m) * kp[i]);
+    if (!g.pk[i]) own += 2 * plane[i];
+  }
   void* buf = nullptr;
   cudaError_t ce = cudaSuccess;
-  const size_t own = (PA ? 0 : 2 * a_plane) + (PB ? 0 : 2 * b_plane);
   if (own && (ce = scratch_alloc(&buf, own * sizeof(float), s)) != cudaSuccess)
     return cuda_fail(ce, "split-TF32 planes");
   ScratchGuard free_buf(buf, s);
-  float* pa = PA ? static_cast<float*>(PA->planes) : static_cast<float*>(buf);
-  float* pb = PB ? static_cast<float*>(PB->planes) : static_cast<float*>(buf) + (PA ? 0 : 2 * a_plane);
-  const F32View va{static_cast<const float*>(g.a.ptr), g.a.rs, g.a.cs, g.m, pa};
-  const F32View vb{static_cast<const float*>(g.b.ptr), g.b.cs, g.b.rs, g.n, pb};
-  if (!PA && !PB && !g.staging) {
-    const F32View both[2] = {va, vb};
-    tf32_operand_planes(both, 2, g.k, kp, s);
+  float* planes[2];
+  for (int i = 0; i < 2; ++i)
+    planes[i] = g.pk[i] ? static_cast<float*>(g.pk[i]->planes)
+                        : static_cast<float*>(buf) + (i && !g.pk[0] ? 2 * plane[0] : 0);
+  const F32View views[2] = {{static_cast<const float*>(g.a.ptr), g.a.rs, g.a.cs, g.m, planes[0]},
+                            {static_cast<const float*>(g.b.ptr), g.b.cs, g.b.rs, g.n, planes[1]}};
+  if (!g.pk[0] && !g.pk[1] && !g.staging) {
+    tf32_operand_planes(views, 2, g.k, kp[0], s);
   } else {
     // each operand's split waits only for that operand
-    if (!PA) {
-      if ((ce = wait_operand(g, 0, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
-      tf32_operand_planes(&va, 1, g.k, kp, s);
-    }
-    if (!PB) {
-      if ((ce = wait_operand(g, 1, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
-      tf32_operand_planes(&vb, 1, g.k, kp, s);
+    for (int i = 0; i < 2; ++i) {
+      if (g.pk[i]) continue;
+      if ((ce = wait_operand(g, i, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
+      tf32_operand_planes(&views[i], 1, g.k, kp[i], s);
     }
   }
 
   CUtensorMap tmA, tmB, tmB_half;
-  {
-    uint64_t dims[3] = {(uint64_t)g.k, (uint64_t)g.m, 2};
-    uint64_t strides[2] = {(uint64_t)kpa * 4, (uint64_t)a_plane * 4};
-    uint32_t box[3] = {32, (uint32_t)sp::BM, 1};  // 128-byte k-blocks
-    int rc = encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, pa, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    uint64_t dimsb[3] = {(uint64_t)g.k, (uint64_t)g.n, 2};
-    uint64_t stridesb[2] = {(uint64_t)kpb * 4, (uint64_t)b_plane * 4};
-    uint32_t boxb[3] = {32, (uint32_t)sp::BN, 1};
-    rc = encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, pb, dimsb, stridesb, boxb, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    uint32_t boxh[3] = {32, (uint32_t)(sp::BN / 2), 1};  // one CTA's half of the B tile for the pair kernel
-    rc = encode_tiled(&tmB_half, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, pb, dimsb, stridesb, boxh,
-                      CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-  }
+  auto map = [&](CUtensorMap* m, int i, int64_t R, int box_rows) {
+    const uint64_t dims[3] = {(uint64_t)g.k, (uint64_t)R, 2};
+    const uint64_t strides[2] = {(uint64_t)kp[i] * 4, (uint64_t)plane[i] * 4};
+    const uint32_t box[3] = {32, (uint32_t)box_rows, 1};  // 128-byte k-blocks
+    return encode_tiled(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, planes[i], dims, strides, box,
+                        CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  int rc = map(&tmA, ia, rows, sp::BM);
+  if (!rc) rc = map(&tmB, ib, cols, sp::BN);
+  if (!rc) rc = map(&tmB_half, ib, cols, sp::BN / 2);  // one CTA's half of the B tile for the pair kernel
+  if (rc) return rc;
 
   sp::Params p;
   memset(&p, 0, sizeof(p));
-  p.m = g.m;
-  p.n = g.n;
+  p.m = rows;
+  p.n = cols;
   p.kelems = 32;
   p.kblocks = (int)ceil_div(g.k, 32);
-  p.tiles_m = (int)ceil_div(g.m, sp::BM);
-  p.tiles_n = (int)ceil_div(g.n, sp::BN);
+  p.tiles_m = (int)ceil_div(rows, sp::BM);
+  p.tiles_n = (int)ceil_div(cols, sp::BN);
   p.ngroups = 1;
   p.group_begin[0] = 0;
   p.group_begin[1] = 3;
   // small cross terms first, then hi*hi
-  p.pair_a[0] = 1; p.pair_b[0] = 0;  // A_lo * B_hi
-  p.pair_a[1] = 0; p.pair_b[1] = 1;  // A_hi * B_lo
+  p.pair_a[0] = !flip; p.pair_b[0] = flip;  // A_lo * B_hi
+  p.pair_a[1] = flip; p.pair_b[1] = !flip;  // A_hi * B_lo
   p.pair_a[2] = 0; p.pair_b[2] = 0;  // A_hi * B_hi
   // 256 k per tensor-core accumulation (8 k-blocks of one pair), then an RN
   // add in registers; chunks never span pairs
@@ -131,8 +135,8 @@ int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   p.alpha_f = (float)g.alpha;
   p.beta_f = (float)g.beta;
   p.c32 = static_cast<float*>(g.c.ptr);
-  p.rsc = g.c.rs;
-  p.csc = g.c.cs;
+  p.rsc = flip ? g.c.cs : g.c.rs;
+  p.csc = flip ? g.c.rs : g.c.cs;
   p.status = ds->status;
 
   // the epilogue reads C

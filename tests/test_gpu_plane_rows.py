@@ -1,5 +1,5 @@
-"""Row strides of the operand planes (whole 32-byte sectors, or 16 bytes under a scratch limit) change
-no result."""
+"""Row strides of the operand planes (whole 32-byte sectors, or 16 bytes under a scratch limit) and
+the tile roles of split TF32 change no result."""
 import ctypes
 
 import numpy as np
@@ -30,9 +30,9 @@ def test_row_strides_give_the_same_bits(gpu, mode, k):
     C0 = np.asfortranarray(C0)
     want = gu.gemm_device(gpu, A, B, C0, -1.0, 0.5, precision=prec, slices=s)
     ref, mag = ou.dd_gemm(A.astype(np.float64), B.astype(np.float64), C0.astype(np.float64), -1.0, 0.5)
-    # 4 slices: operands rounded at 2^-33 of a row's or column's maximum
-    tol = 2 * (k + 2) * 2.0**-24 * mag if dt == np.float32 else 2 * (k + 2) * 2.0**-53 * mag + k * 2.0 ** (1 - 8 * s)
-    assert np.all(np.abs(want - ref) <= tol)
+    if dt == np.float64:
+        # 4 slices: operands rounded at 2^-33 of a row's or column's maximum
+        assert np.all(np.abs(want - ref) <= 2 * (k + 2) * 2.0**-53 * mag + k * 2.0 ** (1 - 8 * s))
     # host operands under a budget that leaves the call no free scratch: 16-byte rows
     gpu.momms_set_staging_budget(300 << 20)
     try:
@@ -56,3 +56,21 @@ def test_row_strides_give_the_same_bits(gpu, mode, k):
         assert np.array_equal(tc.cpu().numpy(), want)
     finally:
         gpu.momms_packed_destroy(pack)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 3), (64, 1000, 40), (1000, 64, 40), (129, 257, 300), (513, 300, 1025)])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_tf32_bits_do_not_depend_on_the_order_of_c(gpu, shape, beta):
+    """C by rows runs as C^T = B^T A^T: the same products and sums, whatever C's strides."""
+    m, n, k = shape
+    A, B, C0 = _operands(np.random.default_rng(m + n + k), m, n, k, np.float32)
+    outs = []
+    for view in (np.zeros((n, m), np.float32).T, np.zeros((m, n + 3), np.float32)[:, :n],
+                 np.zeros((2 * m, 3 * n), np.float32)[::2, ::3], np.zeros((3 * n, 2 * m), np.float32).T[::2, ::3]):
+        view[...] = C0
+        outs.append(np.array(gu.gemm_device(gpu, A, B, view, 1.5, beta, precision=mg.PREC_SPLIT_TF32)))
+    ref, mag = ou.dd_gemm(A.astype(np.float64), B.astype(np.float64), C0.astype(np.float64), 1.5, beta)
+    # both operands' splits and the dropped lo*lo term: 3 * 2^-22 of each product
+    assert np.all(np.abs(outs[0] - ref) <= (2 * (k + 2) * 2.0**-24 + 3 * 2.0**-22) * mag)
+    for o in outs[1:]:
+        assert np.array_equal(o, outs[0])
