@@ -312,9 +312,10 @@ typedef struct {
   int32_t slices;         /* OZAKI: slice count used (chosen or given) */
   int32_t pairs;          /* OZAKI: slice products formed (tensor-core GEMMs) */
   int32_t groups;         /* OZAKI: accumulation groups */
-  int32_t splits;         /* plain paths: k splits */
+  int32_t splits;         /* plain paths and split TF32: k splits */
   int32_t slice_variant;  /* tensor-core paths: slice kernel variant run: 0 = one CTA per tile,
-                             2 = CTA pairs with one cta_group::2 MMA (1 is unused) */
+                             2 = CTA pairs with one cta_group::2 MMA, 3 = a cluster of
+                             CTAs per tile, each a range of k (1 is unused) */
   double bound_rel_err;   /* OZAKI with an automatic slice count: a rigorous bound on
                              max_ij |dC_ij| / (|A||B|)_ij of the product, over every entry (-1 otherwise) */
 } momms_call_info;

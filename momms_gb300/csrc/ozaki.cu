@@ -1966,7 +1966,7 @@ int ozaki_batch_launch(OzakiBatch* b, cudaStream_t s, int max_sms) {
   if (max_sms > 0) clusters = std::max(1, std::min(clusters, max_sms / 2));
   sp::GroupTable gt{b->d_params, b->d_maps, (int)b->probs.size(), b->units};
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = sp::cluster2_config(sp::pair_smem<sp::EPI_OZAKI>(), attr);
+  cudaLaunchConfig_t cfg = sp::cluster_config(2, sp::pair_smem<sp::EPI_OZAKI>(), attr);
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(b->units, clusters)));
   cfg.stream = s;
   cudaError_t e;

@@ -7,6 +7,7 @@
 // Markidis et al. 2018, Ootomo & Yokota 2022). The small cross terms are
 // accumulated first. The result stays inside the f32 componentwise bound
 // |dC| <= 2k u_32 (|A||B|) that the plain FFMA path meets.
+#include <algorithm>
 #include <cstdlib>
 
 #include "internal.h"
@@ -39,6 +40,31 @@ struct Tf32SplitOp {
     out[1] = make_uint2(__float_as_uint(l0), __float_as_uint(l1));
   }
 };
+
+int64_t tiles(int64_t rows, int64_t cols) { return ceil_div(rows, sp::BM) * ceil_div(cols, sp::BN); }
+
+// CTAs per tile where the tiles are fewer than the GPU has room for: the split
+// of k (1: none) whose waves end first, from 0.33 us per k-block of a pair and
+// 5 us per wave, 7 with the reduction. Measured (us, 1 / 2 / 4 / 8 CTAs, the
+// pair kernel for 1): 512^3 32 / 26 / 22 / 20; 1024^3 52 / 37 / 29 / 54;
+// 1500^3 73 / 54 / 62 / 101; 2048^3 102 / 114 / 127 / 189; 2560^3 212 / 200 /
+// 225 / 333; 64 x 64 x 4096 139 / 77 / 47 / 31.
+int split_ctas(int64_t m, int64_t n, int kblocks, int sms) {
+  const int64_t pairs = ceil_div(m, 2 * sp::BM) * ceil_div(n, sp::BN), units = std::min(tiles(m, n), tiles(n, m));
+  if (pairs > sms) return 1;
+  double best = 0.92 * (double)ceil_div(pairs, sms / 2) * (3 * 0.33 * kblocks + 5.0);
+  int ctas = 1;
+  for (int z = 2; z <= 8 && z <= kblocks; z *= 2) {
+    const int fit = sp::split_clusters<1>(z);
+    if (fit < 1) break;
+    const double t = (double)ceil_div(units, fit) * (3 * 0.33 * (double)ceil_div(kblocks, z) + 7.0);
+    if (t < best) {
+      best = t;
+      ctas = z;
+    }
+  }
+  return ctas;
+}
 }  // namespace
 
 int set_attrs_tf32() {
@@ -62,11 +88,17 @@ void tf32_operand_planes(const F32View* v, int count, int64_t K, int64_t kp, cud
 int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   DeviceState* ds = device_state();
   if (!ds) return MOMMS_ERR_NO_DEVICE;
+  // Few tiles: a cluster of CTAs per tile. The same split for every block of a
+  // streamed product and for either orientation, so that neither changes a bit.
+  const int kblocks = (int)ceil_div(g.k, 32);
+  const int ctas = split_ctas(g.whole_m ? g.whole_m : g.m, g.whole_n ? g.whole_n : g.n, kblocks, ds->sm_count);
   // The epilogue's lanes hold consecutive rows of the tile, so C is taken
   // transposed (C^T = B^T A^T) where its columns are the closer ones: 32-lane
   // stores of one line instead of 32 (6000 x 3001 x 4099, C by rows: 627 ->
-  // 543 us). Every product and the order of the sums stay the same.
-  const bool flip = std::llabs(g.c.cs) < std::llabs(g.c.rs);
+  // 543 us); a split product takes the orientation of fewer tiles. Every
+  // product and the order of the sums stay the same.
+  const int64_t fewer = ctas > 1 ? tiles(g.n, g.m) - tiles(g.m, g.n) : 0;
+  const bool flip = fewer ? fewer < 0 : std::llabs(g.c.cs) < std::llabs(g.c.rs);
   const int ia = flip ? 1 : 0, ib = 1 - ia;  // the operand (0 = A, 1 = B) that gives the tile's rows, columns
   const int64_t rows = flip ? g.n : g.m, cols = flip ? g.m : g.n;
   // packed operands (momms_pack) bring their planes
@@ -117,7 +149,7 @@ int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   p.m = rows;
   p.n = cols;
   p.kelems = 32;
-  p.kblocks = (int)ceil_div(g.k, 32);
+  p.kblocks = kblocks;
   p.tiles_m = (int)ceil_div(rows, sp::BM);
   p.tiles_n = (int)ceil_div(cols, sp::BN);
   p.ngroups = 1;
@@ -143,8 +175,10 @@ int launch_sgemm_tf32x3(const DevGemm& g, cudaStream_t s) {
   if ((ce = wait_operand(g, 2, s)) != cudaSuccess) return cuda_fail(ce, "operand staging");
   {
     KernelTimer kt(MOMMS_KERNEL_SLICE_TF32, s);
-    int variant = 0;
-    ce = sp::launch_slice<1, sp::EPI_F32>(tmA, tmB, tmB_half, p, ds->sm_count, s, &variant);
+    int variant = sp::SLICE_SPLIT;
+    call_info().splits = ctas;
+    if (ctas > 1) ce = sp::launch_slice_split<1>(tmA, tmB, p, ctas, s);
+    else ce = sp::launch_slice<1, sp::EPI_F32>(tmA, tmB, tmB_half, p, ds->sm_count, s, &variant);
     if (ce != cudaSuccess) return cuda_fail(ce, "split-TF32 slice launch");
     call_info().slice_variant = variant;
   }

@@ -475,7 +475,43 @@ __device__ __forceinline__ bool float_groups(const Params& p, int g0, int g1, in
   return true;
 }
 
-template <int KIND, int EPI>
+// C's columns [c0, c1) of a tile from the sums of the cluster's CTAs (each
+// BM x BN by columns at `part` of its shared memory), added in rank order.
+// A warp takes one column at a time, a lane four of its rows.
+__device__ __forceinline__ void reduce_columns(const Params& p, const float* part, int64_t row0, int64_t col0, int c0,
+                                               int c1, int ranks, int warp, int lane) {
+  const int64_t row = row0 + lane * 4;
+  const int rows = (int)min((int64_t)4, p.m - row);
+  for (int c = c0 + warp; c < c1; c += THREADS / 32) {
+    if (col0 + c >= p.n) break;
+    float* cp = p.c32 + row * p.rsc + (col0 + c) * p.csc;
+    float old[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (p.beta_f != 0.0f) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q < rows) old[q] = cp[q * p.rsc];
+    }
+    const float* src = part + c * BM + lane * 4;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int r = 0; r < ranks; ++r) {
+      const float4 w = ld_cluster_f4(mapa_shared(src, (uint32_t)r));
+      v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
+    }
+    const float out[4] = {v.x * p.alpha_f, v.y * p.alpha_f, v.z * p.alpha_f, v.w * p.alpha_f};
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q < rows) cp[q * p.rsc] = p.beta_f == 0.0f ? out[q] : fmaf(p.beta_f, old[q], out[q]);
+  }
+}
+
+// Split (EPI_F32, few tiles): a cluster of CTAs per tile, each with a range of
+// the k-blocks of every pair. Each CTA leaves its sums in shared memory, and
+// reduces a range of the tile's columns over the cluster, in rank order. One
+// CTA's chain of MMAs bounds such a product (0.33 us per k-block of a pair):
+// split-TF32 1024 x 1024 x 1024 52 -> 29 us as 4 CTAs per tile. The exchange
+// through the cluster's shared memory needs no scratch and no second kernel.
+template <int KIND, int EPI, bool SPLIT = false>
 __global__ void __launch_bounds__(THREADS, 1)
     slice_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ Params p) {
@@ -491,8 +527,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // work units: output tiles (times group chunks), one CTA each
-  const int64_t unit0 = (int64_t)blockIdx.x;
-  const int64_t unit_step = (int64_t)gridDim.x;
+  const int64_t unit0 = SPLIT ? (int64_t)cluster_id_x() : (int64_t)blockIdx.x;
+  const int64_t unit_step = SPLIT ? (int64_t)cluster_count_x() : (int64_t)gridDim.x;
+  const int rank = SPLIT ? (int)cluster_ctarank() : 0, ranks = SPLIT ? (int)cluster_nctarank() : 1;
+  const int kb0 = p.kblocks * rank / ranks, kb1 = p.kblocks * (rank + 1) / ranks;
   const int units_m = p.tiles_m;
   // work unit t: tile (pair) t % tile_units, groups [g_begin(t), g_end(t)) -
   // group-major, so that units in flight read the same digit planes
@@ -547,7 +585,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         coords(t % tile_units, tm, tn);
         for (int g = g_begin(t); g < g_end(t); ++g) {
           for (int pi = p.group_begin[g]; pi < p.group_begin[g + 1]; ++pi) {
-            for (int kb = 0; kb < p.kblocks; ++kb) {
+            for (int kb = kb0; kb < kb1; ++kb) {
               if (!mbar_wait_bounded(&empty[stage], ph ^ 1)) {
                 report_status(p.status, DEV_TIMEOUT_EMPTY);
                 *abort_flag = 1;
@@ -595,7 +633,7 @@ __global__ void __launch_bounds__(THREADS, 1)
               buf ^= 1;
               open = false;
             }
-            for (int st = 0; st < p.kblocks;) {
+            for (int st = kb0; st < kb1;) {
               if (open && load + w > p.chunk_cap) {
                 tc::commit(&tfull[buf]);
                 acc_ph[buf] ^= 1;
@@ -615,7 +653,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 open = fresh = true;
               }
               // the k-blocks of this pair that still fit in the open chunk
-              const int s0 = st, s1 = min(p.kblocks, st + (p.chunk_cap - load) / w);
+              const int s0 = st, s1 = min(kb1, st + (p.chunk_cap - load) / w);
               for (; st < s1; ++st) {
                 if (!mbar_wait_bounded(&full[stage], ph)) {
                   report_status(p.status, DEV_TIMEOUT_FULL);
@@ -669,7 +707,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       coords(t % tile_units, tm, tn);
       const int64_t row = (int64_t)tm * BM + r_local;
       const int64_t col0 = (int64_t)tn * BN + h * EPI_COLS;
-      if (EPI == EPI_F32) prefetch_c_rows<EPI_COLS>(p, (int64_t)tm * BM + q * 32, col0, lane);
+      if (EPI == EPI_F32 && !SPLIT) prefetch_c_rows<EPI_COLS>(p, (int64_t)tm * BM + q * 32, col0, lane);
       // the next finished chunk's TMEM address (~0: timed out), and its release
       auto wait = [&]() -> uint32_t {
         if (!mbar_wait_bounded(&tfull[buf], acc_ph[buf])) {
@@ -687,7 +725,22 @@ __global__ void __launch_bounds__(THREADS, 1)
         acc_ph[buf] ^= 1;
         buf ^= 1;
       };
-      if constexpr (EPI == EPI_OZAKI) {
+      if constexpr (SPLIT) {
+        // one unit per cluster; the stages are free once its chunks are done
+        float S[EPI_COLS];
+#pragma unroll
+        for (int j = 0; j < EPI_COLS; ++j) S[j] = 0.0f;
+        const int chunks = p.group_begin[1] * ((kb1 - kb0 + p.chunk_cap - 1) / p.chunk_cap);
+        for (int c = 0; c < chunks; ++c) {
+          const uint32_t taddr = wait();
+          if (taddr == ~0u) goto epi_done;
+          drain_chunk<EPI, EPI_COLS>(taddr, S);
+          release();
+        }
+        float* part = reinterpret_cast<float*>(smem) + h * EPI_COLS * BM + r_local;
+#pragma unroll
+        for (int j = 0; j < EPI_COLS; ++j) part[j * BM] = S[j];
+      } else if constexpr (EPI == EPI_OZAKI) {
         if (!ozaki_groups<EPI_COLS>(p, g_begin(t), g_end(t), row, col0, tm, tn, h * EPI_COLS, r_local, wait, release))
           goto epi_done;
       } else {
@@ -700,6 +753,14 @@ __global__ void __launch_bounds__(THREADS, 1)
   // reconverge each warp (its lane 0 may have run a role loop alone) before
   // the CTA-wide barrier, which requires whole warps
   __syncwarp();
+  if constexpr (SPLIT) {
+    cluster_sync();  // every CTA's sums are in place
+    int tm, tn;
+    coords(unit0, tm, tn);
+    reduce_columns(p, reinterpret_cast<const float*>(smem), (int64_t)tm * BM, (int64_t)tn * BN, BN * rank / ranks,
+                   BN * (rank + 1) / ranks, ranks, warp, lane);
+    cluster_sync();  // before any of them is gone
+  }
   tc::fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -1052,6 +1113,10 @@ inline cudaError_t set_slice_attrs() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(slice_gemm_pair_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              pair_smem<EPI>());
+  if constexpr (EPI == EPI_F32)
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(slice_gemm_kernel<KIND, EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               SMEM_BYTES);
   if (e == cudaSuccess && EPI == EPI_OZAKI)
     e = cudaFuncSetAttribute(slice_gemm_pair_kernel<KIND, EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              pair_smem<EPI>());
@@ -1059,16 +1124,17 @@ inline cudaError_t set_slice_attrs() {
 }
 
 // Kernel variants: 0 = one CTA per tile, 2 = CTA pairs with cta_group::2 MMA
+// 3 = a cluster of CTAs per tile, each a range of k
 // (1 is not used: it was a cluster kernel sharing B tiles by multicast loads).
-enum { SLICE_SINGLE = 0, SLICE_PAIR = 2 };
+enum { SLICE_SINGLE = 0, SLICE_PAIR = 2, SLICE_SPLIT = 3 };
 
-inline cudaLaunchConfig_t cluster2_config(int smem, cudaLaunchAttribute* attr) {
+inline cudaLaunchConfig_t cluster_config(int ctas, int smem, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2);
+  cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = (size_t)smem;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = (unsigned)ctas;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -1093,7 +1159,7 @@ inline int slice_variant(int* clusters) {
     int v = SLICE_SINGLE, n = 0;
     if (want_pair) {
       cudaLaunchAttribute attr[1];
-      cudaLaunchConfig_t cfg = cluster2_config(pair_smem<EPI>(), attr);
+      cudaLaunchConfig_t cfg = cluster_config(2, pair_smem<EPI>(), attr);
       int c = 0;
       if (cudaOccupancyMaxActiveClusters(&c, (const void*)slice_gemm_pair_kernel<KIND, EPI>, &cfg) != cudaSuccess) {
         cudaGetLastError();
@@ -1110,6 +1176,38 @@ inline int slice_variant(int* clusters) {
   }
   *clusters = cache_n[dev].load();
   return cache_v[dev].load();
+}
+
+// How many clusters of `ctas` of the split kernel fit the current device at
+// once; queried once per device and size (0: none).
+template <int KIND>
+inline int split_clusters(int ctas) {
+  static std::atomic<int> cache[64][4];  // the count + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::atomic<int>& c = cache[dev][ctas == 8 ? 3 : ctas / 2];
+  int n = c.load();
+  if (!n) {
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = cluster_config(ctas, SMEM_BYTES, attr);
+    if (cudaOccupancyMaxActiveClusters(&n, (const void*)slice_gemm_kernel<KIND, EPI_F32, true>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    c.store(++n);
+  }
+  return n - 1;
+}
+
+// The split kernel: clusters of `ctas`, one per tile.
+template <int KIND>
+inline cudaError_t launch_slice_split(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& p, int ctas,
+                                      cudaStream_t s) {
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = cluster_config(ctas, SMEM_BYTES, attr);
+  cfg.gridDim = dim3((unsigned)((int64_t)p.tiles_m * p.tiles_n * ctas));
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, slice_gemm_kernel<KIND, EPI_F32, true>, tmA, tmB, p);
 }
 
 // Launches the slice kernel. The pair kernel needs at least two m-tiles (its
@@ -1168,7 +1266,7 @@ inline cudaError_t launch_slice(const CUtensorMap& tmA, const CUtensorMap& tmB_f
   const int64_t units = tile_units * ((p.ngroups + q.gchunk - 1) / q.gchunk);
   if (v == SLICE_PAIR) {
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = cluster2_config(pair_smem<EPI>(), attr);
+    cudaLaunchConfig_t cfg = cluster_config(2, pair_smem<EPI>(), attr);
     cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(units, clusters)));
     cfg.stream = s;
     return cudaLaunchKernelEx(&cfg, slice_gemm_pair_kernel<KIND, EPI>, tmA, tmB_half, q, GroupTable{});

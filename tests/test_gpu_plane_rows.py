@@ -74,3 +74,16 @@ def test_tf32_bits_do_not_depend_on_the_order_of_c(gpu, shape, beta):
     assert np.all(np.abs(outs[0] - ref) <= (2 * (k + 2) * 2.0**-24 + 3 * 2.0**-22) * mag)
     for o in outs[1:]:
         assert np.array_equal(o, outs[0])
+
+
+# one and several CTAs per tile (k-blocks of 32 dealt unevenly), tiles of a few rows and columns
+@pytest.mark.parametrize("shape", [(1, 1, 33), (3, 5, 300), (130, 258, 4099), (513, 511, 257), (700, 700, 333),
+                                   (1500, 1400, 700), (2300, 2100, 100)])
+@pytest.mark.parametrize("order", ["F", "C"])
+def test_tf32_split_over_a_cluster(gpu, shape, order):
+    m, n, k = shape
+    A, B, C0 = _operands(np.random.default_rng(m + k), m, n, k, np.float32)
+    C = gu.gemm_device(gpu, A, B, np.array(C0, order=order), -1.0, 1.0, precision=mg.PREC_SPLIT_TF32)
+    rows = np.unique(np.linspace(0, m - 1, 40).astype(int))
+    ref, mag = ou.dd_gemm(A[rows].astype(np.float64), B.astype(np.float64), C0[rows].astype(np.float64), -1.0, 1.0)
+    assert np.all(np.abs(C[rows] - ref) <= (2 * (k + 2) * 2.0**-24 + 3 * 2.0**-22) * mag)
