@@ -107,6 +107,13 @@ __host__ __device__ __forceinline__ float remainder_of(float t, float p, float i
   return fma_f(-q, p, t);
 }
 
+// Digits (|d| <= 128) taken in pairs d + 256 d' (|.| <= 32896) for the residue of
+// a number of ns digits: as many as keep the sum of pairs and digits times
+// 2^(8 i) mod p (at most 127 in magnitude; modulo 256 zero from i = 1 on) within
+// 2^24: four pairs above the first reach 16.74 of 16.78 million, five would not,
+// and nor would four and three or more single digits.
+constexpr int pairs_of_digits(int ns) { return ns <= 10 ? ns / 2 : 4; }
+
 template <int L>
 __host__ __device__ __forceinline__ float residue_of_limbs(const float (&f)[L], const Modulus& m) {
   float t = f[0];

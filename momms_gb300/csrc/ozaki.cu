@@ -809,7 +809,8 @@ int crt_moduli(int ns, double sum) {
 //    all of k: what decides for few tiles), and per group and entry what of
 //    the epilogue they do not hide: 0.53 ps (digits: 4 bytes of plane), 0.2 ps;
 //  * recombination 7.4 ps per entry (7 digit groups), 10.4 ps (16 moduli);
-//  * operand planes 2 bytes per slice or modulus, 8 read, at 6 TB/s.
+//  * operand planes 2 bytes per slice or modulus, 8 read, at 6 TB/s;
+//  * 3 us for the launch that packed operands need only for residues.
 // Both forms, 7 slices, ms per call: 8192 x 8192 x 128 1.33 (digits) and 1.40,
 // x 256 1.61 and 1.56, x 1024 3.17 and 2.48, x 8192 20.9 and 13.1; 65536 x 256 x
 // 256 0.64 and 0.75; the slice kernel alone at 512^3 0.030 and 0.014.
@@ -818,13 +819,13 @@ bool crt_applies(int ns, int64_t m, int64_t n, int64_t k) {
   const int N = crt_moduli(ns, k);
   Schedule sc;
   if (!ozaki_schedule(ns, k, &sc)) return true;
-  constexpr double kPairs = 76.0, kStep = 0.26e6;  // ps
+  constexpr double kPairs = 76.0, kStep = 0.26e6, kPackedPass = 3e6;  // ps
   const double mn = (double)m * n, ops = (double)(m + n) * k;
   const double tiles = (double)(ceil_div(m, 256) * ceil_div(n, 256)), steps = (double)ceil_div(k, 64) * kStep;
   auto products = [&](double pairs, double longest) { return steps * std::max(pairs * tiles / kPairs, longest); };
   const double digits = products(sc.np, ns) + mn * (0.53 * sc.ng + 2.7 + 0.67 * sc.ng) + ops * (8 + 2 * ns) / 6.0;
   const double residues = products(N, 1.0) + mn * (0.2 * N + 0.65 * N) + ops * (8 + 2 * N) / 6.0;
-  return residues < digits;
+  return residues + kPackedPass < digits;
 }
 
 // Scratch of an emulated product, operand planes and group planes: the digit
@@ -850,7 +851,7 @@ int crt_per_pass(int ns, int N, int64_t m, int64_t n, int64_t k, bool tight) {
   return (int)ceil_div(N, passes);
 }
 
-// Residue planes l0..l1-1 of the sides, or of a packed operand's digits.
+// Residue planes l0..l1-1 of the sides, or of packed operands' digits.
 void crt_planes(int ns, const Side* sides, int count, int64_t K, __half* const* out, int64_t ldp,
                 const int64_t* plane_elems, bool from_max, int l0, int l1, cudaStream_t s) {
   KernelTimer kt(MOMMS_KERNEL_PREP, s);
@@ -872,12 +873,22 @@ void crt_planes(int ns, const Side* sides, int count, int64_t K, __half* const* 
     default: refuse_launch(cudaErrorInvalidValue);
   }
 }
-void crt_planes_of_pack(const PackedOperand& P, int64_t R, __half* out, int l0, int l1, int sm_count, cudaStream_t s) {
+void crt_planes_of_packs(const PackedOperand* const* P, const int64_t* R, __half* const* out, int l0, int l1,
+                         int sm_count, cudaStream_t s) {
+  crt::PackedDigits v{};
+  int count = 0, ns = 0;
+  for (int i = 0; i < 2; ++i) {
+    if (!P[i]) continue;
+    v.digits[count] = static_cast<const __half*>(P[i]->planes);
+    v.elems[count] = R[i] * P[i]->kp;
+    v.out[count++] = out[i];
+    ns = P[i]->np;
+  }
+  if (!count) return;
   KernelTimer kt(MOMMS_KERNEL_PREP, s);
-  const __half* d = static_cast<const __half*>(P.planes);
-  switch (P.np) {
+  switch (ns) {
 #define X(NS) \
-  case NS: crt::launch_residues_of_digits<NS>(d, R * P.kp, out, l0, l1, sm_count, s); break;
+  case NS: crt::launch_residues_of_digits<NS>(v, count, l0, l1, sm_count, s); break;
     MOMMS_CRT_NS(X)
 #undef X
     default: refuse_launch(cudaErrorInvalidValue);
@@ -1421,10 +1432,14 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
 
   // row maxima, bound sums and exponents of the unpacked operands
   void* ebuf = nullptr;
-  if ((ce = scratch_alloc(&ebuf, row_work_bytes(m, n), s)) != cudaSuccess) return cuda_fail(ce, "Ozaki exponents");
+  RowWork rw{};
+  if (!PA || !PB) {
+    if ((ce = scratch_alloc(&ebuf, row_work_bytes(m, n), s)) != cudaSuccess) return cuda_fail(ce, "Ozaki exponents");
+    rw = row_work_carve(ebuf, m, n);
+  }
   ScratchGuard free_ebuf(ebuf, s);
-  const RowWork rw = row_work_carve(ebuf, m, n);
-  if ((ce = cudaMemsetAsync(ebuf, 0, row_work_zero_bytes(m, n), s)) != cudaSuccess) return cuda_fail(ce, "Ozaki exponents");
+  if (ebuf && (ce = cudaMemsetAsync(ebuf, 0, row_work_zero_bytes(m, n), s)) != cudaSuccess)
+    return cuda_fail(ce, "Ozaki exponents");
   const double* A = static_cast<const double*>(g.a.ptr);
   const double* B = static_cast<const double*>(g.b.ptr);
   const Side sides[2] = {side_a(g, rw.maxbits, rw.exps), side_b(g, rw.maxbits + m, rw.exps + m)};
@@ -1571,8 +1586,9 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     const int64_t pes[2] = {(int64_t)a_plane, (int64_t)b_plane};
     const int first = PA ? 1 : 0, count = (PA ? 0 : 1) + (together ? 1 : 0);
     if (crt) {
-      if (PA) crt_planes_of_pack(*PA, m, outs[0], l0, l1, ds->sm_count, s);
-      if (PB) crt_planes_of_pack(*PB, n, outs[1], l0, l1, ds->sm_count, s);
+      const PackedOperand* const packs[2] = {PA, PB};
+      const int64_t rows[2] = {m, n};
+      crt_planes_of_packs(packs, rows, outs, l0, l1, ds->sm_count, s);
       if (count) crt_planes(ns, sides + first, count, k, outs + first, kp, pes + first, from_max, l0, l1, s);
       crt_slice_params(m, k, l0, l1, &p);
     } else if (count) {

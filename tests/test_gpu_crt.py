@@ -72,3 +72,44 @@ def test_passes_and_packs_give_the_same_bits(gpu):
         mg.check(gpu.momms_packed_destroy(h), gpu)
     bits = ctypes.c_uint32(0)
     assert gpu.momms_device_status(ctypes.byref(bits)) == mg.OK and bits.value == 0
+
+
+@pytest.mark.parametrize("s", [5, 7, 9, 10, 11, 15])
+def test_residues_of_packed_digits(gpu, s):
+    """Digits are combined in pairs before they meet the moduli: the bits of the plain call, with
+    entries whose digits are all at either end of their range among them."""
+    m, n, k = 520, 700, 333
+    rng = np.random.default_rng(s)
+    ends = np.array([sum(d * 256.0 ** -(i + 1) for i in range(6)) for d in (127, 128, -127, -128)])
+    ops = []
+    for shape in ((m, k), (k, n)):
+        x = rng.uniform(-1, 1, shape) * 0.49
+        x[rng.uniform(size=shape) < 0.3] = rng.choice(ends)
+        ops.append(np.asfortranarray(x))
+    A, B = ops
+    want, info = _call(gpu, A, B, np.zeros((m, n), order="F"), s)
+    assert info.pairs < s * (s + 1) // 2 or s == 5
+    packs = []
+    for role, x in ((mg.ROLE_A, A), (mg.ROLE_B, B)):
+        t, rs, cs = gu.to_device(x)
+        h = ctypes.c_void_p()
+        mg.check(gpu.momms_pack(mg.DTYPE_F64, mg.PREC_OZAKI, role, x.shape[0], x.shape[1],
+                                ctypes.byref(mg.Operand(t.data_ptr(), rs, cs, mg.MEM_DEVICE, 0)), s, None,
+                                ctypes.byref(h)), gpu)
+        packs.append(h)
+    try:
+        for use in ((True, True), (True, False), (False, True)):
+            tc, crs, ccs = gu.to_device(np.zeros((m, n), order="F"))
+            dev = [gu.to_device(x) for x in (A, B)]
+            d = gu.make_desc(mg.DTYPE_F64, m, n, k, 1.0, 0.0, (dev[0][0].data_ptr(),) + dev[0][1:],
+                             (dev[1][0].data_ptr(),) + dev[1][1:], (tc.data_ptr(), crs, ccs),
+                             precision=mg.PREC_OZAKI, slices=s)
+            if use[0]:
+                d.a = mg.Operand(packs[0].value, 0, 0, mg.MEM_PACKED, 0)
+            if use[1]:
+                d.b = mg.Operand(packs[1].value, 0, 0, mg.MEM_PACKED, 0)
+            mg.check(gpu.momms_gemm(ctypes.byref(d), None), gpu)
+            assert np.array_equal(tc.cpu().numpy(), want)
+    finally:
+        for h in packs:
+            gpu.momms_packed_destroy(h)
