@@ -97,6 +97,8 @@ struct PackedDigits {
 template <int NS>
 __global__ void __launch_bounds__(256)
     residues_of_digits_kernel(const __grid_constant__ PackedDigits P, int l0, int l1) {
+  dependency_wait();
+  dependents_may_start();
   const __half* __restrict__ digits = P.digits[blockIdx.y];
   __half* __restrict__ out = P.out[blockIdx.y];
   const int64_t elems = P.elems[blockIdx.y];
@@ -145,7 +147,7 @@ template <int NS>
 void launch_residues_of_digits(const PackedDigits& p, int count, int l0, int l1, int sm_count, cudaStream_t s) {
   const int64_t most = count > 1 ? (p.elems[0] > p.elems[1] ? p.elems[0] : p.elems[1]) : p.elems[0];
   const int64_t blocks = std::min<int64_t>(ceil_div_dev(most / 8, 256), (int64_t)sm_count * 8);
-  residues_of_digits_kernel<NS><<<dim3((unsigned)blocks, (unsigned)count), 256, 0, s>>>(p, l0, l1);
+  launch_dependent(residues_of_digits_kernel<NS>, dim3((unsigned)blocks, (unsigned)count), 256, 0, s, p, l0, l1);
 }
 
 struct CombineParams {
@@ -173,6 +175,7 @@ struct CombineParams {
 // 342 instructions per entry and 1.32 ms at 8192^2 with 16 moduli).
 template <int NW, int N>
 __global__ void __launch_bounds__(256, NW == 4 ? 4 : (NW <= 6 ? 3 : 2)) combine_kernel(const __grid_constant__ CombineParams p) {
+  dependency_wait();
   const int64_t row = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (row >= p.m) return;
   const int er = p.row_exp[row];

@@ -50,6 +50,7 @@ struct One {
 __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
     dgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ Params p) {
+  dependency_wait_few();
   dgemm_body(One{p, &tmA, &tmB}, p.next, p.status);
 }
 
@@ -161,7 +162,7 @@ int launch_dgemm_dmma(const DevGemm& g, cudaStream_t s) {
   const int grid = (int)std::min<int64_t>(plan.units(), slots);
   {
     KernelTimer kt(MOMMS_KERNEL_DGEMM_DMMA, s);
-    dgemm_kernel<<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, p);
+    launch_dependent(dgemm_kernel, dim3((unsigned)grid), THREADS, SMEM_BYTES, s, tmA, tmB, p);
   }
   note_launch();
   ce = launch_status();

@@ -471,6 +471,7 @@ __global__ void __launch_bounds__(256, WIDE ? 2 : 4) combine_kernel(const __grid
   // group sums whose loads are issued together: NS, else every group of up
   // to 8 (narrow) or 16 (wide) groups
   constexpr int kBatch = NS > 0 ? NS : (WIDE ? 16 : 8);
+  dependency_wait();
   int64_t rows[2], roff[2];
   int er[2];
 #pragma unroll
@@ -760,23 +761,23 @@ int launch_combine(CombineParams cp, int64_t j0, int64_t j1, int sm_count, cudaS
     KernelTimer kt(MOMMS_KERNEL_COMBINE, Y);
     const dim3 grid((unsigned)bx, (unsigned)by);
     switch (cp.levels ? cp.levels : (cp.wide ? -1 : 0)) {
-      case -1: combine_kernel<true, 0><<<grid, 256, 0, Y>>>(cp); break;
-      case 13: combine_kernel<true, 13><<<grid, 256, 0, Y>>>(cp); break;
-      case 14: combine_kernel<true, 14><<<grid, 256, 0, Y>>>(cp); break;
-      case 15: combine_kernel<true, 15><<<grid, 256, 0, Y>>>(cp); break;
-      case 1: combine_kernel<false, 1><<<grid, 256, 0, Y>>>(cp); break;
-      case 2: combine_kernel<false, 2><<<grid, 256, 0, Y>>>(cp); break;
-      case 3: combine_kernel<false, 3><<<grid, 256, 0, Y>>>(cp); break;
-      case 4: combine_kernel<false, 4><<<grid, 256, 0, Y>>>(cp); break;
-      case 5: combine_kernel<false, 5><<<grid, 256, 0, Y>>>(cp); break;
-      case 6: combine_kernel<false, 6><<<grid, 256, 0, Y>>>(cp); break;
-      case 7: combine_kernel<false, 7><<<grid, 256, 0, Y>>>(cp); break;
-      case 8: combine_kernel<false, 8><<<grid, 256, 0, Y>>>(cp); break;
-      case 9: combine_kernel<false, 9><<<grid, 256, 0, Y>>>(cp); break;
-      case 10: combine_kernel<false, 10><<<grid, 256, 0, Y>>>(cp); break;
-      case 11: combine_kernel<false, 11><<<grid, 256, 0, Y>>>(cp); break;
-      case 12: combine_kernel<false, 12><<<grid, 256, 0, Y>>>(cp); break;
-      default: combine_kernel<false, 0><<<grid, 256, 0, Y>>>(cp); break;
+      case -1: launch_dependent(combine_kernel<true, 0>, grid, 256, 0, Y, cp); break;
+      case 13: launch_dependent(combine_kernel<true, 13>, grid, 256, 0, Y, cp); break;
+      case 14: launch_dependent(combine_kernel<true, 14>, grid, 256, 0, Y, cp); break;
+      case 15: launch_dependent(combine_kernel<true, 15>, grid, 256, 0, Y, cp); break;
+      case 1: launch_dependent(combine_kernel<false, 1>, grid, 256, 0, Y, cp); break;
+      case 2: launch_dependent(combine_kernel<false, 2>, grid, 256, 0, Y, cp); break;
+      case 3: launch_dependent(combine_kernel<false, 3>, grid, 256, 0, Y, cp); break;
+      case 4: launch_dependent(combine_kernel<false, 4>, grid, 256, 0, Y, cp); break;
+      case 5: launch_dependent(combine_kernel<false, 5>, grid, 256, 0, Y, cp); break;
+      case 6: launch_dependent(combine_kernel<false, 6>, grid, 256, 0, Y, cp); break;
+      case 7: launch_dependent(combine_kernel<false, 7>, grid, 256, 0, Y, cp); break;
+      case 8: launch_dependent(combine_kernel<false, 8>, grid, 256, 0, Y, cp); break;
+      case 9: launch_dependent(combine_kernel<false, 9>, grid, 256, 0, Y, cp); break;
+      case 10: launch_dependent(combine_kernel<false, 10>, grid, 256, 0, Y, cp); break;
+      case 11: launch_dependent(combine_kernel<false, 11>, grid, 256, 0, Y, cp); break;
+      case 12: launch_dependent(combine_kernel<false, 12>, grid, 256, 0, Y, cp); break;
+      default: launch_dependent(combine_kernel<false, 0>, grid, 256, 0, Y, cp); break;
     }
   }
   note_launch();
@@ -957,7 +958,7 @@ int launch_crt_combine(crt::CombineParams& cp, int ns, int64_t j0, int64_t j1, i
     const dim3 grid((unsigned)bx, (unsigned)by);
     // the moduli that ns slices take for k from kCrtMinK to kMaxK
     switch (ns * 100 + cp.moduli) {
-#define X(NS, N) case NS * 100 + N: crt::combine_kernel<crt::words_of(NS), N><<<grid, 256, 0, Y>>>(cp); break;
+#define X(NS, N) case NS * 100 + N: launch_dependent(crt::combine_kernel<crt::words_of(NS), N>, grid, 256, 0, Y, cp); break;
       X(5, 12) X(5, 13) X(6, 14) X(6, 15) X(7, 16) X(7, 17) X(8, 18) X(8, 19) X(9, 20) X(9, 21) X(10, 22) X(10, 23)
       X(11, 24) X(11, 25) X(11, 26) X(12, 27) X(12, 28) X(13, 29) X(13, 30) X(14, 31) X(14, 32) X(14, 33) X(15, 34)
       X(15, 35)
@@ -1981,7 +1982,7 @@ int ozaki_batch_launch(OzakiBatch* b, cudaStream_t s, int max_sms) {
     return fail(MOMMS_ERR_UNSUPPORTED, "grouped emulated launches need CTA pairs on this device");
   if (max_sms > 0) clusters = std::max(1, std::min(clusters, max_sms / 2));
   sp::GroupTable gt{b->d_params, b->d_maps, (int)b->probs.size(), b->units};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = sp::cluster_config(2, sp::pair_smem<sp::EPI_OZAKI>(), attr);
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(b->units, clusters)));
   cfg.stream = s;

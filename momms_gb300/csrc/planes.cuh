@@ -137,6 +137,8 @@ struct Views {
 template <typename Body>
 __global__ void __launch_bounds__(THREADS) views_kernel(const __grid_constant__ Views<typename Body::Tin> vs,
                                                         const __grid_constant__ Body body) {
+  dependency_wait();
+  dependents_may_start();
   const unsigned first = vs.v[0].nx * vs.v[0].ny;
   const int z = blockIdx.x >= first ? 1 : 0;
   const View<typename Body::Tin>& v = vs.v[z];
@@ -151,6 +153,8 @@ __global__ void __launch_bounds__(THREADS) views_kernel(const __grid_constant__ 
 template <typename Body, bool R_CONTIG>
 __global__ void __launch_bounds__(THREADS) view_kernel(const __grid_constant__ View<typename Body::Tin> v, int z,
                                                        const __grid_constant__ Body body) {
+  dependency_wait();
+  dependents_may_start();
   body.template run<R_CONTIG>(v, z, BlockPlace{blockIdx.x % v.nx, blockIdx.x / v.nx, v.ny});
 }
 __host__ __device__ constexpr int run_rows(int lg) { return (THREADS / 32) << (5 - lg); }
@@ -262,13 +266,12 @@ int launch_views(Views<typename Body::Tin> vs, int count, const Body& body, cuda
     grid += v.nx * v.ny;
   }
   if (blocks < kFewBlocks && count > 1) {
-    views_kernel<Body><<<grid, THREADS, 0, s>>>(vs, body);
+    launch_dependent(views_kernel<Body>, dim3(grid), THREADS, 0, s, vs, body);
     return 1;
   }
   for (int i = 0; i < count; ++i) {
     const View<typename Body::Tin>& v = vs.v[i];
-    if (v.r_contig) view_kernel<Body, true><<<v.nx * v.ny, THREADS, 0, s>>>(v, i, body);
-    else view_kernel<Body, false><<<v.nx * v.ny, THREADS, 0, s>>>(v, i, body);
+    launch_dependent(v.r_contig ? view_kernel<Body, true> : view_kernel<Body, false>, dim3(v.nx * v.ny), THREADS, 0, s, v, i, body);
   }
   return count;
 }

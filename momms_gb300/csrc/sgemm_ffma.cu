@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(Tile<TM>::THREADS, Tile<TM>::CTAS_PER_SM)
     sgemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ float4 ffma_smem[];
   __shared__ int s_last;
+  dependency_wait_few();
   const Operands& o = p.o;
   const int64_t units = p.sched.units();
   for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(Small::THREADS, Small::CTAS_PER_SM)
     sgemm_small_kernel(const __grid_constant__ Params p) {
   extern __shared__ float4 ffma_smem[];
   __shared__ int s_last;
+  dependency_wait_few();
   const int64_t units = p.sched.units();
   for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
     int tm, tn, sp;
@@ -175,11 +177,13 @@ int sgemm_ffma_impl(const DevGemm& g0, cudaStream_t s, void* (&scratch)[3]) {
     if (small) {
       static const Kern kSmall[2][2] = {{sgemm_small_kernel<false, false>, sgemm_small_kernel<false, true>},
                                         {sgemm_small_kernel<true, false>, sgemm_small_kernel<true, true>}};
-      kSmall[a_xc][b_xc]<<<grid, Small::THREADS, Small::SMEM_BYTES, s>>>(p);
+      launch_dependent(kSmall[a_xc][b_xc], dim3((unsigned)grid), Small::THREADS, Small::SMEM_BYTES, s, p);
     } else if (cfg.tile == 1)
-      kernel_table<64>()[a_xc][b_xc][li][si]<<<grid, Tile<64>::THREADS, Tile<64>::SMEM_BYTES, s>>>(p);
+      launch_dependent(kernel_table<64>()[a_xc][b_xc][li][si], dim3((unsigned)grid), Tile<64>::THREADS,
+                       Tile<64>::SMEM_BYTES, s, p);
     else
-      kernel_table<128>()[a_xc][b_xc][li][si]<<<grid, Tile<128>::THREADS, Tile<128>::SMEM_BYTES, s>>>(p);
+      launch_dependent(kernel_table<128>()[a_xc][b_xc][li][si], dim3((unsigned)grid), Tile<128>::THREADS,
+                       Tile<128>::SMEM_BYTES, s, p);
   }
   note_launch();
   ce = launch_status();

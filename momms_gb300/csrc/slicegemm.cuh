@@ -568,6 +568,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait_few();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -870,6 +871,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   cluster_sync();  // the pair's barriers exist before any remote arrival
   tc::fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait_few();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -1137,8 +1139,10 @@ inline cudaLaunchConfig_t cluster_config(int ctas, int smem, cudaLaunchAttribute
   attr[0].val.clusterDim.x = (unsigned)ctas;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cfg;
 }
 
@@ -1158,7 +1162,7 @@ inline int slice_variant(int* clusters) {
     const bool want_pair = !(env && env[0] == '0');
     int v = SLICE_SINGLE, n = 0;
     if (want_pair) {
-      cudaLaunchAttribute attr[1];
+      cudaLaunchAttribute attr[2];
       cudaLaunchConfig_t cfg = cluster_config(2, pair_smem<EPI>(), attr);
       int c = 0;
       if (cudaOccupancyMaxActiveClusters(&c, (const void*)slice_gemm_pair_kernel<KIND, EPI>, &cfg) != cudaSuccess) {
@@ -1188,7 +1192,7 @@ inline int split_clusters(int ctas) {
   std::atomic<int>& c = cache[dev][ctas == 8 ? 3 : ctas / 2];
   int n = c.load();
   if (!n) {
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = cluster_config(ctas, SMEM_BYTES, attr);
     if (cudaOccupancyMaxActiveClusters(&n, (const void*)slice_gemm_kernel<KIND, EPI_F32, true>, &cfg) != cudaSuccess) {
       cudaGetLastError();
@@ -1203,7 +1207,7 @@ inline int split_clusters(int ctas) {
 template <int KIND>
 inline cudaError_t launch_slice_split(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& p, int ctas,
                                       cudaStream_t s) {
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = cluster_config(ctas, SMEM_BYTES, attr);
   cfg.gridDim = dim3((unsigned)((int64_t)p.tiles_m * p.tiles_n * ctas));
   cfg.stream = s;
@@ -1265,15 +1269,14 @@ inline cudaError_t launch_slice(const CUtensorMap& tmA, const CUtensorMap& tmB_f
   }
   const int64_t units = tile_units * ((p.ngroups + q.gchunk - 1) / q.gchunk);
   if (v == SLICE_PAIR) {
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = cluster_config(2, pair_smem<EPI>(), attr);
     cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(units, clusters)));
     cfg.stream = s;
     return cudaLaunchKernelEx(&cfg, slice_gemm_pair_kernel<KIND, EPI>, tmA, tmB_half, q, GroupTable{});
   }
   const int grid = (int)std::min<int64_t>(units, sm_count);
-  slice_gemm_kernel<KIND, EPI><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB_full, q);
-  return cudaGetLastError();
+  return launch_dependent(slice_gemm_kernel<KIND, EPI>, dim3((unsigned)grid), THREADS, SMEM_BYTES, s, tmA, tmB_full, q);
 }
 
 }  // namespace sp
