@@ -154,8 +154,7 @@ __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol
 // which hides less of its launch). After the kernel's own wait, so that at most
 // one kernel is ahead, and only in kernels that leave most of the GPU free or
 // end all at once: blocks that start as others end sit where those ended, two
-// long ones on one SM (FFMA 4096 x 4096 x 4096 2544 -> 2889 us, digits 8192 x
-// 8192 x 256 1426 -> 1483).
+// long ones on one SM (FFMA 4096 x 4096 x 4096 2544 -> 2889 us).
 constexpr unsigned kFewCtas = 76;
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dependency_wait_few() {

@@ -178,13 +178,42 @@ __device__ __forceinline__ void drain_chunk(uint32_t taddr, EpiAcc<EPI> (&S)[NC]
 // The maxima need only be upper bounds, so a quotient is a product with the
 // hardware's approximate reciprocal (at most one unit of 2^-23 off), and each
 // maximum is raised by 2^-18 at the end, which covers that and the roundings:
-// six instructions per entry. (With upward-rounded quotients formed where they
+// six instructions per entry with the sum's own. (With upward-rounded quotients formed where they
 // could raise the maximum, and column sums by shuffle, the epilogue took 25 of
 // the 30 us of a 512 x 512 x 512 bound, 0.23 ms at 8192 x 8192 x 64.)
+//
+// The sums of magnitudes are read before the tile's product is there
+// (bound_sums), and the posted maxima all at once: each is a trip to L2 or
+// beyond that nothing else would hide. With the columns past n set apart and a
+// reciprocal without denormals (20 instructions per entry before): 512 x 512 x
+// 512 16.4 -> 14.2 us, 8192 x 8192 x 256 100 -> 67.
+struct BoundSums {
+  float sa = 0.0f, mb = 0.0f;  // this row's sum; the largest column sum this lane read
+};
 template <int NC>
-__device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t col0, const float (&S)[NC], float* sb) {
+__device__ __forceinline__ BoundSums bound_sums(const Params& p, int64_t row, int64_t col0, float* sb) {
+  BoundSums b;
+  if (p.count_only) return b;
+  const int lane = threadIdx.x & 31, nvalid = (int)min((int64_t)NC, max((int64_t)0, p.n - col0));
+  unsigned long long w[NC / 32], a = 0;
+#pragma unroll
+  for (int q = 0; q < NC / 32; ++q) w[q] = 32 * q + lane < nvalid ? p.msum_b[col0 + 32 * q + lane] : 0;
+  if (row < p.m) a = p.msum_a[row];
+#pragma unroll
+  for (int q = 0; q < NC / 32; ++q) {
+    const float v = __fmul_ru(__ull2float_ru(w[q]), 0x1p-40f);
+    sb[32 * q + lane] = v;
+    b.mb = fmaxf(b.mb, v);
+  }
+  b.sa = __fmul_ru(__ull2float_ru(a), 0x1p-40f);
+  __syncwarp();
+  return b;
+}
+template <int NC>
+__device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t col0, float (&S)[NC],
+                                           const BoundSums& sums, float* sb) {
   const int lane = threadIdx.x & 31;
-  float m1 = 0.0f, m2 = 0.0f, ma = 0.0f, mb = 0.0f;
+  float m1 = 0.0f, m2 = 0.0f, ma = sums.sa, mb = sums.mb;
   unsigned cnt = 0;
   // columns of this tile inside C (the same for the whole warp)
   const int nvalid = (int)min((int64_t)NC, max((int64_t)0, p.n - col0));
@@ -195,26 +224,23 @@ __device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t
       for (int j = 0; j < NC; ++j) cnt += (j < nvalid && S[j] > 0.0f) ? 1u : 0u;
     }
   } else {
-#pragma unroll
-    for (int q = 0; q < NC / 32; ++q) {
-      const float v = 32 * q + lane < nvalid ? __fmul_ru(__ull2float_ru(p.msum_b[col0 + 32 * q + lane]), 0x1p-40f) : 0.0f;
-      sb[32 * q + lane] = v;
-      mb = fmaxf(mb, v);
-    }
-    __syncwarp();
     if (rv) {
-      const float sa = ma = __fmul_ru(__ull2float_ru(p.msum_a[row]), 0x1p-40f);
+      const float sa = sums.sa;
       float smin = INFINITY;
+      // columns past n count as covered
+      if (nvalid < NC) {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) S[j] = j < nvalid ? S[j] : INFINITY;
+      }
 #pragma unroll
       for (int j = 0; j < NC; j += 4) {
         const float4 b4 = *reinterpret_cast<const float4*>(sb + j);
         const float b[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          // columns past n count as covered
-          const float s = j + q < nvalid ? S[j + q] : INFINITY;
-          float r;
-          asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(s));
+          const float s = S[j + q];
+          float r;  // a sum that flushes to zero takes the row through the other loop
+          asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
           m1 = fmaxf(m1, (sa + b[q]) * r);
           smin = fminf(smin, s);
         }
@@ -262,10 +288,11 @@ __device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t
     // at 8192 x 8192 x 64 they cost most of the kernel).
     if (!p.count_only) {
       const volatile unsigned* cur = p.bound_out;
-      if (__float_as_uint(m1) > cur[0]) atomicMax(&p.bound_out[0], __float_as_uint(m1));
-      if (__float_as_uint(m2) > cur[1]) atomicMax(&p.bound_out[1], __float_as_uint(m2));
-      if (__float_as_uint(ma) > cur[4]) atomicMax(&p.bound_out[4], __float_as_uint(ma));
-      if (__float_as_uint(mb) > cur[5]) atomicMax(&p.bound_out[5], __float_as_uint(mb));
+      const unsigned c0 = cur[0], c1 = cur[1], c4 = cur[4], c5 = cur[5];
+      if (__float_as_uint(m1) > c0) atomicMax(&p.bound_out[0], __float_as_uint(m1));
+      if (__float_as_uint(m2) > c1) atomicMax(&p.bound_out[1], __float_as_uint(m2));
+      if (__float_as_uint(ma) > c4) atomicMax(&p.bound_out[4], __float_as_uint(ma));
+      if (__float_as_uint(mb) > c5) atomicMax(&p.bound_out[5], __float_as_uint(mb));
     }
     if (cnt) atomicAdd(p.bound_count, (unsigned long long)cnt);
   }
@@ -439,6 +466,8 @@ __device__ __forceinline__ bool float_groups(const Params& p, int g0, int g1, in
   // per-thread FP32 sums of finished chunks, rounded to nearest, which keeps
   // the tensor core's internal accumulation to one chunk at a time
   float S[NC];
+  BoundSums sums;
+  if constexpr (EPI == EPI_BOUND) sums = bound_sums<NC>(p, row, col0, sb);
 #pragma unroll
   for (int j = 0; j < NC; ++j) S[j] = 0.0f;
   for (int g = g0; g < g1; ++g) {
@@ -449,7 +478,7 @@ __device__ __forceinline__ bool float_groups(const Params& p, int g0, int g1, in
       release();
     }
   }
-  if constexpr (EPI == EPI_BOUND) bound_tile<NC>(p, row, col0, S, sb);
+  if constexpr (EPI == EPI_BOUND) bound_tile<NC>(p, row, col0, S, sums, sb);
   if (EPI == EPI_F32 && row < p.m) {
     // C is read 8 columns at a time, every load of a group issued before
     // the first use (one memory round trip per group, not per element)
