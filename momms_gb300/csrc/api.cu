@@ -131,8 +131,8 @@ DeviceState* device_state() {
   return &d;
 }
 
-cudaError_t scratch_alloc_raw(void** ptr, size_t bytes, cudaStream_t s) {
-  if (fault_take(MOMMS_FAULT_ALLOC)) return cudaErrorMemoryAllocation;
+namespace {
+cudaError_t pool_alloc(void** ptr, size_t bytes, cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
     cudaGetLastError();
@@ -141,6 +141,19 @@ cudaError_t scratch_alloc_raw(void** ptr, size_t bytes, cudaStream_t s) {
   DeviceState* d = (cs == cudaStreamCaptureStatusNone) ? device_state() : nullptr;
   if (d && d->pool) return cudaMallocFromPoolAsync(ptr, bytes, d->pool, s);
   return cudaMallocAsync(ptr, bytes, s);
+}
+}  // namespace
+
+cudaError_t scratch_alloc_raw(void** ptr, size_t bytes, cudaStream_t s) {
+  if (fault_take(MOMMS_FAULT_ALLOC)) return cudaErrorMemoryAllocation;
+  return pool_alloc(ptr, bytes, s);
+}
+
+void* scratch_if_room(size_t bytes, cudaStream_t s) {
+  void* p = nullptr;
+  if (pool_alloc(&p, bytes, s) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -348,7 +348,7 @@ int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_
       P.o = Operands{static_cast<const float*>(va.ptr), va.rs, va.cs, static_cast<const float*>(vb.ptr), vb.rs,
                      vb.cs, d.m, d.n, d.k, a_xc, b_xc, vec};
       P.e = Epi{d.m, d.n, (float)d.alpha, (float)d.beta, static_cast<float*>(d.c.ptr), d.c.rs, d.c.cs};
-      const PlainCfg cfg = plain_cfg(MOMMS_DTYPE_F32, d.m, d.n, d.k, ds->sm_count);
+      const PlainCfg cfg = f32_cfg(d.m, d.n, d.k, ds->sm_count);
       const int TMv = cfg.tile == 1 ? 64 : 128;
       if (!offsets_fit_32(P.o)) p->sg[cfg.tile].wide = true;
       P.tiles_m = (int)ceil_div(d.m, TMv);

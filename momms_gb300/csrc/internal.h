@@ -33,6 +33,14 @@ inline cudaError_t scratch_alloc(T** ptr, size_t bytes, cudaStream_t s) {
   return scratch_alloc_raw(reinterpret_cast<void**>(ptr), bytes, s);
 }
 
+// Scratch that a call can do without: null where the device has no room.
+void* scratch_if_room(size_t bytes, cudaStream_t s);
+template <typename T>
+inline bool scratch_alloc_if_room(T** ptr, size_t bytes, cudaStream_t s) {
+  *ptr = static_cast<T*>(scratch_if_room(bytes, s));
+  return *ptr != nullptr;
+}
+
 // Returns a stream-ordered scratch allocation to the pool, in order on `s`,
 // when it goes out of scope: on every return path of a launcher.
 struct ScratchGuard {
@@ -228,7 +236,7 @@ constexpr int kOzakiMaxSlices = 15;
 int launch_dgemm_ozaki(const DevGemm& g, double target_rel_err, int slices, int* slices_used, cudaStream_t s);
 // Bytes of operand and group planes a call holds: `tight`, never above the
 // digit form's; otherwise the residue form may take kFreeScratch instead.
-constexpr size_t kFreeScratch = 512u << 20;
+constexpr size_t kFreeScratch = 1024u << 20;
 double ozaki_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight);
 // Exponents of the R rows of a view x (element (r, p) at x[r*sr + p*sp],
 // p < K) into exps[R], using maxbits[R] as scratch; and the ns digit planes
@@ -262,15 +270,15 @@ struct DmmaOrient {
 };
 DmmaOrient dmma_orient(const DevMat& v, int64_t rows, int64_t cols, bool x_is_rows);
 
-// Launch configuration of a plain problem: the output tile (f32: 0 = 128 x
-// 128, 1 = 64 x 64; f64: 0) and the k-split count, from the tuning table
+// Launch configuration of a plain f32 problem: the output tile (0 = 128 x
+// 128, 1 = 64 x 64) and the k-split count, from the tuning table
 // (momms_autotune, keyed by shape bucket) or the model. Depends only on the
 // shape and the SM count.
 struct PlainCfg {
   int tile;
   int splits;
 };
-PlainCfg plain_cfg(int dtype, int64_t m, int64_t n, int64_t k, int sm_count);
+PlainCfg f32_cfg(int64_t m, int64_t n, int64_t k, int sm_count);
 
 // How a plain f64 problem is cut: square output tiles of ts = 32, 16 or 8, k
 // in `splits` ranges of kb_split k-blocks of 16. Depends only on the shape, the tuning table and

@@ -842,8 +842,10 @@ double crt_scratch(int per, int moduli, int64_t m, int64_t n, int64_t k, bool ti
 }
 // The residue form keeps to the digit form's scratch (or kFreeScratch bytes, unless
 // `tight`) by walking the moduli in several passes, each with its own operand
-// planes: at 8192^3 two passes of 9 and 8 moduli instead of 4.6 GB of planes,
-// for one more read of the operands (0.2 of 13 ms).
+// planes: at 8192^3 two passes of 8 moduli instead of 4.6 GB of planes, for one
+// more read of the operands (0.2 of 13 ms). Where a call is small a second pass
+// shows: 3704 x 74 x 4325 (523 MB at once) 444 us in two, 420 in one;
+// 2600 x 2600 x 2600 796 and 758.
 int crt_per_pass(int ns, int N, int64_t m, int64_t n, int64_t k, bool tight) {
   const double limit = std::max(digit_scratch(ns, m, n, k, tight), tight ? 0.0 : (double)kFreeScratch);
   int per = N;
@@ -1523,17 +1525,6 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   // residue planes in passes of `per` moduli.
   const bool crt = crt_applies(ns, g.whole_m ? g.whole_m : m, g.whole_n ? g.whole_n : n, k);
   const int N = crt ? crt_moduli(ns, sum_most) : ns;
-  const int per = crt ? crt_per_pass(ns, N, m, n, k, g.tight) : ns;
-  const int passes = (int)ceil_div(N, per);
-  const bool own_a = crt || !PA, own_b = crt || !PB;
-  __half* planes_buf = nullptr;
-  const size_t own = (own_a ? (size_t)per * a_plane : 0) + (own_b ? (size_t)per * b_plane : 0);
-  if (own && (ce = scratch_alloc(&planes_buf, own * sizeof(__half), s)) != cudaSuccess)
-    return cuda_fail(ce, "Ozaki slice planes");
-  ScratchGuard free_planes(planes_buf, s);
-  const __half* pa = own_a ? planes_buf : static_cast<const __half*>(PA->planes);
-  const __half* pb = own_b ? planes_buf + (own_a ? (size_t)per * a_plane : 0) : static_cast<const __half*>(PB->planes);
-
   if (k > kMaxK) return fail(MOMMS_ERR_UNSUPPORTED, "Ozaki emulation supports k <= %lld per launch", (long long)kMaxK);
   sp::Params p;
   Schedule sch;
@@ -1551,6 +1542,22 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   const size_t plane = (size_t)mpad * (size_t)round_up(n, (int64_t)sp::BN), word = crt ? 1 : sizeof(int);
   if ((ce = scratch_alloc(&sbuf, (size_t)ng * plane * word, s)) != cudaSuccess) return cuda_fail(ce, "Ozaki group sums");
   ScratchGuard free_sbuf(sbuf, s);
+  // The operand planes of a pass. The residue form's free scratch is taken
+  // only where there is room for it, else the passes it gets by with.
+  const bool own_a = crt || !PA, own_b = crt || !PB;
+  auto own_bytes = [&](int count) {
+    return sizeof(__half) * (size_t)count * ((own_a ? a_plane : 0) + (own_b ? b_plane : 0));
+  };
+  int per = crt ? crt_per_pass(ns, N, m, n, k, g.tight) : ns;
+  const int least = crt ? crt_per_pass(ns, N, m, n, k, true) : per;
+  __half* planes_buf = nullptr;
+  if (least < per && !scratch_alloc_if_room(&planes_buf, own_bytes(per), s)) per = least;
+  if (!planes_buf && own_bytes(per) && (ce = scratch_alloc(&planes_buf, own_bytes(per), s)) != cudaSuccess)
+    return cuda_fail(ce, "Ozaki slice planes");
+  ScratchGuard free_planes(planes_buf, s);
+  const int passes = (int)ceil_div(N, per);
+  const __half* pa = own_a ? planes_buf : static_cast<const __half*>(PA->planes);
+  const __half* pb = own_b ? planes_buf + (own_a ? (size_t)per * a_plane : 0) : static_cast<const __half*>(PB->planes);
   CombineParams cp;
   crt::CombineParams ccp;
   if (crt) crt_combine_params(g, ns, N, sbuf, (int64_t)plane, mpad, rexp, cexp, &ccp);

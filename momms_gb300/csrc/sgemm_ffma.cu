@@ -141,7 +141,7 @@ int sgemm_ffma_impl(const DevGemm& g0, cudaStream_t s, void* (&scratch)[3]) {
                  g.b.cs, g.m, g.n, g.k, a_xc, b_xc, vec};
   p.e = Epi{g.m, g.n, (float)g.alpha, (float)g.beta, static_cast<float*>(g.c.ptr), g.c.rs, g.c.cs};
   // the tile and split count of this shape (tuning table or model)
-  const PlainCfg cfg = plain_cfg(MOMMS_DTYPE_F32, g.m, g.n, g.k, ds->sm_count);
+  const PlainCfg cfg = f32_cfg(g.m, g.n, g.k, ds->sm_count);
   const int64_t kblocks = ceil_div(g.k, BK), kb_split = ceil_div(kblocks, cfg.splits);
   const int splits = (int)ceil_div(kblocks, kb_split);
   // Fewer units of 128 x 128 than SMs (few tiles and a short k): 32 x 32 tiles

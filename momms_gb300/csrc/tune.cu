@@ -65,19 +65,14 @@ bool lookup(int dtype, int prec, int64_t m, int64_t n, int64_t k, PlainCfg* out)
 int clamp_splits(int s, int64_t kblocks) { return std::max(1, (int)std::min<int64_t>(s, std::max<int64_t>(1, kblocks))); }
 }  // namespace
 
-PlainCfg plain_cfg(int dtype, int64_t m, int64_t n, int64_t k, int sm_count) {
+PlainCfg f32_cfg(int64_t m, int64_t n, int64_t k, int sm_count) {
   const int64_t kblocks = ceil_div(k, 16);
   PlainCfg c;
-  if (lookup(dtype, MOMMS_PREC_PLAIN, m, n, k, &c)) {
+  if (lookup(MOMMS_DTYPE_F32, MOMMS_PREC_PLAIN, m, n, k, &c)) {
     c.splits = clamp_splits(c.splits, kblocks);
     return c;
   }
-  if (dtype == MOMMS_DTYPE_F64) {
-    c.tile = 0;
-    c.splits = f64_plan(m, n, k, sm_count).splits;
-    return c;
-  }
-  // f32: the 128 x 128 tile (two CTAs per SM), split while its tiles leave
+  // the 128 x 128 tile (two CTAs per SM), split while its tiles leave
   // CTA slots idle. The 64 x 64 tile is chosen only by the tuner: as the
   // model's choice for every shape whose large tiles leave slots idle it took
   // the f32 part of the 512-problem batch from 0.65 to 0.85 ms (a second
