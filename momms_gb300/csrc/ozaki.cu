@@ -811,7 +811,11 @@ int crt_moduli(int ns, double sum) {
 //    the epilogue they do not hide: 0.53 ps (digits: 4 bytes of plane), 0.2 ps;
 //  * recombination 7.4 ps per entry (7 digit groups), 10.4 ps (16 moduli);
 //  * operand planes 2 bytes per slice or modulus, 8 read, at 6 TB/s;
-//  * 3 us for the launch that packed operands need only for residues.
+//  * packed operands have their digits, and no residues: 2 bytes read per
+//    slice and written per modulus, at 9 TB/s (much of it stays in L2).
+// The residue form has to be faster either way, by 3 us where operands are not
+// packed: 3776 x 247 x 2224 from packs, 8 slices, 115 us by digits and 156 by
+// residues, 1000 x 1000 x 1000, 7 slices, 62 and 56.
 // Both forms, 7 slices, ms per call: 8192 x 8192 x 128 1.33 (digits) and 1.40,
 // x 256 1.61 and 1.56, x 1024 3.17 and 2.48, x 8192 20.9 and 13.1; 65536 x 256 x
 // 256 0.64 and 0.75; the slice kernel alone at 512^3 0.030 and 0.014.
@@ -820,13 +824,14 @@ bool crt_applies(int ns, int64_t m, int64_t n, int64_t k) {
   const int N = crt_moduli(ns, k);
   Schedule sc;
   if (!ozaki_schedule(ns, k, &sc)) return true;
-  constexpr double kPairs = 76.0, kStep = 0.26e6, kPackedPass = 3e6;  // ps
+  constexpr double kPairs = 76.0, kStep = 0.26e6, kMargin = 3e6;  // ps
   const double mn = (double)m * n, ops = (double)(m + n) * k;
   const double tiles = (double)(ceil_div(m, 256) * ceil_div(n, 256)), steps = (double)ceil_div(k, 64) * kStep;
   auto products = [&](double pairs, double longest) { return steps * std::max(pairs * tiles / kPairs, longest); };
-  const double digits = products(sc.np, ns) + mn * (0.53 * sc.ng + 2.7 + 0.67 * sc.ng) + ops * (8 + 2 * ns) / 6.0;
-  const double residues = products(N, 1.0) + mn * (0.2 * N + 0.65 * N) + ops * (8 + 2 * N) / 6.0;
-  return residues + kPackedPass < digits;
+  const double digits = products(sc.np, ns) + mn * (0.53 * sc.ng + 2.7 + 0.67 * sc.ng);
+  const double residues = products(N, 1.0) + mn * (0.2 * N + 0.65 * N);
+  return residues + ops * (8 + 2 * N) / 6.0 + kMargin < digits + ops * (8 + 2 * ns) / 6.0 &&
+         residues + ops * (2 * ns + 2 * N) / 9.0 < digits;
 }
 
 // Scratch of an emulated product, operand planes and group planes: the digit
@@ -844,8 +849,8 @@ double crt_scratch(int per, int moduli, int64_t m, int64_t n, int64_t k, bool ti
 // `tight`) by walking the moduli in several passes, each with its own operand
 // planes: at 8192^3 two passes of 8 moduli instead of 4.6 GB of planes, for one
 // more read of the operands (0.2 of 13 ms). Where a call is small a second pass
-// shows: 3704 x 74 x 4325 (523 MB at once) 444 us in two, 420 in one;
-// 2600 x 2600 x 2600 796 and 758.
+// shows: 2600 x 2600 x 2600 786 us in two, 754 in one, 4096 x 1024 x 4096 728
+// and 678.
 int crt_per_pass(int ns, int N, int64_t m, int64_t n, int64_t k, bool tight) {
   const double limit = std::max(digit_scratch(ns, m, n, k, tight), tight ? 0.0 : (double)kFreeScratch);
   int per = N;
