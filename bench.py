@@ -693,7 +693,7 @@ def run_ours(args):
     # column chunk of C, each over its share of the columns
     slice_per_step = max(1, round(slice_n / max(1, args.steps)))
     tc_flops_per_launch = info.pairs * flops / slice_per_step
-    slice_traffic = profile_traffic("slice_gemm_ozaki_8192")  # one unchunked 8192^3 launch
+    slice_traffic = profile_traffic("slice_gemm_ozaki_8192")  # all slice launches of one 8192^3 call
     if slice_traffic is not None:
         slice_traffic /= slice_per_step
     slice_avg = slice_ms / max(1, slice_n)
@@ -718,8 +718,8 @@ def run_ours(args):
         "vs_baseline": None, "dtype": "f64",
         "data": f"synthetic: uniform[-1,1] from seed {SEED}, column-major, C initialised like A and B",
         "config": {"workload": WORKLOAD.replace("8192", str(size)), "m": m, "n": n, "k": k,
-                   "precision": "emulated FP64 (Ozaki: 8-bit digit slices as fp16 on tcgen05, exact int32 "
-                                "digit sums, FP64 recombination); slice count chosen per call for the "
+                   "precision": "emulated FP64 (Ozaki: 8-bit slices, products modulo coprime p <= 256 or by "
+                                "digits as fp16 on tcgen05, exact, one rounding); slice count chosen per call for the "
                                 "default FP64-level target",
                    "slices": info.slices, "slice_products": info.pairs,
                    "l2": "inputs larger than L2 (512 MiB per operand vs 129 MB L2); no flush",

@@ -117,9 +117,9 @@ int momms_sgemm(int64_t m, int64_t n, int64_t k, const float* alpha, const float
  * Same arguments, same kernel and same tile / split-k plan as momms_dgemm, but
  * all of A, B and C must already be device memory, and A and B must each have
  * unit stride along one index with the other stride a multiple of 2 elements
- * and a 16-byte aligned base (other layouts would need a repack copy). The
+ * and a 16-byte aligned base (momms_dgemm takes any layout). The
  * split-k scratch is one device-global array of MOMMS_NOALLOC_SCRATCH_BYTES
- * (160 partial tiles of 128 x 128 doubles plus 1024 tile counters) and 1 KB of
+ * (the room of 160 partial tiles of 128 x 128 doubles plus 1024 tile counters) and 1 KB of
  * further counters that every GPU loading this library holds until the process
  * exits; a problem whose
  * split-k plan needs more than that is rejected with MOMMS_ERR_INVALID_ARG.
@@ -291,7 +291,7 @@ typedef struct {
   int32_t splits;     /* chosen k-split count */
   int32_t candidates; /* configurations timed */
   float best_ms;      /* time of the chosen configuration */
-  int32_t tile;       /* chosen output tile: 0 = 128 x 128, 1 = the small tile (f32: 64 x 64) */
+  int32_t tile;       /* chosen output tile: f32 0 = 128 x 128, 1 = 64 x 64; f64 0 */
 } momms_tune_result;
 int momms_autotune(const momms_gemm_desc* desc, momms_tune_result* out, void* stream);
 /* Tunes every shape bucket of a batch once (the bucket's first plain problem
@@ -310,8 +310,8 @@ int momms_tune_clear(void);
 typedef struct {
   int32_t precision;      /* momms_precision actually run */
   int32_t slices;         /* OZAKI: slice count used (chosen or given) */
-  int32_t pairs;          /* OZAKI: slice products formed (tensor-core GEMMs) */
-  int32_t groups;         /* OZAKI: accumulation groups */
+  int32_t pairs;          /* OZAKI: tensor-core products formed: slice pairs, or one per modulus */
+  int32_t groups;         /* OZAKI: accumulation groups (or moduli) */
   int32_t splits;         /* plain paths and split TF32: k splits */
   int32_t slice_variant;  /* tensor-core paths: slice kernel variant run: 0 = one CTA per tile,
                              2 = CTA pairs with one cta_group::2 MMA, 3 = a cluster of
