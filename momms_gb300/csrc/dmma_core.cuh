@@ -401,16 +401,7 @@ struct Unit {
   int tm, tn, sp;
 };
 
-// A persistent CTA over a source of units (Src: total(), and unit(u, fn) which
-// calls fn(problem, A map, B map, Unit) with problem a DProblem).
-// With `next` units are handed out dynamically: the producer warp takes the
-// next unit from the global counter (numbered costliest first, so this is
-// longest-processing-time-first list scheduling by the actual durations; a
-// static deal of 4096 equal units over 608 CTAs left one SM in four with 28
-// units against 26.9 on average: 1.055 against 1.095 TFLOP/s at 2048^3).
-// Without, the CTA takes units blockIdx.x, blockIdx.x + gridDim.x, ...
-// Either way the producer tags the first stage it fills for a unit with the
-// unit's index, which the DMMA warps read when they reach that stage; -1 ends.
+// One problem, as the kernels see it.
 struct DProblem {
   int64_t m, n, k;
   Operand a, b;
@@ -422,6 +413,16 @@ struct DProblem {
   unsigned* counters;  // splits > 1: [tiles], zero on entry and on exit
 };
 
+// A persistent CTA over a source of units (Src: total(), and unit(u, fn) which
+// calls fn(problem, A map, B map, Unit) with problem a DProblem).
+// With `next` units are handed out dynamically: the producer warp takes the
+// next unit from the global counter (numbered costliest first, so this is
+// longest-processing-time-first list scheduling by the actual durations; a
+// static deal of 4096 equal units over 608 CTAs left one SM in four with 28
+// units against 26.9 on average: 1.055 against 1.095 TFLOP/s at 2048^3).
+// Without, the CTA takes units blockIdx.x, blockIdx.x + gridDim.x, ...
+// Either way the producer tags the first stage it fills for a unit with the
+// unit's index, which the DMMA warps read when they reach that stage; -1 ends.
 template <typename Src>
 __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* next, unsigned* status) {
   extern __shared__ uint8_t smem_raw[];
