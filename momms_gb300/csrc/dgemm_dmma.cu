@@ -14,7 +14,7 @@
 // slab; both stay inside |dC| <= 2k u (|A||B|).
 //
 // Bound by GB300's FP64 rate (about 1.1 TFLOP/s per GPU): see dmma_core.cuh
-// for why the tile is 32 x 32 and f64_plan (tune.cu) for how units are cut.
+// for why the tile is 32 x 32 and f64_plan.h for how units are cut.
 #include <stdio.h>
 #include <string.h>
 
@@ -142,7 +142,7 @@ int launch_dgemm_dmma(const DevGemm& g, cudaStream_t s) {
   // units than CTAs
   const int64_t slots = (int64_t)CTAS_PER_SM * ds->sm_count;
   const bool dynamic = plan.units() > slots;
-  const size_t part_bytes = plan.splits > 1 ? (size_t)plan.units() * TILE_ELEMS * 8 : 0;
+  const size_t part_bytes = (size_t)plan.partial_elems() * sizeof(double);
   const size_t zero_bytes = (dynamic ? 2 * sizeof(unsigned long long) : 0) +
                             (plan.splits > 1 ? (size_t)plan.tiles() * sizeof(unsigned) : 0);
   void* ws = nullptr;
@@ -299,12 +299,14 @@ extern "C" int momms_dgemm_noalloc(int64_t m, int64_t n, int64_t k, const double
 
   // The same plan as momms_dgemm, so both give the same result.
   const F64Plan plan = f64_plan(g.m, g.n, g.k, nd->sm_count);
-  if (plan.splits > 1 && !f64_split_fits(m, n, plan.splits))
+  const size_t part_bytes = (size_t)plan.partial_elems() * sizeof(double);
+  if (plan.splits > 1 && (!f64_split_fits(m, n, plan.splits) || part_bytes > kNoallocPartialBytes ||
+                          (size_t)plan.tiles() > kNoallocCounterSlots))
     return fail(MOMMS_ERR_INVALID_ARG,
-                "this problem needs %lld split-k partial tiles of 128x128 doubles; the no-alloc scratch holds %zu "
-                "(%d bytes)",
-                (long long)(ceil_div(m, 128) * ceil_div(n, 128) * plan.splits), kNoallocPartialTiles,
-                (int)MOMMS_NOALLOC_SCRATCH_BYTES);
+                "this problem needs %lld split-k partial tiles of 128x128 doubles (%zu bytes, %lld counters); the "
+                "no-alloc scratch holds %zu (%zu bytes, %zu counters)",
+                (long long)(ceil_div(m, 128) * ceil_div(n, 128) * plan.splits), part_bytes, (long long)plan.tiles(),
+                kNoallocPartialTiles, kNoallocPartialBytes, kNoallocCounterSlots);
   Params p;
   CUtensorMap tmA, tmB;
   // waits report in the no-alloc status word, not the library's allocated one

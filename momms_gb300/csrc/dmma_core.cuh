@@ -10,7 +10,7 @@
 // spread over the warps), one producer warp, k-blocks of 16 in a 5-stage ring
 // and four CTAs per SM: a CTA's epilogue and pipeline fill run under the other
 // three's DMMAs. A problem may step its tiles by 16 or 8 instead of 32 (`ts`,
-// see f64_plan): then every warp takes the whole tile for one k step of 4
+// see f64_plan.h): then every warp takes the whole tile for one k step of 4
 // of each k-block, and the four partial sums meet in shared memory. (One
 // block per warp over all of k ran the FP64 pipe at 0.70 of its rate, 0.72
 // TFLOP/s at 1024^3 against 1.09 for four blocks per warp: a warp needs
@@ -37,7 +37,6 @@ constexpr int OP_STAGE = TILE * BK * 8;  // bytes of one operand's k-block
 constexpr int SUB = BK * 128;  // one 16-wide sub-tile of an x-contiguous operand
 constexpr int RED_BYTES = CONSUMER_WARPS * 16 * 16 * 8;  // the warps' partial sums of a 16-stepped tile
 constexpr int SMEM_BYTES = 1024 + STAGES * 2 * OP_STAGE + RED_BYTES + 2 * STAGES * 8 + 16;
-constexpr int TILE_ELEMS = TILE * TILE;  // doubles of one split-k partial tile
 
 // Byte offset of element (r, kk) in a k-contiguous tile: rows of 16 doubles
 // (128 bytes), 128B swizzle (16-byte chunk index XOR row mod 8).
@@ -293,15 +292,16 @@ __device__ __forceinline__ void reduce_warps(double (&acc)[2][2][2], double* red
 
 // Epilogue of one unit. With splits == 1 the tile goes straight to C.
 // Otherwise this split's partial tile is published in `tile_partials`
-// ([splits][TILE_ELEMS], thread-interleaved), and the last split to arrive on
+// ([splits][ts * ts], thread-interleaved: at steps of 16 a thread owns two
+// outputs, at steps of 8 the first warp's threads do), and the last split to arrive on
 // `counter` sums all partials in split order 0..splits-1 (a fixed order: the
 // result does not depend on which CTA finishes last), writes C and resets
 // the counter to zero.
 //
 // A thread owns eight outputs; their loads (C for beta != 0, the partials two
 // splits at a time) are issued before the first value is used.
-__device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2][2][2], const Place& p, int splits,
-                                            int sp, double* tile_partials, unsigned* counter, int ctid,
+__device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2][2][2], const Place& p, int ts,
+                                            int splits, int sp, double* tile_partials, unsigned* counter, int ctid,
                                             int* s_last) {
   // output u = 4i + 2j + q of this thread
   auto live = [&](int u) { return p.row + 16 * (u >> 2) < p.row_end && p.col + 16 * ((u >> 1) & 1) + (u & 1) < p.col_end; };
@@ -327,10 +327,11 @@ __device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2]
     return;
   }
   // Partials exist only for the tile's entries inside C.
-  double* part = tile_partials + (size_t)sp * TILE_ELEMS;
+  const int elems = ts * ts, own = ts > 8 ? CONSUMERS : 32;
+  double* part = tile_partials + (size_t)sp * elems;
 #pragma unroll
   for (int u = 0; u < 8; ++u)
-    if (live(u)) part[u * CONSUMERS + ctid] = v[u];
+    if (live(u)) part[u * own + ctid] = v[u];
   __threadfence();
   consumer_sync();
   if (ctid == 0) {
@@ -342,7 +343,7 @@ __device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2]
     __threadfence();
     constexpr int T = 2;  // splits loaded together
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = live(u) ? __ldcg(tile_partials + u * CONSUMERS + ctid) : 0.0;
+    for (int u = 0; u < 8; ++u) v[u] = live(u) ? __ldcg(tile_partials + u * own + ctid) : 0.0;
     for (int t0 = 1; t0 < splits; t0 += T) {
       double w[T][8];
 #pragma unroll
@@ -350,7 +351,7 @@ __device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2]
 #pragma unroll
         for (int u = 0; u < 8; ++u)
           w[t][u] = (t0 + t < splits && live(u))
-                        ? __ldcg(tile_partials + (size_t)(t0 + t) * TILE_ELEMS + u * CONSUMERS + ctid)
+                        ? __ldcg(tile_partials + (size_t)(t0 + t) * elems + u * own + ctid)
                         : 0.0;
 #pragma unroll
       for (int t = 0; t < T; ++t)
@@ -409,7 +410,7 @@ struct DProblem {
   int tiles_m, tiles_n, splits, ts;
   int64_t kb_split;
   int64_t unit_begin;  // grouped launches: the problem's first unit
-  double* partials;    // splits > 1: [tiles][splits][TILE_ELEMS]
+  double* partials;    // splits > 1: [tiles][splits][ts * ts]
   unsigned* counters;  // splits > 1: [tiles], zero on entry and on exit
 };
 
@@ -488,8 +489,8 @@ __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* n
                         run_blocks(P.ts), acc, status);
       if (!ok) return;
       if (P.ts <= 16) reduce_warps(acc, sm.red, warp, lane);
-      finish_unit(P.e, acc, at, P.splits, w.sp,
-                  P.splits > 1 ? P.partials + (size_t)w.tile * P.splits * TILE_ELEMS : nullptr,
+      finish_unit(P.e, acc, at, P.ts, P.splits, w.sp,
+                  P.splits > 1 ? P.partials + (size_t)w.tile * P.splits * (P.ts * P.ts) : nullptr,
                   P.splits > 1 ? P.counters + w.tile : nullptr, threadIdx.x, sm.s_last);
     });
     if (!ok) return;

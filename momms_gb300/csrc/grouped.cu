@@ -292,7 +292,7 @@ int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_
         // offsets until the buffers exist
         P.partials = reinterpret_cast<double*>(parts * sizeof(double));
         P.counters = reinterpret_cast<unsigned*>(ctrs * sizeof(unsigned));
-        parts += fp.units() * TILE_ELEMS;
+        parts += fp.partial_elems();
         ctrs += fp.tiles();
       }
       probs.push_back(P);

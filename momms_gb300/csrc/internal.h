@@ -7,6 +7,7 @@
 #include <string>
 
 #include "../../include/momms_gpu.h"
+#include "f64_plan.h"
 
 namespace momms {
 
@@ -280,16 +281,8 @@ struct PlainCfg {
 };
 PlainCfg f32_cfg(int64_t m, int64_t n, int64_t k, int sm_count);
 
-// How a plain f64 problem is cut: square output tiles of ts = 32, 16 or 8, k
-// in `splits` ranges of kb_split k-blocks of 16. Depends only on the shape, the tuning table and
-// the SM count.
-struct F64Plan {
-  int ts, tiles_m, tiles_n, splits;
-  int64_t kb_split;
-  int64_t tiles() const { return (int64_t)tiles_m * tiles_n; }
-  int64_t units() const { return tiles() * splits; }
-  double unit_cost;  // FP64-pipe clocks of one SM per unit
-};
+// The plan of a plain f64 problem (f64_plan.h), with the tuning table's split
+// count where it has one.
 F64Plan f64_plan(int64_t m, int64_t n, int64_t k, int sm_count);
 namespace dmma {
 struct DProblem;
@@ -297,13 +290,6 @@ struct DProblem;
 // The kernels' description of a problem under a plan (partials and counters
 // are the caller's), with the tensor maps of the operands TMA stages.
 int dmma_problem(const DevGemm& g, const F64Plan& plan, dmma::DProblem* P, CUtensorMap* tmA, CUtensorMap* tmB);
-// What a split plan of the model may use, the same for every caller: partial
-// tiles within 160 of 128 x 128 doubles (counted on the 128 grid), and the
-// 1280 counters that two splits of so many 32 x 32 tiles take.
-constexpr int64_t kSplitTileCap = 160, kSplitCounterCap = 1280;
-inline bool f64_split_fits(int64_t m, int64_t n, int splits) {
-  return ((m + 127) / 128) * ((n + 127) / 128) * splits <= kSplitTileCap;
-}
 
 // Emulated problems of a plan run together: each problem's preparation and
 // recombination, and ONE persistent slice-kernel launch (CTA pairs) over all

@@ -9,7 +9,7 @@
 // scratch output) is keyed by shape bucket: ceil(log2) of m, n and k, so a
 // tuned shape covers every problem within a factor of two of it and a batch
 // of uneven problems hits tuned entries. Shapes without an entry use a model
-// (f64_plan; f32: the large tile, and k split only while the tiles leave CTA
+// (f64_plan.h; f32: the large tile, and k split only while the tiles leave CTA
 // slots idle, keeping at least 8 k-blocks per split).
 #include <stdio.h>
 #include <string.h>
@@ -61,8 +61,6 @@ bool lookup(int dtype, int prec, int64_t m, int64_t n, int64_t k, PlainCfg* out)
   *out = it->second;
   return true;
 }
-
-int clamp_splits(int s, int64_t kblocks) { return std::max(1, (int)std::min<int64_t>(s, std::max<int64_t>(1, kblocks))); }
 }  // namespace
 
 PlainCfg f32_cfg(int64_t m, int64_t n, int64_t k, int sm_count) {
@@ -83,58 +81,10 @@ PlainCfg f32_cfg(int64_t m, int64_t n, int64_t k, int sm_count) {
   return c;
 }
 
-// The f64 plan minimises the FP64 pipe's time on the busiest SM plus what a
-// split costs at its end. One SM takes 128 clocks per 8 x 8 x 4 DMMA whatever
-// the tile, so the sum per SM (units dealt round-robin, the SM's four CTAs
-// sharing the pipe) is what balance can change: tiles of 32 where they are
-// many, of 16 (8, for a few dozen rows and columns) or k splits where a last
-// wave would be thin or SMs would idle. Splitting adds one FP64 addition per output and split, and
-// a partial write, a fence, an atomic and the last arriver's reads in series
-// (about 3 us).
 F64Plan f64_plan(int64_t m, int64_t n, int64_t k, int sm_count) {
-  constexpr double kBlockStep = 128.0, kUnitFill = 300.0, kSplitTail = 6000.0, kSplitTailEach = 200.0;
-  const int64_t kblocks = ceil_div(k, 16), ksteps = ceil_div(k, 4);
   PlainCfg forced;
   const bool tuned = lookup(MOMMS_DTYPE_F64, MOMMS_PREC_PLAIN, m, n, k, &forced);
-  F64Plan best{};
-  double best_t = -1.0;
-  for (int ts = 32; ts >= 8; ts /= 2) {
-    F64Plan p{};
-    p.ts = ts;
-    p.tiles_m = (int)ceil_div(m, ts);
-    p.tiles_n = (int)ceil_div(n, ts);
-    const int64_t tiles = p.tiles();
-    const double blocks = (double)std::min<int64_t>(ceil_div(m, 8), ts / 8) * std::min<int64_t>(ceil_div(n, 8), ts / 8);
-    const int most = !tuned && tiles > kSplitCounterCap ? 1 : (int)std::min<int64_t>(32, kblocks);
-    // a tuned split count is kept as it is: smaller tiles only where its
-    // counters still fit
-    if (tuned && ts < 32 && clamp_splits(forced.splits, kblocks) > 1 && tiles > kSplitCounterCap) break;
-    int prev = 0;
-    for (int want = 1; want <= most; ++want) {
-      if (tuned) want = clamp_splits(forced.splits, kblocks);
-      p.kb_split = ceil_div(kblocks, want);
-      p.splits = (int)ceil_div(kblocks, p.kb_split);
-      if (!tuned && p.splits > 1 && !f64_split_fits(m, n, p.splits)) break;
-      if (p.splits != prev) {
-        prev = p.splits;
-        const double steps = (double)std::min<int64_t>(4 * p.kb_split, ksteps);
-        // warps with one block of their own keep the pipe at 0.7 of its rate
-        const double rate = ts == 8 || (ts == 32 && m <= 16 && n <= 16) ? 0.7 : 1.0;
-        // per output: alpha and beta (or nothing), and the four warps' sum
-        p.unit_cost = blocks * (kBlockStep / rate * steps + (p.splits == 1 ? 64.0 : 0.0) + (ts < 32 ? 96.0 : 0.0)) + kUnitFill;
-        double t = (double)ceil_div(p.units(), sm_count) * p.unit_cost;
-        if (p.splits > 1)
-          t += kSplitTail + kSplitTailEach * p.splits +
-               (double)ceil_div(tiles, sm_count) * blocks * 32.0 * (p.splits + 1);
-        if (best_t < 0.0 || t < best_t) {
-          best_t = t;
-          best = p;
-        }
-      }
-      if (tuned) break;
-    }
-  }
-  return best;
+  return f64_model(m, n, k, sm_count, tuned ? std::max(1, forced.splits) : 0);
 }
 
 }  // namespace momms
