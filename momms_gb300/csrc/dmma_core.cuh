@@ -125,10 +125,16 @@ __device__ __forceinline__ void stage_tma(const Operand& o, const CUtensorMap* m
 // x staged per operand and k-block for tiles stepped by ts.
 __host__ __device__ constexpr int stage_extent(int ts) { return ts > 16 ? TILE : 16; }
 
+// Arrivals on a stage's full barrier: every producer lane, once its own copies
+// have landed, and lane 0 once more by an ordinary arrival. That one releases
+// lane 0's plain stores (the unit's tag): a cp.async arrival is made when the
+// copies land and orders no other store of its thread.
+constexpr unsigned FULL_ARRIVALS = 33;
+
 // Producer warp: k-blocks [kb0, kb1) of the output tile whose first row and
-// column are m0, n0. Every lane arrives on the stage's full barrier (count 32)
-// once its own copies have landed; lane 0 adds the TMA bytes. Returns false
-// if a bounded wait expired.
+// column are m0, n0. Every lane arrives on the stage's full barrier once its
+// own copies have landed; lane 0 adds the TMA bytes, and releases what it
+// stored before (FULL_ARRIVALS). Returns false if a bounded wait expired.
 __device__ __forceinline__ bool produce_unit(const CUtensorMap* tmA, const CUtensorMap* tmB, const Operand& a,
                                              const Operand& b, int64_t m, int64_t n, int64_t k, int ts, int64_t m0,
                                              int64_t n0, int64_t kb0, int64_t kb1, uint8_t* sA, uint8_t* sB,
@@ -157,6 +163,7 @@ __device__ __forceinline__ bool produce_unit(const CUtensorMap* tmA, const CUten
     if (!b.tma) stage_async(b, b_dst, n0, kc, ext, n, k, lane);
     if (a.tma && b.tma) mbar_arrive(&full[stage]);
     else mbar_arrive_cp_async(&full[stage]);
+    if (lane == 0) mbar_arrive(&full[stage]);
     if (++stage == STAGES) {
       stage = 0;
       phase ^= 1;
@@ -387,7 +394,7 @@ __device__ __forceinline__ Smem setup_smem(uint8_t* smem_raw) {
   s.s_last = reinterpret_cast<int*>(s.empty + STAGES);
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
-      mbar_init(&s.full[i], 32);
+      mbar_init(&s.full[i], FULL_ARRIVALS);
       mbar_init(&s.empty[i], CONSUMER_WARPS);
     }
     fence_barrier_init();
@@ -436,8 +443,8 @@ __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* n
   if (warp == CONSUMER_WARPS) {
     bool ok = true;
     // a tag is written while its stage is free (every DMMA warp read the
-    // previous tag before releasing it) and published by lane 0's arrival on
-    // the stage (release) to the warps' wait (acquire)
+    // previous tag before releasing it) and published by lane 0's ordinary
+    // arrival on the stage (release) to the warps' wait (acquire)
     auto tag = [&](long long u) {
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(&sm.empty[stage], phase ^ 1));
       if (ok && lane == 0) s_stage_unit[stage] = u;
@@ -460,6 +467,7 @@ __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* n
     if (ok) {
       tag(-1);
       if (ok) mbar_arrive(&sm.full[stage]);
+      if (ok && lane == 0) mbar_arrive(&sm.full[stage]);
     }
     cp_async_wait_all();
     if (next && lane == 0) {

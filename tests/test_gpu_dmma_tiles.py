@@ -62,3 +62,26 @@ def test_grouped_mixed_staging_equals_single(gpu):
         assert np.array_equal(keep[i][2][0].cpu().numpy(), expected[i]), i
     bits = ctypes.c_uint32(0)
     assert gpu.momms_device_status(ctypes.byref(bits)) == mg.OK and bits.value == 0
+
+
+@pytest.mark.parametrize("layouts", ["odd odd", "col odd", "odd col", "strided strided"])
+@pytest.mark.parametrize("shape", [(1601, 1503, 23), (2003, 997, 49), (407, 3001, 16)])
+def test_many_short_units_by_either_staging(gpu, shape, layouts):
+    """Several units of one to four k-blocks per CTA: every unit's index travels with its first
+    stage, whichever way the stage is filled. The bits are those of 16-byte aligned copies."""
+    m, n, k = shape
+    la, lb = layouts.split()
+    rng = np.random.default_rng(m + n + k)
+    A, B = _operand(rng, m, k, la), _operand(rng, k, n, lb)
+    C0 = np.asfortranarray(rng.uniform(-1, 1, (m, n)))
+
+    def aligned(x):  # column-major, columns an even number of elements apart
+        y = np.zeros((x.shape[0] + x.shape[0] % 2, x.shape[1]), order="F")
+        y[:x.shape[0]] = x
+        return y[:x.shape[0]]
+
+    want = gu.gemm_device(gpu, aligned(A), aligned(B), C0)
+    for _ in range(3):
+        assert np.array_equal(gu.gemm_device(gpu, A, B, C0), want)
+    ref, mag = ou.dd_gemm(np.asfortranarray(A), np.asfortranarray(B), C0)
+    assert ou.bound_ratio(want, ref, mag, k, U64) <= 1.0
