@@ -109,7 +109,7 @@ int dmma_problem(const DevGemm& g, const F64Plan& plan, dmma::DProblem* P, CUten
   P->m = g.m, P->n = g.n, P->k = g.k;
   P->e = dmma::Epi{g.m, g.n, g.alpha, g.beta, static_cast<double*>(g.c.ptr), g.c.rs, g.c.cs};
   P->tiles_m = plan.tiles_m, P->tiles_n = plan.tiles_n;
-  P->splits = plan.splits, P->ts = plan.ts;
+  P->splits = plan.splits, P->ts = plan.ts, P->run = plan.run;
   P->kb_split = plan.kb_split;
   // A: rows m, cols k, x = m. B: rows k, cols n, x = n.
   const int rc = dmma_operand(g.a, g.m, g.k, true, plan.ts, &P->a, tmA);

@@ -208,14 +208,9 @@ __device__ __forceinline__ Place place_of(int64_t m0, int64_t n0, int ts, int64_
   return p;
 }
 
-// A warp's sums over k are taken in runs of this many k-blocks (256 products per
-// entry), each added to the running total: the error then grows no further with
-// the length of a unit (against 64 bits, one chain and runs: 1999 x 1501 x 2753
-// 8.8e-16 and 5.3e-16, 1728 x 253 x 3153 1.9e-15 and 5.5e-16), for 0.5 % of the
-// time (1024^3 2048 -> 2059 us; runs of 128 cost 1.5-2 %).
-__device__ __forceinline__ int run_blocks(int ts) { return ts <= 16 ? 64 : 16; }
-
-// Consumer: accumulate k-blocks [kb0, kb1) of the current unit into acc.
+// Consumer: accumulate k-blocks [kb0, kb1) of the current unit into acc, each
+// run of `run` k-blocks in a chain of its own that is then added to the total
+// (F64Plan::run).
 // Blocks entirely outside the output and k steps past K are not multiplied
 // (both would add zeros). Returns false if a bounded wait expired.
 __device__ __forceinline__ bool consume_unit(int a_xc, int b_xc, int64_t k, int64_t kb0, int64_t kb1, const Place& p,
@@ -414,7 +409,7 @@ struct DProblem {
   int64_t m, n, k;
   Operand a, b;
   Epi e;
-  int tiles_m, tiles_n, splits, ts;
+  int tiles_m, tiles_n, splits, ts, run;
   int64_t kb_split;
   int64_t unit_begin;  // grouped launches: the problem's first unit
   double* partials;    // splits > 1: [tiles][splits][ts * ts]
@@ -494,7 +489,7 @@ __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* n
       const Place at = place_of((int64_t)w.tm * P.ts, (int64_t)w.tn * P.ts, P.ts, P.m, P.n, warp, lane);
       double acc[2][2][2] = {};
       ok = consume_unit(P.a.xc, P.b.xc, P.k, w.kb0, w.kb1, at, sm.sA, sm.sB, sm.full, sm.empty, stage, phase, lane,
-                        run_blocks(P.ts), acc, status);
+                        P.run, acc, status);
       if (!ok) return;
       if (P.ts <= 16) reduce_warps(acc, sm.red, warp, lane);
       finish_unit(P.e, acc, at, P.ts, P.splits, w.sp,

@@ -22,6 +22,7 @@ inline bool f64_split_fits(int64_t m, int64_t n, int splits) {
 struct F64Plan {
   int ts, tiles_m, tiles_n, splits;
   int64_t kb_split;
+  int run;  // k-blocks whose products a warp sums in one chain (f64_run)
   int64_t tiles() const { return (int64_t)tiles_m * tiles_n; }
   int64_t units() const { return tiles() * splits; }
   // doubles of a split's partial tiles, one of ts x ts per unit
@@ -31,6 +32,43 @@ struct F64Plan {
 
 inline int clamp_splits(int s, int64_t kblocks) {
   return std::max(1, (int)std::min<int64_t>(s, std::max<int64_t>(1, kblocks)));
+}
+
+// A warp sums its products of `run` k-blocks in one chain (16 products an entry
+// and k-block, or 4 where the tile's four warps share each k-block: steps of 16
+// and 8), the runs in turn, then the warps, then the splits. For products of
+// either sign the mean square error of such a sum is proportional to
+//   chain + runs + splits (+ 5 for the four warps),
+// each of runs and splits counted where there is more than one. The run is the
+// longest chain, at most 256 products, whose error is no larger than that of
+// the same product cut on the 128 x 128 grid, k split while tiles leave SMs idle
+// and each range keeps two k-blocks: every run costs one addition per entry,
+// 0.5 % of the time at 256 products and 3 % at 32. (256 throughout had 2.2 times
+// the error of that grid's split at 384 x 384 x 512, 1.8 times at 384 x 384 x 1024.)
+// A tuned split count is what that grid would use as well: 256 products.
+inline int f64_run(const F64Plan& p, int64_t m, int64_t n, int64_t k, int sm_count, bool tuned) {
+  const int per = p.ts > 16 ? 16 : 4;  // products of an entry per k-block and warp
+  if (tuned) return 256 / per;
+  auto div_up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+  const int64_t kblocks = div_up(k, 16), tiles = div_up(m, 128) * div_up(n, 128);
+  const int64_t ranges = tiles < sm_count
+                             ? std::max<int64_t>(1, std::min<int64_t>({sm_count / tiles, kblocks / 2, 32}))
+                             : 1;
+  const int64_t kb_range = div_up(kblocks, ranges), used = div_up(kblocks, kb_range);
+  const int64_t most = std::min(k, 16 * kb_range) + (used > 1 ? used : 0);
+  int best = 1;
+  int64_t best_error = INT64_MAX;
+  for (int run = 256 / per; run >= 1; --run) {
+    const int64_t runs = div_up(std::min(p.kb_split, kblocks), run);
+    const int64_t error = std::min<int64_t>(run, std::min(p.kb_split, kblocks)) * per + (runs > 1 ? runs : 0) +
+                          (p.splits > 1 ? p.splits : 0) + (per == 4 ? 5 : 0);
+    if (error <= most) return run;
+    if (error < best_error) {
+      best_error = error;
+      best = run;
+    }
+  }
+  return best;
 }
 
 // The f64 plan minimises the FP64 pipe's time on the busiest SM plus what a
@@ -83,6 +121,7 @@ inline F64Plan f64_model(int64_t m, int64_t n, int64_t k, int sm_count, int tune
       if (tuned) break;
     }
   }
+  best.run = f64_run(best, m, n, k, sm_count, tuned != 0);
   return best;
 }
 
