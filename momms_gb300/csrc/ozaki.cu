@@ -38,6 +38,7 @@
 
 #include "internal.h"
 #include "crt_kernels.cuh"
+#include "emulated_forms.cuh"
 #include "exact_round.cuh"
 #include "ozaki_elem.cuh"
 #include "planes.cuh"
@@ -46,21 +47,11 @@
 namespace momms {
 namespace {
 
-constexpr int kDigitBits = elem::kDigitBits;
+using namespace forms;
 using elem::abs_bits;
 using elem::exponent_of_max;
 using elem::magnitude;
 using elem::offset_digits;
-// k per launch (kOzakiMaxK): the largest product of two digits is 2^16, so a
-// single pair's int32 sum stays below 2^31 for up to 511 k-blocks of 64
-constexpr int64_t kMaxK = kOzakiMaxK;
-static_assert((kMaxK / 64) * 64 * (1ll << (2 * kDigitBits)) < (1ll << 31), "int32 digit sums must stay exact");
-// an int32 group sum's bound (sums of the pairs' worst cases)
-constexpr double kGroupLimit = 2147483647.0;
-// one TMEM chunk's bound: integers up to 2^24 are exact in FP32
-constexpr double kChunkBound = 16777216.0;
-// the residue form runs from this k (crt_applies)
-constexpr int64_t kCrtMinK = 128;
 
 // Everything in the pre-pass runs on integer bit patterns: GB300's FP64 pipe
 // is about 1 TFLOP/s, so FP64 arithmetic per element would dominate.
@@ -638,62 +629,6 @@ int set_attrs_ozaki() {
 }
 
 namespace {
-// The slice-product schedule for ns slices over k: diagonals d = t + u from
-// the smallest weight (d = ns+1) to the largest (d = 2), each diagonal's pairs
-// (t, d-t) in t order, cut into accumulation groups whose worst-case int32
-// sums (k * 2^bits_t * 2^bits_u over the group's pairs; the top digit has
-// `bits` bits, the centred ones bits-1) stay within kGroupLimit. A group's
-// A TMEM chunk keeps its sum within kChunkBound: a k-block of pair (t, u)
-// adds at most 64 * 2^bits_t * 2^bits_u, so a pair's weight is that product
-// in units of 2^10 and a chunk's capacity kChunkBound / 64 / 2^10 (a lone
-// pair: 4, 8 or 16 k-blocks of 64 for 8-bit digits; at small k one chunk
-// spans several pairs of a group).
-constexpr int kChunkUnitLog2 = 10;
-constexpr int kChunkCap = (int)(kChunkBound / 64.0) >> kChunkUnitLog2;
-struct Schedule {
-  int np = 0, ng = 0;
-  uint8_t pair_a[sp::MAX_PAIRS], pair_b[sp::MAX_PAIRS];
-  int group_begin[sp::MAX_GROUPS + 1];
-  int pair_w[sp::MAX_PAIRS];
-  uint8_t level[sp::MAX_GROUPS];  // d - 2
-};
-
-bool ozaki_schedule(int ns, int64_t k, Schedule* sc) {
-  const int bits = kDigitBits;
-  const int64_t kblocks = ceil_div(std::min<int64_t>(std::max<int64_t>(k, 1), kMaxK), 64);
-  const double kspan = (double)kblocks * 64.0;
-  auto prod = [&](int t, int u) { return ldexp(1.0, (t == 1 ? bits : bits - 1) + (u == 1 ? bits : bits - 1)); };
-  sc->np = sc->ng = 0;
-  for (int d = ns + 1; d >= 2; --d) {
-    double gsum = 0.0;
-    bool open = false;
-    for (int t = 1; t <= ns; ++t) {
-      const int u = d - t;
-      if (u < 1 || u > ns) continue;
-      const double pb = prod(t, u);
-      if (open && gsum + kspan * pb > kGroupLimit) open = false;  // this pair starts the next group
-      if (!open) {
-        if (sc->ng >= sp::MAX_GROUPS) return false;
-        sc->group_begin[sc->ng] = sc->np;
-        sc->level[sc->ng] = (uint8_t)(d - 2);
-        ++sc->ng;
-        gsum = 0.0;
-        open = true;
-      }
-      if (sc->np >= sp::MAX_PAIRS) return false;
-      sc->pair_a[sc->np] = (uint8_t)(t - 1);
-      sc->pair_b[sc->np] = (uint8_t)(u - 1);
-      sc->pair_w[sc->np] = std::max(1, (int)ldexp(pb, -kChunkUnitLog2));
-      ++sc->np;
-      gsum += kspan * pb;
-    }
-  }
-  sc->group_begin[sc->ng] = sc->np;
-  return true;
-}
-}  // namespace
-
-namespace {
 // The slice kernel's parameters of an ns-slice product over k (rows m): the
 // schedule's pairs and groups, the TMEM chunk rule. Sizes along n, the output
 // planes and the status word are the caller's.
@@ -789,75 +724,6 @@ int launch_combine(CombineParams cp, int64_t j0, int64_t j1, int sm_count, cudaS
 namespace {
 // ---- The residue form (crt_elem.cuh) ---------------------------------------
 #define MOMMS_CRT_NS(X) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15)
-
-// Moduli that hold an ns-slice product whose sums of scaled magnitudes
-// (sum_p |a_ip b_pj| 2^-e_i 2^-f_j, at most k) stay within `sum`: P > 2 |R|,
-// |R| <= sum 2^(16 ns), with 2 % to spare for the quotient's rounding
-// (crt::kFracBits). More moduli than R needs do not change the result.
-int crt_moduli(int ns, double sum) {
-  const double need = 16.0 * ns + log2(std::max(sum, (double)kCrtMinK)) + 1.0 + 0.03;
-  double have = 0.0;
-  int n = 0;
-  while (n < crt::kMaxModuli && have < need) have += log2((double)crt::kModuli[n++]);
-  return n;
-}
-// Whether an ns-slice product runs by residues: where the model below says it
-// is the faster form. From the sizes alone (those of the whole product, where
-// it is streamed in blocks), so that a product gives the same bits alone, in a
-// batch, streamed and from packed operands. The rates are measured ones:
-//  * slice products: 0.26 us per 256 x 256 x 64 step of a CTA pair, 76 pairs,
-//    a group's steps in series (7 pairs of digits, or one modulus, each over
-//    all of k: what decides for few tiles), and per group and entry what of
-//    the epilogue they do not hide: 0.53 ps (digits: 4 bytes of plane), 0.2 ps;
-//  * recombination 7.4 ps per entry (7 digit groups), 10.4 ps (16 moduli);
-//  * operand planes 2 bytes per slice or modulus, 8 read, at 6 TB/s;
-//  * packed operands have their digits, and no residues: 2 bytes read per
-//    slice and written per modulus, at 9 TB/s (much of it stays in L2).
-// The residue form has to be faster either way, by 3 us where operands are not
-// packed: 3776 x 247 x 2224 from packs, 8 slices, 115 us by digits and 156 by
-// residues, 1000 x 1000 x 1000, 7 slices, 62 and 56.
-// Both forms, 7 slices, ms per call: 8192 x 8192 x 128 1.33 (digits) and 1.40,
-// x 256 1.61 and 1.56, x 1024 3.17 and 2.48, x 8192 20.9 and 13.1; 65536 x 256 x
-// 256 0.64 and 0.75; the slice kernel alone at 512^3 0.030 and 0.014.
-bool crt_applies(int ns, int64_t m, int64_t n, int64_t k) {
-  if (ns < 5 || k < kCrtMinK) return false;
-  const int N = crt_moduli(ns, k);
-  Schedule sc;
-  if (!ozaki_schedule(ns, k, &sc)) return true;
-  constexpr double kPairs = 76.0, kStep = 0.26e6, kMargin = 3e6;  // ps
-  const double mn = (double)m * n, ops = (double)(m + n) * k;
-  const double tiles = (double)(ceil_div(m, 256) * ceil_div(n, 256)), steps = (double)ceil_div(k, 64) * kStep;
-  auto products = [&](double pairs, double longest) { return steps * std::max(pairs * tiles / kPairs, longest); };
-  const double digits = products(sc.np, ns) + mn * (0.53 * sc.ng + 2.7 + 0.67 * sc.ng);
-  const double residues = products(N, 1.0) + mn * (0.2 * N + 0.65 * N);
-  return residues + ops * (8 + 2 * N) / 6.0 + kMargin < digits + ops * (8 + 2 * ns) / 6.0 &&
-         residues + ops * (2 * ns + 2 * N) / 9.0 < digits;
-}
-
-// Scratch of an emulated product, operand planes and group planes: the digit
-// form's, or the residue form's with `per` moduli per pass.
-double plane_bytes(int64_t m, int64_t n) { return (double)round_up(m, sp::BM) * (double)round_up(n, sp::BN); }
-double digit_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
-  Schedule sc;
-  const double ng = ozaki_schedule(ns, k, &sc) ? sc.ng : sp::MAX_GROUPS;
-  return 2.0 * ns * (double)(m + n) * (double)plane_row(std::min(k, kMaxK), 8, tight) + 4.0 * ng * plane_bytes(m, n);
-}
-double crt_scratch(int per, int moduli, int64_t m, int64_t n, int64_t k, bool tight) {
-  return 2.0 * per * (double)(m + n) * (double)plane_row(std::min(k, kMaxK), 8, tight) + moduli * plane_bytes(m, n);
-}
-// The residue form keeps to the digit form's scratch (or kFreeScratch bytes, unless
-// `tight`) by walking the moduli in several passes, each with its own operand
-// planes: at 8192^3 two passes of 8 moduli instead of 4.6 GB of planes, for one
-// more read of the operands (0.2 of 13 ms). Where a call is small a second pass
-// shows: 2600 x 2600 x 2600 786 us in two, 754 in one, 4096 x 1024 x 4096 728
-// and 678.
-int crt_per_pass(int ns, int N, int64_t m, int64_t n, int64_t k, bool tight) {
-  const double limit = std::max(digit_scratch(ns, m, n, k, tight), tight ? 0.0 : (double)kFreeScratch);
-  int per = N;
-  while (per > 1 && crt_scratch(per, N, m, n, k, tight) > limit) --per;
-  const int passes = (int)ceil_div(N, per);
-  return (int)ceil_div(N, passes);
-}
 
 // Residue planes l0..l1-1 of the sides, or of packed operands' digits.
 void crt_planes(int ns, const Side* sides, int count, int64_t K, __half* const* out, int64_t ldp,
@@ -989,10 +855,12 @@ int plane_map(CUtensorMap* map, const void* base, int64_t k, int64_t rows, int p
 }  // namespace
 
 double ozaki_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
-  const double d = digit_scratch(ns, m, n, k, tight);
+  const Sizes z = sizes_of(m, n, k, tight);
+  const double d = digit_scratch(ns, k, z);
   const int64_t kk = std::min(k, kMaxK);
   if (!crt_applies(ns, m, n, kk)) return d;
-  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, crt_moduli(ns, kk), m, n, kk, tight), crt_moduli(ns, kk), m, n, kk, tight));
+  const int N = crt_moduli(ns, kk);
+  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, N, kk, z, free_scratch(ns, kk, z, tight)), N, z));
 }
 
 namespace {
@@ -1526,40 +1394,55 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   // row strides of the planes: a packed operand's are the pack's
   const int64_t kp = plane_row(k, 8, g.tight), kpa = PA ? PA->kp : kp, kpb = PB ? PB->kp : kp;
   const size_t a_plane = (size_t)m * kpa, b_plane = (size_t)n * kpb;
-  // The form: digit planes (one pass; packed operands bring theirs), or
-  // residue planes in passes of `per` moduli.
-  const bool crt = crt_applies(ns, g.whole_m ? g.whole_m : m, g.whole_n ? g.whole_n : n, k);
-  const int N = crt ? crt_moduli(ns, sum_most) : ns;
   if (k > kMaxK) return fail(MOMMS_ERR_UNSUPPORTED, "Ozaki emulation supports k <= %lld per launch", (long long)kMaxK);
-  sp::Params p;
-  Schedule sch;
-  if (!crt && !slice_params(ns, m, k, &p, &sch))
-    return fail(MOMMS_ERR_UNSUPPORTED, "Ozaki schedule needs too many groups");
-  const int np = crt ? N : sch.np, ng = crt ? N : sch.ng;
-  call_info().slices = ns;
-  call_info().pairs = np;
-  call_info().groups = ng;
-
-  char* sbuf = nullptr;
   // group planes tile-blocked (sp::Params::sbuf): m and n padded to whole
   // 128 x 256 tiles, each tile one contiguous block of int32 or residue bytes
   const int64_t mpad = round_up(m, (int64_t)sp::BM);
-  const size_t plane = (size_t)mpad * (size_t)round_up(n, (int64_t)sp::BN), word = crt ? 1 : sizeof(int);
-  if ((ce = scratch_alloc(&sbuf, (size_t)ng * plane * word, s)) != cudaSuccess) return cuda_fail(ce, "Ozaki group sums");
-  ScratchGuard free_sbuf(sbuf, s);
-  // The operand planes of a pass. The residue form's free scratch is taken
-  // only where there is room for it, else the passes it gets by with.
-  const bool own_a = crt || !PA, own_b = crt || !PB;
-  auto own_bytes = [&](int count) {
-    return sizeof(__half) * (size_t)count * ((own_a ? a_plane : 0) + (own_b ? b_plane : 0));
-  };
-  int per = crt ? crt_per_pass(ns, N, m, n, k, g.tight) : ns;
-  const int least = crt ? crt_per_pass(ns, N, m, n, k, true) : per;
+  const size_t plane = (size_t)mpad * (size_t)round_up(n, (int64_t)sp::BN);
+  const Sizes z{(double)(a_plane + b_plane), (double)((PA ? 0 : a_plane) + (PB ? 0 : b_plane)), (double)plane};
+  // The form: digit planes (one pass; packed operands bring theirs), or
+  // residue planes in passes of `per` moduli. What the residue form takes beyond
+  // the digit form's scratch is taken only where there is room for it, else the
+  // passes it gets by with; from packs, whose digits are there, the digits where
+  // there is no room for its least pass either.
+  bool crt = crt_applies(ns, g.whole_m ? g.whole_m : m, g.whole_n ? g.whole_n : n, k);
+  int N = 0, ng = 0, per = 0;
+  sp::Params p;
+  Schedule sch;
+  char* sbuf = nullptr;
   __half* planes_buf = nullptr;
-  if (least < per && !scratch_alloc_if_room(&planes_buf, own_bytes(per), s)) per = least;
-  if (!planes_buf && own_bytes(per) && (ce = scratch_alloc(&planes_buf, own_bytes(per), s)) != cudaSuccess)
-    return cuda_fail(ce, "Ozaki slice planes");
-  ScratchGuard free_planes(planes_buf, s);
+  ScratchGuard free_sbuf(nullptr, s), free_planes(nullptr, s);
+  bool own_a, own_b;
+  for (;;) {
+    N = crt ? crt_moduli(ns, sum_most) : ns;
+    if (!crt && !slice_params(ns, m, k, &p, &sch))
+      return fail(MOMMS_ERR_UNSUPPORTED, "Ozaki schedule needs too many groups");
+    ng = crt ? N : sch.ng;
+    ce = scratch_alloc(&sbuf, (size_t)ng * plane * (crt ? 1 : sizeof(int)), s);
+    if (ce != cudaSuccess) return cuda_fail(ce, "Ozaki group sums");
+    free_sbuf.p = sbuf;
+    own_a = crt || !PA, own_b = crt || !PB;
+    auto own_bytes = [&](int count) {
+      return sizeof(__half) * (size_t)count * ((own_a ? a_plane : 0) + (own_b ? b_plane : 0));
+    };
+    per = crt ? crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, g.tight)) : ns;
+    const int least = crt ? crt_per_pass(ns, N, k, z, 0.0) : per;
+    if (least < per && !scratch_alloc_if_room(&planes_buf, own_bytes(per), s)) per = least;
+    if (planes_buf || !own_bytes(per)) break;
+    if (!crt || (!PA && !PB)) {
+      if ((ce = scratch_alloc(&planes_buf, own_bytes(per), s)) != cudaSuccess) return cuda_fail(ce, "Ozaki slice planes");
+      break;
+    }
+    if (scratch_alloc_if_room(&planes_buf, own_bytes(per), s)) break;
+    crt = false;
+    free_sbuf.p = nullptr;
+    cudaFreeAsync(sbuf, s);
+  }
+  free_planes.p = planes_buf;
+  const size_t word = crt ? 1 : sizeof(int);
+  call_info().slices = ns;
+  call_info().pairs = crt ? N : sch.np;
+  call_info().groups = ng;
   const int passes = (int)ceil_div(N, per);
   const __half* pa = own_a ? planes_buf : static_cast<const __half*>(PA->planes);
   const __half* pb = own_b ? planes_buf + (own_a ? (size_t)per * a_plane : 0) : static_cast<const __half*>(PB->planes);
@@ -1859,7 +1742,10 @@ bool ozaki_batchable(const DevGemm& g, int slices) {
         g.k > 0))
     return false;
   // residues only where one pass holds them all
-  return !crt_applies(slices, g.m, g.n, g.k) || crt_per_pass(slices, crt_moduli(slices, g.k), g.m, g.n, g.k, false) == crt_moduli(slices, g.k);
+  if (!crt_applies(slices, g.m, g.n, g.k)) return true;
+  const Sizes z = sizes_of(g.m, g.n, g.k, false);
+  const int N = crt_moduli(slices, g.k);
+  return crt_per_pass(slices, N, g.k, z, free_scratch(slices, g.k, z, false)) == N;
 }
 
 void ozaki_batch_destroy(OzakiBatch* b) {

@@ -113,3 +113,58 @@ def test_residues_of_packed_digits(gpu, s):
     finally:
         for h in packs:
             gpu.momms_packed_destroy(h)
+
+
+def _pack(gpu, role, x, s):
+    t, rs, cs = gu.to_device(x)
+    h = ctypes.c_void_p()
+    mg.check(gpu.momms_pack(mg.DTYPE_F64, mg.PREC_OZAKI, role, x.shape[0], x.shape[1],
+                            ctypes.byref(mg.Operand(t.data_ptr(), rs, cs, mg.MEM_DEVICE, 0)), s, None, ctypes.byref(h)), gpu)
+    return h
+
+
+def _packed_call(gpu, packs, A, B, C0, s):
+    """C0 + A B with the operands of `packs` (None: unpacked)."""
+    import torch
+    m, n, k = A.shape[0], B.shape[1], A.shape[1]
+    (ta, *sa), (tb, *sb), (tc, *sc) = (gu.to_device(x) for x in (A, B, C0))
+    d = gu.make_desc(mg.DTYPE_F64, m, n, k, 1.0, 1.0, (ta.data_ptr(), *sa), (tb.data_ptr(), *sb), (tc.data_ptr(), *sc),
+                     precision=mg.PREC_OZAKI, mem=mg.MEM_DEVICE, slices=s)
+    if packs[0]:
+        d.a = mg.Operand(packs[0].value, 0, 0, mg.MEM_PACKED, 0)
+    if packs[1]:
+        d.b = mg.Operand(packs[1].value, 0, 0, mg.MEM_PACKED, 0)
+    mg.check(gpu.momms_gemm(ctypes.byref(d), None), gpu)
+    info = mg.CallInfo()
+    gpu.momms_last_info(ctypes.byref(info))
+    torch.cuda.synchronize()
+    return tc.cpu().numpy(), info
+
+
+@pytest.mark.parametrize("which", ["none", "a", "b", "ab"])
+def test_without_room_for_more_scratch(gpu, monkeypatch, which):
+    """Where the device has no room beyond the digit form's scratch: the same bits in more passes;
+    from packs, whose digits are there, the digit form."""
+    m, n, k, s = 1300, 1027, 1025, 7
+    rng = np.random.default_rng(77)
+    A = np.asfortranarray(rng.uniform(-1, 1, (m, k)))
+    B = np.asfortranarray(rng.uniform(-1, 1, (k, n)))
+    C0 = np.zeros((m, n), order="F")
+    packs = [_pack(gpu, mg.ROLE_A, A, s) if "a" in which.replace("none", "") else None,
+             _pack(gpu, mg.ROLE_B, B, s) if "b" in which else None]
+    try:
+        want, info = _packed_call(gpu, packs, A, B, C0, s)
+        assert info.pairs < s * (s + 1) // 2
+        monkeypatch.setenv("MOMMS_FREE_SCRATCH", "0")
+        got, info = _packed_call(gpu, packs, A, B, C0, s)
+    finally:
+        for h in packs:
+            if h:
+                mg.check(gpu.momms_packed_destroy(h), gpu)
+    if which == "none":
+        assert info.pairs < s * (s + 1) // 2 and np.array_equal(got, want)
+        return
+    assert info.pairs == s * (s + 1) // 2
+    # digits rounded at 2^-(8s+1), the diagonals past s + 1 left out, one rounding
+    ref, _ = ou.dd_gemm(A, B, C0)
+    assert np.all(np.abs(got - ref) <= 1.01 * (2.0**-53 * np.abs(ref) + 2.0 ** (-8 * s - 1) * k * (2 + (s - 1) / 2)))
