@@ -5,6 +5,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "crt_elem.cuh"
 #include "internal.h"
@@ -160,6 +161,27 @@ inline int crt_per_pass(int ns, int N, int64_t k, const Sizes& z, double free) {
 // nine times). `tight`: nothing.
 inline double free_scratch(int ns, int64_t k, const Sizes& z, bool tight) {
   return tight ? 0.0 : std::max((double)kFreeScratch, digit_scratch(ns, k, Sizes{z.ops, z.ops, z.c}));
+}
+
+// A plan holds the scratch of the problems it runs in one slice launch for as
+// long as it lives, residues in one pass. Which of its problems do: those that
+// add least beyond the digit form, while the sum stays within `limit` (a plan of
+// eight 4096 x 1024 x 4096 products would hold 5.9 GB for 3.3 by digits). The
+// others, the largest, run on their own, each in scratch that the next reuses.
+inline double batch_extra(int ns, int64_t m, int64_t n, int64_t k) {
+  if (!crt_applies(ns, m, n, k)) return 0.0;
+  const Sizes z = sizes_of(m, n, k, false);
+  const int N = crt_moduli(ns, k);
+  return std::max(0.0, crt_scratch(N, N, z) - digit_scratch(ns, k, z));
+}
+inline std::vector<char> batch_members(const std::vector<double>& extra, double limit) {
+  std::vector<size_t> order(extra.size());
+  for (size_t i = 0; i < order.size(); ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return extra[x] < extra[y]; });
+  std::vector<char> in(extra.size(), 0);
+  double sum = 0.0;
+  for (size_t i : order) in[i] = (sum += extra[i]) <= limit;
+  return in;
 }
 
 }  // namespace forms

@@ -412,21 +412,31 @@ int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_
   {
     std::vector<DevGemm> gs;
     std::vector<int> sl;
-    std::vector<PlanProblem> rest;
-    for (PlanProblem& pp : p->other) {
+    std::vector<size_t> at;
+    for (size_t i = 0; i < p->other.size(); ++i) {
+      const PlanProblem& pp = p->other[i];
       const DevGemm g = devgemm_of(pp.d);
-      if (pp.d.precision == MOMMS_PREC_OZAKI && ozaki_batchable(g, pp.slices)) {
-        gs.push_back(g);
-        sl.push_back(pp.slices);
-      } else {
-        rest.push_back(pp);
-      }
+      if (pp.d.precision != MOMMS_PREC_OZAKI || !ozaki_batchable(g, pp.slices)) continue;
+      gs.push_back(g);
+      sl.push_back(pp.slices);
+      at.push_back(i);
+    }
+    const std::vector<char> in = ozaki_batch_members(gs.data(), sl.data(), (int)gs.size());
+    std::vector<char> joined(p->other.size(), 0);
+    size_t count = 0;
+    for (size_t i = 0; i < gs.size(); ++i) {
+      if (!in[i]) continue;
+      joined[at[i]] = 1;
+      gs[count] = gs[i];
+      sl[count++] = sl[i];
     }
     int clusters = 0;
-    if (gs.size() >= 2 && sp_pairs_available(&clusters)) {
-      const int rc = ozaki_batch_create(gs.data(), sl.data(), (int)gs.size(), async ? async_stream : nullptr, async,
-                                        &p->ozb);
+    if (count >= 2 && sp_pairs_available(&clusters)) {
+      const int rc = ozaki_batch_create(gs.data(), sl.data(), (int)count, async ? async_stream : nullptr, async, &p->ozb);
       if (rc) { plan_free(p); return rc; }
+      std::vector<PlanProblem> rest;
+      for (size_t i = 0; i < p->other.size(); ++i)
+        if (!joined[i]) rest.push_back(p->other[i]);
       p->other = rest;
     }
   }

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/momms_gpu.h"
 #include "f64_plan.h"
@@ -299,6 +300,8 @@ int dmma_problem(const DevGemm& g, const F64Plan& plan, dmma::DProblem* P, CUten
 // with a fixed slice count, unpacked operands and k within one launch.
 struct OzakiBatch;
 bool ozaki_batchable(const DevGemm& g, int slices);
+// Which of `count` qualifying problems a plan runs together, within its scratch.
+std::vector<char> ozaki_batch_members(const DevGemm* gs, const int* slices, int count);
 // True when this device can run the CTA-pair slice kernel (*clusters: pairs at once).
 bool sp_pairs_available(int* clusters);
 int ozaki_batch_create(const DevGemm* gs, const int* slices, int count, cudaStream_t s, bool async, OzakiBatch** out);

@@ -1748,6 +1748,12 @@ bool ozaki_batchable(const DevGemm& g, int slices) {
   return crt_per_pass(slices, N, g.k, z, free_scratch(slices, g.k, z, false)) == N;
 }
 
+std::vector<char> ozaki_batch_members(const DevGemm* gs, const int* slices, int count) {
+  std::vector<double> extra;
+  for (int i = 0; i < count; ++i) extra.push_back(batch_extra(slices[i], gs[i].m, gs[i].n, gs[i].k));
+  return batch_members(extra, (double)kFreeScratch);
+}
+
 void ozaki_batch_destroy(OzakiBatch* b) {
   if (!b) return;
   auto release = [&](void* p) {

@@ -49,6 +49,19 @@ int main() {
   z.own = 0.0;
   expect(crt_scratch(crt_per_pass(7, 17, 8192, z, 0.0), 17, z) <= 1.9e9, "packs", 7, 8192, 8192, 8192);
   for (int i = 0; i < 20000; ++i) check(5 + i % 11, size(32, 20000), size(32, 20000), size(128, 32704));
+  // plans: what their problems hold together beyond the digit form
+  for (int trial = 0; trial < 300; ++trial) {
+    std::vector<double> extra;
+    double together = 0.0;
+    const int count = 1 + (int)(rnd() * 60);
+    for (int i = 0; i < count; ++i) extra.push_back(batch_extra(5 + (int)(rnd() * 6), size(64, 5000), size(64, 5000), size(64, 5000)));
+    const std::vector<char> in = batch_members(extra, (double)kFreeScratch);
+    double left = 0.0;
+    for (int i = 0; i < count; ++i) (in[i] ? together : left) += extra[i];
+    expect(together <= (double)kFreeScratch, "plan", 0, count, 0, 0);
+    expect(together + left > (double)kFreeScratch || left == 0.0, "all of a small plan", 0, count, 0, 0);
+  }
+  expect(batch_extra(7, 4096, 1024, 4096) * 8 > (double)kFreeScratch, "known plan", 7, 4096, 1024, 4096);
   if (failures) return printf("%d failures\n", failures), 1;
   puts("OK");
   return 0;

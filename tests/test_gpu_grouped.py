@@ -190,3 +190,28 @@ def test_emulated_problems_share_one_slice_launch(gpu):
         for i in range(len(shapes)):
             assert np.array_equal(keep[i][2].cpu().numpy(), expected[i]), (rep, i)
     mg.check(gpu.momms_plan_destroy(plan), gpu)
+
+
+def test_plan_of_large_emulated_problems_bounds_its_scratch(gpu):
+    """Eight emulated problems whose residue planes would add 2.6 GB to what the digit form holds: the
+    plan holds at most 1 GB more, and every result has the bits of the problem alone."""
+    import torch
+    m, n, k, s, count = 4096, 1024, 4096, 7, 8
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    a, b = (torch.rand(shape, dtype=torch.float64, device="cuda", generator=gen) - 0.5 for shape in ((k, m), (n, k)))
+    cs = [torch.zeros((n, m), dtype=torch.float64, device="cuda") for _ in range(count + 1)]
+    descs = (mg.GemmDesc * (count + 1))(*[
+        gu.make_desc(mg.DTYPE_F64, m, n, k, 1.0, 0.0, (a.data_ptr(), 1, m), (b.data_ptr(), 1, k), (c.data_ptr(), 1, m),
+                     precision=mg.PREC_OZAKI, mem=mg.MEM_DEVICE, slices=s) for c in cs])
+    mg.check(gpu.momms_gemm(ctypes.byref(descs[count]), None), gpu)  # alone
+    torch.cuda.synchronize()
+    plan = ctypes.c_void_p()
+    free = torch.cuda.mem_get_info()[0]
+    mg.check(gpu.momms_plan_create(descs, count, ctypes.byref(plan)), gpu)
+    held = free - torch.cuda.mem_get_info()[0]
+    assert held <= count * (2 * s * (m + n) * k + 4 * s * m * n) + (1 << 30) + (64 << 20)
+    mg.check(gpu.momms_plan_launch(plan, None), gpu)
+    torch.cuda.synchronize()
+    for c in cs[:count]:
+        assert torch.equal(c, cs[count])
+    mg.check(gpu.momms_plan_destroy(plan), gpu)
