@@ -163,6 +163,17 @@ inline double free_scratch(int ns, int64_t k, const Sizes& z, bool tight) {
   return tight ? 0.0 : std::max((double)kFreeScratch, digit_scratch(ns, k, Sizes{z.ops, z.ops, z.c}));
 }
 
+// The most an ns-slice product takes, whatever its operands (an automatic count
+// may need fewer moduli than k asks for, and then more of them fit a pass).
+inline double emulated_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
+  const Sizes z = sizes_of(m, n, k, tight);
+  const double d = digit_scratch(ns, k, z);
+  const int64_t kk = std::min(k, kMaxK);
+  if (!crt_applies(ns, m, n, kk) || tight) return d;
+  const int N = crt_moduli(ns, (double)kk);
+  return std::max(d, std::min(crt_scratch(N, N, z), free_scratch(ns, kk, z, false)));
+}
+
 // A plan holds the scratch of the problems it runs in one slice launch for as
 // long as it lives, residues in one pass. Which of its problems do: those that
 // add least beyond the digit form, while the sum stays within `limit` (a plan of

@@ -133,6 +133,12 @@ __global__ void __launch_bounds__(ffma::Tile<TM>::THREADS, ffma::Tile<TM>::CTAS_
 struct PlanProblem {
   momms_gemm_desc d;
   int slices;  // Ozaki: frozen slice count
+  bool tight;  // DevGemm::tight
+  DevGemm gemm() const {
+    DevGemm g = devgemm_of(d);
+    g.tight = tight;
+    return g;
+  }
 };
 
 struct Plan {
@@ -233,7 +239,8 @@ int plan_zero(Plan* p, void* dst, size_t bytes) {
   return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "plan workspace");
 }
 
-int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_t async_stream, bool async) {
+int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_t async_stream, bool async,
+                const char* tight) {
   *out = nullptr;
   if (!descs || count < 0) return fail(MOMMS_ERR_INVALID_ARG, "descs is null or count < 0");
   DeviceState* ds = device_state();
@@ -260,7 +267,7 @@ int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_
     if (d.m == 0 || d.n == 0 || d.k == 0) continue;
     if (d.precision == MOMMS_PREC_PLAIN && d.dtype == MOMMS_DTYPE_F64) dlist.push_back(i);
     else if (d.precision == MOMMS_PREC_PLAIN) slist.push_back(i);
-    else p->other.push_back(PlanProblem{d, d.slices});
+    else p->other.push_back(PlanProblem{d, d.slices, tight && tight[i]});
   }
 
   // ---- f64 group ----
@@ -415,7 +422,7 @@ int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_
     std::vector<size_t> at;
     for (size_t i = 0; i < p->other.size(); ++i) {
       const PlanProblem& pp = p->other[i];
-      const DevGemm g = devgemm_of(pp.d);
+      const DevGemm g = pp.gemm();
       if (pp.d.precision != MOMMS_PREC_OZAKI || !ozaki_batchable(g, pp.slices)) continue;
       gs.push_back(g);
       sl.push_back(pp.slices);
@@ -494,7 +501,7 @@ int plan_launch(Plan* p, cudaStream_t s, int max_sms) {
     if (rc) return rc;
   }
   for (PlanProblem& pp : p->other) {
-    const DevGemm g = devgemm_of(pp.d);
+    const DevGemm g = pp.gemm();
     int rc;
     if (pp.d.precision == MOMMS_PREC_OZAKI) {
       int used = 0;
@@ -522,7 +529,7 @@ int momms_plan_create(const momms_gemm_desc* descs, int count, momms_plan* out) 
   if (!out) return momms::fail(MOMMS_ERR_INVALID_ARG, "out is null");
   *out = nullptr;
   momms::Plan* p = nullptr;
-  int rc = momms::plan_create(descs, count, &p, nullptr, false);
+  int rc = momms::plan_create(descs, count, &p, nullptr, false, nullptr);
   if (rc) return rc;
   *out = new momms_plan_s{p};
   return MOMMS_OK;

@@ -324,7 +324,9 @@ int set_attrs_ozaki();
 // are stream-ordered on `stream` (no device-wide synchronisation); otherwise
 // plan_create is synchronous.
 struct Plan;
-int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_t stream, bool async);
+// `tight` (may be null): the problems that run with DevGemm::tight.
+int plan_create(const momms_gemm_desc* descs, int count, Plan** out, cudaStream_t stream, bool async,
+                const char* tight);
 // max_sms > 0 caps the persistent grids, leaving SMs for concurrent work.
 int plan_launch(Plan* p, cudaStream_t s, int max_sms);
 void plan_destroy(Plan* p);

@@ -855,12 +855,7 @@ int plane_map(CUtensorMap* map, const void* base, int64_t k, int64_t rows, int p
 }  // namespace
 
 double ozaki_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
-  const Sizes z = sizes_of(m, n, k, tight);
-  const double d = digit_scratch(ns, k, z);
-  const int64_t kk = std::min(k, kMaxK);
-  if (!crt_applies(ns, m, n, kk)) return d;
-  const int N = crt_moduli(ns, kk);
-  return std::max(tight ? d : 0.0, crt_scratch(crt_per_pass(ns, N, kk, z, free_scratch(ns, kk, z, tight)), N, z));
+  return emulated_scratch(ns, m, n, k, tight);
 }
 
 namespace {
@@ -1743,9 +1738,9 @@ bool ozaki_batchable(const DevGemm& g, int slices) {
     return false;
   // residues only where one pass holds them all
   if (!crt_applies(slices, g.m, g.n, g.k)) return true;
-  const Sizes z = sizes_of(g.m, g.n, g.k, false);
+  const Sizes z = sizes_of(g.m, g.n, g.k, g.tight);
   const int N = crt_moduli(slices, g.k);
-  return crt_per_pass(slices, N, g.k, z, free_scratch(slices, g.k, z, false)) == N;
+  return crt_per_pass(slices, N, g.k, z, free_scratch(slices, g.k, z, g.tight)) == N;
 }
 
 std::vector<char> ozaki_batch_members(const DevGemm* gs, const int* slices, int count) {
@@ -1810,7 +1805,7 @@ int ozaki_batch_create(const DevGemm* gs, const int* slices, int count, cudaStre
       break;
     }
     const int ng = P.crt ? P.planes_each : sch.ng;
-    P.kp = plane_row(k, 8, false);
+    P.kp = plane_row(k, 8, P.g.tight);
     P.a_plane = (size_t)m * P.kp;
     P.b_plane = (size_t)n * P.kp;
     const int64_t mpad = round_up(m, (int64_t)sp::BM);

@@ -39,6 +39,7 @@ namespace {
 struct Request {
   momms_gemm_desc d;
   size_t footprint = 0;
+  bool tight = false;  // admitted on the tight footprint
   double flops = 0.0;
   double est_s = 0.0;
   double submit_s = 0.0, start_s = 0.0, done_s = 0.0;
@@ -72,15 +73,15 @@ double estimate_s(const momms_gemm_desc& d) {
   return flops / rate;
 }
 
-// Operands and work space. A request whose work space would pass the budget
-// only in the larger form it may take (work_bytes) is charged the whole budget.
-size_t footprint_of(const momms_gemm_desc& d, uint64_t budget) {
+// Operands and work space. A request whose work space passes the budget only in
+// the larger form it may take (work_bytes) runs, and is charged, in the tight one.
+size_t footprint_of(const momms_gemm_desc& d, uint64_t budget, bool* tight) {
   const size_t es = d.dtype == MOMMS_DTYPE_F64 ? 8 : 4;
   const double m = (double)d.m, n = (double)d.n, k = (double)d.k;
   const size_t ops = (size_t)(es * (m * k + k * n + m * n));
   const size_t most = ops + work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k, false);
-  if (most <= budget) return most;
-  return std::max<size_t>(ops + work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k, true), budget);
+  *tight = most > budget;
+  return *tight ? ops + work_bytes(d.dtype, d.precision, d.slices, d.m, d.n, d.k, true) : most;
 }
 
 }  // namespace
@@ -203,6 +204,7 @@ struct Server {
         Batch b;
         b.stream = sidx;
         std::vector<momms_gemm_desc> descs;
+        std::vector<char> tight;
         double est = 0.0;
         const bool big_slot = big_inflight < (int)streams.size() - 1 || streams.size() == 1;
         for (auto it = ready.begin(); it != ready.end() && (int)b.ids.size() < cfg.max_batch;) {
@@ -211,7 +213,7 @@ struct Server {
             if (b.ids.empty() && big_slot) {
               b.big = true;
               b.ids.push_back(*it);
-              descs.push_back(r.d);
+              descs.push_back(r.d), tight.push_back(r.tight);
               r.start_s = now();
               ready.erase(it);
               break;
@@ -222,7 +224,7 @@ struct Server {
           if (!b.ids.empty() && est + r.est_s > kQuantumS) break;
           est += r.est_s;
           b.ids.push_back(*it);
-          descs.push_back(r.d);
+          descs.push_back(r.d), tight.push_back(r.tight);
           r.start_s = now();
           it = ready.erase(it);
         }
@@ -239,7 +241,7 @@ struct Server {
                    (unsigned long long)next_batch, descs.size(), sidx);
           nvtxRangePushA(msg);
         }
-        int rc = plan_create(descs.data(), (int)descs.size(), &b.plan, s, true);
+        int rc = plan_create(descs.data(), (int)descs.size(), &b.plan, s, true, tight.data());
         cudaError_t e = cudaSuccess;
         if (!rc) {
           e = cudaEventCreate(&b.ev_start);
@@ -346,7 +348,8 @@ int momms_server_submit(momms_server server, const momms_gemm_desc* desc, uint64
         return fail(MOMMS_ERR_INVALID_ARG, "served requests keep their operands resident in device memory");
       }
     }
-  const size_t fp = footprint_of(*desc, sv->cfg.hbm_budget_bytes);
+  bool tight = false;
+  const size_t fp = footprint_of(*desc, sv->cfg.hbm_budget_bytes, &tight);
   std::lock_guard<std::mutex> lk(sv->mu);
   if (sv->stop) return fail(MOMMS_ERR_SHUTDOWN, "server is stopping");
   if (fp > sv->cfg.hbm_budget_bytes) {
@@ -360,6 +363,7 @@ int momms_server_submit(momms_server server, const momms_gemm_desc* desc, uint64
   Request r;
   r.d = *desc;
   r.footprint = fp;
+  r.tight = tight;
   r.flops = 2.0 * (double)desc->m * (double)desc->n * (double)desc->k;
   r.est_s = estimate_s(*desc);
   r.submit_s = sv->now();

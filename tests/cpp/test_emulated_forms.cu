@@ -31,6 +31,11 @@ static void check(int ns, int64_t m, int64_t n, int64_t k) {
       if (!packs) expect(crt_scratch(least, N, z) <= digits, "within the digit form", ns, m, n, k);
       expect(crt_scratch(most, N, z) <= std::max(digits, free_scratch(ns, k, z, tight)) || most == 1, "free scratch", ns, m, n, k);
       if (tight) expect(most == least, "tight", ns, m, n, k);
+      // what admission and streaming charge for it, whatever number of moduli the data need
+      for (int moduli = crt_moduli(ns, 1.0); moduli <= N; ++moduli) {
+        const int per = crt_per_pass(ns, moduli, k, z, free_scratch(ns, k, z, tight));
+        expect(crt_scratch(per, moduli, z) <= emulated_scratch(ns, m, n, k, tight), "charge", ns, m, n, k);
+      }
     }
 }
 

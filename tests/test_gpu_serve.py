@@ -169,3 +169,45 @@ def test_emulated_requests_of_a_batch_share_one_slice_launch(gpu):
     assert slice_launches.value == len(batches) < len(reqs)
     for (d, dev, host), exp in zip(reqs, expected):
         assert np.array_equal(dev[2].cpu().numpy(), exp)
+
+
+TIGHT_REQUEST = """
+import ctypes, sys
+import torch
+import momms_gb300 as mg
+from tests import gpu_util as gu
+lib = mg.load_library()
+m, n, k, s, budget = 4096, 1024, 4096, 7, 700 << 20
+gen = torch.Generator(device="cuda").manual_seed(3)
+a, b = (torch.rand(x, dtype=torch.float64, device="cuda", generator=gen) - 0.5 for x in ((k, m), (n, k)))
+served, alone = (torch.zeros((n, m), dtype=torch.float64, device="cuda") for _ in range(2))
+descs = [gu.make_desc(mg.DTYPE_F64, m, n, k, 1.0, 0.0, (a.data_ptr(), 1, m), (b.data_ptr(), 1, k), (c.data_ptr(), 1, m),
+                      precision=mg.PREC_OZAKI, mem=mg.MEM_DEVICE, slices=s) for c in (served, alone)]
+cfg = mg.ServerConfig(hbm_budget_bytes=budget, max_batch=4, max_inflight=1, queue_capacity=8)
+srv, rid = ctypes.c_void_p(), ctypes.c_uint64()
+mg.check(lib.momms_server_create(ctypes.byref(cfg), ctypes.byref(srv)), lib)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+mg.check(lib.momms_server_submit(srv, ctypes.byref(descs[0]), ctypes.byref(rid)), lib)
+mg.check(lib.momms_server_wait(srv, rid, 60.0, None), lib)
+held = free - torch.cuda.mem_get_info()[0]  # the scratch pool keeps what it grew by
+mg.check(lib.momms_server_destroy(srv), lib)
+mg.check(lib.momms_gemm(ctypes.byref(descs[1]), None), lib)
+torch.cuda.synchronize()
+operands = 8 * (m * k + k * n + m * n)
+print(held, budget - operands, torch.equal(served, alone))
+assert torch.equal(served, alone)
+assert held <= budget - operands + (64 << 20)
+"""
+
+
+def test_request_admitted_on_its_tight_footprint_keeps_to_it(gpu):
+    """A request whose larger scratch passes the budget runs in the smaller one it was charged for, with
+    the bits of the call alone. In a process of its own: the scratch pool starts empty."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", TIGHT_REQUEST], cwd=root, capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, PYTHONPATH=root))
+    assert r.returncode == 0, r.stdout + r.stderr
