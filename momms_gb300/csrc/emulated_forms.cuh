@@ -158,11 +158,14 @@ inline int crt_per_pass(int ns, int N, int64_t k, const Sizes& z, double free) {
 // What a call may take where the device has room for it: kFreeScratch, and as
 // much again as the digits that packed operands bring (in passes within the
 // digit form's own scratch, 8192 x 8192 x 8192 from packs re-reads the digits
-// nine times). `tight`: nothing.
-inline double free_scratch(int ns, int64_t k, const Sizes& z, bool tight) {
-  return tight ? 0.0 : std::max((double)kFreeScratch, digit_scratch(ns, k, Sizes{z.ops, z.ops, z.c}));
+// nine times). A call under stream capture has its scratch allocated when its
+// graph is launched, where no second choice is left: kCapturedScratch, enough
+// for one pass of the small calls to which a pass matters. `tight`: nothing.
+constexpr double kCapturedScratch = 256.0 * (1 << 20);
+inline double free_scratch(int ns, int64_t k, const Sizes& z, bool tight, bool captured) {
+  if (tight) return 0.0;
+  return captured ? kCapturedScratch : std::max((double)kFreeScratch, digit_scratch(ns, k, Sizes{z.ops, z.ops, z.c}));
 }
-
 // The most an ns-slice product takes, whatever its operands (an automatic count
 // may need fewer moduli than k asks for, and then more of them fit a pass).
 inline double emulated_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tight) {
@@ -171,7 +174,7 @@ inline double emulated_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tig
   const int64_t kk = std::min(k, kMaxK);
   if (!crt_applies(ns, m, n, kk) || tight) return d;
   const int N = crt_moduli(ns, (double)kk);
-  return std::max(d, std::min(crt_scratch(N, N, z), free_scratch(ns, kk, z, false)));
+  return std::max(d, std::min(crt_scratch(N, N, z), free_scratch(ns, kk, z, false, false)));
 }
 
 // A plan holds the scratch of the problems it runs in one slice launch for as

@@ -1270,7 +1270,8 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   }
   Staging* stg = g.staging;
   const bool defer_b = stg && stg->deferred[1], defer_c = stg && stg->deferred[2];
-  const int nch = (cap == cudaStreamCaptureStatusNone && ds->aux) ? column_chunks(m, n, k, defer_b || defer_c) : 1;
+  const bool captured = cap != cudaStreamCaptureStatusNone;
+  const int nch = (!captured && ds->aux) ? column_chunks(m, n, k, defer_b || defer_c) : 1;
   int64_t cut[kMaxChunks + 1];
   column_cuts(n, nch, defer_b || defer_c, cut);
   const bool choose = ns_fixed == 0 && slices <= 0;
@@ -1420,8 +1421,8 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     auto own_bytes = [&](int count) {
       return sizeof(__half) * (size_t)count * ((own_a ? a_plane : 0) + (own_b ? b_plane : 0));
     };
-    per = crt ? crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, g.tight)) : ns;
-    const int least = crt ? crt_per_pass(ns, N, k, z, 0.0) : per;
+    per = crt ? crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, g.tight, captured)) : ns;
+    const int least = crt && !captured ? crt_per_pass(ns, N, k, z, 0.0) : per;
     if (least < per && !scratch_alloc_if_room(&planes_buf, own_bytes(per), s)) per = least;
     if (planes_buf || !own_bytes(per)) break;
     if (!crt || (!PA && !PB)) {
@@ -1740,7 +1741,7 @@ bool ozaki_batchable(const DevGemm& g, int slices) {
   if (!crt_applies(slices, g.m, g.n, g.k)) return true;
   const Sizes z = sizes_of(g.m, g.n, g.k, g.tight);
   const int N = crt_moduli(slices, g.k);
-  return crt_per_pass(slices, N, g.k, z, free_scratch(slices, g.k, z, g.tight)) == N;
+  return crt_per_pass(slices, N, g.k, z, free_scratch(slices, g.k, z, g.tight, false)) == N;
 }
 
 std::vector<char> ozaki_batch_members(const DevGemm* gs, const int* slices, int count) {

@@ -24,16 +24,19 @@ static void check(int ns, int64_t m, int64_t n, int64_t k) {
       const double row = (double)plane_row(k, 8, tight);
       z.own = ((packs & 1 ? 0.0 : (double)m) + (packs & 2 ? 0.0 : (double)n)) * row;
       const double digits = digit_scratch(ns, k, z);
-      const int least = crt_per_pass(ns, N, k, z, 0.0), most = crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, tight));
+      const int least = crt_per_pass(ns, N, k, z, 0.0), most = crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, tight, false));
       expect(least >= 1 && least <= most && most <= N, "passes", ns, m, n, k);
       // one modulus per pass is the least there is: from packs it can be more than their digit form takes
       expect(crt_scratch(least, N, z) <= digits || (packs && least == 1), "least passes", ns, m, n, k);
       if (!packs) expect(crt_scratch(least, N, z) <= digits, "within the digit form", ns, m, n, k);
-      expect(crt_scratch(most, N, z) <= std::max(digits, free_scratch(ns, k, z, tight)) || most == 1, "free scratch", ns, m, n, k);
+      expect(crt_scratch(most, N, z) <= std::max(digits, free_scratch(ns, k, z, tight, false)) || most == 1, "free scratch", ns, m, n, k);
       if (tight) expect(most == least, "tight", ns, m, n, k);
+      // under capture: at most 256 MB beyond the digit form
+      const int captured = crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, tight, true));
+      expect(crt_scratch(captured, N, z) <= std::max(digits, 256.0 * (1 << 20)) || (packs && captured == 1), "captured", ns, m, n, k);
       // what admission and streaming charge for it, whatever number of moduli the data need
       for (int moduli = crt_moduli(ns, 1.0); moduli <= N; ++moduli) {
-        const int per = crt_per_pass(ns, moduli, k, z, free_scratch(ns, k, z, tight));
+        const int per = crt_per_pass(ns, moduli, k, z, free_scratch(ns, k, z, tight, false));
         expect(crt_scratch(per, moduli, z) <= emulated_scratch(ns, m, n, k, tight), "charge", ns, m, n, k);
       }
     }

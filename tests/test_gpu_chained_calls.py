@@ -71,3 +71,35 @@ def test_chained_calls_give_the_bits_of_separate_ones(gpu, mode, n, w):
         graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(x, y) for x, y in zip(got, want))
+
+
+def test_captured_emulated_call_bounds_its_scratch(gpu):
+    """A graph's scratch is allocated when it is launched: a captured call stays within the digit form's
+    (or 256 MB), in more passes and with the bits of the call outside."""
+    import torch
+    m, n, k, slices = 4096, 1024, 4096, 7
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    a, b = (torch.rand(x, dtype=torch.float64, device="cuda", generator=gen) - 0.5 for x in ((k, m), (n, k)))
+    want, got = (torch.zeros((n, m), dtype=torch.float64, device="cuda") for _ in range(2))
+    s = torch.cuda.Stream()
+
+    def call(c):
+        d = mg.GemmDesc()
+        d.dtype, d.precision, d.slices = mg.DTYPE_F64, mg.PREC_OZAKI, slices
+        d.m, d.n, d.k, d.alpha, d.beta = m, n, k, 1.0, 0.0
+        d.a, d.b, d.c = (mg.Operand(x.data_ptr(), 1, ld, mg.MEM_DEVICE, 0) for x, ld in ((a, m), (b, k), (c, m)))
+        mg.check(gpu.momms_gemm(ctypes.byref(d), ctypes.c_void_p(s.cuda_stream)), gpu)
+
+    torch.cuda.synchronize()
+    call(want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        call(got)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    graph.replay()
+    torch.cuda.synchronize()
+    held = free - torch.cuda.mem_get_info()[0]
+    assert torch.equal(got, want)
+    assert held <= 2 * slices * (m + n) * k + 4 * slices * m * n + (64 << 20)
