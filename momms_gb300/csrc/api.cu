@@ -120,6 +120,12 @@ DeviceState* device_state() {
       cuda_fail(e, "library stream");
       return nullptr;
     }
+    unsigned* words = nullptr;
+    if (cudaMallocHost(&words, 64 * kHostWordSlots) != cudaSuccess) {
+      cudaGetLastError();  // read-backs go to pageable memory
+      words = nullptr;
+    }
+    d.host_words = words;
     d.copy_stream = cs;
     d.copy_stream2 = cs2;
     d.aux = aux;

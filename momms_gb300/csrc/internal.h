@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -22,6 +23,39 @@ struct DeviceState {
   cudaStream_t copy_stream2 = nullptr;  // device->host copies (streamed calls, C write-back)
   cudaStream_t aux = nullptr;           // second compute stream of column-chunked emulated calls
   cudaStream_t aux2 = nullptr;          // emulated calls: the guaranteed bound and, under it, recombinations
+  unsigned* host_words = nullptr;       // pinned, kHostWordSlots slots of 64 bytes (HostWords)
+  std::atomic<uint64_t> host_words_used{0};
+};
+
+// 64 bytes of pinned host memory for the length of one read-back (a copy to
+// pageable memory is staged by the driver): a slot of what the device's set-up
+// allocated, since a call must not allocate pinned memory itself (another thread
+// may be capturing a stream, which the allocation would break). Beyond
+// kHostWordSlots read-backs at once, memory of its own, not pinned.
+constexpr int kHostWordSlots = 64;
+class HostWords {
+ public:
+  explicit HostWords(DeviceState* d) : d_(d) {
+    uint64_t used = d->host_words_used.load();
+    while (d->host_words && used != ~0ull) {
+      const int i = __builtin_ctzll(~used);
+      if (d->host_words_used.compare_exchange_weak(used, used | 1ull << i)) {
+        slot_ = i;
+        break;
+      }
+    }
+  }
+  ~HostWords() {
+    if (slot_ >= 0) d_->host_words_used.fetch_and(~(1ull << slot_));
+  }
+  HostWords(const HostWords&) = delete;
+  HostWords& operator=(const HostWords&) = delete;
+  unsigned* get() { return slot_ >= 0 ? d_->host_words + 16 * slot_ : own_; }
+
+ private:
+  DeviceState* d_;
+  int slot_ = -1;
+  unsigned own_[16] = {};
 };
 
 // Stream-ordered scratch allocation (free with cudaFreeAsync) from the

@@ -1124,25 +1124,11 @@ int enqueue_bound_kernel(const BoundWork& w, int64_t m, int64_t n, int64_t k, bo
 // term below FP32's range (relative to 2^(e_i+f_j)): no slice count can vouch
 // for it. Entries with no nonzero term are exact (their digits are all zero).
 // Synchronises `s`.
-// Pinned words the calling thread reads results into: a copy to pageable
-// memory is staged by the driver.
-struct PinnedWords {
-  unsigned* p = nullptr;
-  PinnedWords() {
-    if (cudaMallocHost(&p, 64) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-  }
-  ~PinnedWords() {
-    if (p) cudaFreeHost(p);
-  }
-};
 int bound_result(const BoundWork& w, const Side (&sides)[2], int64_t m, int64_t n, int64_t k, DeviceState* ds,
                  cudaStream_t s, float* q1, float* q2, bool* uncovered, double* sum_most = nullptr) {
-  static thread_local PinnedWords pinned;
-  unsigned local[kBoundWords] = {0, 0, 0, 0};
-  unsigned* words = pinned.p ? pinned.p : local;
+  HostWords host(ds);
+  unsigned* words = host.get();
+  static_assert(kBoundWords <= 16, "64 bytes");
   cudaError_t ce = cudaMemcpyAsync(words, w.out, kBoundWords * sizeof(unsigned), cudaMemcpyDeviceToHost, s);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
   if (ce != cudaSuccess) return cuda_fail(ce, "Ozaki bound");

@@ -103,3 +103,49 @@ def test_captured_emulated_call_bounds_its_scratch(gpu):
     held = free - torch.cuda.mem_get_info()[0]
     assert torch.equal(got, want)
     assert held <= 2 * slices * (m + n) * k + 4 * slices * m * n + (64 << 20)
+
+
+def test_a_thread_that_called_may_end_during_a_capture(gpu):
+    """A thread whose automatic call read a result back ends while another one captures a stream in the
+    global mode (torch's default): nothing is left to free that would break the capture."""
+    import threading
+
+    import torch
+    n = 384
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    a, b = (torch.rand((n, n), dtype=torch.float64, device="cuda", generator=gen) - 0.5 for _ in range(2))
+    cs = [torch.zeros((n, n), dtype=torch.float64, device="cuda") for _ in range(2)]
+    s = torch.cuda.Stream()
+
+    def call(c, stream, slices):
+        d = mg.GemmDesc()
+        d.dtype, d.precision, d.slices = mg.DTYPE_F64, mg.PREC_OZAKI, slices  # 0: chosen from the data
+        d.m = d.n = d.k = n
+        d.alpha, d.beta = 1.0, 0.0
+        d.a, d.b, d.c = (mg.Operand(x.data_ptr(), 1, n, mg.MEM_DEVICE, 0) for x in (a, b, c))
+        return gpu.momms_gemm(ctypes.byref(d), ctypes.c_void_p(stream.cuda_stream))
+
+    called, end, results = threading.Event(), threading.Event(), []
+
+    def other():
+        results.append(call(cs[0], torch.cuda.Stream(), 0))
+        called.set()
+        end.wait(60)
+
+    torch.cuda.synchronize()
+    assert call(cs[1], s, 7) == mg.OK
+    torch.cuda.synchronize()
+    want = cs[1].clone()
+    th = threading.Thread(target=other)
+    th.start()
+    assert called.wait(60) and results == [mg.OK]
+    cs[1].zero_()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        assert call(cs[1], s, 7) == mg.OK
+        end.set()
+        th.join()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(cs[1], want)
