@@ -51,7 +51,7 @@ inline bool ozaki_schedule(int ns, int64_t k, Schedule* sc) {
   const int bits = kDigitBits;
   const int64_t kblocks = ceil_div(std::min<int64_t>(std::max<int64_t>(k, 1), kMaxK), 64);
   const double kspan = (double)kblocks * 64.0;
-  auto prod = [&](int t, int u) { return ldexp(1.0, (t == 1 ? bits : bits - 1) + (u == 1 ? bits : bits - 1)); };
+  auto prod = [&](int t, int u) { return 1 << ((t == 1 ? bits : bits - 1) + (u == 1 ? bits : bits - 1)); };
   sc->np = sc->ng = 0;
   for (int d = ns + 1; d >= 2; --d) {
     double gsum = 0.0;
@@ -59,7 +59,7 @@ inline bool ozaki_schedule(int ns, int64_t k, Schedule* sc) {
     for (int t = 1; t <= ns; ++t) {
       const int u = d - t;
       if (u < 1 || u > ns) continue;
-      const double pb = prod(t, u);
+      const int pb = prod(t, u);
       if (open && gsum + kspan * pb > kGroupLimit) open = false;  // this pair starts the next group
       if (!open) {
         if (sc->ng >= sp::MAX_GROUPS) return false;
@@ -72,7 +72,7 @@ inline bool ozaki_schedule(int ns, int64_t k, Schedule* sc) {
       if (sc->np >= sp::MAX_PAIRS) return false;
       sc->pair_a[sc->np] = (uint8_t)(t - 1);
       sc->pair_b[sc->np] = (uint8_t)(u - 1);
-      sc->pair_w[sc->np] = std::max(1, (int)ldexp(pb, -kChunkUnitLog2));
+      sc->pair_w[sc->np] = std::max(1, pb >> kChunkUnitLog2);
       ++sc->np;
       gsum += kspan * pb;
     }
@@ -143,28 +143,29 @@ inline double digit_scratch(int ns, int64_t k, const Sizes& z) {
   return 2.0 * ns * z.own + 4.0 * ng * z.c;
 }
 inline double crt_scratch(int per, int N, const Sizes& z) { return 2.0 * per * z.ops + N * z.c; }
-// The residue form keeps to the digit form's scratch, or to `free` bytes, by
+// The residue form keeps to `limit` bytes, the digit form's scratch or more, by
 // walking the moduli in several passes, each with its own operand planes: at
 // 8192^3 two passes of 8 moduli instead of 4.6 GB of planes, for one more read
 // of the operands (0.2 of 13 ms). Where a call is small a second pass shows:
 // 2600 x 2600 x 2600 786 us in two, 754 in one, 4096 x 1024 x 4096 728 and 678.
-inline int crt_per_pass(int ns, int N, int64_t k, const Sizes& z, double free) {
-  const double limit = std::max(digit_scratch(ns, k, z), free);
+inline int crt_per_pass(int N, const Sizes& z, double limit) {
   int per = N;
   while (per > 1 && crt_scratch(per, N, z) > limit) --per;
   const int passes = (int)ceil_div(N, per);
   return (int)ceil_div(N, passes);
 }
-// What a call may take where the device has room for it: kFreeScratch, and as
-// much again as the digits that packed operands bring (in passes within the
+// What a call may take where the device has room for it, `digits` the digit
+// form's scratch: kFreeScratch, or the digits that packed operands bring on top (in passes within the
 // digit form's own scratch, 8192 x 8192 x 8192 from packs re-reads the digits
 // nine times). A call under stream capture has its scratch allocated when its
 // graph is launched, where no second choice is left: kCapturedScratch, enough
-// for one pass of the small calls to which a pass matters. `tight`: nothing.
+// for one pass of the small calls to which a pass matters. `tight`: no more
+// than the digit form's.
 constexpr double kCapturedScratch = 256.0 * (1 << 20);
-inline double free_scratch(int ns, int64_t k, const Sizes& z, bool tight, bool captured) {
-  if (tight) return 0.0;
-  return captured ? kCapturedScratch : std::max((double)kFreeScratch, digit_scratch(ns, k, Sizes{z.ops, z.ops, z.c}));
+inline double scratch_limit(int ns, const Sizes& z, double digits, bool tight, bool captured) {
+  if (tight) return digits;
+  if (captured) return std::max(digits, kCapturedScratch);
+  return std::max(digits + 2.0 * ns * (z.ops - z.own), (double)kFreeScratch);
 }
 // The most an ns-slice product takes, whatever its operands (an automatic count
 // may need fewer moduli than k asks for, and then more of them fit a pass).
@@ -174,7 +175,7 @@ inline double emulated_scratch(int ns, int64_t m, int64_t n, int64_t k, bool tig
   const int64_t kk = std::min(k, kMaxK);
   if (!crt_applies(ns, m, n, kk) || tight) return d;
   const int N = crt_moduli(ns, (double)kk);
-  return std::max(d, std::min(crt_scratch(N, N, z), free_scratch(ns, kk, z, false, false)));
+  return std::max(d, std::min(crt_scratch(N, N, z), scratch_limit(ns, z, d, false, false)));
 }
 
 // A plan holds the scratch of the problems it runs in one slice launch for as

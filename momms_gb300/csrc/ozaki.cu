@@ -1407,8 +1407,9 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     auto own_bytes = [&](int count) {
       return sizeof(__half) * (size_t)count * ((own_a ? a_plane : 0) + (own_b ? b_plane : 0));
     };
-    per = crt ? crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, g.tight, captured)) : ns;
-    const int least = crt && !captured ? crt_per_pass(ns, N, k, z, 0.0) : per;
+    const double digits = crt ? digit_scratch(ns, k, z) : 0.0;
+    per = crt ? crt_per_pass(N, z, scratch_limit(ns, z, digits, g.tight, captured)) : ns;
+    const int least = crt && !captured ? crt_per_pass(N, z, digits) : per;
     if (least < per && !scratch_alloc_if_room(&planes_buf, own_bytes(per), s)) per = least;
     if (planes_buf || !own_bytes(per)) break;
     if (!crt || (!PA && !PB)) {
@@ -1727,7 +1728,7 @@ bool ozaki_batchable(const DevGemm& g, int slices) {
   if (!crt_applies(slices, g.m, g.n, g.k)) return true;
   const Sizes z = sizes_of(g.m, g.n, g.k, g.tight);
   const int N = crt_moduli(slices, g.k);
-  return crt_per_pass(slices, N, g.k, z, free_scratch(slices, g.k, z, g.tight, false)) == N;
+  return crt_per_pass(N, z, scratch_limit(slices, z, digit_scratch(slices, g.k, z), g.tight, false)) == N;
 }
 
 std::vector<char> ozaki_batch_members(const DevGemm* gs, const int* slices, int count) {

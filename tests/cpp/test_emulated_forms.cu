@@ -24,19 +24,20 @@ static void check(int ns, int64_t m, int64_t n, int64_t k) {
       const double row = (double)plane_row(k, 8, tight);
       z.own = ((packs & 1 ? 0.0 : (double)m) + (packs & 2 ? 0.0 : (double)n)) * row;
       const double digits = digit_scratch(ns, k, z);
-      const int least = crt_per_pass(ns, N, k, z, 0.0), most = crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, tight, false));
+      const double limit = scratch_limit(ns, z, digits, tight, false);
+      const int least = crt_per_pass(N, z, digits), most = crt_per_pass(N, z, limit);
       expect(least >= 1 && least <= most && most <= N, "passes", ns, m, n, k);
       // one modulus per pass is the least there is: from packs it can be more than their digit form takes
       expect(crt_scratch(least, N, z) <= digits || (packs && least == 1), "least passes", ns, m, n, k);
       if (!packs) expect(crt_scratch(least, N, z) <= digits, "within the digit form", ns, m, n, k);
-      expect(crt_scratch(most, N, z) <= std::max(digits, free_scratch(ns, k, z, tight, false)) || most == 1, "free scratch", ns, m, n, k);
+      expect(crt_scratch(most, N, z) <= limit || most == 1, "free scratch", ns, m, n, k);
       if (tight) expect(most == least, "tight", ns, m, n, k);
       // under capture: at most 256 MB beyond the digit form
-      const int captured = crt_per_pass(ns, N, k, z, free_scratch(ns, k, z, tight, true));
+      const int captured = crt_per_pass(N, z, scratch_limit(ns, z, digits, tight, true));
       expect(crt_scratch(captured, N, z) <= std::max(digits, 256.0 * (1 << 20)) || (packs && captured == 1), "captured", ns, m, n, k);
       // what admission and streaming charge for it, whatever number of moduli the data need
       for (int moduli = crt_moduli(ns, 1.0); moduli <= N; ++moduli) {
-        const int per = crt_per_pass(ns, moduli, k, z, free_scratch(ns, k, z, tight, false));
+        const int per = crt_per_pass(moduli, z, limit);
         expect(crt_scratch(per, moduli, z) <= emulated_scratch(ns, m, n, k, tight), "charge", ns, m, n, k);
       }
     }
@@ -55,7 +56,7 @@ int main() {
   // 8192 x 8192 x 8192 from packs of 7 digits: the digit form's 1.9 GB of group sums, not its 3.8 GB with planes
   Sizes z = sizes_of(8192, 8192, 8192, false);
   z.own = 0.0;
-  expect(crt_scratch(crt_per_pass(7, 17, 8192, z, 0.0), 17, z) <= 1.9e9, "packs", 7, 8192, 8192, 8192);
+  expect(crt_scratch(crt_per_pass(17, z, digit_scratch(7, 8192, z)), 17, z) <= 1.9e9, "packs", 7, 8192, 8192, 8192);
   for (int i = 0; i < 20000; ++i) check(5 + i % 11, size(32, 20000), size(32, 20000), size(128, 32704));
   // plans: what their problems hold together beyond the digit form
   for (int trial = 0; trial < 300; ++trial) {
