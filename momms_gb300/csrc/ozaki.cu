@@ -1094,12 +1094,6 @@ int enqueue_bound_kernel(const BoundWork& w, int64_t m, int64_t n, int64_t k, bo
   p.merge_pairs = 0;
   p.msum_a = w.sum_a;
   p.msum_b = w.sum_b;
-  // The FP32 sum of non-negative exact bf16 products, accumulated by the
-  // tensor core (alignment and truncation at most a few units of 2^-24 per
-  // step), is taken to lose at most max(k, 64) 2^-21 of itself.
-  const double lbs = 1.0 - (double)std::max<int64_t>(k, 64) * ldexp(1.0, -21);
-  p.lb_scale = (float)lbs;
-  if ((double)p.lb_scale > lbs) p.lb_scale = nextafterf(p.lb_scale, 0.0f);  // rounded down
   p.kf = (float)k;
   p.bound_out = w.out;
   p.bound_count = reinterpret_cast<unsigned long long*>(w.out + 2);
@@ -1116,6 +1110,17 @@ int enqueue_bound_kernel(const BoundWork& w, int64_t m, int64_t n, int64_t k, bo
   return ce == cudaSuccess ? MOMMS_OK : cuda_fail(ce, "Ozaki bound launch");
 }
 
+// q1 and q2 from the maxima of the quotients by S (slicegemm.cuh, bound_tile).
+// The FP32 sum of non-negative exact bf16 products, accumulated by the tensor
+// core (alignment and truncation at most a few units of 2^-24 per step), is taken
+// to lose at most max(k, 64) 2^-21 of itself; q1's reciprocals are at most 2^-23
+// short, and the last factor covers the FP64 roundings here.
+void bound_quotients(float max1, float max2, int64_t k, double* q1, double* q2) {
+  const double up = (1.0 + 0x1p-48) / (1.0 - (double)std::max<int64_t>(k, 64) * ldexp(1.0, -21));
+  *q1 = (double)max1 * (1.0 + 0x1p-23) * (1.0 + 0x1p-45) * up;
+  *q2 = (double)max2 * up;
+}
+
 // The bound's result, once the bound kernel is enqueued on `s`: the two
 // maxima, and whether some entry is uncovered. The kernel counts the entries
 // whose lower bound is zero (none, for dense data); if there are any, a
@@ -1125,15 +1130,17 @@ int enqueue_bound_kernel(const BoundWork& w, int64_t m, int64_t n, int64_t k, bo
 // for it. Entries with no nonzero term are exact (their digits are all zero).
 // Synchronises `s`.
 int bound_result(const BoundWork& w, const Side (&sides)[2], int64_t m, int64_t n, int64_t k, DeviceState* ds,
-                 cudaStream_t s, float* q1, float* q2, bool* uncovered, double* sum_most = nullptr) {
+                 cudaStream_t s, double* q1, double* q2, bool* uncovered, double* sum_most = nullptr) {
   HostWords host(ds);
   unsigned* words = host.get();
   static_assert(kBoundWords <= 16, "64 bytes");
   cudaError_t ce = cudaMemcpyAsync(words, w.out, kBoundWords * sizeof(unsigned), cudaMemcpyDeviceToHost, s);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
   if (ce != cudaSuccess) return cuda_fail(ce, "Ozaki bound");
-  memcpy(q1, &words[0], 4);
-  memcpy(q2, &words[1], 4);
+  float max1, max2;
+  memcpy(&max1, &words[0], 4);
+  memcpy(&max2, &words[1], 4);
+  bound_quotients(max1, max2, k, q1, q2);
   if (sum_most) {
     // |a'_ip|, |b'_pj| <= 1, so an entry's sum is at most its row's and its
     // column's; a scaled integer may exceed the element by half a unit (2^-41 at
@@ -1349,14 +1356,14 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     rc = enqueue_magnitudes(sides, 2, k, mags, bw.kp, sums, from_max, s);
     from_max = false;
     if (!rc) rc = enqueue_bound_kernel(bw, m, n, k, false, ds->status, ds->sm_count, s);
-    float q1f = 0.0f, q2f = 0.0f;
+    double q1 = 0.0, q2 = 0.0;
     bool uncovered = false;
     if (!rc)
-      rc = bound_result(bw, sides, m, n, k, ds, s, &q1f, &q2f, &uncovered, &sum_most);
+      rc = bound_result(bw, sides, m, n, k, ds, s, &q1, &q2, &uncovered, &sum_most);
     if (rc) return rc;
     bool reachable = false;
-    ns = guaranteed_slices(target, q1f, q2f, uncovered, &reachable);
-    call_info().bound_rel_err = uncovered ? HUGE_VAL : guaranteed_bound(ns, q1f, q2f);
+    ns = guaranteed_slices(target, q1, q2, uncovered, &reachable);
+    call_info().bound_rel_err = uncovered ? HUGE_VAL : guaranteed_bound(ns, q1, q2);
     if (!reachable) verdict = MOMMS_ERR_TARGET_UNREACHABLE;
   } else if (automatic) {
     // A's magnitudes; B at the sampled columns, and their exponents
@@ -1558,19 +1565,19 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
   // chunk's magnitudes are in; the host reads the two maxima. Nothing has
   // written C yet, so a count that misses the target is simply redone.
   int redo = 0;
-  float q1f = 0.0f, q2f = 0.0f;
+  double q1 = 0.0, q2 = 0.0;
   bool uncovered = false;
   if (verify && !rc) {
     rc = enqueue_bound_kernel(bw, m, n, k, false, ds->status, ds->sm_count, V);
     if (!rc)
-      rc = bound_result(bw, sides, m, n, k, ds, V, &q1f, &q2f, &uncovered);
+      rc = bound_result(bw, sides, m, n, k, ds, V, &q1, &q2, &uncovered);
     if (!rc) {
       bool reachable = false;
-      const int need = guaranteed_slices(target, q1f, q2f, uncovered, &reachable);
+      const int need = guaranteed_slices(target, q1, q2, uncovered, &reachable);
       if (need > ns) {
         redo = need;  // more slices: redo with that count (C untouched)
       } else {
-        call_info().bound_rel_err = uncovered ? HUGE_VAL : guaranteed_bound(ns, q1f, q2f);
+        call_info().bound_rel_err = uncovered ? HUGE_VAL : guaranteed_bound(ns, q1, q2);
         if (!reachable) verdict = MOMMS_ERR_TARGET_UNREACHABLE;
       }
     }
@@ -1613,7 +1620,7 @@ int launch_dgemm_ozaki(const DevGemm& g, double target, int slices, int* slices_
     const int use = std::min(redo, kOzakiMaxSlices);
     rc = launch_dgemm_ozaki(g, target, use, slices_used, s);
     if (rc) return rc;
-    const double b = uncovered ? HUGE_VAL : guaranteed_bound(use, q1f, q2f);
+    const double b = uncovered ? HUGE_VAL : guaranteed_bound(use, q1, q2);
     call_info().bound_rel_err = b;
     return b > target_or_fp64(target) ? MOMMS_ERR_TARGET_UNREACHABLE : MOMMS_OK;
   }
@@ -1666,7 +1673,7 @@ int ozaki_choose_slices(const momms_gemm_desc& d, int* slices, cudaStream_t s) {
     if (!rc) rc = enqueue_absmax(sides, 2, g.k, s);
     if (!rc) rc = enqueue_magnitudes(sides, 2, g.k, mags, bw.kp, sums, true, s);
     if (!rc) rc = enqueue_bound_kernel(bw, m, n, g.k, false, ds->status, ds->sm_count, s);
-    float q1 = 0.0f, q2 = 0.0f;
+    double q1 = 0.0, q2 = 0.0;
     bool uncovered = false;
     if (!rc) rc = bound_result(bw, sides, m, n, g.k, ds, s, &q1, &q2, &uncovered);
     if (!rc) {

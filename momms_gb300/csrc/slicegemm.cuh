@@ -106,11 +106,11 @@ struct Params {
     float p, inv;
   } mod[MAX_MODULI];
   // EPI_BOUND: row sums of the scaled magnitudes of A (m) and B's columns
-  // (n) in units of 2^-40, each term rounded up; the lower-bound factor for
-  // the accumulation; k; the two maxima (bit patterns of non-negative floats)
+  // (n) in units of 2^-40, each term rounded up; k; the maxima (bit patterns of
+  // non-negative floats)
   const unsigned long long* msum_a;
   const unsigned long long* msum_b;
-  float lb_scale, kf;
+  float kf;
   unsigned* bound_out;                // [0], [1]: the maxima; [4], [5]: the largest row sum of A's and B's magnitudes
   unsigned long long* bound_count;  // entries counted
   int count_only;
@@ -175,12 +175,15 @@ __device__ __forceinline__ void drain_chunk(uint32_t taddr, EpiAcc<EPI> (&S)[NC]
 // and posted to the maxima. Every lane calls it (rows past m contribute 0).
 // `sb`: shared memory for this warp's NC column sums.
 //
-// The maxima need only be upper bounds, so a quotient is a product with the
-// hardware's approximate reciprocal (at most one unit of 2^-23 off), and each
-// maximum is raised by 2^-18 at the end, which covers that and the roundings:
-// six instructions per entry with the sum's own. (With upward-rounded quotients formed where they
-// could raise the maximum, and column sums by shuffle, the epilogue took 25 of
-// the 30 us of a 512 x 512 x 512 bound, 0.23 ms at 8192 x 8192 x 64.)
+// The maxima are of quotients by S, upward but for the reciprocal: q1's are
+// products with the hardware's approximate one (at most one unit in the last
+// place off, 2^-23), six instructions per entry with the sum's own. The host
+// raises them by that and scales S down to its lower bound in FP64
+// (bound_quotients). In all they are above the entries' own by at most 2^-21, as
+// four upward-rounded FP32 operations would leave them. (Those, formed where they
+// could raise the maximum, and column sums by shuffle took 25 of the 30 us of a
+// 512 x 512 x 512 bound, 0.23 ms at 8192 x 8192 x 64; a second look at the
+// entries near the maximum, for the exact one, cost 1-4 us of 14.)
 //
 // The sums of magnitudes are read before the tile's product is there
 // (bound_sums), and the posted maxima all at once: each is a trip to L2 or
@@ -241,7 +244,7 @@ __device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t
           const float s = S[j + q];
           float r;  // a sum that flushes to zero takes the row through the other loop
           asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
-          m1 = fmaxf(m1, (sa + b[q]) * r);
+          m1 = fmaxf(m1, __fmul_ru(__fadd_ru(sa, b[q]), r));
           smin = fminf(smin, s);
         }
       }
@@ -258,7 +261,7 @@ __device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t
 #pragma unroll
           for (int q = 0; q < NC; ++q) s = q == j ? S[q] : s;
           if (s > 0.0f) {
-            m1 = fmaxf(m1, __fdiv_ru(sa + sb[j], s));
+            m1 = fmaxf(m1, __fdiv_ru(__fadd_ru(sa, sb[j]), s));
             smin = fminf(smin, s);
           } else {
             ++cnt;
@@ -266,10 +269,6 @@ __device__ __forceinline__ void bound_tile(const Params& p, int64_t row, int64_t
         }
       }
       if (smin < INFINITY) m2 = __fdiv_ru(p.kf, smin);
-      // the lower bound is S times lb_scale
-      const float up = __fdiv_ru(1.0f + 0x1p-18f, p.lb_scale);
-      m1 = __fmul_ru(m1, up);
-      m2 = __fmul_ru(m2, up);
     }
     __syncwarp();  // before the next tile's column sums
   }

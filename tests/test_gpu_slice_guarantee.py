@@ -204,3 +204,30 @@ def test_every_slice_count_up_to_the_most(gpu):
     for s in range(1, 9):
         assert errs[s] < errs[s - 1] / 16, (s + 1, errs)
     assert max(errs[9:]) <= 2 * U64, errs  # 10 slices and more: FP64 rounding of C only
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 300, 256), (513, 700, 192), (1100, 1300, 128)])
+def test_reported_bound_is_as_tight_as_upward_quotients(gpu, m, n, k):
+    """Magnitudes of four bits, so that the bound's sums are exact in FP32: bound_rel_err is above the
+    formula's own value by no more than four upward roundings of 2^-23."""
+    rng = np.random.default_rng(m)
+
+    def operand(shape, axis):
+        x = rng.integers(1, 13, shape) / 16.0 * 2.0 ** -rng.integers(0, 3, shape)  # multiples of 2^-6, below 1
+        if axis:
+            x[:, 0] = 0.75
+        else:
+            x[0, :] = 0.75
+        return np.asfortranarray(x * rng.choice([-1.0, 1.0], shape))
+
+    A, B = operand((m, k), 1), operand((k, n), 0)
+    rc, _ = _run(gpu, A, B, 0.0)
+    assert rc == mg.OK
+    info = _info(gpu)
+    L = (np.abs(A) @ np.abs(B)) * (1.0 - max(k, 64) * 2.0**-21)  # multiples of 2^-12 below 2^8: exact sums
+    q1 = ((np.abs(A).sum(1)[:, None] + np.abs(B).sum(0)[None, :]) / L).max()
+    q2 = k / L.min()
+    s = info.slices
+    u = 2.0 ** (-8 * s - 1)
+    want = u * (q1 + (0.5 * (s - 1) * (256.0 / 255.0) + u) * q2)
+    assert want * (1 - 1e-13) <= info.bound_rel_err <= want * (1 + 2.0**-21)
