@@ -210,9 +210,18 @@ bool on_device(const void* ptr) {
 
 }  // namespace
 
+// Shared memory of the f64 kernel where its launch is capped to some of the SMs:
+// more than half of an SM's, so that it has one CTA on each. The CTAs of a grid
+// are spread over all SMs that can take one: four small ones for each SM of the
+// cap ran on every SM, and a request whose kernel needs a whole SM waited for the
+// large one beside it to end (emulated 512 x 512 x 512 beside f64 4096 x 4096 x
+// 2048: 52 ms instead of 0.09).
+constexpr int kCappedSmem = 116 * 1024;
+static_assert(kCappedSmem > dmma::SMEM_BYTES && 2 * (kCappedSmem + 1024) > 228 * 1024, "one CTA per SM");
+
 int set_attrs_grouped() {
   cudaError_t e = cudaFuncSetAttribute(grouped::dgemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       dmma::SMEM_BYTES);
+                                       kCappedSmem);
   return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "cudaFuncSetAttribute(grouped)");
 }
 
@@ -469,10 +478,11 @@ int plan_launch(Plan* p, cudaStream_t s, int max_sms) {
   if (ds->device != p->device) return fail(MOMMS_ERR_INVALID_ARG, "plan belongs to device %d", p->device);
   cudaError_t e;
   if (p->nd) {
-    const int sms = (max_sms > 0 && max_sms < ds->sm_count) ? max_sms : ds->sm_count;
-    const int grid = (int)std::min<int64_t>(p->d_units, (int64_t)dmma::CTAS_PER_SM * sms);
+    const bool capped = max_sms > 0 && max_sms < ds->sm_count;
+    const int64_t ctas = capped ? max_sms : (int64_t)dmma::CTAS_PER_SM * ds->sm_count;
+    const int grid = (int)std::min<int64_t>(p->d_units, ctas);
     KernelTimer kt(MOMMS_KERNEL_DGEMM_DMMA, s);
-    grouped::dgemm_grouped_kernel<<<grid, dmma::THREADS, dmma::SMEM_BYTES, s>>>(
+    grouped::dgemm_grouped_kernel<<<grid, dmma::THREADS, capped ? kCappedSmem : dmma::SMEM_BYTES, s>>>(
         p->d_maps, p->d_probs, p->nd, p->d_units, p->d_next, ds->status);
     note_launch();
     if ((e = launch_status()) != cudaSuccess) return cuda_fail(e, "grouped f64 launch");

@@ -211,3 +211,45 @@ def test_request_admitted_on_its_tight_footprint_keeps_to_it(gpu):
     r = subprocess.run([sys.executable, "-c", TIGHT_REQUEST], cwd=root, capture_output=True, text=True, timeout=300,
                        env=dict(os.environ, PYTHONPATH=root))
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("kind", ["ozaki", "tf32", "f64"])
+def test_small_requests_finish_beside_a_large_f64_one(gpu, kind):
+    """A large plain f64 request leaves SMs free: one that arrives while it runs is finished long before
+    it, also by kernels that take whole SMs."""
+    import torch
+    n = 4096
+
+    def request(m, prec, dtype=torch.float64, slices=0):
+        ops = [torch.rand((m, m), dtype=dtype, device="cuda") - 0.5 for _ in range(3)]
+        d = gu.make_desc(mg.DTYPE_F64 if dtype == torch.float64 else mg.DTYPE_F32, m, m, m, 1.0, 0.0,
+                         *((x.data_ptr(), 1, m) for x in ops), precision=prec, mem=mg.MEM_DEVICE, slices=slices)
+        return d, ops
+
+    large = request(n, mg.PREC_PLAIN)
+    small = {"ozaki": lambda: request(512, mg.PREC_OZAKI, slices=7), "f64": lambda: request(200, mg.PREC_PLAIN),
+             "tf32": lambda: request(1024, mg.PREC_SPLIT_TF32, torch.float32)}[kind]()
+    cfg = mg.ServerConfig(hbm_budget_bytes=8 << 30, max_batch=4, max_inflight=3, queue_capacity=16)
+    srv = ctypes.c_void_p()
+    mg.check(gpu.momms_server_create(ctypes.byref(cfg), ctypes.byref(srv)), gpu)
+    torch.cuda.synchronize()
+
+    def submit(r):
+        rid = ctypes.c_uint64(0)
+        mg.check(gpu.momms_server_submit(srv, ctypes.byref(r[0]), ctypes.byref(rid)), gpu)
+        return rid.value
+
+    def wait(rid):
+        info = mg.RequestInfo()
+        mg.check(gpu.momms_server_wait(srv, rid, 60.0, ctypes.byref(info)), gpu)
+        return info
+
+    for r in (small, small):  # first calls of a process load kernels
+        wait(submit(r))
+    first = submit(large)  # 0.17 s
+    time.sleep(0.01)
+    s = wait(submit(small))
+    b = wait(first)
+    mg.check(gpu.momms_server_destroy(srv), gpu)
+    assert b.device_start_ms < s.device_start_ms
+    assert s.device_end_ms < b.device_end_ms - 0.2 * (b.device_end_ms - b.device_start_ms)
