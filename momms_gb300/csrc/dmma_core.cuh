@@ -37,6 +37,8 @@ constexpr int OP_STAGE = TILE * BK * 8;  // bytes of one operand's k-block
 constexpr int SUB = BK * 128;  // one 16-wide sub-tile of an x-contiguous operand
 constexpr int RED_BYTES = CONSUMER_WARPS * 16 * 16 * 8;  // the warps' partial sums of a 16-stepped tile
 constexpr int SMEM_BYTES = 1024 + STAGES * 2 * OP_STAGE + RED_BYTES + 2 * STAGES * 8 + 16;
+constexpr int GROUP_SMEM = (SMEM_BYTES - 1024 + 1023) / 1024 * 1024;  // from one group's shared memory to the next's
+constexpr int smem_bytes(int groups) { return SMEM_BYTES + (groups - 1) * GROUP_SMEM; }
 
 // Byte offset of element (r, kk) in a k-contiguous tile: rows of 16 doubles
 // (128 bytes), 128B swizzle (16-byte chunk index XOR row mod 8).
@@ -55,7 +57,10 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMERS) : "memory"); }
+// Among the DMMA warps of one group (dgemm_body).
+__device__ __forceinline__ void consumer_sync(int group) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(CONSUMERS) : "memory");
+}
 
 // How the kernels read an operand: xc, the staged layout (x contiguous); tma,
 // through the tensor map, else element (x, k) at ptr[x*sx + k*sk].
@@ -278,10 +283,10 @@ __device__ __forceinline__ bool consume_unit(int a_xc, int b_xc, int64_t k, int6
 
 // ts 16 and 8: the four warps' partial sums of the tile, added in warp order;
 // each warp is left with its block in acc[0][0].
-__device__ __forceinline__ void reduce_warps(double (&acc)[2][2][2], double* red, int warp, int lane) {
+__device__ __forceinline__ void reduce_warps(double (&acc)[2][2][2], double* red, int warp, int lane, int group) {
 #pragma unroll
   for (int u = 0; u < 8; ++u) red[(warp * 8 + u) * 32 + lane] = acc[u >> 2][(u >> 1) & 1][u & 1];
-  consumer_sync();
+  consumer_sync(group);
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     double v = red[(2 * warp + q) * 32 + lane];
@@ -289,7 +294,7 @@ __device__ __forceinline__ void reduce_warps(double (&acc)[2][2][2], double* red
     for (int w = 1; w < CONSUMER_WARPS; ++w) v += red[(w * 8 + 2 * warp + q) * 32 + lane];
     acc[0][0][q] = v;
   }
-  consumer_sync();  // read before the next unit's sums are written
+  consumer_sync(group);  // read before the next unit's sums are written
 }
 
 // Epilogue of one unit. With splits == 1 the tile goes straight to C.
@@ -304,7 +309,7 @@ __device__ __forceinline__ void reduce_warps(double (&acc)[2][2][2], double* red
 // splits at a time) are issued before the first value is used.
 __device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2][2][2], const Place& p, int ts,
                                             int splits, int sp, double* tile_partials, unsigned* counter, int ctid,
-                                            int* s_last) {
+                                            int group, int* s_last) {
   // output u = 4i + 2j + q of this thread
   auto live = [&](int u) { return p.row + 16 * (u >> 2) < p.row_end && p.col + 16 * ((u >> 1) & 1) + (u & 1) < p.col_end; };
   auto cptr = [&](int u) {
@@ -335,12 +340,12 @@ __device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2]
   for (int u = 0; u < 8; ++u)
     if (live(u)) part[u * own + ctid] = v[u];
   __threadfence();
-  consumer_sync();
+  consumer_sync(group);
   if (ctid == 0) {
     unsigned prev = atomicAdd(counter, 1u);
     *s_last = (prev == (unsigned)(splits - 1)) ? 1 : 0;
   }
-  consumer_sync();
+  consumer_sync(group);
   if (*s_last) {
     __threadfence();
     constexpr int T = 2;  // splits loaded together
@@ -365,7 +370,7 @@ __device__ __forceinline__ void finish_unit(const Epi& e, const double (&acc)[2]
     update(v);
     if (ctid == 0) *counter = 0u;
   }
-  consumer_sync();
+  consumer_sync(group);
 }
 
 // Shared-memory carve-up and barrier initialisation common to the kernels.
@@ -378,8 +383,9 @@ struct Smem {
   int* s_last;
 };
 
-__device__ __forceinline__ Smem setup_smem(uint8_t* smem_raw) {
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+__device__ __forceinline__ Smem setup_smem(uint8_t* smem_raw, int group, int tid) {
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023)) +
+                  group * GROUP_SMEM;
   Smem s;
   s.sA = smem;
   s.sB = smem + STAGES * OP_STAGE;
@@ -387,7 +393,7 @@ __device__ __forceinline__ Smem setup_smem(uint8_t* smem_raw) {
   s.full = reinterpret_cast<uint64_t*>(s.sB + STAGES * OP_STAGE + RED_BYTES);
   s.empty = s.full + STAGES;
   s.s_last = reinterpret_cast<int*>(s.empty + STAGES);
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&s.full[i], FULL_ARRIVALS);
       mbar_init(&s.empty[i], CONSUMER_WARPS);
@@ -417,7 +423,9 @@ struct DProblem {
 };
 
 // A persistent CTA over a source of units (Src: total(), and unit(u, fn) which
-// calls fn(problem, A map, B map, Unit) with problem a DProblem).
+// calls fn(problem, A map, B map, Unit) with problem a DProblem), or GROUPS of
+// such CTAs, each with its own warps, barriers and shared memory, as one: where
+// they have to be on one SM.
 // With `next` units are handed out dynamically: the producer warp takes the
 // next unit from the global counter (numbered costliest first, so this is
 // longest-processing-time-first list scheduling by the actual durations; a
@@ -426,12 +434,14 @@ struct DProblem {
 // Without, the CTA takes units blockIdx.x, blockIdx.x + gridDim.x, ...
 // Either way the producer tags the first stage it fills for a unit with the
 // unit's index, which the DMMA warps read when they reach that stage; -1 ends.
-template <typename Src>
+template <int GROUPS = 1, typename Src>
 __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* next, unsigned* status) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ long long s_stage_unit[STAGES];
-  const Smem sm = setup_smem(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ long long s_units[GROUPS][STAGES];
+  const int group = GROUPS > 1 ? threadIdx.x / THREADS : 0, tid = threadIdx.x - group * THREADS;
+  long long* const s_stage_unit = s_units[group];
+  const Smem sm = setup_smem(smem_raw, group, tid);
+  const int warp = tid >> 5, lane = tid & 31;
   const long long total = src.total();
   int stage = 0;
   uint32_t phase = 0;
@@ -445,7 +455,7 @@ __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* n
       if (ok && lane == 0) s_stage_unit[stage] = u;
       if (!ok && lane == 0) report_status(status, DEV_TIMEOUT_EMPTY);
     };
-    for (long long u = blockIdx.x;; u += gridDim.x) {
+    for (long long u = (long long)blockIdx.x * GROUPS + group;; u += (long long)gridDim.x * GROUPS) {
       if (next) {
         if (lane == 0) u = (long long)atomicAdd(next, 1ull);
         u = __shfl_sync(0xffffffffu, u, 0);
@@ -466,10 +476,10 @@ __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* n
     }
     cp_async_wait_all();
     if (next && lane == 0) {
-      // the last CTA out resets the counters for the next launch
+      // the last group out resets the counters for the next launch
       __threadfence();
       const unsigned long long done = atomicAdd(next + 1, 1ull);
-      if (done == (unsigned long long)gridDim.x - 1) {
+      if (done == (unsigned long long)gridDim.x * GROUPS - 1) {
         next[0] = 0ull;
         next[1] = 0ull;
         __threadfence();
@@ -491,10 +501,10 @@ __device__ __forceinline__ void dgemm_body(const Src& src, unsigned long long* n
       ok = consume_unit(P.a.xc, P.b.xc, P.k, w.kb0, w.kb1, at, sm.sA, sm.sB, sm.full, sm.empty, stage, phase, lane,
                         P.run, acc, status);
       if (!ok) return;
-      if (P.ts <= 16) reduce_warps(acc, sm.red, warp, lane);
+      if (P.ts <= 16) reduce_warps(acc, sm.red, warp, lane, group);
       finish_unit(P.e, acc, at, P.ts, P.splits, w.sp,
                   P.splits > 1 ? P.partials + (size_t)w.tile * P.splits * (P.ts * P.ts) : nullptr,
-                  P.splits > 1 ? P.counters + w.tile : nullptr, threadIdx.x, sm.s_last);
+                  P.splits > 1 ? P.counters + w.tile : nullptr, tid, group, sm.s_last);
     });
     if (!ok) return;
   }

@@ -72,10 +72,16 @@ struct Many {
 
 // Every plain f64 problem's units, dealt dynamically (dgemm_body); the last
 // CTA resets the unit counter, so a captured plan relaunches as is.
-__global__ void __launch_bounds__(dmma::THREADS, dmma::CTAS_PER_SM)
+// GROUPS = CTAS_PER_SM: an SM's CTAs as one, for launches capped to some of the
+// SMs. The CTAs of a grid are spread over all SMs that can take one: four small
+// ones for each SM of the cap ran on every SM, and a request whose kernel needs a
+// whole SM waited for the large one beside it to end (emulated 512 x 512 x 512
+// beside f64 4096 x 4096 x 2048: 52 ms, 0.07 as one CTA on each SM of the cap).
+template <int GROUPS>
+__global__ void __launch_bounds__(dmma::THREADS * GROUPS, dmma::CTAS_PER_SM / GROUPS)
     dgemm_grouped_kernel(const CUtensorMap* __restrict__ maps, const DProblem* __restrict__ probs, int nprobs,
                          int64_t total_units, unsigned long long* next_unit, unsigned* status) {
-  dmma::dgemm_body(Many{maps, probs, nprobs, total_units}, next_unit, status);
+  dmma::dgemm_body<GROUPS>(Many{maps, probs, nprobs, total_units}, next_unit, status);
 }
 
 template <int TM, typename Off>
@@ -210,18 +216,12 @@ bool on_device(const void* ptr) {
 
 }  // namespace
 
-// Shared memory of the f64 kernel where its launch is capped to some of the SMs:
-// more than half of an SM's, so that it has one CTA on each. The CTAs of a grid
-// are spread over all SMs that can take one: four small ones for each SM of the
-// cap ran on every SM, and a request whose kernel needs a whole SM waited for the
-// large one beside it to end (emulated 512 x 512 x 512 beside f64 4096 x 4096 x
-// 2048: 52 ms instead of 0.09).
-constexpr int kCappedSmem = 116 * 1024;
-static_assert(kCappedSmem > dmma::SMEM_BYTES && 2 * (kCappedSmem + 1024) > 228 * 1024, "one CTA per SM");
-
 int set_attrs_grouped() {
-  cudaError_t e = cudaFuncSetAttribute(grouped::dgemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kCappedSmem);
+  cudaError_t e = cudaFuncSetAttribute(grouped::dgemm_grouped_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       dmma::smem_bytes(1));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(grouped::dgemm_grouped_kernel<dmma::CTAS_PER_SM>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, dmma::smem_bytes(dmma::CTAS_PER_SM));
   return e == cudaSuccess ? MOMMS_OK : cuda_fail(e, "cudaFuncSetAttribute(grouped)");
 }
 
@@ -479,11 +479,14 @@ int plan_launch(Plan* p, cudaStream_t s, int max_sms) {
   cudaError_t e;
   if (p->nd) {
     const bool capped = max_sms > 0 && max_sms < ds->sm_count;
-    const int64_t ctas = capped ? max_sms : (int64_t)dmma::CTAS_PER_SM * ds->sm_count;
-    const int grid = (int)std::min<int64_t>(p->d_units, ctas);
     KernelTimer kt(MOMMS_KERNEL_DGEMM_DMMA, s);
-    grouped::dgemm_grouped_kernel<<<grid, dmma::THREADS, capped ? kCappedSmem : dmma::SMEM_BYTES, s>>>(
-        p->d_maps, p->d_probs, p->nd, p->d_units, p->d_next, ds->status);
+    auto launch = [&](auto kernel, int groups, int64_t ctas) {
+      const int grid = (int)std::min<int64_t>(ceil_div(p->d_units, groups), ctas);
+      kernel<<<grid, dmma::THREADS * groups, dmma::smem_bytes(groups), s>>>(p->d_maps, p->d_probs, p->nd, p->d_units,
+                                                                            p->d_next, ds->status);
+    };
+    if (capped) launch(grouped::dgemm_grouped_kernel<dmma::CTAS_PER_SM>, dmma::CTAS_PER_SM, max_sms);
+    else launch(grouped::dgemm_grouped_kernel<1>, 1, (int64_t)dmma::CTAS_PER_SM * ds->sm_count);
     note_launch();
     if ((e = launch_status()) != cudaSuccess) return cuda_fail(e, "grouped f64 launch");
   }
