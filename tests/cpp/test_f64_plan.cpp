@@ -25,7 +25,9 @@ static void check(int64_t m, int64_t n, int64_t k, int sms, int tuned) {
   ok = ok && threads * outputs == p.ts * p.ts;
   // the scratch of calls that cannot allocate: 160 tiles of 128 x 128 doubles and 1280 counters
   const bool split = p.splits > 1;
-  const bool room = !split || (p.partial_elems() <= 160 * 128 * 128 && p.tiles() <= 1280);
+  // (with a launch's unit counters, also within the 21 MB that admission and streaming charge for it)
+  const bool room = !split || (p.partial_elems() <= 160 * 128 * 128 && p.tiles() <= 1280 &&
+                               p.partial_elems() * 8 + p.tiles() * 4 + 16 <= 21 * 1024 * 1024);
   if (!tuned) ok = ok && room;  // a tuned plan may ask for more, and is refused there
   else if (split && momms::f64_split_fits(m, n, p.splits)) ok = ok && room;
   if (!ok && failures++ < 10)
