@@ -161,7 +161,7 @@ inline int crt_per_pass(int N, const Sizes& z, double limit) {
 // graph is launched, where no second choice is left: kCapturedScratch, enough
 // for one pass of the small calls to which a pass matters. `tight`: no more
 // than the digit form's.
-constexpr double kCapturedScratch = 256.0 * (1 << 20);
+constexpr double kCapturedScratch = 512.0 * (1 << 20);
 inline double scratch_limit(int ns, const Sizes& z, double digits, bool tight, bool captured) {
   if (tight) return digits;
   if (captured) return std::max(digits, kCapturedScratch);

@@ -32,9 +32,9 @@ static void check(int ns, int64_t m, int64_t n, int64_t k) {
       if (!packs) expect(crt_scratch(least, N, z) <= digits, "within the digit form", ns, m, n, k);
       expect(crt_scratch(most, N, z) <= limit || most == 1, "free scratch", ns, m, n, k);
       if (tight) expect(most == least, "tight", ns, m, n, k);
-      // under capture: at most 256 MB beyond the digit form
+      // under capture: at most the digit form's or 512 MB
       const int captured = crt_per_pass(N, z, scratch_limit(ns, z, digits, tight, true));
-      expect(crt_scratch(captured, N, z) <= std::max(digits, 256.0 * (1 << 20)) || (packs && captured == 1), "captured", ns, m, n, k);
+      expect(crt_scratch(captured, N, z) <= std::max(digits, 512.0 * (1 << 20)) || (packs && captured == 1), "captured", ns, m, n, k);
       // what admission and streaming charge for it, whatever number of moduli the data need
       for (int moduli = crt_moduli(ns, 1.0); moduli <= N; ++moduli) {
         const int per = crt_per_pass(moduli, z, limit);

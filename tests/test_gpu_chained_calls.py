@@ -75,7 +75,7 @@ def test_chained_calls_give_the_bits_of_separate_ones(gpu, mode, n, w):
 
 def test_captured_emulated_call_bounds_its_scratch(gpu):
     """A graph's scratch is allocated when it is launched: a captured call stays within the digit form's
-    (or 256 MB), in more passes and with the bits of the call outside."""
+    (or 512 MB), in more passes and with the bits of the call outside."""
     import torch
     m, n, k, slices = 4096, 1024, 4096, 7
     gen = torch.Generator(device="cuda").manual_seed(6)
@@ -102,7 +102,7 @@ def test_captured_emulated_call_bounds_its_scratch(gpu):
     torch.cuda.synchronize()
     held = free - torch.cuda.mem_get_info()[0]
     assert torch.equal(got, want)
-    assert held <= 2 * slices * (m + n) * k + 4 * slices * m * n + (64 << 20)
+    assert held <= max(2 * slices * (m + n) * k + 4 * slices * m * n, 512 << 20) + (64 << 20)
 
 
 def test_a_thread_that_called_may_end_during_a_capture(gpu):
