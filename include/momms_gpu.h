@@ -152,7 +152,9 @@ int momms_noalloc_status(uint32_t* bits);
  * skips that operand's pre-pass; an emulated call with a packed operand uses
  * the pack's slice count (both packs must agree) and needs no host round
  * trip to choose one, so it can be captured in a CUDA graph. Results are
- * bit-identical to the unpacked call with the same slice count. The
+ * bit-identical to the unpacked call with the same slice count (only where the
+ * device has no room for the residue form's scratch does an emulated call run
+ * by its packs' digits instead, within the same error bound). The
  * reference's counterpart is its Hierarch matrix type (src/matrix/hierarch.rs:
  * 18-140), which stores an operand in the blocked layout the algorithm walks
  * so that no packing happens at run time.
@@ -199,9 +201,10 @@ int momms_stream_plan(const momms_gemm_desc* desc, uint64_t budget, int64_t* mb,
  * Many independent GEMMs run as one persistent kernel per dtype: every plain
  * f64 problem's tiles (and k-splits) are work units of one DMMA kernel, every
  * plain f32 problem's of one FFMA kernel per output tile size; the slice
- * products of all emulated (Ozaki) problems with unpacked operands and k up to
- * 32704 are work units of one tcgen05 kernel (each problem's digit planes are
- * prepared and its recombination run by its own small kernels); split-TF32
+ * products of the emulated (Ozaki) problems with unpacked operands and k up to
+ * 32704 are work units of one tcgen05 kernel (each problem's operand planes are
+ * prepared and its recombination run by its own small kernels), as far as what
+ * they hold beyond the digit form's scratch stays within 1 GB; split-TF32
  * and other emulated problems run their own kernel sequences. Each problem is planned from its own
  * shape only (tile, split-k: the tuning table or the model), so a problem
  * gives bit-identical results alone (momms_gemm) and in any batch. Plans take
